@@ -303,40 +303,108 @@ __global__ void __launch_bounds__(32 * kReduceRows) ReducePartialsKernel(const f
 }
 
 // SwiGLU on gu [rows, 2 * f] (gate = columns [0, f), up = columns [f, 2f)): out = silu(gate) * up.
-__global__ void SwigluFwdKernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, size_t rows, int f)
+//
+// Streaming kernels bound by HBM (6 bytes per output element forward, 10 backward).  Every thread takes VECS vectors
+// kSwiThreads apart and requests all of them before the first is used (8 resp. 6 16-byte loads in flight); the flat
+// vector index is divided by the row length once per thread, not once per vector, in 32 bits where the size allows.
+// Measured at 4096 x 28672 against a grid-stride loop with one vector and a 64-bit division per step: forward 137.6 ->
+// 104.1 us (705 MB, 6.8 TB/s), backward 201.0 -> 172.5 us (1174 MB, 6.8 TB/s); at 4096 x 3584 22.7 -> 18.2 and 28.9 ->
+// 25.2 us.  The division is the hardware's approximate one (two ulp), the result is rounded to 8 bits.
+constexpr int kSwiThreads = 256;
+constexpr int kSwiFwdVecs = 4, kSwiBwdVecs = 2;
+__device__ __forceinline__ void RowOf(size_t i, uint32_t perRow, bool fits32, size_t* row, uint32_t* v)
 {
-    const size_t nVecRow = (size_t)f / 8;
-    const size_t total = rows * nVecRow;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row = i / nVecRow, v = i % nVecRow;
-        float g[8], u[8], o[8];
-        Unpack8(reinterpret_cast<const uint4*>(gu + row * 2 * f)[v], g);
-        Unpack8(reinterpret_cast<const uint4*>(gu + row * 2 * f + f)[v], u);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
-        reinterpret_cast<uint4*>(out + row * f)[v] = Pack8(o);
+    if (fits32) {
+        const uint32_t r = (uint32_t)i / perRow;
+        *row = r;
+        *v = (uint32_t)i - r * perRow;
+    } else {
+        *row = i / perRow;
+        *v = (uint32_t)(i - *row * perRow);
     }
 }
-__global__ void SwigluBwdKernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dgu,
-                                size_t rows, int f)
+__device__ __forceinline__ float Sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
+template <int VECS>
+__global__ void __launch_bounds__(kSwiThreads) SwigluFwdKernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, size_t rows, int f)
 {
-    const size_t nVecRow = (size_t)f / 8;
+    const uint32_t nVecRow = (uint32_t)f / 8;
     const size_t total = rows * nVecRow;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row = i / nVecRow, v = i % nVecRow;
-        float g[8], u[8], d[8], dg[8], du[8];
-        Unpack8(reinterpret_cast<const uint4*>(gu + row * 2 * f)[v], g);
-        Unpack8(reinterpret_cast<const uint4*>(gu + row * 2 * f + f)[v], u);
-        Unpack8(reinterpret_cast<const uint4*>(dout + row * f)[v], d);
+    size_t i = (size_t)blockIdx.x * (kSwiThreads * VECS) + threadIdx.x, row;
+    uint32_t v;
+    RowOf(i, nVecRow, total <= 0xFFFFFFFFull, &row, &v);
+    uint4 g[VECS], u[VECS];
+    uint32_t vs[VECS];
+    size_t rs[VECS];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float sig = 1.f / (1.f + __expf(-g[k]));
-            const float silu = g[k] * sig;
-            dg[k] = d[k] * u[k] * sig * (1.f + g[k] * (1.f - sig));
-            du[k] = d[k] * silu;
+    for (int k = 0; k < VECS; ++k, i += kSwiThreads) {
+        rs[k] = row;
+        vs[k] = v;
+        if (i < total) {
+            const uint4* p = reinterpret_cast<const uint4*>(gu + row * 2 * f);
+            g[k] = p[v];
+            u[k] = p[nVecRow + v];
+        } else {
+            vs[k] = 0xFFFFFFFFu;
         }
-        reinterpret_cast<uint4*>(dgu + row * 2 * f)[v] = Pack8(dg);
-        reinterpret_cast<uint4*>(dgu + row * 2 * f + f)[v] = Pack8(du);
+        v += kSwiThreads;
+        if (v >= nVecRow) { const uint32_t q = v / nVecRow; row += q; v -= q * nVecRow; }
+    }
+#pragma unroll
+    for (int k = 0; k < VECS; ++k) {
+        if (vs[k] == 0xFFFFFFFFu) break;
+        float fg[8], fu[8], o[8];
+        Unpack8(g[k], fg);
+        Unpack8(u[k], fu);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = fg[e] * Sigmoid(fg[e]) * fu[e];
+        reinterpret_cast<uint4*>(out + rs[k] * f)[vs[k]] = Pack8(o);
+    }
+}
+template <int VECS>
+__global__ void __launch_bounds__(kSwiThreads) SwigluBwdKernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
+                                                               __nv_bfloat16* __restrict__ dgu, size_t rows, int f)
+{
+    const uint32_t nVecRow = (uint32_t)f / 8;
+    const size_t total = rows * nVecRow;
+    size_t i = (size_t)blockIdx.x * (kSwiThreads * VECS) + threadIdx.x, row;
+    uint32_t v;
+    RowOf(i, nVecRow, total <= 0xFFFFFFFFull, &row, &v);
+    uint4 g[VECS], u[VECS], d[VECS];
+    uint32_t vs[VECS];
+    size_t rs[VECS];
+#pragma unroll
+    for (int k = 0; k < VECS; ++k, i += kSwiThreads) {
+        rs[k] = row;
+        vs[k] = v;
+        if (i < total) {
+            const uint4* p = reinterpret_cast<const uint4*>(gu + row * 2 * f);
+            g[k] = p[v];
+            u[k] = p[nVecRow + v];
+            d[k] = reinterpret_cast<const uint4*>(dout + row * f)[v];
+        } else {
+            vs[k] = 0xFFFFFFFFu;
+        }
+        v += kSwiThreads;
+        if (v >= nVecRow) { const uint32_t q = v / nVecRow; row += q; v -= q * nVecRow; }
+    }
+#pragma unroll
+    for (int k = 0; k < VECS; ++k) {
+        if (vs[k] == 0xFFFFFFFFu) break;
+        float fg[8], fu[8], fd[8], dg[8], du[8];
+        Unpack8(g[k], fg);
+        Unpack8(u[k], fu);
+        Unpack8(d[k], fd);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float sig = Sigmoid(fg[e]);
+            const float silu = fg[e] * sig;
+            dg[e] = fd[e] * fu[e] * sig * (1.f + fg[e] * (1.f - sig));
+            du[e] = fd[e] * silu;
+        }
+        uint4* q = reinterpret_cast<uint4*>(dgu + rs[k] * 2 * f);
+        q[vs[k]] = Pack8(dg);
+        q[nVecRow + vs[k]] = Pack8(du);
     }
 }
 
@@ -398,6 +466,11 @@ HcclResult CheckLaunch(const char* what)
     if (e != cudaSuccess) { HCCL_ERROR("%s launch failed: %s", what, cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
+// Several vectors per thread only where two blocks per SM remain with them; below that one each, which spreads the work
+// over more SMs (128 x 3584: 4.2 us either way, the launch).
+bool SwigluBig(size_t vecs) { return vecs >= (size_t)SmCount() * 2 * kSwiThreads * kSwiFwdVecs; }
+size_t SwigluBlocks(size_t vecs, int vecsPerThread) { return (vecs + (size_t)kSwiThreads * vecsPerThread - 1) / ((size_t)kSwiThreads * vecsPerThread); }
+
 int ElementwiseGrid(size_t items)
 {
     size_t blocks = (items + 255) / 256;
@@ -472,7 +545,12 @@ HcclResult HcclFusedSwigluFwd(const void* gu, void* out, uint64_t rows, uint32_t
     CHK_PTR_NULL(gu); CHK_PTR_NULL(out);
     if (f == 0 || f % 8 != 0 || !Aligned16(gu) || !Aligned16(out)) return HCCL_E_PARA;
     if (rows == 0) return HCCL_SUCCESS;
-    SwigluFwdKernel<<<ElementwiseGrid(rows * (f / 8)), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f);
+    const size_t vecs = rows * (f / 8);
+    const bool big = SwigluBig(vecs);
+    const size_t blocks = SwigluBlocks(vecs, big ? kSwiFwdVecs : 1);
+    if (blocks > 0x7FFFFFFFull) return HCCL_E_PARA;
+    if (big) SwigluFwdKernel<kSwiFwdVecs><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f);
+    else SwigluFwdKernel<1><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f);
     return CheckLaunch("SwigluFwd");
 }
 
@@ -481,8 +559,12 @@ HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint6
     CHK_PTR_NULL(gu); CHK_PTR_NULL(dout); CHK_PTR_NULL(dgu);
     if (f == 0 || f % 8 != 0 || !Aligned16(gu) || !Aligned16(dout) || !Aligned16(dgu)) return HCCL_E_PARA;
     if (rows == 0) return HCCL_SUCCESS;
-    SwigluBwdKernel<<<ElementwiseGrid(rows * (f / 8)), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout,
-                                                                                      (__nv_bfloat16*)dgu, rows, (int)f);
+    const size_t vecs = rows * (f / 8);
+    const bool big = SwigluBig(vecs);
+    const size_t blocks = SwigluBlocks(vecs, big ? kSwiBwdVecs : 1);
+    if (blocks > 0x7FFFFFFFull) return HCCL_E_PARA;
+    if (big) SwigluBwdKernel<kSwiBwdVecs><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, rows, (int)f);
+    else SwigluBwdKernel<1><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, rows, (int)f);
     return CheckLaunch("SwigluBwd");
 }
 

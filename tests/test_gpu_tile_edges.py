@@ -46,3 +46,30 @@ def test_add_rms_norm_groups(rows, hidden, with_delta):
     # without the residual gradient a row of 8 elements is a difference of nearly equal terms: the fp32 terms of size |dh|
     # are what the error is relative to
     assert (x.grad.double() - dx).norm().item() <= ONE_ROUNDING * dx.norm().item() + 1e-6 * d_h.double().norm().item()
+
+
+# vectors per thread: one (small) and several, rows shorter than a block's stretch, ragged ends
+@pytest.mark.parametrize("rows,f", [(1, 8), (3, 264), (700, 56), (1031, 3592), (4097, 1024)])
+def test_swiglu_blocks(rows, f):
+    g = torch.Generator(device="cuda").manual_seed(rows + f)
+    x, dy = _rnd(g, rows, 2 * f, std=2.0).requires_grad_(), _rnd(g, rows, f)
+    y = fused.swiglu(x)
+    y.backward(dy)
+    x64 = x.detach().double().requires_grad_()
+    a, b = x64.chunk(2, dim=-1)
+    y64 = a * torch.sigmoid(a) * b
+    assert _rel(y.detach(), y64.detach()) <= ONE_ROUNDING
+    assert _rel(x.grad, torch.autograd.grad(y64, x64, dy.double())[0]) <= ONE_ROUNDING
+
+
+def test_swiglu_extremes():
+    """Gates whose sigmoid saturates, infinities and NaN give what the expression gives."""
+    gate = torch.tensor([-1e30, -200.0, -88.5, -20.0, 0.0, 20.0, 90.0, 1e30], device="cuda")
+    x = torch.cat((gate, torch.full((8,), 2.0, device="cuda"))).bfloat16().view(1, 16)
+    want = fused.swiglu_reference(x.double())
+    got = fused.swiglu(x).double()
+    assert torch.isfinite(got).all()
+    torch.testing.assert_close(got, want, rtol=8e-3, atol=1e-30)
+    x = torch.tensor([[float("nan")] + [float("inf")] * 7 + [1.0] * 8], device="cuda").bfloat16()
+    got = fused.swiglu(x)
+    assert torch.isnan(got[0, 0]) and torch.isinf(got[0, 1:]).all()

@@ -73,3 +73,22 @@ def test_swiglu_extremes():
     x = torch.tensor([[float("nan")] + [float("inf")] * 7 + [1.0] * 8], device="cuda").bfloat16()
     got = fused.swiglu(x)
     assert torch.isnan(got[0, 0]) and torch.isinf(got[0, 1:]).all()
+
+
+# heads per thread: four, two, one, a last group that is not full; rows per block: many, one, one in several passes
+@pytest.mark.parametrize("s,heads,d,extra", [(1, 1, 16, 0), (9, 2, 64, 128), (33, 3, 128, 0), (130, 5, 64, 16), (7, 64, 128, 2048), (3, 130, 256, 0)])
+def test_rope_head_groups(s, heads, d, extra):
+    g = torch.Generator(device="cuda").manual_seed(s + heads)
+    x = _rnd(g, s, heads * d + extra)[:, :heads * d].view(s, heads, d).requires_grad_()
+    ang = torch.rand(s, d // 2, device="cuda", generator=g) * 6.28
+    cos, sin, dy = ang.cos().contiguous(), ang.sin().contiguous(), _rnd(g, s, heads, d)
+    y = fused.rope(x, cos, sin)
+    dx = torch.autograd.grad(y, x, dy)[0]
+    c, n, h = cos.double()[:, None], sin.double()[:, None], d // 2
+
+    def turn(t, sign):
+        a, b = t.double()[..., :h], t.double()[..., h:]
+        return torch.cat((a * c - sign * b * n, b * c + sign * a * n), dim=-1)
+
+    assert _rel(y.detach(), turn(x.detach(), 1)) <= ONE_ROUNDING
+    assert _rel(dx, turn(dy, -1)) <= ONE_ROUNDING

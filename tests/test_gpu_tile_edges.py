@@ -10,6 +10,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 from hccl_b200.ops import fused
+from hccl_b200.ops.moe import expert_offsets
 
 ONE_ROUNDING = 2.0 ** -8 + 1e-4
 
@@ -92,3 +93,15 @@ def test_rope_head_groups(s, heads, d, extra):
 
     assert _rel(y.detach(), turn(x.detach(), 1)) <= ONE_ROUNDING
     assert _rel(dx, turn(dy, -1)) <= ONE_ROUNDING
+
+
+# shared counters and global ones, one round of the scan and many, one block and several passes over the ids
+@pytest.mark.parametrize("pairs,experts", [(1, 1), (2047, 256), (2049, 257), (300000, 4096), (5000, 4097), (40000, 65536)])
+def test_expert_offsets_ranges(pairs, experts):
+    g = torch.Generator(device="cuda").manual_seed(pairs)
+    idx = torch.randint(-1, experts + 1, (pairs,), device="cuda", generator=g, dtype=torch.int32)
+    ok = idx[(idx >= 0) & (idx < experts)].long()
+    ref = torch.zeros(experts + 1, dtype=torch.int64, device="cuda")
+    ref[1:] = torch.bincount(ok, minlength=experts).cumsum(0)
+    for _ in range(2):
+        assert torch.equal(expert_offsets(idx, experts).long(), ref)

@@ -23,11 +23,28 @@ namespace hccl {
 
 namespace {
 
-constexpr int kMoeThreads = 256;
+constexpr int kMoeThreads = 512;
+constexpr int kMoeWarps = kMoeThreads / 32;
 
 // ------------------------------------------------------------------ count + local positions
 // counts[e] = number of (token, k) pairs routed to global expert e; pos[t * K + k] = rank of the pair among this
-// rank's pairs for the same expert.
+// rank's pairs for the same expert.  Up to kMoeCountOneBlock pairs (a decode step, a short prompt) one block counts in
+// shared memory and writes every count; more pairs are spread over blocks that share cleared global counters.
+constexpr int kMoeCountOneBlock = 16384;
+__global__ void __launch_bounds__(1024) MoeCountOneBlockKernel(const int32_t* __restrict__ topkIdx, int nPairs, int nExperts, uint32_t* __restrict__ counts,
+                                                               uint32_t* __restrict__ pos)
+{
+    __shared__ uint32_t s_count[kMoeMaxExperts];
+    for (int e = threadIdx.x; e < nExperts; e += blockDim.x) s_count[e] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nPairs; i += blockDim.x) {
+        const int e = topkIdx[i];
+        pos[i] = (e >= 0 && e < nExperts) ? atomicAdd(&s_count[e], 1u) : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nExperts; e += blockDim.x) counts[e] = s_count[e];
+}
 __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, int nExperts, uint32_t* __restrict__ counts,
                                uint32_t* __restrict__ pos)
 {
@@ -38,123 +55,130 @@ __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, 
 }
 
 // ------------------------------------------------------------------ dispatch
+// Bound by the bytes written (topk fp8 copies of every row, over NVLink to the peers).  A WARP owns a token: a lane
+// takes 16 elements of the row (two 16-byte loads), eight lanes share a 128-element block's maximum, and the lane
+// quantises its 16 elements in registers and stores them to all topk destinations, 512 contiguous bytes per warp and
+// destination.  No block-wide step inside a token, so all warps' loads and stores overlap; with a block per token and
+// its three barriers a rank of 256 tokens spent four fifths of the time waiting for one row at a time.
 struct DispatchBody {
     using Args = MoeDispatchArgs;
     static constexpr int kThreads = kMoeThreads;
     __device__ static void Run(const DevComm& c, const Args& a, int b, int nb)
     {
-        extern __shared__ uint32_t s_dyn[];   // unused: static arrays below
         __shared__ uint32_t s_cnt[kMaxDevRanks * kMoeMaxExperts];   // [src][expert]
         __shared__ uint32_t s_base[kMoeMaxExperts];                 // slot base in the destination rank for (expert, src = me)
-        __shared__ float s_scale[64];                               // up to 64 blocks of 128 -> hidden <= 8192
-        __shared__ uint4 s_row[8192 / 16];                          // the quantised row: hidden <= 8192 bytes of fp8
-        __shared__ uint64_t s_dst[kMoeMaxTopk];                     // (destination rank, slot) of the row's copies
         OpHead(c, b);
         const int p = c.nRanks, me = c.rank;
         const int E = a.nExperts, perRank = E / p;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint64_t e0 = LoadEpoch(c, b);
         // phase 0: publish my counts in every rank's table, row `me` (each block row owns a private copy of the table)
-        for (int q = 0; q < p; ++q) {
-            uint32_t* tbl = a.table[q] + ((size_t)b * kMaxDevRanks + me) * kMoeMaxExperts;
-            for (int e = threadIdx.x; e < E; e += blockDim.x) tbl[e] = a.counts[e];
+        for (int i = threadIdx.x; i < p * E; i += kThreads) {
+            const int q = i / E, e = i - q * E;
+            a.table[q][((size_t)b * kMaxDevRanks + me) * kMoeMaxExperts + e] = a.counts[e];
         }
         bool ok = RankBarrier(c, b, 0, e0 + 1, K_MOE_DISPATCH);
         // phase 1: slot bases.  Destination rank d = e / perRank holds its experts one after the other; inside an expert the
         // sources are ordered by rank.
         const uint32_t* mine = a.table[me] + (size_t)b * kMaxDevRanks * kMoeMaxExperts;
-        for (int i = threadIdx.x; i < p * E; i += blockDim.x) s_cnt[(i / E) * kMoeMaxExperts + (i % E)] = mine[(size_t)(i / E) * kMoeMaxExperts + (i % E)];
-        __syncthreads();
-        for (int e = threadIdx.x; e < E; e += blockDim.x) {
-            const int d = e / perRank;
-            uint32_t base = 0;
-            for (int e2 = d * perRank; e2 < e; ++e2)
-                for (int s = 0; s < p; ++s) base += s_cnt[s * kMoeMaxExperts + e2];
-            for (int s = 0; s < me; ++s) base += s_cnt[s * kMoeMaxExperts + e];
-            s_base[e] = base;
+        for (int i = threadIdx.x; i < p * E; i += kThreads) {
+            const int s = i / E, e = i - s * E;
+            s_cnt[s * kMoeMaxExperts + e] = mine[(size_t)s * kMoeMaxExperts + e];
         }
         __syncthreads();
-        if (b == 0) {
-            // what this rank receives: per local expert total and the running offsets (for the grouped GEMM that follows)
-            for (int le = threadIdx.x; le <= perRank; le += blockDim.x) {
-                uint32_t off = 0;
-                for (int e2 = 0; e2 < le; ++e2)
-                    for (int s = 0; s < p; ++s) off += s_cnt[s * kMoeMaxExperts + me * perRank + e2];
-                a.recvOffsets[le] = off;
-                if (le == perRank && off > a.capacity) ReportWaitFailure(c, K_MOE_DISPATCH, b, 0, me, a.capacity, off, DEV_ERR_BOUNDS);
-            }
-        }
-        // phase 2: token rows
-        const int H = a.hidden, nScale = H / 128, vecPerRow = H / 8;      // uint4 of 8 bf16
-        for (int t = b; t < a.nTokens && ok; t += nb) {
-            const uint4* row = reinterpret_cast<const uint4*>(a.x + (size_t)t * H);
-            // amax per 128-element block: 16 vectors per block, one vector per thread per pass
-            for (int v0 = 0; v0 < vecPerRow; v0 += blockDim.x) {
-                const int v = v0 + threadIdx.x;
-                float amax = 0.f;
-                if (v < vecPerRow) {
-                    const uint4 raw = row[v];
-                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float2 f = __bfloat1622float2(h[k]);
-                        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+        // one warp per destination rank scans its experts, 32 at a time
+        for (int d = warp; d < p; d += kMoeWarps) {
+            uint32_t run = 0;
+            for (int le0 = 0; le0 < perRank; le0 += 32) {
+                const int le = le0 + lane, e = d * perRank + le;
+                uint32_t total = 0, before = 0;
+                if (le < perRank) {
+                    for (int s = 0; s < p; ++s) {
+                        const uint32_t n = s_cnt[s * kMoeMaxExperts + e];
+                        total += n;
+                        if (s < me) before += n;
                     }
                 }
-                // 16 consecutive lanes cover one block of 128
+                uint32_t incl = total;
 #pragma unroll
-                for (int o = 8; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                if (v < vecPerRow && (threadIdx.x & 15) == 0) s_scale[v / 16] = fmaxf(amax, 1e-10f) / 448.f;
-            }
-            __syncthreads();
-            // quantise the row ONCE into shared memory (16 bytes of fp8 = 16 elements = 2 input vectors per thread) ...
-            for (int w = threadIdx.x; w < H / 16; w += blockDim.x) {
-                const float inv = 1.f / s_scale[(w * 16) / 128];
-                const uint4 r0 = row[2 * w], r1 = row[2 * w + 1];
-                const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&r0);
-                const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&r1);
-                uint32_t outw[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const __nv_bfloat162* h = j < 2 ? h0 + 2 * j : h1 + 2 * (j - 2);
-                    const float2 fa = __bfloat1622float2(h[0]), fb = __bfloat1622float2(h[1]);
-                    const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(fa.x * inv, fa.y * inv), __NV_SATFINITE, __NV_E4M3);
-                    const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(fb.x * inv, fb.y * inv), __NV_SATFINITE, __NV_E4M3);
-                    outw[j] = (uint32_t)lo | ((uint32_t)hi << 16);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += up;
                 }
-                s_row[w] = make_uint4(outw[0], outw[1], outw[2], outw[3]);
+                const uint32_t off = run + incl - total;            // where the expert starts in rank d's receive buffer
+                if (le < perRank) {
+                    s_base[e] = off + before;
+                    if (b == 0 && d == me) a.recvOffsets[le] = off;  // for the grouped GEMM that follows
+                }
+                run += __shfl_sync(0xffffffffu, incl, 31);
             }
-            // ... and where its topk copies go
-            if (threadIdx.x < a.topk) {
-                const int pair = t * a.topk + threadIdx.x;
+            if (b == 0 && d == me && lane == 0) {
+                a.recvOffsets[perRank] = run;
+                if (run > a.capacity) ReportWaitFailure(c, K_MOE_DISPATCH, b, 0, me, a.capacity, run, DEV_ERR_BOUNDS);
+            }
+        }
+        __syncthreads();
+        // phase 2: token rows.  16 elements per lane: nPiece is a multiple of 8 (hidden is one of 128).
+        const int H = a.hidden, nScale = H / 128, nPiece = H / 16;
+        constexpr int U = 2;                                        // pieces a lane requests before it quantises the first
+        for (int t = b + warp * nb; t < a.nTokens && ok; t += nb * kMoeWarps) {
+            // lane k < topk: where the row's k-th copy goes
+            uint64_t sm = ~0ull;
+            if (lane < a.topk) {
+                const int pair = t * a.topk + lane;
                 const int e = a.topkIdx[pair];
-                uint64_t sm = ~0ull;
                 if (e >= 0 && e < E) sm = ((uint64_t)(e / perRank) << 32) | (uint64_t)(s_base[e] + a.pos[pair]);
                 a.slotMap[pair] = sm;
-                s_dst[threadIdx.x] = (sm != ~0ull && (uint32_t)sm < a.capacity) ? sm : ~0ull;      // overflow: reported by the receiver's bounds check above
+                if (sm != ~0ull && (uint32_t)sm >= a.capacity) sm = ~0ull;      // overflow: reported by the receiver's bounds check above
+                if (sm != ~0ull) a.recvSrc[sm >> 32][(uint32_t)sm] = ((uint64_t)me << 32) | (uint32_t)pair;
             }
-            __syncthreads();
-            // then the K copies leave as plain stores from shared memory: every thread has all K destinations' stores of
-            // its piece in flight together
-            for (int w = threadIdx.x; w < H / 16; w += blockDim.x) {
-                const uint4 q = s_row[w];
+            const uint4* row = reinterpret_cast<const uint4*>(a.x + (size_t)t * H);
+            for (int w0 = 0; w0 < nPiece; w0 += 32 * U) {
+                uint4 raw[U][2];
 #pragma unroll
-                for (int k = 0; k < kMoeMaxTopk; ++k) {
-                    if (k >= a.topk) break;
-                    const uint64_t sm = s_dst[k];
-                    if (sm == ~0ull) continue;
-                    reinterpret_cast<uint4*>(a.recvX[sm >> 32] + (size_t)(uint32_t)sm * H)[w] = q;
+                for (int u = 0; u < U; ++u) {
+                    const int w = w0 + u * 32 + lane;
+                    raw[u][0] = raw[u][1] = make_uint4(0, 0, 0, 0);
+                    if (w < nPiece) { raw[u][0] = row[2 * w]; raw[u][1] = row[2 * w + 1]; }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int w = w0 + u * 32 + lane;
+                    float f[16];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[u][j]);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const float2 v = __bfloat1622float2(h[k]);
+                            f[j * 8 + 2 * k] = v.x;
+                            f[j * 8 + 2 * k + 1] = v.y;
+                        }
+                    }
+                    float amax = 0.f;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(f[k]));
+                    // 8 consecutive lanes cover one block of 128
+#pragma unroll
+                    for (int o = 4; o >= 1; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                    const float scale = fmaxf(amax, 1e-10f) / 448.f;
+                    const float inv = 1.f / scale;
+                    uint32_t outw[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j] * inv, f[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+                        const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+                        outw[j] = (uint32_t)lo | ((uint32_t)hi << 16);
+                    }
+                    const uint4 q = make_uint4(outw[0], outw[1], outw[2], outw[3]);
+                    for (int k = 0; k < a.topk; ++k) {
+                        const uint64_t to = __shfl_sync(0xffffffffu, sm, k);
+                        if (to == ~0ull || w >= nPiece) continue;
+                        reinterpret_cast<uint4*>(a.recvX[to >> 32] + (size_t)(uint32_t)to * H)[w] = q;
+                        if ((lane & 7) == 0) a.recvScale[to >> 32][(size_t)(uint32_t)to * nScale + w / 8] = scale;
+                    }
                 }
             }
-            for (int i = threadIdx.x; i < a.topk * nScale; i += blockDim.x) {
-                const int k = i / nScale, sidx = i % nScale;
-                const uint64_t sm = s_dst[k];
-                if (sm != ~0ull) a.recvScale[sm >> 32][(size_t)(uint32_t)sm * nScale + sidx] = s_scale[sidx];
-            }
-            if (threadIdx.x < a.topk) {
-                const uint64_t sm = s_dst[threadIdx.x];
-                if (sm != ~0ull) a.recvSrc[sm >> 32][(uint32_t)sm] = ((uint64_t)me << 32) | (uint32_t)(t * a.topk + threadIdx.x);
-            }
-            __syncthreads();
         }
         RankBarrier(c, b, 0, e0 + 2, K_MOE_DISPATCH);
         StoreEpoch(c, b, e0 + 2);
@@ -163,6 +187,12 @@ struct DispatchBody {
 };
 
 // ------------------------------------------------------------------ combine
+// A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: 32 * kCombinePieces 16-byte pieces of one
+// token's row (a part of a row, so that a few hundred tokens still give every warp of the chip something to load); a
+// lane requests topk loads per piece, two pieces at a time, before it uses the first.  Lane k keeps the k-th copy's
+// address and weight and hands them round by shuffle: eight addresses per lane in registers held the kernel at 8 warps
+// per SM.
+constexpr int kCombinePieces = 4;
 struct CombineBody {
     using Args = MoeCombineArgs;
     static constexpr int kThreads = kMoeThreads;
@@ -172,59 +202,59 @@ struct CombineBody {
         const uint64_t e0 = LoadEpoch(c, b);
         bool ok = RankBarrier(c, b, 0, e0 + 1, K_MOE_COMBINE);      // the peers' expert outputs are final
         const int H = a.hidden, vecPerRow = H / 8;
-        // Two pieces (16 bytes each) of a token row per thread and pass: 2 x topk remote loads are requested before the
-        // first is used (a pull over NVLink is bound by the bytes in flight, not by issue rate).
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int parts = (vecPerRow + 32 * kCombinePieces - 1) / (32 * kCombinePieces);
+        const long long items = (long long)a.nTokens * parts;
         constexpr int U = 2;
-        for (int t = b; t < a.nTokens && ok; t += nb) {
-            float w[kMoeMaxTopk];
-            const __nv_bfloat16* src[kMoeMaxTopk];
-#pragma unroll
-            for (int k = 0; k < kMoeMaxTopk; ++k) {
-                w[k] = 0.f;
-                src[k] = nullptr;
-                if (k < a.topk) {
-                    const uint64_t sm = a.slotMap[t * a.topk + k];
-                    if (sm != ~0ull && (uint32_t)sm < a.capacity) {
-                        w[k] = a.topkWeight[t * a.topk + k];
-                        src[k] = a.y[sm >> 32] + (size_t)(uint32_t)sm * H;
-                    }
+        for (long long it = b + (long long)warp * nb; it < items && ok; it += (long long)nb * kMoeWarps) {
+            const int t = (int)(it / parts), v00 = (int)(it % parts) * 32 * kCombinePieces;
+            float wk = 0.f;
+            unsigned long long srcK = 0;                            // 0: the copy was dropped
+            if (lane < a.topk) {
+                const uint64_t sm = a.slotMap[(size_t)t * a.topk + lane];
+                if (sm != ~0ull && (uint32_t)sm < a.capacity) {
+                    wk = a.topkWeight[(size_t)t * a.topk + lane];
+                    srcK = reinterpret_cast<unsigned long long>(a.y[sm >> 32] + (size_t)(uint32_t)sm * H);
                 }
             }
-            for (int v0 = threadIdx.x; v0 < vecPerRow; v0 += U * blockDim.x) {
+#pragma unroll
+            for (int i = 0; i < kCombinePieces; i += U) {
+                const int v0 = v00 + i * 32 + lane;
                 uint4 raw[U][kMoeMaxTopk];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int v = v0 + u * blockDim.x;
+                for (int k = 0; k < kMoeMaxTopk; ++k) {
+                    const uint4* src = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, srcK, k));
 #pragma unroll
-                    for (int k = 0; k < kMoeMaxTopk; ++k) {
+                    for (int u = 0; u < U; ++u) {
                         raw[u][k] = make_uint4(0, 0, 0, 0);
-                        if (k < a.topk && v < vecPerRow && src[k] != nullptr) raw[u][k] = reinterpret_cast<const uint4*>(src[k])[v];
+                        if (src != nullptr && v0 + u * 32 < vecPerRow) raw[u][k] = src[v0 + u * 32];
                     }
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int v = v0 + u * blockDim.x;
-                    if (v >= vecPerRow) continue;
                     float acc[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
 #pragma unroll
                     for (int k = 0; k < kMoeMaxTopk; ++k) {
+                        const float w = __shfl_sync(0xffffffffu, wk, k);
                         if (k < a.topk) {
                             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[u][k]);
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
                                 const float2 f = __bfloat1622float2(h[j]);
-                                acc[2 * j] += w[k] * f.x;
-                                acc[2 * j + 1] += w[k] * f.y;
+                                acc[2 * j] += w * f.x;
+                                acc[2 * j + 1] += w * f.y;
                             }
                         }
                     }
-                    uint4 o;
-                    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+                    if (v0 + u * 32 < vecPerRow) {
+                        uint4 o;
+                        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                    reinterpret_cast<uint4*>(a.out + (size_t)t * H)[v] = o;
+                        for (int j = 0; j < 4; ++j) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+                        reinterpret_cast<uint4*>(a.out + (size_t)t * H)[v0 + u * 32] = o;
+                    }
                 }
             }
         }
@@ -249,6 +279,10 @@ HcclResult LaunchMoe(const LaunchTarget& t, const typename Body::Args& a, int nB
 
 HcclResult LaunchMoeCount(const int32_t* topkIdx, int nPairs, int nExperts, uint32_t* counts, uint32_t* pos, cudaStream_t stream)
 {
+    if (nPairs <= kMoeCountOneBlock) {
+        MoeCountOneBlockKernel<<<1, 1024, 0, stream>>>(topkIdx, nPairs, nExperts, counts, pos);
+        return cudaGetLastError() == cudaSuccess ? HCCL_SUCCESS : HCCL_E_RUNTIME;
+    }
     CHK_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (size_t)nExperts, stream));
     const int blocks = nPairs >= 1 << 16 ? 64 : 16;
     MoeCountKernel<<<blocks, 256, 0, stream>>>(topkIdx, nPairs, nExperts, counts, pos);

@@ -105,3 +105,51 @@ def test_expert_offsets_ranges(pairs, experts):
     ref[1:] = torch.bincount(ok, minlength=experts).cumsum(0)
     for _ in range(2):
         assert torch.equal(expert_offsets(idx, experts).long(), ref)
+
+
+# rows of one 128-element block and of a part of a warp's stretch, one token and more tokens than warps, dropped pairs,
+# the counting kernel of one block and of many
+@pytest.mark.parametrize("p,tokens,hidden,experts,topk", [(2, 3, 128, 2, 1), (2, 70, 1152, 16, 3), (4, 40, 8192, 64, 8), (2, 5000, 256, 8, 4)])
+def test_moe_dispatch_and_combine_edges(p, tokens, hidden, experts, topk):
+    import hccl_b200 as hb
+    from hccl_b200 import Communicator
+    from hccl_b200.ops.moe import MoeDispatcher
+
+    comms = Communicator.emulated(p, hb.make_config(buffer_mib=8))
+    cap = 2 * tokens * topk * p
+    disp = [MoeDispatcher(c, tokens, hidden, topk, experts, capacity=cap) for c in comms]
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    xs = [_rnd(g, tokens, hidden) for _ in comms]
+    idx = [torch.topk(torch.randn(tokens, experts, device="cuda", generator=g), min(topk, experts), dim=-1)[1].int().contiguous() for _ in comms]
+    idx[0][tokens // 2, -1] = -1                                     # a dropped pair
+    ws = [torch.rand(tokens, topk, device="cuda", generator=g) + 0.1 for _ in comms]
+    res = [d.dispatch(x, i) for d, x, i in zip(disp, xs, idx)]
+    torch.cuda.synchronize()
+    per = experts // p
+    for r in range(p):
+        want = torch.stack([(torch.stack([(i == r * per + e).sum() for i in idx])).sum() for e in range(per)]).cumsum(0)
+        assert res[r].offsets[0] == 0 and torch.equal(res[r].offsets[1:].long(), want)
+        n = int(want[-1])
+        src = res[r].src_info[:n]
+        rank, pair = src >> 32, src & 0xFFFFFFFF
+        rows = torch.stack(xs)[rank, pair // topk].float().view(n, hidden // 128, 128)
+        # the scale and the bytes, bit for bit: fp32 maximum / 448, then the hardware's conversion
+        scale = rows.abs().amax(-1).clamp_min(1e-10) / 448.0
+        assert torch.equal(res[r].scales[:n], scale)
+        want8 = (rows * (1.0 / scale).unsqueeze(-1)).to(torch.float8_e4m3fn).view(n, hidden)
+        assert torch.equal(res[r].x_fp8[:n].view(torch.uint8), want8.view(torch.uint8))
+        assert torch.equal(torch.stack(idx)[rank, pair // topk, pair % topk].long(),
+                           torch.repeat_interleave(torch.arange(per, device="cuda"), res[r].offsets.long().diff()) + r * per)
+        disp[r].y.copy_(torch.randn(cap, hidden, device="cuda", generator=g))
+    out = [d.combine(w) for d, w in zip(disp, ws)]
+    torch.cuda.synchronize()
+    y = torch.stack([d.y for d in disp]).double()
+    for r in range(p):
+        slot = res[r].slot_map.view(tokens, topk)
+        keep = slot != -1
+        rows = y[(slot >> 32).clamp_min(0), (slot & 0xFFFFFFFF) * keep]
+        ref = (rows * (ws[r].double() * keep).unsqueeze(-1)).sum(1)
+        assert _rel(out[r], ref) <= ONE_ROUNDING
+    assert comms[0].async_error() == hb.Result.SUCCESS
+    for c in comms:
+        c.destroy()

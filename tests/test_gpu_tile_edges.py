@@ -133,8 +133,9 @@ def test_moe_dispatch_and_combine_edges(p, tokens, hidden, experts, topk):
         src = res[r].src_info[:n]
         rank, pair = src >> 32, src & 0xFFFFFFFF
         rows = torch.stack(xs)[rank, pair // topk].float().view(n, hidden // 128, 128)
-        # the scale and the bytes, bit for bit: fp32 maximum / 448, then the hardware's conversion
-        scale = rows.abs().amax(-1).clamp_min(1e-10) / 448.0
+        # the scale and the bytes, bit for bit: fp32 maximum / 448 (a tensor: torch multiplies by the reciprocal of a number)
+        amax = rows.abs().amax(-1).clamp_min(1e-10)
+        scale = amax / torch.full_like(amax, 448.0)
         assert torch.equal(res[r].scales[:n], scale)
         want8 = (rows * (1.0 / scale).unsqueeze(-1)).to(torch.float8_e4m3fn).view(n, hidden)
         assert torch.equal(res[r].x_fp8[:n].view(torch.uint8), want8.view(torch.uint8))

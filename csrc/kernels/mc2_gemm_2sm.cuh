@@ -182,6 +182,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const int tilesM2 = (g.M + 255) / 256;
         const int nTiles = tilesM2 * g.tilesN;
         const int kBlocks = (g.K + kBK - 1) / kBK;
+        // bytes of a stage in both CTAs.  An MN-major half tile of B comes in boxes of 64 columns, whole ones: at a
+        // half width that is no multiple of 64 the last box brings columns of the neighbouring half (or tile) along,
+        // which the MMA, BN wide, does not read.
+        const uint32_t txBytes = (uint32_t)(2 * (L::kABytes + (B_MN ? (BN / 2 + 63) / 64 * 64 : BN / 2) * kBK * 2));
 
         if (warp == 0) {
             // ===== TMA producer (both CTAs): own 128 rows of A, own 128 rows of B, completion on the LEADER's full barrier
@@ -218,7 +222,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         uint8_t* sa = smem + stage * L::kStageBytes;
                         uint8_t* sb = sa + L::kABytes;
                         const uint32_t leaderFull = SmemAddr(&fullBar[stage]) & kPeerBitMask;
-                        if (crank == 0) MbarExpectTx(&fullBar[stage], (uint32_t)(2 * (L::kABytes + (BN / 2) * kBK * 2)));
+                        if (crank == 0) MbarExpectTx(&fullBar[stage], txBytes);
                         if (!A_MN) {
                             if (g.l2HintA != 0) TmaLoad2D2SmHint(sa, mapA, leaderFull, kb * kBK, rowA, polA);
                             else TmaLoad2D2Sm(sa, mapA, leaderFull, kb * kBK, rowA);

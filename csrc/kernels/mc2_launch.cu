@@ -258,6 +258,25 @@ uint32_t* PlainCtl()
     return p;
 }
 
+// Column tile width of a plain two-SM matmul: the one with the least (waves x time of a tile).  A k-block of a 256 x bn tile
+// takes as long as bn + 96 columns of math (the rest is the fill of the 128 rows of A and the turn of the ring; measured per
+// wave at K = 8192: 34.5, 36.7, 44.8, 47.5 us for 160, 192, 224, 256).  MN-major B is filled in whole boxes of 64 columns, so
+// 160, 192 and 224 bring as many bytes as 256 and two thirds of the difference stay (43.1, 43.7, 46.3, 47.0 us); they pay
+// where they save a wave: 4096 x 3584 x 8192 217.7 us with 128, 178.6 with 224, 179.6 with 256; 1024 x 28672 x 8192 464.7 us
+// with 128, 334.7 with 224; 8192 x 3584 x 4096 228.5 with 128, 165.8 with 224.
+int TwoSmColumnTile(int tilesM2, uint64_t n, int pairs, bool bMn)
+{
+    int best = 256;
+    double bestCost = 1e30;
+    for (int cand : {256, 224, 192, 160, 128}) {
+        const int loaded = bMn ? 2 * ((cand / 2 + 63) / 64 * 64) : cand;
+        const int waves = (tilesM2 * (int)((n + cand - 1) / cand) + pairs - 1) / pairs;
+        const double cost = (double)waves * ((cand + 2 * loaded) / 3.0 + 96);
+        if (cost < bestCost - 1e-9) { bestCost = cost; best = cand; }
+    }
+    return best;
+}
+
 HcclResult CheckShapes(uint64_t m, uint64_t n, uint64_t k)
 {
     if (m == 0 || n == 0 || k == 0 || m > (1u << 30) || n > (1u << 30) || k > (1u << 30)) return HCCL_E_PARA;
@@ -376,20 +395,10 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     DevComm dummy;
     memset(&dummy, 0, sizeof(dummy));
     if (bn == 256 && Use2Sm() && m >= 256) {
-        // Column tile width: the widest tile is the most efficient one, but a last wave that is mostly empty costs a
-        // whole tile time; pick the width that minimises (waves x width).  MN-major B is loaded in 64-column boxes, so
-        // its half tile has to be a multiple of 64.
         const int pairs = (SmCount() & ~1) / 2;
         const int tilesM2 = (int)((m + 255) / 256);
-        int bestBn = 256;
-        double bestCost = 1e30;
-        for (int cand : {256, 224, 192, 160, 128}) {
-            if (bMn && (cand / 2) % 64 != 0) continue;
-            const int tn = (int)((n + cand - 1) / cand);
-            const int waves = (tilesM2 * tn + pairs - 1) / pairs;
-            const double cost = (double)waves * (cand + 12);      // narrower tiles amortise the fixed per-tile work less well
-            if (cost < bestCost - 1e-9) { bestCost = cost; bestBn = cand; }
-        }
+        const int bestBn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
+        const double bestCost = (double)((tilesM2 * (int)((n + bestBn - 1) / bestBn) + pairs - 1) / pairs) * (bestBn + 12);
         // wide tiles: the same search over (waves x width) with two column tiles per work item
         {
             int wideBn = 0;

@@ -9,7 +9,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from hccl_b200.ops import fused
+from hccl_b200.ops import fused, mc2
 from hccl_b200.ops.moe import expert_offsets
 
 ONE_ROUNDING = 2.0 ** -8 + 1e-4
@@ -154,3 +154,23 @@ def test_moe_dispatch_and_combine_edges(p, tokens, hidden, experts, topk):
     assert comms[0].async_error() == hb.Result.SUCCESS
     for c in comms:
         c.destroy()
+
+
+def _check_matmul(m, n, k, ta, tb):
+    g = torch.Generator(device="cuda").manual_seed(m * 31 + n * 7 + k)
+    a, b = _rnd(g, *((k, m) if ta else (m, k))), _rnd(g, *((n, k) if tb else (k, n)))
+    out = torch.full((m + 1, n), 7.0, device="cuda", dtype=torch.bfloat16)       # the last row must stay
+    mc2.matmul(a, b, trans_a=ta, trans_b=tb, out=out[:m])
+    ref = (a.double().t() if ta else a.double()) @ (b.double() if not tb else b.double().t())
+    assert _rel(out[:m], ref) <= ONE_ROUNDING
+    assert (out[m] == 7.0).all()
+
+
+LAYOUTS = [(False, True), (False, False), (True, True), (True, False)]
+
+
+# column tiles whose half is no multiple of 64 (224, 192 and 160 wide), a ragged last one, full and partial row tiles
+@pytest.mark.parametrize("ta", [False, True])
+@pytest.mark.parametrize("m,n,k", [(4096, 3584, 128), (1024, 8192, 192), (2304, 7104, 64), (1000, 10232, 136)])
+def test_wide_matmul_with_kn_weight(m, n, k, ta):
+    _check_matmul(m, n, k, ta, False)

@@ -8,6 +8,7 @@
 #include "../core/cuda_driver.h"
 #include "../core/log.h"
 #include "mc2_gemm_2sm_wide.cuh"
+#include "mc2_gemm_splitk.cuh"
 
 namespace hccl {
 
@@ -136,6 +137,29 @@ HcclResult LaunchGemm2SmWide(const CUtensorMap& ta, const CUtensorMap& tb, const
     cfg.stream = stream;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, g);
     if (e != cudaSuccess) { HCCL_ERROR("wide two-SM matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
+}
+
+template <bool W_MN, bool X_MN>
+HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& g, int tiles, int split, cudaStream_t stream)
+{
+    auto kernel = GemmSplitKernel<W_MN, X_MN>;
+    const int smem = SplitSmemBytes(g.bt);
+    CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = (unsigned)split;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tw, tx, g);
+    if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 
@@ -373,32 +397,61 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     CHK_RET(CheckShapes(m, n, k));
     const bool aMn = transA != 0, bMn = transB == 0;
     if (aMn && m % 8 != 0) return HCCL_E_PARA;
-    const int tilesM = (int)((m + kBM - 1) / kBM);
-    // narrow column tiles when the wide ones would leave most SMs idle
+    const int tilesM = (int)((m + kBM - 1) / kBM), tilesM2 = (int)((m + 255) / 256);
+    const int pairs = (SmCount() & ~1) / 2;
+    // narrow: 256-wide column tiles would leave most SMs idle
     const bool narrow = (uint64_t)tilesM * ((n + 255) / 256) < (uint64_t)SmCount() * 3 / 4;
-    const int bn = narrow ? 128 : 256;
+    // Two-SM tiles: outputs that fill the chip with 256 x 256 tiles, and from 129 rows on those that fill four fifths of the
+    // pairs with 256 x 128 ones if the inner dimension is long (us, before on the one-SM kernel -> two-SM: 200 x 10240 x
+    // 8192 84.5 -> 45.0, 200 x 57344 x 8192 331.0 -> 199.8, 300 x 8192 x 8192 88.1 -> 49.0, 256 x 8192 x 8192 49.2 -> 40.9,
+    // 512 x 4096 x 4096 26.6 -> 23.1, 1000 x 2048 x 2048 16.5 -> 16.1; with fewer tiles the split kernel is ahead: 300 x
+    // 2048 x 4096 22.4 against 16.5).
+    const bool twoSm = Use2Sm() && ((!narrow && m >= 256) || (m > 128 && k >= 2048 && (uint64_t)tilesM2 * ((n + 127) / 128) * 5 >= (uint64_t)pairs * 4));
+    // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
+    // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
+    // long (400 x 1024 x 1024: 10.3 us against 9.2 on the one-SM kernel, 300 x 2048 x 4096: 16.5 against 24.7).
+    if (!twoSm && (m <= 96 || (narrow && (m <= 128 || k >= 4096)))) {
+        SplitArgs g;
+        memset(&g, 0, sizeof(g));
+        g.M = (int)m; g.N = (int)n; g.K = (int)k;
+        g.out = (__nv_bfloat16*)out;
+        // token tile: all of them up to 128, else equal tiles of at most 128 (MN-major activations come in 64-column boxes)
+        const int unit = aMn ? 64 : 16, parts = (int)((m + kSplitMaxBt - 1) / kSplitMaxBt);
+        g.bt = ((int)((m + parts - 1) / parts) + unit - 1) / unit * unit;
+        g.tilesM = (int)((m + g.bt - 1) / g.bt);
+        g.stages = SplitStages(g.bt);
+        g.ctl = PlainCtl();
+        if (!g.ctl) return HCCL_E_MEMORY;
+        // two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile)
+        const int tiles = g.tilesM * (int)((n + 127) / 128), kBlocks = (int)((k + kBK - 1) / kBK);
+        const int split = std::max(1, std::min({kSplitMaxCluster, 2 * SmCount() / tiles, kBlocks / 4}));
+        CUtensorMap tw, tx;
+        CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, 128, kBK));
+        CHK_RET(aMn ? MakeMap(&tx, a, k, m, kBK, 64) : MakeMap(&tx, a, m, k, (uint32_t)g.bt, kBK));
+        if (!bMn && !aMn) return LaunchGemmSplit<false, false>(tw, tx, g, tiles, split, stream);
+        if (!bMn && aMn) return LaunchGemmSplit<false, true>(tw, tx, g, tiles, split, stream);
+        if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, split, stream);
+        return LaunchGemmSplit<true, true>(tw, tx, g, tiles, split, stream);
+    }
     CUtensorMap ta, tb;
     CHK_RET(MapA(&ta, a, m, k, aMn));
-    CHK_RET(MapB(&tb, b, n, k, bMn, bn));
     GemmArgs g;
     memset(&g, 0, sizeof(g));
     g.M = (int)m; g.N = (int)n; g.K = (int)k;
     g.out = (__nv_bfloat16*)out;
     g.ldc = (int)n;
-    g.tilesM = tilesM;
-    g.tilesN = (int)((n + bn - 1) / bn);
     g.ctl = PlainCtl();
     if (!g.ctl) return HCCL_E_MEMORY;
     g.nRanks = 1;
-    const int grid = std::min(SmCount(), g.tilesM * g.tilesN);
-    g.nGemmCtas = grid;
     DevComm dummy;
     memset(&dummy, 0, sizeof(dummy));
-    if (bn == 256 && Use2Sm() && m >= 256) {
-        const int pairs = (SmCount() & ~1) / 2;
-        const int tilesM2 = (int)((m + 255) / 256);
+    if (twoSm) {
         const int bestBn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
-        const double bestCost = (double)((tilesM2 * (int)((n + bestBn - 1) / bestBn) + pairs - 1) / pairs) * (bestBn + 12);
+        g.bn = bestBn;
+        g.tilesN = (int)((n + bestBn - 1) / bestBn);
+        // B is split between the two CTAs of a pair: each loads half of the B rows of a tile
+        CHK_RET(MapB(&tb, b, n, k, bMn, bestBn / 2));
+        const double bestCost = (double)((tilesM2 * g.tilesN + pairs - 1) / pairs) * (bestBn + 12);
         // wide tiles: the same search over (waves x width) with two column tiles per work item
         {
             int wideBn = 0;
@@ -425,10 +478,6 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
                 return LaunchGemm2SmWide<true, true>(ta, tb, g, grid2, stream);
             }
         }
-        g.bn = bestBn;
-        g.tilesN = (int)((n + bestBn - 1) / bestBn);
-        // B is split between the two CTAs of a pair: each loads half of the B rows of a tile
-        CHK_RET(MapB(&tb, b, n, k, bMn, bestBn / 2));
         // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
         // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next
         // to the stream of the other, it is loaded "evict last", the streamed one "evict first", and the band covers
@@ -446,11 +495,16 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
                 g.rasterGroup = std::max(1, std::min(8, pairs / std::max(1, g.tilesN)));   // all columns of B in flight together
             }
         }
-        const int pairsWanted = tilesM2 * g.tilesN;
-        const int grid2 = std::min(SmCount() & ~1, 2 * pairsWanted);
+        const int grid2 = std::min(2 * pairs, 2 * tilesM2 * g.tilesN);
         g.nGemmCtas = grid2;
         return DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid2, false, stream);
     }
+    const int bn = narrow ? 128 : 256;
+    g.tilesM = tilesM;
+    g.tilesN = (int)((n + bn - 1) / bn);
+    CHK_RET(MapB(&tb, b, n, k, bMn, bn));
+    const int grid = std::min(SmCount(), g.tilesM * g.tilesN);
+    g.nGemmCtas = grid;
     if (bn == 128) return DispatchLayout<128, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid, false, stream);
     return DispatchLayout<256, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid, false, stream);
 }

@@ -174,3 +174,13 @@ LAYOUTS = [(False, True), (False, False), (True, True), (True, False)]
 @pytest.mark.parametrize("m,n,k", [(4096, 3584, 128), (1024, 8192, 192), (2304, 7104, 64), (1000, 10232, 136)])
 def test_wide_matmul_with_kn_weight(m, n, k, ta):
     _check_matmul(m, n, k, ta, False)
+
+
+# token tiles of 16 .. 128 and several of them, k-blocks fewer and more than the CTAs of a cluster, ragged N and K
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("m,n,k", [(8, 8, 8), (16, 128, 64), (24, 136, 256), (64, 1024, 520), (128, 248, 2048), (136, 1000, 1032), (304, 640, 4096),
+                                   (1, 264, 1024), (17, 8192, 1024)])
+def test_small_output_matmul(m, n, k, ta, tb):
+    if ta and m % 8:
+        pytest.skip("transposed A needs M % 8 == 0")
+    _check_matmul(m, n, k, ta, tb)

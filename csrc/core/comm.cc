@@ -420,9 +420,6 @@ HcclResult EmuGroup::Create(int nRanks, const HcclCommConfig* cfg, std::vector<C
     CHK_RET(SymAllocLocalGroup(nRanks, kSlabDataOff + data, &g->slabs_));
     g->maxBlocksPerRank_ = EmuMaxBlocksPerRank(nRanks);
     CHK_CUDA(cudaMalloc(&g->dComms_, sizeof(DevComm) * (size_t)nRanks));
-    CHK_CUDA(cudaHostAlloc((void**)&g->hArgs_, kRing * kArgSlotBytes * (size_t)nRanks, cudaHostAllocDefault));
-    CHK_CUDA(cudaMalloc(&g->dArgs_, kRing * kArgSlotBytes * (size_t)nRanks));
-    for (int i = 0; i < kRing; ++i) CHK_CUDA(cudaEventCreateWithFlags(&g->ringEvents_[i], cudaEventDisableTiming));
     comms->clear();
     g->hostComms_.resize((size_t)nRanks);
     for (int r = 0; r < nRanks; ++r) {
@@ -442,9 +439,6 @@ EmuGroup::~EmuGroup()
 {
     cudaDeviceSynchronize();
     if (dComms_) cudaFree(dComms_);
-    if (hArgs_) cudaFreeHost(hArgs_);
-    if (dArgs_) cudaFree(dArgs_);
-    for (int i = 0; i < kRing; ++i) if (ringEvents_[i]) cudaEventDestroy(ringEvents_[i]);
 }
 
 void EmuGroup::Release(CommImpl*)
@@ -461,7 +455,7 @@ HcclResult EmuGroup::Post(int rank, const void* args, size_t argBytes, int nBloc
                           cudaStream_t stream)
 {
     std::lock_guard<std::mutex> lk(mu_);
-    if (argBytes > kArgSlotBytes || rank < 0 || rank >= nRanks_) return HCCL_E_INTERNAL;
+    if (rank < 0 || rank >= nRanks_) return HCCL_E_INTERNAL;
     // One FIFO per rank: a rank may run ahead (an operator that needs several loops posts several launches before
     // the next rank is called); a launch is issued whenever every rank has an entry at the head of its queue.
     PendingPost post;
@@ -487,22 +481,16 @@ HcclResult EmuGroup::Post(int rank, const void* args, size_t argBytes, int nBloc
             for (auto& q : queues_) q.clear();
             return HCCL_E_INTERNAL;
         }
-        // the slot is free once the launch that used it last has consumed its arguments
-        if (cudaEventQuery(ringEvents_[ringHead_]) == cudaErrorNotReady) CHK_CUDA(cudaEventSynchronize(ringEvents_[ringHead_]));
-        char* slot = hArgs_ + (size_t)ringHead_ * kArgSlotBytes * (size_t)nRanks_;
-        char* dslot = dArgs_ + (size_t)ringHead_ * kArgSlotBytes * (size_t)nRanks_;
-        for (int r = 0; r < nRanks_; ++r) memcpy(slot + (size_t)r * ab, queues_[(size_t)r].front().args.data(), ab);
+        // the kernel's second parameter: one argument struct per possible rank
+        launchArgs_.assign(ab * (size_t)kMaxDevRanks, 0);
+        for (int r = 0; r < nRanks_; ++r) memcpy(launchArgs_.data() + (size_t)r * ab, queues_[(size_t)r].front().args.data(), ab);
         const void* fn = first.kernel;
         const int th = first.threads;
         for (auto& q : queues_) q.pop_front();
-        CHK_CUDA(cudaMemcpyAsync(dslot, slot, ab * (size_t)nRanks_, cudaMemcpyHostToDevice, stream));
         const DevComm* dc = dComms_;
-        const void* da = dslot;
-        void* kargs[3] = {(void*)&dc, (void*)&da, (void*)&nb};
+        void* kargs[3] = {(void*)&dc, (void*)launchArgs_.data(), (void*)&nb};
         cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)(nb * nRanks_)), dim3((unsigned)th), kargs, 0, stream);
         if (e != cudaSuccess) { HCCL_ERROR("cooperative launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
-        CHK_CUDA(cudaEventRecord(ringEvents_[ringHead_], stream));
-        ringHead_ = (ringHead_ + 1) % kRing;
     }
 }
 

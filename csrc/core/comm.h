@@ -161,13 +161,7 @@ private:
     int alive_ = 0;
     std::mutex mu_;
     DevComm* dComms_ = nullptr;            // device array [nRanks]
-    // ring of argument slots (pinned host + device), each holds nRanks * kArgSlotBytes
-    static constexpr int kRing = 64;
-    static constexpr size_t kArgSlotBytes = 4096;
-    char* hArgs_ = nullptr;
-    char* dArgs_ = nullptr;
-    cudaEvent_t ringEvents_[kRing] = {nullptr};
-    int ringHead_ = 0;
+    std::vector<char> launchArgs_;         // the ranks' arguments side by side (EmuArgs), copied by the launch itself
     // launches posted by individual ranks and not yet issued
     struct PendingPost { const void* kernel; int nBlocks, threads; std::vector<char> args; };
     std::vector<std::deque<PendingPost>> queues_;

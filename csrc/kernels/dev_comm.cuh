@@ -284,12 +284,23 @@ __global__ void __launch_bounds__(Body::kThreads) CollKernel(DevComm c, typename
 {
     Body::Run(c, a, (int)blockIdx.x, (int)gridDim.x);
 }
+// All ranks' arguments travel in the kernel's parameter space (a few kilobytes, 13 for the largest), as a single rank's
+// do: a launch needs no staging copy in front of it and nothing has to outlive the call that made it.
+template <class Args> struct EmuArgs { Args rank[kMaxDevRanks]; };
 template <class Body>
 __global__ void __launch_bounds__(Body::kThreads)
-    CollKernelEmu(const DevComm* cs, const typename Body::Args* as, int blocksPerRank)
+    CollKernelEmu(const DevComm* cs, const __grid_constant__ EmuArgs<typename Body::Args> as, int blocksPerRank)
 {
+    static_assert(sizeof(EmuArgs<typename Body::Args>) <= 32 * 1024 - 64, "kernel parameters are limited to 32764 bytes");
     const int r = (int)blockIdx.x / blocksPerRank;
-    Body::Run(cs[r], as[r], (int)blockIdx.x % blocksPerRank, blocksPerRank);
+    // the bodies index their arguments by rank: this rank's go to shared memory, where that is one load
+    using Args = typename Body::Args;
+    static_assert(sizeof(Args) % sizeof(uint64_t) == 0, "copied as 64-bit words");
+    __shared__ uint64_t s_args[sizeof(Args) / sizeof(uint64_t)];
+    const uint64_t* mine = reinterpret_cast<const uint64_t*>(&as.rank[r]);
+    for (int i = threadIdx.x; i < (int)(sizeof(Args) / sizeof(uint64_t)); i += Body::kThreads) s_args[i] = mine[i];
+    __syncthreads();
+    Body::Run(cs[r], *reinterpret_cast<const Args*>(s_args), (int)blockIdx.x % blocksPerRank, blocksPerRank);
 }
 #endif
 

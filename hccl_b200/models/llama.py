@@ -84,9 +84,7 @@ class DecoderLayer(torch.nn.Module):
         x, h = fused.add_rms_norm(x, delta, self.attn_norm, cfg.norm_eps, use_kernels=k_)
         qkv = self.qkv(h)                                                     # [S, (hq + 2 hkv) * D]
         s = qkv.shape[0]
-        q = fused.rope(qkv[:, :self.hq * d].view(s, self.hq, d), cos, sin, use_kernels=k_)
-        k = fused.rope(qkv[:, self.hq * d:(self.hq + self.hkv) * d].view(s, self.hkv, d), cos, sin, use_kernels=k_)
-        v = qkv[:, (self.hq + self.hkv) * d:].view(s, self.hkv, d)
+        q, k, v = fused.rope_qkv(qkv, cos, sin, self.hq, self.hkv, use_kernels=k_)
         attn = F.scaled_dot_product_attention(q.transpose(0, 1)[None], k.transpose(0, 1)[None], v.transpose(0, 1)[None], is_causal=True,
                                               enable_gqa=self.hq != self.hkv)
         attn = attn[0].transpose(0, 1).reshape(s, self.hq * d)

@@ -4,6 +4,7 @@
 * ``swiglu(gate_up)`` -> ``silu(gate) * up`` for ``gate_up = [gate | up]`` along the last dimension
 * ``rope(x, cos, sin)`` -> rotary embedding ("rotate halves") of ``x [S, heads, D]``; ``x`` may be a column slice
   of a wider projection output (row stride larger than ``heads * D``)
+* ``rope_qkv(qkv, cos, sin, hq, hkv)`` -> ``(q, k, v)`` of a projection output ``[S, (hq + 2 hkv) * D]`` with q and k rotated
 
 CUDA bf16 tensors run the hand-written kernels (csrc/kernels/fused_elementwise.cu); anything else (CPU tensors, other
 dtypes, hidden > 8192) takes the equivalent PyTorch expression, which is also the reference the tests compare against.
@@ -150,6 +151,46 @@ class _Rope(torch.autograd.Function):
         return dx, None, None
 
 
+class _RopeQkv(torch.autograd.Function):
+    """Query, key and value heads of one projection output.  The backward pass writes the three gradients side by side into
+    one tensor; slicing the output instead makes autograd fill three zero tensors of its full size and add them up."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, hq, hkv):
+        s, d = qkv.shape[0], qkv.shape[1] // (hq + 2 * hkv)
+        out = []
+        for first, heads in ((0, hq), (hq, hkv)):
+            o = torch.empty((s, heads, d), device=qkv.device, dtype=qkv.dtype)
+            _check(lib.HcclFusedRope(_p(qkv[:, first * d:]), qkv.stride(0), _p(o), heads * d, _p(cos), _p(sin), s, heads, d, 0, _s()), "HcclFusedRope")
+            out.append(o)
+        _count(2)
+        ctx.save_for_backward(cos, sin)
+        ctx.heads = (hq, hkv, d)
+        return out[0], out[1], qkv[:, (hq + hkv) * d:].view(s, hkv, d)
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        cos, sin = ctx.saved_tensors
+        hq, hkv, d = ctx.heads
+        s = cos.shape[0]
+        width = (hq + 2 * hkv) * d
+        like = next(g for g in (dq, dk, dv) if g is not None)
+        dqkv = torch.empty((s, width), device=like.device, dtype=like.dtype)
+        for first, heads, g in ((0, hq, dq), (hq, hkv, dk)):
+            part = dqkv[:, first * d:(first + heads) * d]
+            if g is None:
+                part.zero_()
+                continue
+            # rows and heads as attention left them where the kernel can read that, else a packed copy
+            if not (g.stride(2) == 1 and g.stride(1) == d and g.stride(0) % 8 == 0 and g.data_ptr() % 16 == 0):
+                g = g.contiguous()
+            _check(lib.HcclFusedRope(_p(g), g.stride(0), _p(part), width, _p(cos), _p(sin), s, heads, d, 1, _s()), "HcclFusedRope")
+            _count()
+        part = dqkv[:, (hq + hkv) * d:].view(s, hkv, d)
+        part.copy_(dv) if dv is not None else part.zero_()
+        return dqkv, None, None, None, None
+
+
 # ----------------------------------------------------------------------------- public functions
 def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
     """``x_out = x + delta`` (``delta`` may be None) and ``h = rms_norm(x_out) * weight`` in one pass; returns both."""
@@ -172,3 +213,15 @@ def rope(x, cos, sin, use_kernels: bool = True):
             and x.data_ptr() % 16 == 0 and cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()):
         return _Rope.apply(x, cos, sin)
     return rope_reference(x, cos, sin)
+
+
+def rope_qkv(qkv, cos, sin, hq: int, hkv: int, use_kernels: bool = True):
+    """Splits ``qkv [S, (hq + 2 hkv) * D]`` into heads and rotates q and k: ``([S, hq, D], [S, hkv, D], [S, hkv, D])``."""
+    s, d = qkv.shape[0], qkv.shape[1] // (hq + 2 * hkv)
+    if (use_kernels and _native(qkv) and d % 16 == 0 and hkv > 0 and s > 0 and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
+            and cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.shape == sin.shape == (s, d // 2)
+            and cos.is_contiguous() and sin.is_contiguous()):
+        return _RopeQkv.apply(qkv, cos, sin, hq, hkv)
+    q = rope(qkv[:, :hq * d].view(s, hq, d), cos, sin, use_kernels=use_kernels)
+    k = rope(qkv[:, hq * d:(hq + hkv) * d].view(s, hkv, d), cos, sin, use_kernels=use_kernels)
+    return q, k, qkv[:, (hq + hkv) * d:].view(s, hkv, d)

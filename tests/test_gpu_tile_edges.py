@@ -184,3 +184,23 @@ def test_small_output_matmul(m, n, k, ta, tb):
     if ta and m % 8:
         pytest.skip("transposed A needs M % 8 == 0")
     _check_matmul(m, n, k, ta, tb)
+
+
+# all three gradients, strided ones as attention returns them, and only some of them
+@pytest.mark.parametrize("s,hq,hkv,d", [(1, 1, 1, 16), (65, 8, 2, 64), (130, 16, 16, 128)])
+def test_rope_qkv_matches_the_sliced_form(s, hq, hkv, d):
+    g = torch.Generator(device="cuda").manual_seed(s + hq)
+    base = _rnd(g, s, (hq + 2 * hkv) * d)
+    ang = torch.rand(s, d // 2, device="cuda", generator=g) * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    ups = [_rnd(g, n, s, d).transpose(0, 1) for n in (hq, hkv, hkv)]
+    for used in ((0, 1, 2), (0, 2), (1,)):
+        a, b = base.clone().requires_grad_(), base.clone().requires_grad_()
+        got = fused.rope_qkv(a, cos, sin, hq, hkv)
+        want = (fused.rope(b[:, :hq * d].view(s, hq, d), cos, sin), fused.rope(b[:, hq * d:(hq + hkv) * d].view(s, hkv, d), cos, sin),
+                b[:, (hq + hkv) * d:].view(s, hkv, d))
+        for x, y in zip(got, want):
+            assert torch.equal(x, y)
+        torch.autograd.backward([got[i] for i in used], [ups[i] for i in used])
+        torch.autograd.backward([want[i] for i in used], [ups[i] for i in used])
+        assert torch.equal(a.grad, b.grad)

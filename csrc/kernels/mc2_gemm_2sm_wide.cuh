@@ -1,18 +1,23 @@
 // Wide-tile variant of the two-SM matmul (plain matmul only): a CTA pair works on 256 rows x TWO adjacent column
-// tiles at once, one in each of its two TMEM accumulators, so that every k-block of A is loaded once for 512 output
-// columns instead of once for 256.
+// tiles, one in each of its two TMEM accumulators, so that a k-block of A is loaded once for 512 output columns
+// instead of once for 256.
 //
-// Why: a GPU at its power limit finishes a step when the step's energy has been spent, and with 256 x 256 tiles the
-// shared-memory fill traffic from L2 (64 KiB per pair and k-block, about 11 TB/s at full tensor rate) is a large part
-// of what a matmul spends beyond the tensor cores.  The wide tile needs 48 KiB per CTA and k-block for twice the
-// math (A 16 KiB + two B halves of 16 KiB): a quarter less L2 -> SM traffic per FLOP.  The price: both accumulators
-// belong to the tile in flight, so the epilogue no longer overlaps the next tile's main loop; that is a few percent
-// of a tile when K is in the thousands and too much when it is not, so the launcher picks this kernel only for
-// large K and enough tiles to keep the last wave busy.
+// Why: a GPU at its power limit finishes a matmul when the matmul's energy has been spent, and with 256 x 256 tiles the
+// shared-memory fill traffic from L2 (64 KiB per pair and k-block) is a large part of what is spent beyond the tensor
+// cores.  The wide tile needs 48 KiB per CTA and k-block for twice the math (A 16 KiB + two B halves of 16 KiB): a
+// quarter less L2 -> SM traffic per FLOP.
+//
+// Both accumulators belong to the tile in flight, so the epilogue can only overlap if the two halves end at different
+// times.  They are skewed by `skew` k-blocks: the left half runs k-blocks [0, skew) alone, both run [skew, K) together,
+// the right half catches up with [0, skew) alone.  The left accumulator is drained under the right half's catch-up, the
+// right one under the next tile's left-only stretch; the price is `skew` k-blocks of A loaded twice per tile.
+//
+// Work items: full rounds of wide tiles over all pairs, then the rest as single 256-row x one-column-tile items (at most
+// two per pair, in alternating accumulators), so the launch takes as many column-tile times as the narrow kernel.
 //
 // Pipeline: four stages of 48 KiB; otherwise the roles, barriers and hand-over of mc2_gemm_2sm.cuh (full[stage] in
-// the leader, empty[stage] and tmemFull per CTA through the multicast commit, tmemEmpty in the leader with eight
-// arrivals).
+// the leader, empty[stage] and tmemFull[acc] per CTA through the multicast commit, tmemEmpty[acc] in the leader with
+// eight arrivals).
 #pragma once
 #include "mc2_gemm_2sm.cuh"
 
@@ -29,6 +34,52 @@ struct SmemLayoutWide {
     static constexpr int kTotal = kStagingOff + kEpilogueStagingBytes + 1024;
 };
 
+constexpr int kWideSkew = 12;                         // k-blocks: about the time 256 accumulator columns take to drain
+
+// Item t of the launch -> what a pair does.  Full rounds of wide tiles come first: `wide` of them, a multiple of the
+// pairs; a wide position that is left over becomes two singles, an odd last column tile one.
+struct WideItem { int mt2, nt; bool both; int acc; };
+struct WideOrder {
+    int tilesM2, cols, tilesN, positions, wide, items, nPairs, group;
+    __host__ __device__ WideOrder(int tilesM2_, int tilesN_, int nPairs_, int group_)
+        : tilesM2(tilesM2_), cols(tilesN_ / 2), tilesN(tilesN_), positions(tilesM2_ * (tilesN_ / 2)), nPairs(nPairs_), group(group_)
+    {
+        wide = positions / nPairs * nPairs;
+        items = wide + 2 * (positions - wide) + (tilesN & 1) * tilesM2;
+    }
+    // grouped raster over (256-row tile, pair of column tiles): bands of `group` row tiles, rows fastest
+    __host__ __device__ void Position(int q, int* mt2, int* col) const
+    {
+        const int perBand = group * cols;
+        const int band = q / perBand, rem = q % perBand;
+        const int first = band * group;
+        const int rows = (tilesM2 - first) < group ? (tilesM2 - first) : group;
+        *mt2 = first + rem % rows;
+        *col = rem / rows;
+    }
+    __host__ __device__ WideItem Get(int t) const
+    {
+        WideItem w;
+        int col;
+        if (t < wide) {
+            Position(t, &w.mt2, &col);
+            w.nt = 2 * col; w.both = true; w.acc = 0;
+            return w;
+        }
+        const int s = t - wide, split = 2 * (positions - wide);
+        w.both = false;
+        w.acc = (s / nPairs) & 1;                      // this pair's singles take the accumulators in turn
+        if (s < split) {
+            Position(wide + s / 2, &w.mt2, &col);
+            w.nt = 2 * col + (s & 1);
+        } else {
+            w.mt2 = s - split;
+            w.nt = tilesN - 1;
+        }
+        return w;
+    }
+};
+
 template <bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     GemmKernel2SmWide(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g)
@@ -39,21 +90,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kTileBytes);
     uint64_t* fullBar = bars;                          // [kStagesWide]  (used in the leader)
     uint64_t* emptyBar = bars + kStagesWide;           // [kStagesWide]
-    uint64_t* tmemFull = bars + 2 * kStagesWide;       // one: both accumulators complete together
-    uint64_t* tmemEmpty = bars + 2 * kStagesWide + 1;  // one (used in the leader)
-    uint32_t* tmemBaseSlot = reinterpret_cast<uint32_t*>(bars + 2 * kStagesWide + 2);
+    uint64_t* tmemFull = bars + 2 * kStagesWide;       // [2]
+    uint64_t* tmemEmpty = bars + 2 * kStagesWide + 2;  // [2]            (used in the leader)
+    uint32_t* tmemBaseSlot = reinterpret_cast<uint32_t*>(bars + 2 * kStagesWide + 4);
     volatile uint32_t* abortWord = g.ctl + kCtlAbort;
 
     const int warp = threadIdx.x / 32;
     const int cta = (int)blockIdx.x;
     const uint32_t crank = ClusterCtaRank();
-    const uint32_t launchEpoch = *reinterpret_cast<volatile uint32_t*>(g.ctl + kCtlEpoch) + 1;
 
     constexpr uint32_t kTmemCols = 2 * kBN2;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStagesWide; ++s) { MbarInit(&fullBar[s], 1); MbarInit(&emptyBar[s], 1); }
-        MbarInit(tmemFull, 1);
-        MbarInit(tmemEmpty, 2 * (kEpilogueThreads / 32));
+        for (int a = 0; a < 2; ++a) { MbarInit(&tmemFull[a], 1); MbarInit(&tmemEmpty[a], 2 * (kEpilogueThreads / 32)); }
         MbarInitFence();
         PrefetchTensorMap(&tmA);
         PrefetchTensorMap(&tmB);
@@ -69,20 +118,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const uint32_t tmemBase = *tmemBaseSlot;
     const int BN = g.bn;
     const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;
-    const int tilesM2 = (g.M + 255) / 256;
-    const int tilesNW = (g.tilesN + 1) / 2;             // wide column tiles: (2w, 2w + 1)
-    const int nTiles = tilesM2 * tilesNW;
     const int kBlocks = (g.K + kBK - 1) / kBK;
-    // grouped raster over (256-row tile, wide column tile): bands of g.rasterGroup (default 8) row tiles, rows fastest
-    auto coord = [&](int t, int* mt2, int* ntw) {
-        const int kGroup = g.rasterGroup > 0 ? g.rasterGroup : 8;
-        const int perBand = kGroup * tilesNW;
-        const int band = t / perBand, rem = t % perBand;
-        const int first = band * kGroup;
-        const int rows = (tilesM2 - first) < kGroup ? (tilesM2 - first) : kGroup;
-        *mt2 = first + rem % rows;
-        *ntw = rem / rows;
-    };
+    const WideOrder order((g.M + 255) / 256, g.tilesN, nPairs, g.rasterGroup > 0 ? g.rasterGroup : 8);
+    const int skew = kBlocks / 2 < kWideSkew ? kBlocks / 2 : kWideSkew;
 
     if (warp == 0) {
         // ===== TMA producer (both CTAs)
@@ -90,28 +128,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const uint32_t bHalfBytes = (uint32_t)((BN / 2) * kBK * 2);
-            for (int t = pair; t < nTiles && ok; t += nPairs) {
-                int mt2, ntw;
-                coord(t, &mt2, &ntw);
-                const int mt = mt2 * 2 + (int)crank;
-                const int nt0 = 2 * ntw;
-                const bool second = nt0 + 1 < g.tilesN;
-                for (int kb = 0; kb < kBlocks; ++kb) {
+            // whole boxes of 64 columns for an MN-major half tile of B (see mc2_gemm_2sm.cuh)
+            const uint32_t bHalfBytes = (uint32_t)((B_MN ? (BN / 2 + 63) / 64 * 64 : BN / 2) * kBK * 2);
+            for (int t = pair; t < order.items && ok; t += nPairs) {
+                const WideItem w = order.Get(t);
+                const int mt = w.mt2 * 2 + (int)crank;
+                // steps of a wide item: left only, both, right only; of a single one: its column tile only
+                const int steps = w.both ? kBlocks + skew : kBlocks;
+                for (int i = 0; i < steps; ++i) {
+                    const bool left = !w.both || i < kBlocks, right = w.both && i >= skew;
+                    const int kb = i < kBlocks ? i : i - kBlocks;
                     ok = MbarWait(&emptyBar[stage], phase ^ 1u, abortWord, kWaitLimitNs);
                     if (!ok) break;
                     uint8_t* sa = smem + stage * L::kStageBytes;
                     const uint32_t leaderFull = SmemAddr(&fullBar[stage]) & kPeerBitMask;
-                    if (crank == 0) MbarExpectTx(&fullBar[stage], 2u * ((uint32_t)L::kABytes + (second ? 2u : 1u) * bHalfBytes));
+                    if (crank == 0) MbarExpectTx(&fullBar[stage], 2u * ((uint32_t)L::kABytes + (left && right ? 2u : 1u) * bHalfBytes));
                     if (!A_MN) {
                         TmaLoad2D2Sm(sa, &tmA, leaderFull, kb * kBK, mt * kBM);
                     } else {
 #pragma unroll
                         for (int j = 0; j < kBM / 64; ++j) TmaLoad2D2Sm(sa + j * (64 * kBK * 2), &tmA, leaderFull, mt * kBM + j * 64, kb * kBK);
                     }
-                    for (int h = 0; h < (second ? 2 : 1); ++h) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (!(h == 0 ? left : right)) continue;
                         uint8_t* sb = sa + L::kABytes + h * L::kBBytes;
-                        const int nRow = (nt0 + h) * BN + (int)crank * (BN / 2);
+                        const int nRow = (w.nt + h) * BN + (int)crank * (BN / 2);
                         if (!B_MN) {
                             TmaLoad2D2Sm(sb, &tmB, leaderFull, kb * kBK, nRow);
                         } else {
@@ -134,66 +176,64 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const uint32_t idesc = InstrDescF16(256, BN, true, A_MN, B_MN);
             int stage = 0;
             uint32_t phase = 0;
-            uint32_t accPhase = 0;
+            uint32_t accPhase[2] = {0, 0};
             bool ok = true;
-            for (int t = pair; t < nTiles && ok; t += nPairs) {
-                int mt2, ntw;
-                coord(t, &mt2, &ntw);
-                const bool second = 2 * ntw + 1 < g.tilesN;
-                ok = MbarWait(tmemEmpty, accPhase ^ 1u, abortWord, kWaitLimitNs);
-                if (!ok) break;
-                TcFenceAfter();
-                for (int kb = 0; kb < kBlocks; ++kb) {
-                    ok = MbarWait(&fullBar[stage], phase, abortWord, kWaitLimitNs);
+            for (int t = pair; t < order.items && ok; t += nPairs) {
+                const WideItem w = order.Get(t);
+                const int steps = w.both ? kBlocks + skew : kBlocks;
+                const int first = w.both ? 0 : w.acc;      // accumulator of the left (or only) half
+                for (int i = 0; i < steps; ++i) {
+                    const bool left = !w.both || i < kBlocks, right = w.both && i >= skew;
+                    if (i == 0) ok = MbarWait(&tmemEmpty[first], accPhase[first] ^ 1u, abortWord, kWaitLimitNs);
+                    if (ok && w.both && i == skew) ok = MbarWait(&tmemEmpty[1], accPhase[1] ^ 1u, abortWord, kWaitLimitNs);
+                    if (ok) ok = MbarWait(&fullBar[stage], phase, abortWord, kWaitLimitNs);
                     if (!ok) break;
                     TcFenceAfter();
                     const uint32_t sa = SmemAddr(smem + stage * L::kStageBytes);
                     const uint64_t da = A_MN ? SmemDescMnMajor(sa, 64 * kBK * 2) : SmemDescKMajor(sa);
-                    for (int h = 0; h < (second ? 2 : 1); ++h) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (!(h == 0 ? left : right)) continue;
                         const uint32_t sb = sa + L::kABytes + h * L::kBBytes;
                         const uint64_t db = B_MN ? SmemDescMnMajor(sb, 64 * kBK * 2) : SmemDescKMajor(sb);
-                        const uint32_t tmemD = tmemBase + (uint32_t)(h * kBN2);
+                        const uint32_t tmemD = tmemBase + (uint32_t)((h == 0 ? first : 1) * kBN2);
+                        const int start = h == 0 ? 0 : skew;
 #pragma unroll
                         for (int k = 0; k < kBK / kUmmaK; ++k) {
                             const uint64_t aStep = (uint64_t)((A_MN ? kUmmaK * 128 : kUmmaK * 2) >> 4) * k;
                             const uint64_t bStep = (uint64_t)((B_MN ? kUmmaK * 128 : kUmmaK * 2) >> 4) * k;
-                            UmmaF16_2Sm(tmemD, da + aStep, db + bStep, idesc, (kb | k) != 0 ? 1u : 0u);
+                            UmmaF16_2Sm(tmemD, da + aStep, db + bStep, idesc, (i != start || k != 0) ? 1u : 0u);
                         }
                     }
                     UmmaCommit2Sm(&emptyBar[stage]);
+                    if (i == kBlocks - 1) { UmmaCommit2Sm(&tmemFull[first]); accPhase[first] ^= 1u; }
+                    if (w.both && i == steps - 1) { UmmaCommit2Sm(&tmemFull[1]); accPhase[1] ^= 1u; }
                     if (++stage == kStagesWide) { stage = 0; phase ^= 1u; }
                 }
-                if (!ok) break;
-                UmmaCommit2Sm(tmemFull);
-                accPhase ^= 1u;
             }
         }
     } else {
-        // ===== epilogue warps 2..5 of both CTAs: each CTA drains its own 128 accumulator rows of both column tiles
+        // ===== epilogue warps 2..5 of both CTAs: each CTA drains its own 128 accumulator rows
         const int quarter = warp & 3;
         const int lane = threadIdx.x & 31;
-        uint32_t accPhase = 0;
+        uint32_t accPhase[2] = {0, 0};
         bool ok = true;
-        for (int t = pair; t < nTiles && ok; t += nPairs) {
-            int mt2, ntw;
-            coord(t, &mt2, &ntw);
-            const int mt = mt2 * 2 + (int)crank;
-            ok = MbarWait(tmemFull, accPhase, abortWord, kWaitLimitNs);
-            if (!ok) break;
-            TcFenceAfter();
-            const int row0 = mt * kBM + quarter * 32;
+        for (int t = pair; t < order.items && ok; t += nPairs) {
+            const WideItem w = order.Get(t);
+            const int row0 = (w.mt2 * 2 + (int)crank) * kBM + quarter * 32;
             uint8_t* stg = smem + L::kStagingOff + quarter * kStgWarpBytes;
-            for (int h = 0; h < 2; ++h) {
-                const int nt = 2 * ntw + h;
-                if (nt >= g.tilesN) break;
-                const uint32_t taddr = tmemBase + (uint32_t)(h * kBN2) + ((uint32_t)(quarter * 32) << 16);
-                const int validCols = g.N - nt * BN;
-                DrainTileRows(taddr, BN, stg, lane, validCols, g.M - row0, g.out + (size_t)row0 * g.ldc + (size_t)nt * BN, (size_t)g.ldc);
+            for (int h = 0; h < (w.both ? 2 : 1); ++h) {
+                const int acc = w.both ? h : w.acc, nt = w.nt + h;
+                ok = MbarWait(&tmemFull[acc], accPhase[acc], abortWord, kWaitLimitNs);
+                if (!ok) break;
+                TcFenceAfter();
+                const uint32_t taddr = tmemBase + (uint32_t)(acc * kBN2) + ((uint32_t)(quarter * 32) << 16);
+                DrainTileRows(taddr, BN, stg, lane, g.N - nt * BN, g.M - row0, g.out + (size_t)row0 * g.ldc + (size_t)nt * BN, (size_t)g.ldc);
+                TcFenceBefore();
+                __syncwarp();
+                if (lane == 0) MbarArriveCluster(SmemAddr(&tmemEmpty[acc]) & kPeerBitMask);
+                accPhase[acc] ^= 1u;
             }
-            TcFenceBefore();
-            __syncwarp();
-            if (lane == 0) MbarArriveCluster(SmemAddr(tmemEmpty) & kPeerBitMask);
-            accPhase ^= 1u;
         }
     }
     TcFenceBefore();
@@ -202,16 +242,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (warp == 1) {
         TcFenceAfter();
         TmemDealloc2(tmemBase, kTmemCols);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t ticket = atomicAdd(g.ctl + kCtlTicket, 1u);
-        if (ticket == gridDim.x - 1) {
-            g.ctl[kCtlTicket] = 0;
-            *reinterpret_cast<volatile uint32_t*>(g.ctl + kCtlEpoch) = launchEpoch;
-            __threadfence();
-        }
     }
 }
 

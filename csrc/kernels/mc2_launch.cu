@@ -163,16 +163,16 @@ HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const S
     return HCCL_SUCCESS;
 }
 
-// Wide tiles (two column tiles per CTA pair, see mc2_gemm_2sm_wide.cuh): HCCL_MC2_WIDE=1 whenever the shape allows,
-// HCCL_MC2_WIDE=auto when the inner dimension is long and there are enough tiles to fill the last wave; off otherwise.
-// Measured on the decoder's matmuls the unoverlapped epilogue (about 9 us per 256 accumulator columns) costs more
-// than the saved L2 traffic returns, so the double-buffered 256 x 256 kernel stays the default.
+// Wide tiles (two column tiles per CTA pair, see mc2_gemm_2sm_wide.cuh): where at least two full rounds of them run, so
+// that most of the output gains from the saved L2 traffic, and the inner dimension has 48 k-blocks or more, so that the
+// dozen whose A is loaded twice per tile stay a small part.  HCCL_MC2_WIDE=0 turns them off, 1 takes them wherever one
+// full round runs.
 int WideMode()
 {
     static int v = -2;
     if (v == -2) {
         const char* e = getenv("HCCL_MC2_WIDE");
-        v = e == nullptr ? 0 : (e[0] == 'a' ? -1 : (e[0] == '1' ? 1 : 0));
+        v = e == nullptr || e[0] == 'a' ? -1 : (e[0] == '1' ? 1 : 0);
     }
     return v;
 }
@@ -451,32 +451,14 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         g.tilesN = (int)((n + bestBn - 1) / bestBn);
         // B is split between the two CTAs of a pair: each loads half of the B rows of a tile
         CHK_RET(MapB(&tb, b, n, k, bMn, bestBn / 2));
-        const double bestCost = (double)((tilesM2 * g.tilesN + pairs - 1) / pairs) * (bestBn + 12);
-        // wide tiles: the same search over (waves x width) with two column tiles per work item
-        {
-            int wideBn = 0;
-            double wideCost = 1e30;
-            for (int cand : {256, 224, 192, 160, 128}) {
-                if (bMn && (cand / 2) % 64 != 0) continue;
-                const int tn = (int)((n + cand - 1) / cand);
-                const int items = tilesM2 * ((tn + 1) / 2);
-                const int waves = (items + pairs - 1) / pairs;
-                const double cost = (double)waves * 2.0 * (cand + 12);
-                if (cost < wideCost - 1e-9) { wideCost = cost; wideBn = cand; }
-            }
-            const int wideItems = tilesM2 * (((int)((n + wideBn - 1) / wideBn) + 1) / 2);
-            const bool wideAuto = k >= 4096 && wideItems >= 4 * pairs && wideCost <= bestCost * 1.03;
-            if (WideMode() != 0 && (WideMode() == 1 || wideAuto) && n > (uint64_t)wideBn) {
-                g.bn = wideBn;
-                g.tilesN = (int)((n + wideBn - 1) / wideBn);
-                CHK_RET(MapB(&tb, b, n, k, bMn, wideBn / 2));
-                const int grid2 = std::min(SmCount() & ~1, 2 * wideItems);
-                g.nGemmCtas = grid2;
-                if (!aMn && !bMn) return LaunchGemm2SmWide<false, false>(ta, tb, g, grid2, stream);
-                if (!aMn && bMn) return LaunchGemm2SmWide<false, true>(ta, tb, g, grid2, stream);
-                if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, grid2, stream);
-                return LaunchGemm2SmWide<true, true>(ta, tb, g, grid2, stream);
-            }
+        const WideOrder order(tilesM2, g.tilesN, pairs, 8);
+        if (WideMode() == 1 ? order.wide > 0 : (WideMode() == -1 && order.wide >= 2 * pairs && k >= 48 * kBK)) {
+            const int grid2 = 2 * pairs;
+            g.nGemmCtas = grid2;
+            if (!aMn && !bMn) return LaunchGemm2SmWide<false, false>(ta, tb, g, grid2, stream);
+            if (!aMn && bMn) return LaunchGemm2SmWide<false, true>(ta, tb, g, grid2, stream);
+            if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, grid2, stream);
+            return LaunchGemm2SmWide<true, true>(ta, tb, g, grid2, stream);
         }
         // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
         // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next

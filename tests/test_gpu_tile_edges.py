@@ -176,6 +176,12 @@ def test_wide_matmul_with_kn_weight(m, n, k, ta):
     _check_matmul(m, n, k, ta, False)
 
 
+# two full rounds of wide tiles, then left-over positions and an odd last column tile as single ones; ragged in every direction
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+def test_wide_tile_rounds(ta, tb):
+    _check_matmul(2504, 7800, 3080, ta, tb)
+
+
 # token tiles of 16 .. 128 and several of them, k-blocks fewer and more than the CTAs of a cluster, ragged N and K
 @pytest.mark.parametrize("ta,tb", LAYOUTS)
 @pytest.mark.parametrize("m,n,k", [(8, 8, 8), (16, 128, 64), (24, 136, 256), (64, 1024, 520), (128, 248, 2048), (136, 1000, 1032), (304, 640, 4096),

@@ -58,8 +58,8 @@ __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, 
 // Bound by the bytes written (topk fp8 copies of every row, over NVLink to the peers).  A WARP owns a token: a lane
 // takes 16 elements of the row (two 16-byte loads), eight lanes share a 128-element block's maximum, and the lane
 // quantises its 16 elements in registers and stores them to all topk destinations, 512 contiguous bytes per warp and
-// destination.  No block-wide step inside a token, so all warps' loads and stores overlap; with a block per token and
-// its three barriers a rank of 256 tokens spent four fifths of the time waiting for one row at a time.
+// destination.  No block-wide step inside a token, so all warps' loads and stores overlap.  Measured against a block
+// per token with three barriers, 8 emulated ranks, 256 tokens x 7168, top-8: 130 -> 50 us (150 MB).
 struct DispatchBody {
     using Args = MoeDispatchArgs;
     static constexpr int kThreads = kMoeThreads;
@@ -190,8 +190,8 @@ struct DispatchBody {
 // A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: 32 * kCombinePieces 16-byte pieces of one
 // token's row (a part of a row, so that a few hundred tokens still give every warp of the chip something to load); a
 // lane requests topk loads per piece, two pieces at a time, before it uses the first.  Lane k keeps the k-th copy's
-// address and weight and hands them round by shuffle: eight addresses per lane in registers held the kernel at 8 warps
-// per SM.
+// address and weight and hands them round by shuffle.  Measured against a block per token: 89 -> 90 us (264 MB, the expert
+// rows still being written back: level), 8 emulated ranks, 256 tokens x 7168, top-8.
 constexpr int kCombinePieces = 4;
 struct CombineBody {
     using Args = MoeCombineArgs;

@@ -58,7 +58,7 @@ static __global__ void __launch_bounds__(kRouteThreads) MoeExpertOffsetsKernel(c
     if (!s_last) return;
     __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t run = 0;                               // pairs of all experts before this round's
+    uint32_t run = 0;                               // pairs of all experts before this pass of the loop
     for (uint32_t base = 0; base < nExperts; base += kRouteThreads) {
         const uint32_t e = base + threadIdx.x;
         uint32_t c = 0;
@@ -82,7 +82,7 @@ static __global__ void __launch_bounds__(kRouteThreads) MoeExpertOffsetsKernel(c
         }
         if (e < nExperts) offsets[e] = run + before + incl - c;
         run += all;
-        __syncthreads();                            // s_warp is read before the next round writes it
+        __syncthreads();                            // s_warp is read before the next pass writes it
     }
     if (threadIdx.x == 0) {
         offsets[nExperts] = run;

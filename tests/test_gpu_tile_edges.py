@@ -70,10 +70,33 @@ def test_swiglu_extremes():
     want = fused.swiglu_reference(x.double())
     got = fused.swiglu(x).double()
     assert torch.isfinite(got).all()
-    torch.testing.assert_close(got, want, rtol=8e-3, atol=1e-30)
+    torch.testing.assert_close(got, want, rtol=8e-3, atol=2.0 ** -126)      # the smallest normal number
     x = torch.tensor([[float("nan")] + [float("inf")] * 7 + [1.0] * 8], device="cuda").bfloat16()
     got = fused.swiglu(x)
     assert torch.isnan(got[0, 0]) and torch.isinf(got[0, 1:]).all()
+
+
+@pytest.mark.parametrize("rows", [1, 40])                     # one vector per thread, several
+def test_swiglu_of_every_gate(rows):
+    """All bf16 gates.  Around -88 the exponential is near the largest fp32 number and the result a normal bf16 one; below
+    -88.5 the exponential overflows and the result is 0."""
+    gate = torch.arange(-32768, 32768, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = torch.cat((gate, torch.full_like(gate, 3.0))).repeat(rows, 1).requires_grad_()
+    dy = torch.full((rows, gate.numel()), 2.0, device="cuda", dtype=torch.bfloat16)
+    y = fused.swiglu(x)
+    y.backward(dy)
+    x64 = x.detach().double().requires_grad_()
+    y64 = fused.swiglu_reference(x64)
+    dx = torch.autograd.grad(y64, x64, dy.double())[0]
+    g = gate.float()
+    # 2^-126: the smallest normal number; gradients of gates near the zero of silu's slope cancel, to fp32's last place
+    seen, zero = (g >= -88.5) & (g <= 1e38), (g < -88.75) & torch.isfinite(g)
+    for got, want, extra in ((y.detach(), y64.detach(), 0.0), (x.grad[:, :gate.numel()], dx[:, :gate.numel()], 2e-6), (x.grad[:, gate.numel():], dx[:, gate.numel():], 0.0)):
+        err = (got.double() - want).abs()
+        assert (err[:, seen] <= ONE_ROUNDING * want[:, seen].abs() + 2.0 ** -126 + extra * (g[seen] > -4)).all()
+        assert (got[:, zero] == 0).all()
+    assert torch.isnan(y[:, torch.isnan(g) | (g == float("-inf"))]).all() and torch.isinf(y[:, g == float("inf")]).all()
+    assert torch.equal(torch.signbit(y[0, g == 0]), torch.signbit(g[g == 0]))
 
 
 # heads per thread: four, two, one, a last group that is not full; rows per block: many, one, one in several passes

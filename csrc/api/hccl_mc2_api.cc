@@ -150,6 +150,14 @@ HcclResult HcclMc2Matmul(const void* a, const void* b, void* out, uint64_t m, ui
 {
     return Mc2Matmul(a, b, out, m, n, k, transA, transB, (cudaStream_t)stream);
 }
+// Tests: the matmul with a CTA whose operands never arrive.  `out` must stay as it is where that CTA's tile lies, and the next
+// matmul on the device must return HCCL_E_TIMEOUT.
+HcclResult HcclDebugMatmulStalled(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, int cta,
+                                  uint64_t waitLimitNs, hcclStream_t stream)
+{
+    const Mc2StalledCta stalled = {cta, waitLimitNs};
+    return Mc2Matmul(a, b, out, m, n, k, transA, transB, (cudaStream_t)stream, &stalled);
+}
 HcclResult HcclMc2AllGatherMatmul(const void* aShard, const void* b, void* out, void* gathered, uint64_t mPerRank, uint64_t n, uint64_t k,
                                   int transB, HcclComm comm, hcclStream_t stream)
 {

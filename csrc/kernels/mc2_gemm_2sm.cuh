@@ -248,10 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         if (++stage == kStages2) { stage = 0; phase ^= 1u; }
                     }
                 }
-                if (!ok) {
-                    const uint64_t t0 = TimerNs();
-                    while (TimerNs() - t0 < 200000) {}
-                }
+                if (!ok) GiveUp(g.ctl);
                 MC2_TR(if (g.trace) {
                     uint64_t* w = g.trace + (size_t)cta * kTraceWords;
                     w[TR_PROD_READY_CLK] = (uint64_t)trReady; w[TR_PROD_FIRST_REMOTE_NS] = trFirst; w[TR_PROD_EMPTY_CLK] = (uint64_t)trEmpty;
@@ -298,6 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     UmmaCommit2Sm(&tmemFull[acc]);
                     if (++acc == 2) { acc = 0; accPhase ^= 1u; }
                 }
+                if (!ok) GiveUp(g.ctl);
                 MC2_TR(if (g.trace) {
                     uint64_t* w = g.trace + (size_t)cta * kTraceWords;
                     w[TR_MMA_FULL_CLK] = (uint64_t)trFull; w[TR_MMA_TMEM_CLK] = (uint64_t)trTmem; w[TR_MMA_END_NS] = TimerNs();
@@ -327,7 +325,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (MODE == MODE_AG && pushLeft) pushLeft = CoopPushWhileWaiting(g, launchEpoch, lane, &tmemFull[acc], accPhase);
                 if (MODE == MODE_RS && reduceLeft) reduceLeft = CoopReduceWhileWaiting(g, launchEpoch, lane, &reducePending, &tmemFull[acc], accPhase);
                 MC2_TR(const long long c1 = clock64(); trPush += c1 - c0;)
-                ok = MbarWait(&tmemFull[acc], accPhase, abortWord, kWaitLimitNs);
+                ok = __all_sync(0xFFFFFFFFu, MbarWait(&tmemFull[acc], accPhase, abortWord, kWaitLimitNs));
                 MC2_TR(const long long c2 = clock64(); trWait += c2 - c1;)
                 if (!ok) break;
                 TcFenceAfter();
@@ -369,6 +367,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             MC2_TR(const long long c3 = clock64();)
             if (MODE == MODE_AG && pushLeft) CoopPushDrain(g, launchEpoch, lane);
             if (MODE == MODE_RS && reduceLeft) CoopReduceDrain(g, launchEpoch, lane, &reducePending);
+            if (!ok && lane == 0) GiveUp(g.ctl);
             MC2_TR(trTail = clock64() - c3;
                    if (trMe) {
                        uint64_t* w = g.trace + (size_t)cta * kTraceWords;

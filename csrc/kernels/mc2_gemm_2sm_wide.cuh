@@ -165,10 +165,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if (++stage == kStagesWide) { stage = 0; phase ^= 1u; }
                 }
             }
-            if (!ok) {
-                const uint64_t t0 = TimerNs();
-                while (TimerNs() - t0 < 200000) {}
-            }
+            if (!ok) GiveUp(g.ctl);
         }
     } else if (warp == 1) {
         // ===== MMA issuer: leader CTA only
@@ -211,6 +208,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if (++stage == kStagesWide) { stage = 0; phase ^= 1u; }
                 }
             }
+            if (!ok) GiveUp(g.ctl);
         }
     } else {
         // ===== epilogue warps 2..5 of both CTAs: each CTA drains its own 128 accumulator rows
@@ -224,7 +222,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             uint8_t* stg = smem + L::kStagingOff + quarter * kStgWarpBytes;
             for (int h = 0; h < (w.both ? 2 : 1); ++h) {
                 const int acc = w.both ? h : w.acc, nt = w.nt + h;
-                ok = MbarWait(&tmemFull[acc], accPhase[acc], abortWord, kWaitLimitNs);
+                ok = __all_sync(0xFFFFFFFFu, MbarWait(&tmemFull[acc], accPhase[acc], abortWord, kWaitLimitNs));
                 if (!ok) break;
                 TcFenceAfter();
                 const uint32_t taddr = tmemBase + (uint32_t)(acc * kBN2) + ((uint32_t)(quarter * 32) << 16);
@@ -235,6 +233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 accPhase[acc] ^= 1u;
             }
         }
+        if (!ok && lane == 0) GiveUp(g.ctl);
     }
     TcFenceBefore();
     __syncthreads();

@@ -17,7 +17,8 @@
 // 73.9 -> 26.6, 300 x 2048 x 4096 24.7 -> 16.5; against its 256-wide form 16 x 57344 x 8192 160.6 -> 142.4 (6.6 TB/s), 64
 // x 57344 x 8192 162.3 -> 151.0.
 // Warp roles and waits are those of the other kernels (mc2_gemm.cuh): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5
-// drain the accumulator; every wait is bounded.
+// drain the accumulator; every wait is bounded, and a CTA that gave one up tells its cluster, which then stores nothing of
+// the tile: what its shared memory holds is no partial sum.
 #pragma once
 #include "mc2_gemm.cuh"
 
@@ -38,6 +39,8 @@ struct SplitArgs {
     int tilesM;                // token tiles; the tile index runs over them first, so that they share a weight tile in L2
     int stages;
     uint32_t* ctl;             // control block: the abort word of bounded waits
+    uint64_t waitLimitNs;      // of every wait
+    int stalledCta;            // tests: this CTA's producer loads nothing (-1: none)
 };
 
 __host__ __device__ constexpr int SplitStageBytes(int bt) { return kSplitWBytes + bt * kBK * 2; }
@@ -69,6 +72,13 @@ __device__ __forceinline__ void SplitClusterSync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ uint32_t LdCluster1(uint32_t localAddr, uint32_t rank)
+{
+    uint32_t a, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(localAddr), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
 __device__ __forceinline__ float4 LdCluster4(uint32_t localAddr, uint32_t rank)
 {
     uint32_t a;
@@ -99,6 +109,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
     uint64_t* emptyBar = fullBar + kSplitMaxStages;
     uint64_t* tmemFull = fullBar + 2 * kSplitMaxStages;
     uint32_t* tmemBaseSlot = reinterpret_cast<uint32_t*>(fullBar + 2 * kSplitMaxStages + 1);
+    volatile uint32_t* gaveUp = tmemBaseSlot + 1;      // a role of this CTA left before its work was done
     volatile uint32_t* abortWord = g.ctl + kCtlAbort;
 
     const int warp = threadIdx.x / 32;
@@ -112,6 +123,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
     if (threadIdx.x == 0) {
         for (int s = 0; s < g.stages; ++s) { MbarInit(&fullBar[s], 1); MbarInit(&emptyBar[s], 1); }
         MbarInit(tmemFull, 1);
+        *gaveUp = 0;
         MbarInitFence();
         PrefetchTensorMap(&tmW);
         PrefetchTensorMap(&tmX);
@@ -130,8 +142,8 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int kb = kFirst; kb < kLast; ++kb) {
-                ok = MbarWait(&emptyBar[stage], phase ^ 1u, abortWord, kWaitLimitNs);
+            for (int kb = kFirst; kb < kLast && (int)blockIdx.x != g.stalledCta; ++kb) {
+                ok = MbarWait(&emptyBar[stage], phase ^ 1u, abortWord, g.waitLimitNs);
                 if (!ok) break;
                 uint8_t* sw = smem + stage * stageBytes;
                 uint8_t* sx = sw + kSplitWBytes;
@@ -149,11 +161,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
                 }
                 if (++stage == g.stages) { stage = 0; phase ^= 1u; }
             }
-            if (!ok) {
-                // let copies that were already issued land before the CTA's shared memory goes away
-                const uint64_t t0 = TimerNs();
-                while (TimerNs() - t0 < 200000) {}
-            }
+            if (!ok) { *gaveUp = 1; GiveUp(g.ctl); }
         }
     } else if (warp == 1) {
         if (ElectOne()) {
@@ -162,7 +170,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
             uint32_t phase = 0;
             bool ok = true;
             for (int kb = kFirst; kb < kLast; ++kb) {
-                ok = MbarWait(&fullBar[stage], phase, abortWord, kWaitLimitNs);
+                ok = MbarWait(&fullBar[stage], phase, abortWord, g.waitLimitNs);
                 if (!ok) break;
                 TcFenceAfter();
                 const uint32_t sw = SmemAddr(smem + stage * stageBytes);
@@ -179,12 +187,13 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
                 if (++stage == g.stages) { stage = 0; phase ^= 1u; }
             }
             if (ok) UmmaCommit(tmemFull);
+            else { *gaveUp = 1; GiveUp(g.ctl); }
         }
     } else {
         // accumulator lanes = weight rows (output columns), accumulator columns = tokens; the MMAs that read the ring
         // have completed, so the partial tile may take its place
         const int quarter = warp & 3, lane = threadIdx.x & 31;
-        if (MbarWait(tmemFull, 0, abortWord, kWaitLimitNs)) {
+        if (__all_sync(0xFFFFFFFFu, MbarWait(tmemFull, 0, abortWord, g.waitLimitNs))) {
             TcFenceAfter();
             const uint32_t taddr = tmemBase + ((uint32_t)(quarter * 32) << 16);
             float* part = reinterpret_cast<float*>(smem) + quarter * 32 + lane;
@@ -196,6 +205,9 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
                 for (int j = 0; j < 16; ++j) part[(c + j) * 128] = __uint_as_float(v[j]);
             }
             TcFenceBefore();
+        } else if (lane == 0) {
+            *gaveUp = 1;
+            GiveUp(g.ctl);
         }
     }
     __syncthreads();
@@ -205,6 +217,10 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
         const int tokens = (g.M - row0) < g.bt ? (g.M - row0) : g.bt;
         const int t0 = tokens * crank / split, t1 = tokens * (crank + 1) / split;
         const uint32_t base = SmemAddr(smem);
+        uint32_t lost = 0;
+#pragma unroll
+        for (int r = 0; r < kSplitMaxCluster; ++r)
+            if (r < split) lost |= LdCluster1(SmemAddr(const_cast<uint32_t*>(gaveUp)), (uint32_t)r);
         for (int i = t0 * 32 + (int)threadIdx.x; i < t1 * 32; i += kThreads) {
             const int t = i >> 5, c = (i & 31) * 4;
             float4 p[kSplitMaxCluster];
@@ -215,7 +231,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
 #pragma unroll
             for (int r = 1; r < kSplitMaxCluster; ++r)
                 if (r < split) { s.x += p[r].x; s.y += p[r].y; s.z += p[r].z; s.w += p[r].w; }
-            if (col0 + c < g.N) {                      // N is a multiple of 8
+            if (col0 + c < g.N && lost == 0) {         // N is a multiple of 8
                 __nv_bfloat162 lo = __floats2bfloat162_rn(s.x, s.y), hi = __floats2bfloat162_rn(s.z, s.w);
                 *reinterpret_cast<uint2*>(g.out + (size_t)(row0 + t) * g.N + col0 + c) =
                     make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));

@@ -265,21 +265,48 @@ HcclResult DispatchLayout(bool aMn, bool bMn, const CUtensorMap& ta, const CUten
     return HCCL_E_NOT_SUPPORT;
 }
 
-// Control block for plain matmuls (no communicator): one per device, zeroed once.
-uint32_t* PlainCtl()
+// Control block for plain matmuls (no communicator): one per device, zeroed once.  `gaveUp` is a word of host memory that a
+// kernel sets when one of its waits ran out (GiveUp).
+struct PlainCtl { uint32_t* ctl = nullptr; volatile uint32_t* gaveUp = nullptr; };
+HcclResult GetPlainCtl(PlainCtl* out)
 {
     static std::mutex mu;
-    static std::map<int, uint32_t*> perDev;
+    static std::map<int, PlainCtl> perDev;
     std::lock_guard<std::mutex> lk(mu);
     int dev = 0;
-    cudaGetDevice(&dev);
+    CHK_CUDA(cudaGetDevice(&dev));
     auto it = perDev.find(dev);
-    if (it != perDev.end()) return it->second;
-    uint32_t* p = nullptr;
-    if (cudaMalloc(&p, kMc2CtlWords * sizeof(uint32_t)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, kMc2CtlWords * sizeof(uint32_t));
-    perDev[dev] = p;
-    return p;
+    if (it == perDev.end()) {
+        uint32_t *ctl = nullptr, *host = nullptr;
+        if (cudaHostAlloc((void**)&host, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return HCCL_E_MEMORY;
+        if (cudaMalloc(&ctl, kMc2CtlWords * sizeof(uint32_t)) != cudaSuccess) { cudaFreeHost(host); return HCCL_E_MEMORY; }
+        *host = 0;
+        std::vector<uint32_t> init(kMc2CtlWords, 0);
+        const uint64_t address = (uint64_t)(uintptr_t)host;      // one address space: the device uses the host's pointer
+        memcpy(&init[kCtlHostWord], &address, sizeof(address));
+        // on every stream the first matmul comes after the block is written
+        if (cudaMemcpy(ctl, init.data(), kMc2CtlWords * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+            cudaFree(ctl);
+            cudaFreeHost(host);
+            return HCCL_E_RUNTIME;
+        }
+        it = perDev.emplace(dev, PlainCtl{ctl, host}).first;
+    }
+    *out = it->second;
+    return HCCL_SUCCESS;
+}
+// An earlier matmul on this device gave up a wait: part of its output was not written, and with the abort word up later ones
+// would give up early too.  The call that finds it reports it and starts nothing; the next one runs again.
+HcclResult ReportGaveUp(const PlainCtl& p, cudaStream_t stream)
+{
+    HCCL_ERROR("an earlier matmul on this device gave up a wait; part of its output was not written");
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        *p.gaveUp = 0;
+        CHK_CUDA(cudaMemsetAsync(p.ctl + kCtlAbort, 0, sizeof(uint32_t), stream));
+    }
+    return HCCL_E_TIMEOUT;
 }
 
 // Column tile width of a plain two-SM matmul: the one with the least (waves x time of a tile).  A k-block of a 256 x bn tile
@@ -391,12 +418,16 @@ HcclResult Mc2EnsureState(CommImpl* comm, uint64_t parityBytes)
     return HCCL_SUCCESS;
 }
 
-HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, cudaStream_t stream)
+HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, cudaStream_t stream,
+                     const Mc2StalledCta* stalled)
 {
     CHK_PTR_NULL(a); CHK_PTR_NULL(b); CHK_PTR_NULL(out);
     CHK_RET(CheckShapes(m, n, k));
     const bool aMn = transA != 0, bMn = transB == 0;
     if (aMn && m % 8 != 0) return HCCL_E_PARA;
+    PlainCtl plain;
+    CHK_RET(GetPlainCtl(&plain));
+    if (*plain.gaveUp != 0) return ReportGaveUp(plain, stream);
     const int tilesM = (int)((m + kBM - 1) / kBM), tilesM2 = (int)((m + 255) / 256);
     const int pairs = (SmCount() & ~1) / 2;
     // narrow: 256-wide column tiles would leave most SMs idle
@@ -420,8 +451,9 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         g.bt = ((int)((m + parts - 1) / parts) + unit - 1) / unit * unit;
         g.tilesM = (int)((m + g.bt - 1) / g.bt);
         g.stages = SplitStages(g.bt);
-        g.ctl = PlainCtl();
-        if (!g.ctl) return HCCL_E_MEMORY;
+        g.ctl = plain.ctl;
+        g.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
+        g.stalledCta = stalled != nullptr ? stalled->cta : -1;
         // two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile)
         const int tiles = g.tilesM * (int)((n + 127) / 128), kBlocks = (int)((k + kBK - 1) / kBK);
         const int split = std::max(1, std::min({kSplitMaxCluster, 2 * SmCount() / tiles, kBlocks / 4}));
@@ -433,6 +465,7 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, split, stream);
         return LaunchGemmSplit<true, true>(tw, tx, g, tiles, split, stream);
     }
+    if (stalled != nullptr) return HCCL_E_NOT_SUPPORT;
     CUtensorMap ta, tb;
     CHK_RET(MapA(&ta, a, m, k, aMn));
     GemmArgs g;
@@ -440,8 +473,7 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     g.M = (int)m; g.N = (int)n; g.K = (int)k;
     g.out = (__nv_bfloat16*)out;
     g.ldc = (int)n;
-    g.ctl = PlainCtl();
-    if (!g.ctl) return HCCL_E_MEMORY;
+    g.ctl = plain.ctl;
     g.nRanks = 1;
     DevComm dummy;
     memset(&dummy, 0, sizeof(dummy));

@@ -23,8 +23,10 @@ constexpr int kMc2MaxTiles = 16384;
 constexpr int kMc2AgBlocks = 8 * 512;   // arrival counters of the push-form AllGather: ranks x 128-row blocks per rank
 constexpr int kMc2CtlWords = 16 + 8 * 512;
 
+// Tests of a wait that runs out, on a matmul with few output tiles: CTA `cta` loads nothing, all waits end after waitLimitNs.
+struct Mc2StalledCta { int cta; uint64_t waitLimitNs; };
 HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB,
-                     cudaStream_t stream);
+                     cudaStream_t stream, const Mc2StalledCta* stalled = nullptr);
 HcclResult Mc2AllGatherMatmul(CommImpl* comm, const void* aShard, const void* b, void* out, void* gathered, uint64_t mPerRank,
                               uint64_t n, uint64_t k, int transB, cudaStream_t stream);
 HcclResult Mc2MatmulReduceScatter(CommImpl* comm, const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k,

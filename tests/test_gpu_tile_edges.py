@@ -215,6 +215,29 @@ def test_small_output_matmul(m, n, k, ta, tb):
     _check_matmul(m, n, k, ta, tb)
 
 
+# the stalled CTA alone on its tile, and one of a cluster of four: its peers hold good partials and must not store sums either
+@pytest.mark.parametrize("cta,k", [(0, 128), (0, 2048), (2, 2048)])
+def test_matmul_that_gives_up_a_wait(cta, k):
+    """A CTA whose operands never arrive gives up after a short limit: nothing of its tile is stored, the next matmul on the
+    device reports it, the one after that runs."""
+    import ctypes
+    from hccl_b200 import Result
+    from hccl_b200._lib import lib
+    from hccl_b200.comm import HcclError
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = _rnd(g, 16, k), _rnd(g, 128, k)
+    out = torch.full((16, 128), 7.0, device="cuda", dtype=torch.bfloat16)
+    ptr = [ctypes.c_void_p(t.data_ptr()) for t in (a, b, out)]
+    lib.HcclDebugMatmulStalled.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_uint64] * 3 + [ctypes.c_int] * 3 + [ctypes.c_uint64, ctypes.c_void_p]
+    assert lib.HcclDebugMatmulStalled(*ptr, 16, 128, k, 0, 1, cta, 1_000_000, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert (out == 7.0).all()
+    with pytest.raises(HcclError) as e:
+        mc2.matmul(a, b)
+    assert e.value.code == Result.E_TIMEOUT
+    _check_matmul(16, 128, k, False, True)
+
+
 # all three gradients, strided ones as attention returns them, and only some of them
 @pytest.mark.parametrize("s,hq,hkv,d", [(1, 1, 1, 16), (65, 8, 2, 64), (130, 16, 16, 128)])
 def test_rope_qkv_matches_the_sliced_form(s, hq, hkv, d):

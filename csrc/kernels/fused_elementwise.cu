@@ -6,11 +6,11 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include "hccl/hccl_fused_ops.h"
 #include "../core/log.h"
+#include "../core/per_device.h"
 
 namespace hccl {
 namespace {
@@ -481,32 +481,14 @@ __global__ void __launch_bounds__(kRopeThreads) RopeKernel(const __nv_bfloat16* 
     }
 }
 
-constexpr int kMaxDevices = 64;
-int CurrentDevice()
+// Lets a norm kernel take the largest ring the norm kernels use.
+template <auto KERNEL> HcclResult AllowNormRing()
 {
-    int dev = 0;
-    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices ? dev : 0;
-}
-int SmCount()
-{
-    static std::atomic<int> count[kMaxDevices];        // asked once per device
-    const int dev = CurrentDevice();
-    int n = count[dev].load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
-        count[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-// Lets `kernel` take the largest ring the norm kernels use; asked once per kernel and device.
-template <int WHICH, class K> HcclResult AllowNormRing(K kernel)
-{
-    static std::atomic<bool> done[kMaxDevices];
-    const int dev = CurrentDevice();
-    if (done[dev].load(std::memory_order_relaxed)) return HCCL_SUCCESS;
-    CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kNormPartBytes + kNormSlots * 3 * 2 * kNormMaxHidden)));
-    done[dev].store(true, std::memory_order_relaxed);
-    return HCCL_SUCCESS;
+    static OncePerDevice once;
+    return once([]() -> HcclResult {
+        CHK_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kNormPartBytes + kNormSlots * 3 * 2 * kNormMaxHidden)));
+        return HCCL_SUCCESS;
+    });
 }
 // As many groups (rows in work at a time) per CTA as kNormThreads hold, but no more than it takes to give every SM rows
 // of its own; one CTA per SM.
@@ -551,7 +533,7 @@ HcclResult HcclFusedAddRmsNormFwd(const void* x, const void* delta, const void* 
     const NormShape n = ShapeNorm(rows, hidden);
     const size_t smem = kNormPartBytes + (size_t)n.groups * kNormSlots * hidden * 2 * (delta ? 2 : 1);
     auto kernel = delta ? AddRmsNormFwdKernel<true> : AddRmsNormFwdKernel<false>;
-    CHK_RET(delta ? AllowNormRing<0>(kernel) : AllowNormRing<1>(kernel));
+    CHK_RET(delta ? AllowNormRing<AddRmsNormFwdKernel<true>>() : AllowNormRing<AddRmsNormFwdKernel<false>>());
     kernel<<<n.ctas, n.groups * n.groupThreads, smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w,
                                                                               (__nv_bfloat16*)xOut, (__nv_bfloat16*)h, (float*)rstd, (int)rows,
                                                                               (int)hidden, n.groupThreads, eps);
@@ -575,7 +557,7 @@ HcclResult HcclFusedRmsNormBwd(const void* dh, const void* x, const void* w, con
     const size_t smem = kNormPartBytes + std::max((size_t)n.groups * kNormSlots * hidden * 2 * (dxExtra ? 3 : 2),
                                                   n.groups > 1 ? (size_t)n.groups * hidden * 4 : (size_t)0);
     auto kernel = dxExtra ? RmsNormBwdKernel<true> : RmsNormBwdKernel<false>;
-    CHK_RET(dxExtra ? AllowNormRing<2>(kernel) : AllowNormRing<3>(kernel));
+    CHK_RET(dxExtra ? AllowNormRing<RmsNormBwdKernel<true>>() : AllowNormRing<RmsNormBwdKernel<false>>());
     kernel<<<nPart, n.groups * n.groupThreads, smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)dh, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                                                          (const float*)rstd, (const __nv_bfloat16*)dxExtra, (__nv_bfloat16*)dx,
                                                                          (float*)dwPartial, (int)rows, (int)hidden, n.groupThreads);

@@ -7,6 +7,7 @@
 #include "../core/comm.h"
 #include "../core/cuda_driver.h"
 #include "../core/log.h"
+#include "../core/per_device.h"
 #include "mc2_gemm_2sm_wide.cuh"
 #include "mc2_gemm_splitk.cuh"
 
@@ -59,15 +60,14 @@ HcclResult MapB(CUtensorMap* map, const void* b, uint64_t n, uint64_t k, bool mn
     return mnMajor ? MakeMap(map, b, k, n, kBK, 64) : MakeMap(map, b, n, k, (uint32_t)bn, kBK);
 }
 
-int SmCount()
+// Lets `kernel` take `bytes` of dynamic shared memory.  KERNEL: its type does not tell kernels of one signature apart.
+template <auto KERNEL> HcclResult AllowSharedMemory(int bytes)
 {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return n;
+    static OncePerDevice once;
+    return once([&]() -> HcclResult {
+        CHK_CUDA(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        return HCCL_SUCCESS;
+    });
 }
 
 template <int BN, bool A_MN, bool B_MN, int MODE>
@@ -75,12 +75,8 @@ HcclResult LaunchGemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
                       cudaStream_t stream, const CUtensorMap* taOwn = nullptr)
 {
     const CUtensorMap& ta2 = taOwn != nullptr ? *taOwn : ta;      // AG: this rank's own shard, read where it is
-    auto kernel = GemmKernel<BN, A_MN, B_MN, MODE>;
-    static bool attrSet = false;
-    if (!attrSet) {
-        CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayout<BN>::kTotal));
-        attrSet = true;
-    }
+    constexpr auto kernel = GemmKernel<BN, A_MN, B_MN, MODE>;
+    CHK_RET(AllowSharedMemory<kernel>(SmemLayout<BN>::kTotal));
     if (cooperative) {
         void* args[5] = {(void*)&ta, (void*)&tb, (void*)&ta2, (void*)&g, (void*)&c};
         cudaError_t e = cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)grid), dim3(kThreads), args, SmemLayout<BN>::kTotal, stream);
@@ -98,12 +94,8 @@ HcclResult LaunchGemm2Sm(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
                          cudaStream_t stream, const CUtensorMap* taOwn = nullptr)
 {
     const CUtensorMap& ta2 = taOwn != nullptr ? *taOwn : ta;
-    auto kernel = GemmKernel2Sm<A_MN, B_MN, MODE>;
-    static bool attrSet = false;
-    if (!attrSet) {
-        CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayout2::kTotal));
-        attrSet = true;
-    }
+    constexpr auto kernel = GemmKernel2Sm<A_MN, B_MN, MODE>;
+    CHK_RET(AllowSharedMemory<kernel>(SmemLayout2::kTotal));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);
@@ -123,12 +115,8 @@ HcclResult LaunchGemm2Sm(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
 template <bool A_MN, bool B_MN>
 HcclResult LaunchGemm2SmWide(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int grid, cudaStream_t stream)
 {
-    auto kernel = GemmKernel2SmWide<A_MN, B_MN>;
-    static bool attrSet = false;
-    if (!attrSet) {
-        CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemLayoutWide::kTotal));
-        attrSet = true;
-    }
+    constexpr auto kernel = GemmKernel2SmWide<A_MN, B_MN>;
+    CHK_RET(AllowSharedMemory<kernel>(SmemLayoutWide::kTotal));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);

@@ -34,8 +34,7 @@ HcclResult HcclMoeCombine(HcclComm comm, const void* y, const float* topkWeight,
 
 // Local routing helper (no communicator): offsets[e] .. offsets[e + 1] is the row range of expert e when this
 // rank's nPairs (token, expert) pairs are grouped by expert; offsets has nExperts + 1 entries in device memory.
-// Ids outside [0, nExperts) are ignored.  Keeps a small device scratch buffer per GPU (allocated on first use);
-// calls on one GPU must be ordered (same stream) because they share it.
+// Ids outside [0, nExperts) are ignored.  Needs no scratch memory: calls may run at the same time on several streams.
 HcclResult HcclMoeExpertOffsets(const int32_t* topkIdx, uint64_t nPairs, uint32_t nExperts, uint32_t* offsets, hcclStream_t stream);
 
 #ifdef __cplusplus

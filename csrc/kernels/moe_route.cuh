@@ -1,100 +1,146 @@
 // Expert histogram + exclusive scan for MoE routing: from the [tokens, topk]
 // expert ids of this rank, the row range every expert's tokens occupy when the
 // (token, expert) pairs are grouped by expert (what a grouped GEMM consumes).
-// The kernel needs `nExperts + 1` 32-bit words of scratch that are zero when it
-// starts: per-expert counters and an exit ticket.  Blocks add their pairs to
-// the counters; the last block to finish turns the counters into offsets and
-// leaves the scratch zeroed again for the next call.
 //
-// Latency bound: a table of 64 Ki pairs is 256 KiB.  A block counts its pairs in
-// shared memory and adds only the sums to the counters (up to kRouteSharedExperts
-// experts; beyond that an expert meets few pairs and the counters take them
-// directly), and the last block scans all counters together, kRouteThreads at a
-// time; one thread that walks them pays a round trip to L2 per expert.  Measured
-// against that: 8192 x 8 pairs and 256 experts 40.8 -> 6.3 us, 16 x 8 24.7 -> 4.3
-// us, 32768 x 8 and 512 experts 82.0 -> 7.2 us, 100000 x 2 and 4096 experts 637 ->
-// 14.5 us, 20000 x 2 and 60000 experts 9156 -> 132 us.
+// One cluster of kRouteCtas CTAs does the whole job, with its counters in
+// shared memory: a launch owns everything it writes, so calls on any number of
+// streams, in graphs and from several threads do not meet.
+//
+// Latency bound: a table of 64 Ki pairs is 256 KiB.  Up to kRouteCounters
+// experts every CTA counts its share of the pairs on its own, and CTA r adds
+// up the CTAs' counters of its eighth of the experts through distributed
+// shared memory; with more experts an expert meets few pairs and its counter
+// lives only in the CTA that owns it, where all CTAs add to it.  Each CTA
+// scans its experts, the CTAs' totals give it its first row.  Measured (back to back on
+// one B200, 6.3 us is what an empty table takes), against blocks that share counters in
+// memory and a last block that scans them: 8192 x 8 pairs and 256 experts 6.3 us both,
+// 32768 x 8 and 512 8.3 both, 100000 x 2 and 4096 14.5 -> 8.3, 20000 x 2 and 60000 131 ->
+// 18.6 us.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace hccl {
 
-constexpr int kRouteThreads = 256;
-constexpr uint32_t kRouteSharedExperts = 4096;      // 16 KiB of counters per block
-constexpr int kRoutePairs = 8;                      // ids a thread requests before it counts the first
+constexpr int kRouteCtas = 8;                       // the largest cluster every GPU grants
+constexpr int kRouteThreads = 1024;
+constexpr uint32_t kRouteCounters = 8192;           // 32 KiB per CTA
+constexpr uint32_t kRouteMaxExperts = kRouteCtas * kRouteCounters;
+static_assert(kRouteThreads == 32 * 32, "one warp total per lane");
+constexpr int kRouteVecs = 4;                       // 16-byte loads a thread requests before it counts the first id
 
-static __global__ void __launch_bounds__(kRouteThreads) MoeExpertOffsetsKernel(const int32_t* __restrict__ topkIdx, uint64_t nPairs, uint32_t nExperts,
-                                                                               uint32_t* __restrict__ scratch, uint32_t* __restrict__ offsets)
+namespace route {
+__device__ __forceinline__ uint32_t ClusterRank()
 {
-    uint32_t* counters = scratch;
-    uint32_t* ticket = scratch + nExperts;
-    __shared__ uint32_t s_count[kRouteSharedExperts];
-    __shared__ uint32_t s_warp[kRouteThreads / 32];
-    __shared__ bool s_last;
-    const bool shared = nExperts <= kRouteSharedExperts;
-    if (shared) {
-        for (uint32_t e = threadIdx.x; e < nExperts; e += kRouteThreads) s_count[e] = 0;
-        __syncthreads();
-    }
-    const uint64_t step = (uint64_t)gridDim.x * kRouteThreads;
-    for (uint64_t i = (uint64_t)blockIdx.x * kRouteThreads + threadIdx.x; i < nPairs; i += step * kRoutePairs) {
-        int32_t e[kRoutePairs];
-#pragma unroll
-        for (int k = 0; k < kRoutePairs; ++k) e[k] = i + k * step < nPairs ? topkIdx[i + k * step] : -1;
-#pragma unroll
-        for (int k = 0; k < kRoutePairs; ++k)
-            if (e[k] >= 0 && (uint32_t)e[k] < nExperts) atomicAdd(shared ? &s_count[e[k]] : &counters[e[k]], 1u);
-    }
-    if (shared) {
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < nExperts; e += kRouteThreads)
-            if (s_count[e] != 0) atomicAdd(&counters[e], s_count[e]);
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t run = 0;                               // pairs of all experts before this pass of the loop
-    for (uint32_t base = 0; base < nExperts; base += kRouteThreads) {
-        const uint32_t e = base + threadIdx.x;
-        uint32_t c = 0;
-        if (e < nExperts) {
-            c = *reinterpret_cast<volatile uint32_t*>(&counters[e]);
-            counters[e] = 0;                        // the scratch is zero again when the kernel ends
-        }
-        uint32_t incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += up;
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        uint32_t before = 0, all = 0;
-#pragma unroll
-        for (int q = 0; q < kRouteThreads / 32; ++q) {
-            if (q < warp) before += s_warp[q];
-            all += s_warp[q];
-        }
-        if (e < nExperts) offsets[e] = run + before + incl - c;
-        run += all;
-        __syncthreads();                            // s_warp is read before the next pass writes it
-    }
-    if (threadIdx.x == 0) {
-        offsets[nExperts] = run;
-        *ticket = 0;
-    }
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
 }
-
-// One block per 2048 pairs (every thread's ids in one request), 64 at most.
-inline int MoeExpertOffsetsBlocks(uint64_t nPairs)
+__device__ __forceinline__ void ClusterBarrier()
 {
-    uint64_t b = (nPairs + kRouteThreads * kRoutePairs - 1) / (kRouteThreads * kRoutePairs);
-    return (int)(b < 1 ? 1 : (b > 64 ? 64 : b));
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t PeerAddr(const uint32_t* p, uint32_t rank)      // `p` of CTA `rank`
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t LoadPeer(const uint32_t* p, uint32_t rank)
+{
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(PeerAddr(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void StorePeer(const uint32_t* p, uint32_t rank, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(PeerAddr(p, rank)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void AddPeer(const uint32_t* p, uint32_t rank)
+{
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], 1;" ::"r"(PeerAddr(p, rank)) : "memory");
+}
+}  // namespace route
+
+static __global__ void __cluster_dims__(kRouteCtas, 1, 1) __launch_bounds__(kRouteThreads)
+    MoeExpertOffsetsKernel(const int32_t* __restrict__ topkIdx, uint64_t nPairs, uint32_t nExperts, uint32_t* __restrict__ offsets)
+{
+    __shared__ uint32_t s_count[kRouteCounters];
+    __shared__ uint32_t s_warp[kRouteThreads / 32];
+    __shared__ uint32_t s_before[kRouteCtas];                    // pairs of the experts of each CTA before this one
+    const uint32_t rank = route::ClusterRank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool everyCta = nExperts <= kRouteCounters;            // every CTA counts all experts
+    const uint32_t perCta = (nExperts + kRouteCtas - 1) / kRouteCtas;
+    const uint32_t nCounters = everyCta ? nExperts : perCta;
+    for (uint32_t e = tid; e < nCounters; e += kRouteThreads) s_count[e] = 0;
+    __syncthreads();
+    if (!everyCta) route::ClusterBarrier();
+    auto count = [&](int32_t id) {
+        const uint32_t e = (uint32_t)id;
+        if (id < 0 || e >= nExperts) return;
+        if (everyCta) atomicAdd(&s_count[e], 1u);
+        else route::AddPeer(&s_count[e % perCta], e / perCta);
+    };
+    const uint64_t me = (uint64_t)rank * kRouteThreads + tid, step = (uint64_t)kRouteCtas * kRouteThreads;
+    const uint64_t nVecs = (reinterpret_cast<uintptr_t>(topkIdx) & 15u) == 0 ? nPairs / 4 : 0;
+    const int4* vecs = reinterpret_cast<const int4*>(topkIdx);
+    for (uint64_t i = me; i < nVecs; i += step * kRouteVecs) {
+        int4 v[kRouteVecs];
+#pragma unroll
+        for (int k = 0; k < kRouteVecs; ++k) v[k] = i + k * step < nVecs ? vecs[i + k * step] : make_int4(-1, -1, -1, -1);
+#pragma unroll
+        for (int k = 0; k < kRouteVecs; ++k) { count(v[k].x); count(v[k].y); count(v[k].z); count(v[k].w); }
+    }
+    // the ids after the last whole vector, or all of them where the table does not start on 16 bytes
+    for (uint64_t i = nVecs * 4 + me; i < nPairs; i += step * kRouteVecs) {
+        int32_t v[kRouteVecs];
+#pragma unroll
+        for (int k = 0; k < kRouteVecs; ++k) v[k] = i + k * step < nPairs ? topkIdx[i + k * step] : -1;
+#pragma unroll
+        for (int k = 0; k < kRouteVecs; ++k) count(v[k]);
+    }
+    route::ClusterBarrier();                                     // every pair is counted
+    // this CTA's experts [first, last), `mine` consecutive ones per thread
+    const uint32_t first = rank * perCta < nExperts ? rank * perCta : nExperts;
+    const uint32_t last = first + perCta < nExperts ? first + perCta : nExperts;
+    const uint32_t mine = (perCta + kRouteThreads - 1) / kRouteThreads;
+    constexpr uint32_t kMost = kRouteCounters / kRouteThreads;
+    uint32_t c[kMost], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kMost; ++j) {
+        const uint32_t e = first + tid * mine + j;
+        c[j] = 0;
+        if (j < mine && e < last) {
+            if (everyCta) {
+#pragma unroll
+                for (uint32_t r = 0; r < kRouteCtas; ++r) c[j] += route::LoadPeer(&s_count[e], r);
+            } else {
+                c[j] = s_count[e - first];
+            }
+        }
+        sum += c[j];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += up;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    const uint32_t ofWarp = s_warp[lane];                        // as many warps as lanes
+    uint32_t run = incl - sum + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? ofWarp : 0u);      // before this thread's, in this CTA
+    const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, ofWarp);
+    if (tid > rank && tid < kRouteCtas) route::StorePeer(&s_before[rank], tid, all);
+    route::ClusterBarrier();                                     // the totals are there; nobody reads a peer after this
+    for (uint32_t r = 0; r < rank; ++r) run += s_before[r];
+#pragma unroll
+    for (uint32_t j = 0; j < kMost; ++j) {
+        const uint32_t e = first + tid * mine + j;
+        if (j < mine && e < last) offsets[e] = run;
+        run += c[j];
+    }
+    if (rank == kRouteCtas - 1 && tid == kRouteThreads - 1) offsets[nExperts] = run;
 }
 
 }  // namespace hccl

@@ -130,6 +130,45 @@ def test_expert_offsets_ranges(pairs, experts):
         assert torch.equal(expert_offsets(idx, experts).long(), ref)
 
 
+def _offsets_of(idx, experts):
+    ok = idx[(idx >= 0) & (idx < experts)].long()
+    return torch.cat((ok.new_zeros(1), torch.bincount(ok, minlength=experts).cumsum(0)))
+
+
+@pytest.mark.parametrize("start", [0, 1, 3])
+@pytest.mark.parametrize("pairs,experts", [(3, 5), (130, 8192), (70001, 8193), (131073, 100)])
+def test_expert_offsets_of_a_table_that_starts_anywhere(pairs, experts, start):
+    g = torch.Generator(device="cuda").manual_seed(pairs)
+    idx = torch.randint(-1, experts + 1, (pairs + start,), device="cuda", generator=g, dtype=torch.int32)[start:]
+    assert torch.equal(expert_offsets(idx, experts).long(), _offsets_of(idx, experts))
+
+
+def test_expert_offsets_on_two_streams_and_in_a_graph():
+    """Calls that run at the same time, with different numbers of experts, on two streams and from a replayed graph."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    tables = [(torch.randint(0, e, (n,), device="cuda", generator=g, dtype=torch.int32), e) for n, e in ((60000, 256), (50000, 57), (40000, 9000))]
+    want = [_offsets_of(i, e) for i, e in tables]
+    streams = [torch.cuda.Stream() for _ in tables]
+    graph, keep = torch.cuda.CUDAGraph(), []
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=streams[2]):
+        for _ in range(20):
+            keep.append(expert_offsets(*tables[2]))
+    got = [[], []]
+    for s in streams:
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(20_000_000)                      # all three start together
+    with torch.cuda.stream(streams[2]):
+        graph.replay()
+    for _ in range(40):
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(expert_offsets(*tables[i]))
+    torch.cuda.synchronize()
+    for outs, ref in ((got[0], want[0]), (got[1], want[1]), (keep, want[2])):
+        assert all(torch.equal(o.long(), ref) for o in outs)
+
+
 # rows of one 128-element block and of a part of a warp's stretch, one token and more tokens than warps, dropped pairs,
 # the counting kernel of one block and of many
 @pytest.mark.parametrize("p,tokens,hidden,experts,topk", [(2, 3, 128, 2, 1), (2, 70, 1152, 16, 3), (4, 40, 8192, 64, 8), (2, 5000, 256, 8, 4)])

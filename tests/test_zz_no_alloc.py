@@ -2,9 +2,8 @@
 
 Who needs it: callers that must not allocate device memory when they ask for routing offsets (every byte already
 belongs to a framework's caching allocator, a serving process forbids cudaMalloc after start-up, or the hidden device
-synchronisation of cudaMalloc is unacceptable on the path).  The variant keeps its counters in an array inside the
-library image, so its results must equal those of HcclMoeExpertOffsets, call after call, although all calls share
-that array.  This file sorts last so that a run stopping at the first failure has already run every other test.
+synchronisation of cudaMalloc is unacceptable on the path).  Its results must equal those of HcclMoeExpertOffsets, call
+after call.  This file sorts last so that a run stopping at the first failure has already run every other test.
 """
 import ctypes
 from pathlib import Path
@@ -35,7 +34,6 @@ def _call(fn, idx, n_experts, out):
 def test_no_alloc_matches_allocating_entry_point_on_consecutive_calls():
     torch.cuda.set_device(0)
     reference, no_alloc = _symbols()
-    # first call on the device (does the one-time address lookup), outside any stream capture
     for call, (tokens, topk, experts) in enumerate([(8192, 8, 256), (8192, 8, 256), (333, 3, 4096), (50000, 4, 17)]):
         g = torch.Generator(device="cuda").manual_seed(100 + call)
         idx = torch.randint(-2, experts, (tokens, topk), device="cuda", generator=g, dtype=torch.int32)

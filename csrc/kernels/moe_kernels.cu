@@ -55,11 +55,12 @@ __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, 
 }
 
 // ------------------------------------------------------------------ dispatch
-// Bound by the bytes written (topk fp8 copies of every row, over NVLink to the peers).  A WARP owns a token: a lane
-// takes 16 elements of the row (two 16-byte loads), eight lanes share a 128-element block's maximum, and the lane
-// quantises its 16 elements in registers and stores them to all topk destinations, 512 contiguous bytes per warp and
-// destination.  No block-wide step inside a token, so all warps' loads and stores overlap.  Measured against a block
-// per token with three barriers, 8 emulated ranks, 256 tokens x 7168, top-8: 130 -> 50 us (150 MB).
+// Bound by the bytes written (topk fp8 copies of every row, over NVLink to the peers).  A WARP owns a token, or a part of
+// one while there are warps for it: a lane takes 16 elements of the row (two 16-byte loads), eight lanes share a
+// 128-element block's maximum, and the lane quantises its 16 elements in registers and stores them to all topk
+// destinations, 512 contiguous bytes per warp and destination.  No block-wide step inside a token, so all warps' loads and
+// stores overlap.  Measured against a block per token with three barriers, 8 emulated ranks, rows of 7168, top-8: 256 tokens
+// (150 MB) 133 -> 52 us, 64 82 -> 33, 8 72 -> 28, 1 28 -> 17 (with whole tokens only 49, 41, 36 and 34 us).
 struct DispatchBody {
     using Args = MoeDispatchArgs;
     static constexpr int kThreads = kMoeThreads;
@@ -121,19 +122,24 @@ struct DispatchBody {
         // phase 2: token rows.  16 elements per lane: nPiece is a multiple of 8 (hidden is one of 128).
         const int H = a.hidden, nScale = H / 128, nPiece = H / 16;
         constexpr int U = 2;                                        // pieces a lane requests before it quantises the first
-        for (int t = b + warp * nb; t < a.nTokens && ok; t += nb * kMoeWarps) {
+        const int nStretch = (nPiece + 32 * U - 1) / (32 * U);
+        const int parts = min(max(nb * kMoeWarps / max(a.nTokens, 1), 1), nStretch), perPart = (nStretch + parts - 1) / parts;
+        const uint32_t items = (uint32_t)a.nTokens * parts;         // at most eight parts of rows that fit the GPU: far below 2^32
+        for (uint32_t it = b + warp * nb; it < items && ok; it += nb * kMoeWarps) {
+            const int t = (int)(it / (uint32_t)parts), part = (int)it - t * parts;
             // lane k < topk: where the row's k-th copy goes
             uint64_t sm = ~0ull;
             if (lane < a.topk) {
                 const int pair = t * a.topk + lane;
                 const int e = a.topkIdx[pair];
                 if (e >= 0 && e < E) sm = ((uint64_t)(e / perRank) << 32) | (uint64_t)(s_base[e] + a.pos[pair]);
-                a.slotMap[pair] = sm;
+                if (part == 0) a.slotMap[pair] = sm;
                 if (sm != ~0ull && (uint32_t)sm >= a.capacity) sm = ~0ull;      // overflow: reported by the receiver's bounds check above
-                if (sm != ~0ull) a.recvSrc[sm >> 32][(uint32_t)sm] = ((uint64_t)me << 32) | (uint32_t)pair;
+                if (sm != ~0ull && part == 0) a.recvSrc[sm >> 32][(uint32_t)sm] = ((uint64_t)me << 32) | (uint32_t)pair;
             }
             const uint4* row = reinterpret_cast<const uint4*>(a.x + (size_t)t * H);
-            for (int w0 = 0; w0 < nPiece; w0 += 32 * U) {
+            const int end = min((part + 1) * perPart * 32 * U, nPiece);
+            for (int w0 = part * perPart * 32 * U; w0 < end; w0 += 32 * U) {
                 uint4 raw[U][2];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {

@@ -170,8 +170,9 @@ def test_expert_offsets_on_two_streams_and_in_a_graph():
 
 
 # rows of one 128-element block and of a part of a warp's stretch, one token and more tokens than warps, dropped pairs,
-# the counting kernel of one block and of many
-@pytest.mark.parametrize("p,tokens,hidden,experts,topk", [(2, 3, 128, 2, 1), (2, 70, 1152, 16, 3), (4, 40, 8192, 64, 8), (2, 5000, 256, 8, 4)])
+# the counting kernel of one block and of many; rows shared by several warps where tokens are few, every group of topk
+@pytest.mark.parametrize("p,tokens,hidden,experts,topk", [(2, 3, 128, 2, 1), (2, 70, 1152, 16, 3), (4, 40, 8192, 64, 8), (2, 5000, 256, 8, 4),
+                                                           (2, 1, 7168, 8, 8), (8, 8, 2048, 16, 2), (2, 9, 7168, 16, 5), (4, 2, 1408, 8, 1)])
 def test_moe_dispatch_and_combine_edges(p, tokens, hidden, experts, topk):
     import hccl_b200 as hb
     from hccl_b200 import Communicator

@@ -193,27 +193,26 @@ struct DispatchBody {
 };
 
 // ------------------------------------------------------------------ combine
-// A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: 32 * kCombinePieces 16-byte pieces of one
-// token's row (a part of a row, so that a few hundred tokens still give every warp of the chip something to load); a
-// lane requests topk loads per piece, two pieces at a time, before it uses the first.  Lane k keeps the k-th copy's
-// address and weight and hands them round by shuffle.  Measured against a block per token: 89 -> 90 us (264 MB, the expert
-// rows still being written back: level), 8 emulated ranks, 256 tokens x 7168, top-8.
+// A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: up to kCombinePieces pieces (32 vectors of 16
+// bytes) of one token's row, fewer while that gives idle warps something to load.  A lane requests up to COPIES loads per
+// piece, UNROLL pieces at a time, before it uses the first: eight loads for every topk, which fit the 128 registers of a
+// thread (sixteen did not, and spilled).  Lane k keeps the k-th copy's address and weight and hands them round by shuffle.
+// Measured against a block per token, 8 emulated ranks, rows of 7168, top-8: 256 tokens (264 MB, the expert rows still being
+// written back) 91 -> 82 us, 64 55 -> 47, 8 45 -> 39, 1 15.6 -> 15.0; rows of 4096, top-2: 256 47 -> 26, 1 12.7 -> 13.0.
 constexpr int kCombinePieces = 4;
 struct CombineBody {
     using Args = MoeCombineArgs;
     static constexpr int kThreads = kMoeThreads;
-    __device__ static void Run(const DevComm& c, const Args& a, int b, int nb)
+    template <int COPIES, int UNROLL>
+    __device__ static void Tokens(const Args& a, int b, int nb)
     {
-        OpHead(c, b);
-        const uint64_t e0 = LoadEpoch(c, b);
-        bool ok = RankBarrier(c, b, 0, e0 + 1, K_MOE_COMBINE);      // the peers' expert outputs are final
-        const int H = a.hidden, vecPerRow = H / 8;
+        const int H = a.hidden, vecPerRow = H / 8, nPieces = (vecPerRow + 31) / 32;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int parts = (vecPerRow + 32 * kCombinePieces - 1) / (32 * kCombinePieces);
-        const long long items = (long long)a.nTokens * parts;
-        constexpr int U = 2;
-        for (long long it = b + (long long)warp * nb; it < items && ok; it += (long long)nb * kMoeWarps) {
-            const int t = (int)(it / parts), v00 = (int)(it % parts) * 32 * kCombinePieces;
+        const uint32_t stride = (uint32_t)nb * kMoeWarps, all = (uint32_t)a.nTokens * nPieces;      // rows fit the GPU: far below 2^32
+        const int perItem = (int)min((all + stride - 1) / stride, (uint32_t)kCombinePieces);
+        const uint32_t parts = perItem > 0 ? (nPieces + perItem - 1) / perItem : 0, items = (uint32_t)a.nTokens * parts;
+        for (uint32_t it = b + warp * nb; it < items; it += stride) {
+            const int t = (int)(it / parts), first = (int)(it - t * parts) * perItem;
             float wk = 0.f;
             unsigned long long srcK = 0;                            // 0: the copy was dropped
             if (lane < a.topk) {
@@ -223,26 +222,25 @@ struct CombineBody {
                     srcK = reinterpret_cast<unsigned long long>(a.y[sm >> 32] + (size_t)(uint32_t)sm * H);
                 }
             }
+            const int end = min((first + perItem) * 32, vecPerRow);
+            for (int v0 = first * 32 + lane; v0 - lane < end; v0 += 32 * UNROLL) {
+                uint4 raw[UNROLL][COPIES];
 #pragma unroll
-            for (int i = 0; i < kCombinePieces; i += U) {
-                const int v0 = v00 + i * 32 + lane;
-                uint4 raw[U][kMoeMaxTopk];
-#pragma unroll
-                for (int k = 0; k < kMoeMaxTopk; ++k) {
+                for (int k = 0; k < COPIES; ++k) {
                     const uint4* src = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, srcK, k));
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
+                    for (int u = 0; u < UNROLL; ++u) {
                         raw[u][k] = make_uint4(0, 0, 0, 0);
-                        if (src != nullptr && v0 + u * 32 < vecPerRow) raw[u][k] = src[v0 + u * 32];
+                        if (src != nullptr && v0 + u * 32 < end) raw[u][k] = src[v0 + u * 32];
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
+                for (int u = 0; u < UNROLL; ++u) {
                     float acc[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
 #pragma unroll
-                    for (int k = 0; k < kMoeMaxTopk; ++k) {
+                    for (int k = 0; k < COPIES; ++k) {
                         const float w = __shfl_sync(0xffffffffu, wk, k);
                         if (k < a.topk) {
                             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[u][k]);
@@ -254,7 +252,7 @@ struct CombineBody {
                             }
                         }
                     }
-                    if (v0 + u * 32 < vecPerRow) {
+                    if (v0 + u * 32 < end) {
                         uint4 o;
                         __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
@@ -264,11 +262,22 @@ struct CombineBody {
                 }
             }
         }
+    }
+    __device__ static void Run(const DevComm& c, const Args& a, int b, int nb)
+    {
+        OpHead(c, b);
+        const uint64_t e0 = LoadEpoch(c, b);
+        if (RankBarrier(c, b, 0, e0 + 1, K_MOE_COMBINE)) {          // the peers' expert outputs are final
+            if (a.topk > 4) Tokens<8, 1>(a, b, nb);
+            else if (a.topk > 2) Tokens<4, 2>(a, b, nb);
+            else Tokens<2, 4>(a, b, nb);
+        }
         RankBarrier(c, b, 0, e0 + 2, K_MOE_COMBINE);                 // nobody overwrites its outputs while a peer still reads
         StoreEpoch(c, b, e0 + 2);
         OpTail(c, b);
     }
 };
+static_assert(kMoeMaxTopk == 8, "CombineBody picks its copies by topk");
 
 template <class Body>
 HcclResult LaunchMoe(const LaunchTarget& t, const typename Body::Args& a, int nBlocks)

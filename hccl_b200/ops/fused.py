@@ -165,6 +165,7 @@ class _RopeQkv(torch.autograd.Function):
             out.append(o)
         _count(2)
         ctx.save_for_backward(cos, sin)
+        ctx.set_materialize_grads(False)        # an output that nothing used has no gradient: its part is filled, not rotated
         ctx.heads = (hq, hkv, d)
         return out[0], out[1], qkv[:, (hq + hkv) * d:].view(s, hkv, d)
 
@@ -174,7 +175,9 @@ class _RopeQkv(torch.autograd.Function):
         hq, hkv, d = ctx.heads
         s = cos.shape[0]
         width = (hq + 2 * hkv) * d
-        like = next(g for g in (dq, dk, dv) if g is not None)
+        like = next((g for g in (dq, dk, dv) if g is not None), None)
+        if like is None:
+            return None, None, None, None, None
         dqkv = torch.empty((s, width), device=like.device, dtype=like.dtype)
         for first, heads, g in ((0, hq, dq), (hq, hkv, dk)):
             part = dqkv[:, first * d:(first + heads) * d]

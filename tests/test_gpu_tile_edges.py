@@ -293,6 +293,8 @@ def test_rope_qkv_matches_the_sliced_form(s, hq, hkv, d):
                 b[:, (hq + hkv) * d:].view(s, hkv, d))
         for x, y in zip(got, want):
             assert torch.equal(x, y)
+        before = fused.LAUNCHES
         torch.autograd.backward([got[i] for i in used], [ups[i] for i in used])
+        assert fused.LAUNCHES - before == len({0, 1} & set(used))           # a rotation for q and k only where one has a gradient
         torch.autograd.backward([want[i] for i in used], [ups[i] for i in used])
         assert torch.equal(a.grad, b.grad)

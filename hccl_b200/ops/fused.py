@@ -210,10 +210,15 @@ def swiglu(gate_up, use_kernels: bool = True):
     return swiglu_reference(gate_up)
 
 
+def _rope_table(t, x) -> bool:
+    """A table the kernel can read for every row of x; others (a row that broadcasts, one on the host) go to PyTorch."""
+    return t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() >= x.shape[0] * (x.shape[-1] // 2)
+
+
 def rope(x, cos, sin, use_kernels: bool = True):
     """x [S, heads, D] (row stride may exceed heads * D), cos / sin fp32 [S, D / 2]."""
     if (use_kernels and _native(x) and x.shape[-1] % 16 == 0 and x.stride(2) == 1 and x.stride(1) == x.shape[-1] and x.stride(0) % 8 == 0
-            and x.data_ptr() % 16 == 0 and cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()):
+            and x.data_ptr() % 16 == 0 and _rope_table(cos, x) and _rope_table(sin, x)):
         return _Rope.apply(x, cos, sin)
     return rope_reference(x, cos, sin)
 
@@ -222,7 +227,7 @@ def rope_qkv(qkv, cos, sin, hq: int, hkv: int, use_kernels: bool = True):
     """Splits ``qkv [S, (hq + 2 hkv) * D]`` into heads and rotates q and k: ``([S, hq, D], [S, hkv, D], [S, hkv, D])``."""
     s, d = qkv.shape[0], qkv.shape[1] // (hq + 2 * hkv)
     if (use_kernels and _native(qkv) and d % 16 == 0 and hkv > 0 and s > 0 and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
-            and cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.shape == sin.shape == (s, d // 2)
+            and cos.is_cuda and sin.is_cuda and cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.shape == sin.shape == (s, d // 2)
             and cos.is_contiguous() and sin.is_contiguous()):
         return _RopeQkv.apply(qkv, cos, sin, hq, hkv)
     q = rope(qkv[:, :hq * d].view(s, hq, d), cos, sin, use_kernels=use_kernels)

@@ -108,3 +108,34 @@ def test_hccl_test_command_line_on_the_host_engine():
         rows = [l.split() for l in r.stdout.splitlines() if l.strip() and not l.startswith("#") and not l.strip().startswith("data_size")]
         assert [int(x[0]) for x in rows] == [1024, 4096, 16384], r.stdout
         assert all(x[3] == "success" for x in rows), r.stdout
+
+
+class _OnGpu(torch.Tensor):
+    """A host tensor that says it lies on a GPU: what the routing of an operator looks at, without a GPU."""
+    is_cuda = True
+
+
+def test_rope_reads_only_tables_that_hold_every_row(monkeypatch):
+    """The rotary kernel reads S rows of D / 2 fp32 cosines and sines: tables on the host, too short ones (a row that
+    broadcasts) and others take the PyTorch expression."""
+    native = []
+    monkeypatch.setattr(fused, "_native", lambda *t, **k: True)
+    monkeypatch.setattr(fused._Rope, "apply", lambda *a: native.append("rope") or a[0])
+    monkeypatch.setattr(fused._RopeQkv, "apply", lambda *a: native.append("qkv") or (a[0],) * 3)
+    s, heads, d = 6, 4, 32
+    x = torch.randn(s, heads, d).bfloat16()
+    qkv = torch.randn(s, (heads + 2) * d).bfloat16()
+    ang = torch.rand(s, d // 2)
+    gpu = lambda t: t.as_subclass(_OnGpu)  # noqa: E731
+    cos, sin = gpu(ang.cos()), gpu(ang.sin())
+    fused.rope(x, cos, sin)
+    fused.rope_qkv(qkv, cos, sin, heads, 1)
+    assert native == ["rope", "qkv"]
+    native.clear()
+    row = gpu(ang.cos()[:1].contiguous())
+    for c, n in ((ang.cos(), sin), (cos, ang.sin()), (row, row), (cos, gpu(ang.sin().double()))):
+        torch.testing.assert_close(fused.rope(x, c, n), fused.rope_reference(x, c, n))
+        fused.rope_qkv(qkv, c, n, heads, 1)
+    assert not native
+    fused.rope(x[:4], cos, sin)                          # a longer table is read from its start
+    assert native == ["rope"]

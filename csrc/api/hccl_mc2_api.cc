@@ -150,6 +150,16 @@ HcclResult HcclMc2Matmul(const void* a, const void* b, void* out, uint64_t m, ui
 {
     return Mc2Matmul(a, b, out, m, n, k, transA, transB, (cudaStream_t)stream);
 }
+// Tests: how a plain matmul would run on a GPU of `sms` SMs under the switches of the process environment.
+HcclResult HcclDebugMatmulPlan(uint64_t m, uint64_t n, uint64_t k, int transA, int transB, uint32_t sms, char* text, uint32_t cap)
+{
+    CHK_PTR_NULL(text);
+    const MatmulPlan p = PlanMatmul(m, n, k, transA != 0, transB == 0, (int)sms, MatmulSwitchesOfEnv());
+    static const char* const names[] = {"split", "one_sm", "two_sm", "wide"};
+    snprintf(text, cap, "route=%s bn=%d tiles=%dx%d grid=%d bt=%d split=%d wide=%d singles=%d hints=%d%d raster=%d", names[(int)p.route], p.bn, p.tilesM,
+             p.tilesN, p.grid, p.bt, p.split, p.wide, p.singles, p.l2HintA, p.l2HintB, p.rasterGroup);
+    return HCCL_SUCCESS;
+}
 // Tests: the matmul with a CTA whose operands never arrive.  `out` must stay as it is where that CTA's tile lies, and the next
 // matmul on the device must return HCCL_E_TIMEOUT.
 HcclResult HcclDebugMatmulStalled(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, int cta,

@@ -151,20 +151,6 @@ HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const S
     return HCCL_SUCCESS;
 }
 
-// Wide tiles (two column tiles per CTA pair, see mc2_gemm_2sm_wide.cuh): where at least two full rounds of them run, so
-// that most of the output gains from the saved L2 traffic, and the inner dimension has 48 k-blocks or more, so that the
-// dozen whose A is loaded twice per tile stay a small part.  HCCL_MC2_WIDE=0 turns them off, 1 takes them wherever one
-// full round runs.
-int WideMode()
-{
-    static int v = -2;
-    if (v == -2) {
-        const char* e = getenv("HCCL_MC2_WIDE");
-        v = e == nullptr || e[0] == 'a' ? -1 : (e[0] == '1' ? 1 : 0);
-    }
-    return v;
-}
-
 template <int MODE>
 HcclResult DispatchLayout2Sm(bool aMn, bool bMn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, const DevComm& c, int grid,
                              bool coop, cudaStream_t s, const CUtensorMap* taOwn = nullptr)
@@ -406,6 +392,93 @@ HcclResult Mc2EnsureState(CommImpl* comm, uint64_t parityBytes)
     return HCCL_SUCCESS;
 }
 
+MatmulSwitches MatmulSwitchesOfEnv()
+{
+    static const MatmulSwitches s = [] {
+        MatmulSwitches v;
+        const char* hints = getenv("HCCL_MC2_L2_HINTS");
+        const char* wide = getenv("HCCL_MC2_WIDE");
+        v.twoSm = Use2Sm();
+        v.l2Hints = hints != nullptr && hints[0] == '1';
+        // the wide kernel takes no hints: asking for them keeps the narrow tiles unless wide ones are asked for as well
+        v.wide = wide == nullptr ? (v.l2Hints ? 0 : -1) : (wide[0] == 'a' ? -1 : (wide[0] == '1' ? 1 : 0));
+        return v;
+    }();
+    return s;
+}
+
+MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw)
+{
+    MatmulPlan p;
+    const int tilesM = (int)((m + kBM - 1) / kBM), tilesM2 = (int)((m + 255) / 256);
+    const int pairs = (sms & ~1) / 2;
+    // narrow: 256-wide column tiles would leave most SMs idle
+    const bool narrow = (uint64_t)tilesM * ((n + 255) / 256) < (uint64_t)sms * 3 / 4;
+    // Two-SM tiles: outputs that fill the chip with 256 x 256 tiles, and from 129 rows on those that fill four fifths of the
+    // pairs with 256 x 128 ones if the inner dimension is long (us, before on the one-SM kernel -> two-SM: 200 x 10240 x
+    // 8192 84.5 -> 45.0, 200 x 57344 x 8192 331.0 -> 199.8, 300 x 8192 x 8192 88.1 -> 49.0, 256 x 8192 x 8192 49.2 -> 40.9,
+    // 512 x 4096 x 4096 26.6 -> 23.1, 1000 x 2048 x 2048 16.5 -> 16.1; with fewer tiles the split kernel is ahead: 300 x
+    // 2048 x 4096 22.4 against 16.5).
+    const bool twoSm = sw.twoSm && ((!narrow && m >= 256) || (m > 128 && k >= 2048 && (uint64_t)tilesM2 * ((n + 127) / 128) * 5 >= (uint64_t)pairs * 4));
+    // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
+    // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
+    // long (400 x 1024 x 1024: 10.3 us against 9.2 on the one-SM kernel, 300 x 2048 x 4096: 16.5 against 24.7).
+    if (!twoSm && (m <= 96 || (narrow && (m <= 128 || k >= 4096)))) {
+        p.route = MatmulRoute::SPLIT;
+        // token tile: all of them up to 128, else equal tiles of at most 128 (MN-major activations come in 64-column boxes)
+        const int unit = aMn ? 64 : 16, parts = (int)((m + kSplitMaxBt - 1) / kSplitMaxBt);
+        p.bt = ((int)((m + parts - 1) / parts) + unit - 1) / unit * unit;
+        p.bn = 128;
+        p.tilesM = (int)((m + p.bt - 1) / p.bt);
+        p.tilesN = (int)((n + 127) / 128);
+        // two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile)
+        const int tiles = p.tilesM * p.tilesN, kBlocks = (int)((k + kBK - 1) / kBK);
+        p.split = std::max(1, std::min({kSplitMaxCluster, 2 * sms / tiles, kBlocks / 4}));
+        p.grid = tiles * p.split;
+        return p;
+    }
+    if (!twoSm) {
+        p.route = MatmulRoute::ONE_SM;
+        p.bn = narrow ? 128 : 256;
+        p.tilesM = tilesM;
+        p.tilesN = (int)((n + p.bn - 1) / p.bn);
+        p.grid = std::min(sms, p.tilesM * p.tilesN);
+        return p;
+    }
+    p.bn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
+    p.tilesN = (int)((n + p.bn - 1) / p.bn);
+    // Wide tiles (two column tiles per CTA pair, see mc2_gemm_2sm_wide.cuh): where at least two full rounds of them run, so
+    // that most of the output gains from the saved L2 traffic, and the inner dimension has 48 k-blocks or more, so that the
+    // dozen whose A is loaded twice per tile stay a small part.
+    const WideOrder order(tilesM2, p.tilesN, pairs, 8);
+    if (sw.wide == 1 ? order.wide > 0 : (sw.wide == -1 && order.wide >= 2 * pairs && k >= 48 * kBK)) {
+        p.route = MatmulRoute::WIDE;
+        p.grid = 2 * pairs;
+        p.wide = order.wide;
+        p.singles = order.items - order.wide;
+        return p;
+    }
+    p.route = MatmulRoute::TWO_SM;
+    p.grid = std::min(2 * pairs, 2 * tilesM2 * p.tilesN);
+    // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
+    // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next
+    // to the stream of the other, it is loaded "evict last", the streamed one "evict first", and the band covers
+    // the whole small operand.  Measured on the decoder's matmuls it did not pay (evict-first lines of the
+    // streamed operand leave before the other row tiles of the wave have read them), so it is off by default.
+    if (sw.l2Hints) {
+        const double bytesA = 2.0 * (double)m * (double)k, bytesB = 2.0 * (double)n * (double)k;
+        const double fits = 72.0 * (1 << 20);
+        if (bytesA <= fits && bytesB > 1.5 * bytesA) {
+            p.l2HintA = 1; p.l2HintB = 2;
+            p.rasterGroup = std::min(tilesM2, 32);            // all rows of A in one band: B is read once
+        } else if (bytesB <= fits && bytesA > 1.5 * bytesB) {
+            p.l2HintA = 2; p.l2HintB = 1;
+            p.rasterGroup = std::max(1, std::min(8, pairs / std::max(1, p.tilesN)));   // all columns of B in flight together
+        }
+    }
+    return p;
+}
+
 HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, cudaStream_t stream,
                      const Mc2StalledCta* stalled)
 {
@@ -416,46 +489,32 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     PlainCtl plain;
     CHK_RET(GetPlainCtl(&plain));
     if (*plain.gaveUp != 0) return ReportGaveUp(plain, stream);
-    const int tilesM = (int)((m + kBM - 1) / kBM), tilesM2 = (int)((m + 255) / 256);
-    const int pairs = (SmCount() & ~1) / 2;
-    // narrow: 256-wide column tiles would leave most SMs idle
-    const bool narrow = (uint64_t)tilesM * ((n + 255) / 256) < (uint64_t)SmCount() * 3 / 4;
-    // Two-SM tiles: outputs that fill the chip with 256 x 256 tiles, and from 129 rows on those that fill four fifths of the
-    // pairs with 256 x 128 ones if the inner dimension is long (us, before on the one-SM kernel -> two-SM: 200 x 10240 x
-    // 8192 84.5 -> 45.0, 200 x 57344 x 8192 331.0 -> 199.8, 300 x 8192 x 8192 88.1 -> 49.0, 256 x 8192 x 8192 49.2 -> 40.9,
-    // 512 x 4096 x 4096 26.6 -> 23.1, 1000 x 2048 x 2048 16.5 -> 16.1; with fewer tiles the split kernel is ahead: 300 x
-    // 2048 x 4096 22.4 against 16.5).
-    const bool twoSm = Use2Sm() && ((!narrow && m >= 256) || (m > 128 && k >= 2048 && (uint64_t)tilesM2 * ((n + 127) / 128) * 5 >= (uint64_t)pairs * 4));
-    // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
-    // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
-    // long (400 x 1024 x 1024: 10.3 us against 9.2 on the one-SM kernel, 300 x 2048 x 4096: 16.5 against 24.7).
-    if (!twoSm && (m <= 96 || (narrow && (m <= 128 || k >= 4096)))) {
+    const MatmulPlan plan = PlanMatmul(m, n, k, aMn, bMn, SmCount(), MatmulSwitchesOfEnv());
+    if (plan.route == MatmulRoute::SPLIT) {
         SplitArgs g;
         memset(&g, 0, sizeof(g));
         g.M = (int)m; g.N = (int)n; g.K = (int)k;
         g.out = (__nv_bfloat16*)out;
-        // token tile: all of them up to 128, else equal tiles of at most 128 (MN-major activations come in 64-column boxes)
-        const int unit = aMn ? 64 : 16, parts = (int)((m + kSplitMaxBt - 1) / kSplitMaxBt);
-        g.bt = ((int)((m + parts - 1) / parts) + unit - 1) / unit * unit;
-        g.tilesM = (int)((m + g.bt - 1) / g.bt);
+        g.bt = plan.bt;
+        g.tilesM = plan.tilesM;
         g.stages = SplitStages(g.bt);
         g.ctl = plain.ctl;
         g.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
         g.stalledCta = stalled != nullptr ? stalled->cta : -1;
-        // two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile)
-        const int tiles = g.tilesM * (int)((n + 127) / 128), kBlocks = (int)((k + kBK - 1) / kBK);
-        const int split = std::max(1, std::min({kSplitMaxCluster, 2 * SmCount() / tiles, kBlocks / 4}));
+        const int tiles = plan.tilesM * plan.tilesN;
         CUtensorMap tw, tx;
         CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, 128, kBK));
         CHK_RET(aMn ? MakeMap(&tx, a, k, m, kBK, 64) : MakeMap(&tx, a, m, k, (uint32_t)g.bt, kBK));
-        if (!bMn && !aMn) return LaunchGemmSplit<false, false>(tw, tx, g, tiles, split, stream);
-        if (!bMn && aMn) return LaunchGemmSplit<false, true>(tw, tx, g, tiles, split, stream);
-        if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, split, stream);
-        return LaunchGemmSplit<true, true>(tw, tx, g, tiles, split, stream);
+        if (!bMn && !aMn) return LaunchGemmSplit<false, false>(tw, tx, g, tiles, plan.split, stream);
+        if (!bMn && aMn) return LaunchGemmSplit<false, true>(tw, tx, g, tiles, plan.split, stream);
+        if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, plan.split, stream);
+        return LaunchGemmSplit<true, true>(tw, tx, g, tiles, plan.split, stream);
     }
     if (stalled != nullptr) return HCCL_E_NOT_SUPPORT;
     CUtensorMap ta, tb;
     CHK_RET(MapA(&ta, a, m, k, aMn));
+    // two-SM tiles: B is split between the two CTAs of a pair, each loads half of the B rows of a tile
+    CHK_RET(MapB(&tb, b, n, k, bMn, plan.route == MatmulRoute::ONE_SM ? plan.bn : plan.bn / 2));
     GemmArgs g;
     memset(&g, 0, sizeof(g));
     g.M = (int)m; g.N = (int)n; g.K = (int)k;
@@ -463,52 +522,24 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     g.ldc = (int)n;
     g.ctl = plain.ctl;
     g.nRanks = 1;
+    g.bn = plan.bn;
+    g.tilesM = plan.tilesM;
+    g.tilesN = plan.tilesN;
+    g.nGemmCtas = plan.grid;
+    g.rasterGroup = plan.rasterGroup;
+    g.l2HintA = plan.l2HintA;
+    g.l2HintB = plan.l2HintB;
     DevComm dummy;
     memset(&dummy, 0, sizeof(dummy));
-    if (twoSm) {
-        const int bestBn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
-        g.bn = bestBn;
-        g.tilesN = (int)((n + bestBn - 1) / bestBn);
-        // B is split between the two CTAs of a pair: each loads half of the B rows of a tile
-        CHK_RET(MapB(&tb, b, n, k, bMn, bestBn / 2));
-        const WideOrder order(tilesM2, g.tilesN, pairs, 8);
-        if (WideMode() == 1 ? order.wide > 0 : (WideMode() == -1 && order.wide >= 2 * pairs && k >= 48 * kBK)) {
-            const int grid2 = 2 * pairs;
-            g.nGemmCtas = grid2;
-            if (!aMn && !bMn) return LaunchGemm2SmWide<false, false>(ta, tb, g, grid2, stream);
-            if (!aMn && bMn) return LaunchGemm2SmWide<false, true>(ta, tb, g, grid2, stream);
-            if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, grid2, stream);
-            return LaunchGemm2SmWide<true, true>(ta, tb, g, grid2, stream);
-        }
-        // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
-        // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next
-        // to the stream of the other, it is loaded "evict last", the streamed one "evict first", and the band covers
-        // the whole small operand.  Measured on the decoder's matmuls it did not pay (evict-first lines of the
-        // streamed operand leave before the other row tiles of the wave have read them), so it is off by default.
-        static const bool l2Hints = [] { const char* e = getenv("HCCL_MC2_L2_HINTS"); return e != nullptr && e[0] == '1'; }();
-        if (l2Hints) {
-            const double bytesA = 2.0 * (double)m * (double)k, bytesB = 2.0 * (double)n * (double)k;
-            const double fits = 72.0 * (1 << 20);
-            if (bytesA <= fits && bytesB > 1.5 * bytesA) {
-                g.l2HintA = 1; g.l2HintB = 2;
-                g.rasterGroup = std::min(tilesM2, 32);            // all rows of A in one band: B is read once
-            } else if (bytesB <= fits && bytesA > 1.5 * bytesB) {
-                g.l2HintA = 2; g.l2HintB = 1;
-                g.rasterGroup = std::max(1, std::min(8, pairs / std::max(1, g.tilesN)));   // all columns of B in flight together
-            }
-        }
-        const int grid2 = std::min(2 * pairs, 2 * tilesM2 * g.tilesN);
-        g.nGemmCtas = grid2;
-        return DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid2, false, stream);
+    if (plan.route == MatmulRoute::WIDE) {
+        if (!aMn && !bMn) return LaunchGemm2SmWide<false, false>(ta, tb, g, plan.grid, stream);
+        if (!aMn && bMn) return LaunchGemm2SmWide<false, true>(ta, tb, g, plan.grid, stream);
+        if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, plan.grid, stream);
+        return LaunchGemm2SmWide<true, true>(ta, tb, g, plan.grid, stream);
     }
-    const int bn = narrow ? 128 : 256;
-    g.tilesM = tilesM;
-    g.tilesN = (int)((n + bn - 1) / bn);
-    CHK_RET(MapB(&tb, b, n, k, bMn, bn));
-    const int grid = std::min(SmCount(), g.tilesM * g.tilesN);
-    g.nGemmCtas = grid;
-    if (bn == 128) return DispatchLayout<128, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid, false, stream);
-    return DispatchLayout<256, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, grid, false, stream);
+    if (plan.route == MatmulRoute::TWO_SM) return DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
+    if (plan.bn == 128) return DispatchLayout<128, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
+    return DispatchLayout<256, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
 }
 
 HcclResult Mc2AllGatherMatmul(CommImpl* comm, const void* aShard, const void* b, void* out, void* gathered, uint64_t mPerRank, uint64_t n,

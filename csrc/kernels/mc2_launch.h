@@ -23,6 +23,23 @@ constexpr int kMc2MaxTiles = 16384;
 constexpr int kMc2AgBlocks = 8 * 512;   // arrival counters of the push-form AllGather: ranks x 128-row blocks per rank
 constexpr int kMc2CtlWords = 16 + 8 * 512;
 
+// How a plain matmul runs, from its sizes, the number of SMs and the switches of the environment.
+enum class MatmulRoute { SPLIT, ONE_SM, TWO_SM, WIDE };
+struct MatmulSwitches {
+    bool twoSm = true;                  // HCCL_MC2_2SM
+    int wide = -1;                      // HCCL_MC2_WIDE: 0 never, 1 wherever one full round runs, -1 by the rule
+    bool l2Hints = false;               // HCCL_MC2_L2_HINTS
+};
+struct MatmulPlan {
+    MatmulRoute route = MatmulRoute::ONE_SM;
+    int bn = 0, tilesM = 0, tilesN = 0, grid = 0;
+    int bt = 0, split = 0;              // SPLIT: tokens per tile, CTAs per tile
+    int wide = 0, singles = 0;          // WIDE: wide items, single ones
+    int rasterGroup = 0, l2HintA = 0, l2HintB = 0;
+};
+MatmulSwitches MatmulSwitchesOfEnv();
+MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw);
+
 // Tests of a wait that runs out, on a matmul with few output tiles: CTA `cta` loads nothing, all waits end after waitLimitNs.
 struct Mc2StalledCta { int cta; uint64_t waitLimitNs; };
 HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB,

@@ -255,6 +255,28 @@ def test_small_output_matmul(m, n, k, ta, tb):
     _check_matmul(m, n, k, ta, tb)
 
 
+@pytest.mark.parametrize("m,n", [(16, 128), (512, 512)])
+def test_matmul_as_the_first_work_of_a_thread(m, n):
+    """A thread that has made no CUDA call yet has no current context; autograd's is one when a matmul is its first work."""
+    import threading
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b = _rnd(g, m, 256), _rnd(g, n, 256)
+    out, want, failed = torch.empty(m, n, device="cuda", dtype=torch.bfloat16), mc2.matmul(a, b), []
+
+    def work():
+        try:
+            mc2.matmul(a, b, out=out)
+        except Exception as e:
+            failed.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    assert torch.equal(out, want)
+
+
 # the stalled CTA alone on its tile, and one of a cluster of four: its peers hold good partials and must not store sums either
 @pytest.mark.parametrize("cta,k", [(0, 128), (0, 2048), (2, 2048)])
 def test_matmul_that_gives_up_a_wait(cta, k):

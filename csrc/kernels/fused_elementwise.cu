@@ -16,6 +16,7 @@ namespace hccl {
 namespace {
 
 constexpr uint32_t kNormMaxHidden = 8192;      // a row stays in the registers of one group of threads
+constexpr uint64_t kNormMaxRows = 0x7FFFFFFF;  // row numbers are 32-bit
 
 __device__ __forceinline__ void Unpack8(const uint4& raw, float* f)
 {
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(kNormThreads, 1) AddRmsNormFwdKernel(const __n
     uint8_t* ring = smem + kNormPartBytes + (size_t)group * kNormSlots * slotBytes;
     const uint32_t ringAddr = (uint32_t)__cvta_generic_to_shared(ring);
     const int first = (int)blockIdx.x * nGroups + group, stride = (int)gridDim.x * nGroups;
-    const int nMine = first < rows ? (rows - first + stride - 1) / stride : 0;
+    const int nMine = first < rows ? (rows - 1 - first) / stride + 1 : 0;
     auto fill = [&](int i) {                          // this thread's vectors of its group's row number i -> slot i % kNormSlots
         if (i < nMine) {
             const size_t off = ((size_t)first + (size_t)i * stride) * hidden;
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(kNormThreads, 1) RmsNormBwdKernel(const __nv_b
     uint8_t* ring = smem + kNormPartBytes + (size_t)group * kNormSlots * slotBytes;
     const uint32_t ringAddr = (uint32_t)__cvta_generic_to_shared(ring);
     const int first = (int)blockIdx.x * nGroups + group, stride = (int)gridDim.x * nGroups;
-    const int nMine = first < rows ? (rows - first + stride - 1) / stride : 0;
+    const int nMine = first < rows ? (rows - 1 - first) / stride + 1 : 0;
     auto fill = [&](int i) {                          // this thread's vectors of its group's row number i -> slot i % kNormSlots
         if (i < nMine) {
             const size_t off = ((size_t)first + (size_t)i * stride) * hidden;
@@ -527,7 +528,7 @@ HcclResult HcclFusedAddRmsNormFwd(const void* x, const void* delta, const void* 
 {
     CHK_PTR_NULL(x); CHK_PTR_NULL(w); CHK_PTR_NULL(h); CHK_PTR_NULL(rstd);
     if (delta != nullptr) CHK_PTR_NULL(xOut);
-    if (hidden == 0 || hidden % 8 != 0 || hidden > kNormMaxHidden) return HCCL_E_PARA;
+    if (hidden == 0 || hidden % 8 != 0 || hidden > kNormMaxHidden || rows > kNormMaxRows) return HCCL_E_PARA;
     if (!Aligned16(x) || !Aligned16(w) || !Aligned16(h) || (delta && (!Aligned16(delta) || !Aligned16(xOut)))) return HCCL_E_PARA;
     if (rows == 0) return HCCL_SUCCESS;
     const NormShape n = ShapeNorm(rows, hidden);
@@ -549,7 +550,7 @@ HcclResult HcclFusedRmsNormBwd(const void* dh, const void* x, const void* w, con
                                void* dw, uint64_t rows, uint32_t hidden, hcclStream_t stream)
 {
     CHK_PTR_NULL(dh); CHK_PTR_NULL(x); CHK_PTR_NULL(w); CHK_PTR_NULL(rstd); CHK_PTR_NULL(dx); CHK_PTR_NULL(dwPartial); CHK_PTR_NULL(dw);
-    if (hidden == 0 || hidden % 8 != 0 || hidden > kNormMaxHidden) return HCCL_E_PARA;
+    if (hidden == 0 || hidden % 8 != 0 || hidden > kNormMaxHidden || rows > kNormMaxRows) return HCCL_E_PARA;
     if (!Aligned16(dh) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dx) || !Aligned16(dwPartial) || (dxExtra && !Aligned16(dxExtra))) return HCCL_E_PARA;
     if (rows == 0) return HCCL_SUCCESS;
     const NormShape n = ShapeNorm(rows, hidden);

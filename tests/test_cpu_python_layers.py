@@ -139,3 +139,13 @@ def test_rope_reads_only_tables_that_hold_every_row(monkeypatch):
     assert not native
     fused.rope(x[:4], cos, sin)                          # a longer table is read from its start
     assert native == ["rope"]
+
+
+def test_norm_kernels_refuse_row_counts_they_cannot_number():
+    """2^31 rows and more are refused before anything is launched (the pointers are never used)."""
+    import ctypes
+    from hccl_b200._lib import lib
+    p = ctypes.c_void_p(4096)
+    for rows in (1 << 31, (1 << 32) + 5):
+        assert lib.HcclFusedAddRmsNormFwd(p, ctypes.c_void_p(0), p, ctypes.c_void_p(0), p, p, rows, 8, 1e-5, ctypes.c_void_p(0)) == 1
+        assert lib.HcclFusedRmsNormBwd(p, p, p, p, ctypes.c_void_p(0), p, p, p, rows, 8, ctypes.c_void_p(0)) == 1

@@ -49,6 +49,19 @@ def test_add_rms_norm_groups(rows, hidden, with_delta):
     assert (x.grad.double() - dx).norm().item() <= ONE_ROUNDING * dx.norm().item() + 1e-6 * d_h.double().norm().item()
 
 
+def test_rms_norm_of_as_many_rows_as_there_are_row_numbers():
+    rows, hidden = 2 ** 31 - 8, 8
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 77 GB")
+    x = torch.empty(rows, hidden, device="cuda", dtype=torch.bfloat16).fill_(3.0)
+    w = torch.arange(1, 9, device="cuda").bfloat16()
+    h = fused.add_rms_norm(x, None, w, 0.0)[1]
+    for part in (h[:10000], h[-10000:]):
+        assert torch.equal(part, w.expand(10000, hidden))
+    del x, h
+    torch.cuda.empty_cache()
+
+
 # vectors per thread: one (small) and several, rows shorter than a block's stretch, ragged ends
 @pytest.mark.parametrize("rows,f", [(1, 8), (3, 264), (700, 56), (1031, 3592), (4097, 1024)])
 def test_swiglu_blocks(rows, f):

@@ -49,6 +49,40 @@ def test_add_rms_norm_groups(rows, hidden, with_delta):
     assert (x.grad.double() - dx).norm().item() <= ONE_ROUNDING * dx.norm().item() + 1e-6 * d_h.double().norm().item()
 
 
+@pytest.mark.parametrize("captured", [False, True])
+def test_norm_backward_on_a_side_stream(captured):
+    """The two launches of the norm's backward pass on a stream of their own, eager and replayed from a graph on other inputs."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    inputs = [[_rnd(g, 700, 2056), _rnd(g, 700, 2056), _rnd(g, 2056), _rnd(g, 700, 2056), _rnd(g, 700, 2056)] for _ in range(2)]
+
+    def grads(x, delta, w, d_out, d_h):
+        x, delta, w = (t.detach().requires_grad_() for t in (x, delta, w))
+        return torch.autograd.grad(fused.add_rms_norm(x, delta, w, 1e-5), [x, delta, w], [d_out, d_h])
+
+    want = [grads(*i) for i in inputs]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    if captured:
+        static = [t.clone() for t in inputs[0]]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            grads(*static)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = grads(*static)
+    for i, ref in zip(inputs, want):
+        with torch.cuda.stream(side):
+            if captured:
+                for t, v in zip(static, i):
+                    t.copy_(v)
+                graph.replay()
+                got = [o.clone() for o in out]
+            else:
+                got = grads(*i)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
 def test_rms_norm_of_as_many_rows_as_there_are_row_numbers():
     rows, hidden = 2 ** 31 - 8, 8
     if torch.cuda.mem_get_info()[0] < 100 << 30:
@@ -256,6 +290,47 @@ def test_wide_matmul_with_kn_weight(m, n, k, ta):
 @pytest.mark.parametrize("ta,tb", LAYOUTS)
 def test_wide_tile_rounds(ta, tb):
     _check_matmul(2504, 7800, 3080, ta, tb)
+
+
+# (m, n, k), single items per pair after the wide ones: a second in the other accumulator, a third back in the first
+WIDE_SINGLES = [((1592, 13400, 3080), 2), ((3080, 8800, 3080), 3)]
+
+
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("shape", [s for s, _ in WIDE_SINGLES])
+def test_wide_tiles_followed_by_several_singles(shape, ta, tb):
+    _check_matmul(*shape, ta, tb)
+
+
+# k-blocks: one (the halves run together), four (skew two), 17 (skew eight), 24 (the first with the full skew)
+WIDE_SHORT_K = [(2504, 7800, k) for k in (64, 200, 1032, 1536)]
+
+
+def test_wide_tiles_with_a_short_inner_dimension():
+    """Shapes that take wide tiles only where HCCL_MC2_WIDE=1 asks for them; the switch is read once per process."""
+    import os
+    import subprocess
+    import sys
+    code = ("import sys; sys.path.insert(0, 'tests'); import test_gpu_tile_edges as t\n"
+            "for shape in t.WIDE_SHORT_K:\n"
+            "    for layout in t.LAYOUTS:\n"
+            "        t._check_matmul(*shape, *layout)\n"
+            "print('checked')")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=root, env={**os.environ, "HCCL_MC2_WIDE": "1"}, timeout=600)
+    assert r.returncode == 0 and "checked" in r.stdout, r.stderr[-3000:]
+
+
+# clusters of three: k-blocks and tokens that three CTAs cannot share evenly
+SPLIT_OF_THREE = [(17, 10000, 840), (40, 12000, 1032), (8, 9608, 960)]
+
+
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("shape", SPLIT_OF_THREE)
+def test_split_matmul_over_three_ctas(shape, ta, tb):
+    if ta and shape[0] % 8:
+        pytest.skip("transposed A needs M % 8 == 0")
+    _check_matmul(*shape, ta, tb)
 
 
 # token tiles of 16 .. 128 and several of them, k-blocks fewer and more than the CTAs of a cluster, ragged N and K

@@ -40,3 +40,16 @@ WIDE_SHAPE = (4096, 57344, 8192)
 def test_switches(env, route, hints):
     p = plan_with(env, *WIDE_SHAPE)
     assert (p["route"], p["hints"]) == (route, hints)
+
+
+def test_the_gpu_tests_reach_the_forms_they_are_named_after():
+    import test_gpu_tile_edges as edges
+    for ta, tb in edges.LAYOUTS:
+        for shape, singles in edges.WIDE_SINGLES:
+            p = plan(*shape, int(ta), int(tb))
+            assert p["route"] == "wide" and -(-int(p["singles"]) // 74) == singles, (shape, p)
+        for shape in edges.SPLIT_OF_THREE:
+            p = plan(*shape, int(ta), int(tb))
+            assert p["route"] == "split" and p["split"] == "3", (shape, p)
+    for shape in edges.WIDE_SHORT_K:
+        assert plan(*shape)["route"] == "two_sm" and plan_with({"HCCL_MC2_WIDE": "1"}, *shape)["route"] == "wide"

@@ -307,13 +307,13 @@ __global__ void __launch_bounds__(32 * kReduceRows) ReducePartialsKernel(const f
 // SwiGLU on gu [rows, 2 * f] (gate = columns [0, f), up = columns [f, 2f)): out = silu(gate) * up.
 //
 // Streaming kernels bound by HBM (6 bytes per output element forward, 10 backward).  Every thread takes VECS vectors
-// kSwiThreads apart and requests all of them before the first is used (8 resp. 6 16-byte loads in flight); the flat
+// kSwiThreads apart and requests all of them before the first is used (4 resp. 6 16-byte loads in flight); the flat
 // vector index is divided by the row length once per thread, not once per vector, in 32 bits where the size allows.
 // Measured at 4096 x 28672 against a grid-stride loop with one vector and a 64-bit division per step: forward 137.6 ->
-// 107.2 us (705 MB, 6.6 TB/s), backward 201.0 -> 172.5 us (1174 MB, 6.8 TB/s); at 4096 x 3584 22.7 -> 18.6 and 28.9 ->
-// 25.4 us.
+// 102.6 us (705 MB, 6.9 TB/s; 106.7 and 107.2 us with three and four vectors, whose registers leave fewer warps for the
+// arithmetic), backward 201.0 -> 172.5 us (1174 MB, 6.8 TB/s); at 4096 x 3584 22.7 -> 16.5 and 28.9 -> 25.5 us.
 constexpr int kSwiThreads = 256;
-constexpr int kSwiFwdVecs = 4, kSwiBwdVecs = 2;
+constexpr int kSwiFwdVecs = 2, kSwiBwdVecs = 2;
 __device__ __forceinline__ void RowOf(size_t i, uint32_t perRow, bool fits32, size_t* row, uint32_t* v)
 {
     if (fits32) {
@@ -330,7 +330,8 @@ __device__ __forceinline__ void RowOf(size_t i, uint32_t perRow, bool fits32, si
 // processor", 1990).  Both sides are scaled by a quarter, which keeps the divisor below 2^126, where its reciprocal is a
 // normal number: __fdividef(1, 1 + e^-x) is 0 for gates around -88, whose results are normal bf16 numbers.  Zeros and
 // infinities have no remainder, their quotient stands.  An exponential that is flushed to zero adds nothing to 1
-// anyway.  With the division operator in its place the forward pass at 4096 x 28672 takes 127.5 instead of 107.2 us.
+// anyway.  With the division operator in its place the forward pass at 4096 x 28672, four vectors per thread, takes
+// 127.5 instead of 107.2 us.
 __device__ __forceinline__ float OverOnePlusExp(float n, float x)
 {
     float e, r;
@@ -511,9 +512,9 @@ HcclResult CheckLaunch(const char* what)
     if (e != cudaSuccess) { HCCL_ERROR("%s launch failed: %s", what, cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
-// Several vectors per thread only where two blocks per SM remain with them; below that one each, which spreads the work
+// Two vectors per thread only where four blocks per SM remain with them; below that one each, which spreads the work
 // over more SMs (128 x 3584: 4.2 us either way, the launch).
-bool SwigluBig(size_t vecs) { return vecs >= (size_t)SmCount() * 2 * kSwiThreads * kSwiFwdVecs; }
+bool SwigluBig(size_t vecs) { return vecs >= (size_t)SmCount() * 4 * kSwiThreads * 2; }
 size_t SwigluBlocks(size_t vecs, int vecsPerThread) { return (vecs + (size_t)kSwiThreads * vecsPerThread - 1) / ((size_t)kSwiThreads * vecsPerThread); }
 
 }  // namespace

@@ -281,8 +281,9 @@ __global__ void __launch_bounds__(kNormThreads, 1) RmsNormBwdKernel(const __nv_b
 
 // dw[h] = sum of the CTAs' partials, in a fixed order.  32 columns per block (one 128-byte line of every partial row),
 // kReduceRows threads share a column's partials and are added through shared memory; at 148 partials of 8192 columns
-// that is 256 blocks of 8 warps instead of one thread per column walking all partials.  Launched so that its blocks
-// are already resident when RmsNormBwdKernel ends.
+// that is 256 blocks of 16 warps instead of one thread per column walking all partials.  The launch is a programmatic
+// dependent of RmsNormBwdKernel, which gives no early trigger and whose CTAs leave no registers for a second block: its
+// blocks start as CTAs of the norm kernel exit, and griddepcontrol.wait holds them until all partials are visible.
 constexpr int kReduceRows = 16;
 __global__ void __launch_bounds__(32 * kReduceRows) ReducePartialsKernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int nPartials, int hidden)
 {
@@ -544,7 +545,9 @@ HcclResult HcclFusedAddRmsNormFwd(const void* x, const void* delta, const void* 
 
 uint32_t HcclFusedRmsNormBwdPartials(uint64_t rows)
 {
-    return (uint32_t)(rows < 296 ? (rows < 1 ? 1 : rows) : 296);       // two CTAs per SM on 148 SMs
+    // the most partial rows that a launch may write: one per row, at most 296.  HcclFusedRmsNormBwd writes one per CTA and
+    // runs one CTA per SM, 148 on a B200; callers keep the size that they have always asked for.
+    return (uint32_t)(rows < 296 ? (rows < 1 ? 1 : rows) : 296);
 }
 
 HcclResult HcclFusedRmsNormBwd(const void* dh, const void* x, const void* w, const void* rstd, const void* dxExtra, void* dx, void* dwPartial,

@@ -12,8 +12,12 @@
 // the right half catches up with [0, skew) alone.  The left accumulator is drained under the right half's catch-up, the
 // right one under the next tile's left-only stretch; the price is `skew` k-blocks of A loaded twice per tile.
 //
-// Work items: full rounds of wide tiles over all pairs, then the rest as single 256-row x one-column-tile items (at most
-// two per pair, in alternating accumulators), so the launch takes as many column-tile times as the narrow kernel.
+// Work items: full rounds of wide tiles over all pairs, then the rest as single 256-row x one-column-tile items in
+// alternating accumulators, so the launch takes as many column-tile times as the narrow kernel.  Left-over positions give
+// a pair at most two singles, an odd last column tile adds one per row tile, spread over the pairs.
+//
+// A column's sum runs over k in the order 0 .. K where it is a left half or a single item, and skew .. K, 0 .. skew where
+// it is a right half: results depend on the shape of the product (not on timing) in the last place of their fp32 sums.
 //
 // Pipeline: four stages of 48 KiB; otherwise the roles, barriers and hand-over of mc2_gemm_2sm.cuh (full[stage] in
 // the leader, empty[stage] and tmemFull[acc] per CTA through the multicast commit, tmemEmpty[acc] in the leader with

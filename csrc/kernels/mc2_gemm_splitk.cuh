@@ -11,7 +11,8 @@
 //     start and end run under its neighbour's main loop;
 //   * each CTA leaves its fp32 partial in its own shared memory ([token][column], the idle stage ring) and, after one
 //     cluster barrier, CTA r adds its share of the tokens over all CTAs in rank order (one fixed order, no atomics, no
-//     workspace) and stores them as bf16, 256 contiguous bytes per token row.
+//     workspace) and stores them as bf16, 256 contiguous bytes per token row.  The order depends on the number of CTAs
+//     per tile and so on the shape: a row's fp32 sum may differ in its last place from that of a call with more rows.
 // Measured against the one-SM kernel on 128 x 128 tiles (us, bf16, weight [N, K]): 16 x 8192 x 8192 47.5 -> 26.8 (5.0
 // TB/s), 64 x 8192 x 8192 48.4 -> 28.8, 16 x 8192 x 1024 12.4 -> 8.4, 128 x 4096 x 4096 26.7 -> 16.5, 32 x 4096 x 14336
 // 73.9 -> 26.6, 300 x 2048 x 4096 24.7 -> 16.5; against its 256-wide form 16 x 57344 x 8192 160.6 -> 142.4 (6.6 TB/s), 64

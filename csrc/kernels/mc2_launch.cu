@@ -601,7 +601,8 @@ HcclResult Mc2AllGatherMatmul(CommImpl* comm, const void* aShard, const void* b,
     else workers = twoSm ? GatherWorkerCtas((g.M / 256) * g.tilesN, 2) : GatherWorkerCtas(g.tilesM * g.tilesN, 1);
     g.nGemmCtas = grid - workers;
     if (twoSm) {
-        // column tile width: fewest (waves x width), as for the plain matmul; MN-major B is loaded in 64-column boxes
+        // column tile width: fewest (waves x (width + 12)); only whole 64-column boxes of MN-major B.  (The plain matmul weighs
+        // its widths by measured wave times, TwoSmColumnTile; this kernel's waves also carry the copies and were not timed so.)
         const int pairs = g.nGemmCtas / 2;
         const int tilesM2 = g.M / 256;
         int bestBn = 256;

@@ -62,7 +62,7 @@ __device__ __forceinline__ void AddPeer(const uint32_t* p, uint32_t rank)
 }
 }  // namespace route
 
-static __global__ void __cluster_dims__(kRouteCtas, 1, 1) __launch_bounds__(kRouteThreads)
+static __global__ void __cluster_dims__(kRouteCtas, 1, 1) __launch_bounds__(kRouteThreads, 1)
     MoeExpertOffsetsKernel(const int32_t* __restrict__ topkIdx, uint64_t nPairs, uint32_t nExperts, uint32_t* __restrict__ offsets)
 {
     __shared__ uint32_t s_count[kRouteCounters];

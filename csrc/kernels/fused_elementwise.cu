@@ -11,6 +11,7 @@
 #include "hccl/hccl_fused_ops.h"
 #include "../core/log.h"
 #include "../core/per_device.h"
+#include "dependent_launch.cuh"
 
 namespace hccl {
 namespace {
@@ -85,6 +86,8 @@ __global__ void __launch_bounds__(kNormThreads, 1) AddRmsNormFwdKernel(const __n
                                                                        __nv_bfloat16* __restrict__ h, float* __restrict__ rstd, int rows, int hidden,
                                                                        int groupThreads, float eps)
 {
+    DependencyWait();
+    AllowDependents();
     extern __shared__ __align__(128) uint8_t smem[];
     const int nVec = hidden / 8;
     const int group = threadIdx.x / groupThreads, nGroups = blockDim.x / groupThreads, tid = threadIdx.x % groupThreads;
@@ -169,6 +172,8 @@ __global__ void __launch_bounds__(kNormThreads, 1) RmsNormBwdKernel(const __nv_b
                                                                    const __nv_bfloat16* __restrict__ dxExtra, __nv_bfloat16* __restrict__ dx,
                                                                    float* __restrict__ dwPartial, int rows, int hidden, int groupThreads)
 {
+    DependencyWait();
+    AllowDependents();
     extern __shared__ __align__(128) uint8_t smem[];
     const int nVec = hidden / 8;
     const int group = threadIdx.x / groupThreads, nGroups = blockDim.x / groupThreads, tid = threadIdx.x % groupThreads;
@@ -281,13 +286,12 @@ __global__ void __launch_bounds__(kNormThreads, 1) RmsNormBwdKernel(const __nv_b
 
 // dw[h] = sum of the CTAs' partials, in a fixed order.  32 columns per block (one 128-byte line of every partial row),
 // kReduceRows threads share a column's partials and are added through shared memory; at 148 partials of 8192 columns
-// that is 256 blocks of 16 warps instead of one thread per column walking all partials.  The launch is a programmatic
-// dependent of RmsNormBwdKernel, which gives no early trigger and whose CTAs leave no registers for a second block: its
-// blocks start as CTAs of the norm kernel exit, and griddepcontrol.wait holds them until all partials are visible.
+// that is 256 blocks of 16 warps instead of one thread per column walking all partials.
 constexpr int kReduceRows = 16;
 __global__ void __launch_bounds__(32 * kReduceRows) ReducePartialsKernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int nPartials, int hidden)
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    DependencyWait();
+    AllowDependents();
     __shared__ float s_sum[kReduceRows][33];
     const int lane = threadIdx.x & 31, r = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -346,6 +350,8 @@ __device__ __forceinline__ float OverOnePlusExp(float n, float x)
 template <int VECS>
 __global__ void __launch_bounds__(kSwiThreads) SwigluFwdKernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, size_t rows, int f)
 {
+    DependencyWait();
+    AllowDependents();
     const uint32_t nVecRow = (uint32_t)f / 8;
     const size_t total = rows * nVecRow;
     size_t i = (size_t)blockIdx.x * (kSwiThreads * VECS) + threadIdx.x, row;
@@ -383,6 +389,8 @@ template <int VECS>
 __global__ void __launch_bounds__(kSwiThreads) SwigluBwdKernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
                                                                __nv_bfloat16* __restrict__ dgu, size_t rows, int f)
 {
+    DependencyWait();
+    AllowDependents();
     const uint32_t nVecRow = (uint32_t)f / 8;
     const size_t total = rows * nVecRow;
     size_t i = (size_t)blockIdx.x * (kSwiThreads * VECS) + threadIdx.x, row;
@@ -442,6 +450,8 @@ __global__ void __launch_bounds__(kRopeThreads) RopeKernel(const __nv_bfloat16* 
                                                            size_t outStride, const float* __restrict__ cosT, const float* __restrict__ sinT,
                                                            size_t rows, int nHeads, int d, float sign, int rowsPerBlock)
 {
+    DependencyWait();
+    AllowDependents();
     const int half = d / 2, vecHalf = half / 8;
     const int headGroups = (nHeads + HEADS - 1) / HEADS, perRow = headGroups * vecHalf;
     const size_t firstRow = (size_t)blockIdx.x * rowsPerBlock;
@@ -507,9 +517,8 @@ NormShape ShapeNorm(uint64_t rows, uint32_t hidden)
     return n;
 }
 bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-HcclResult CheckLaunch(const char* what)
+HcclResult Launched(cudaError_t e, const char* what)
 {
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { HCCL_ERROR("%s launch failed: %s", what, cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -537,10 +546,10 @@ HcclResult HcclFusedAddRmsNormFwd(const void* x, const void* delta, const void* 
     const size_t smem = kNormPartBytes + (size_t)n.groups * kNormSlots * hidden * 2 * (delta ? 2 : 1);
     auto kernel = delta ? AddRmsNormFwdKernel<true> : AddRmsNormFwdKernel<false>;
     CHK_RET(delta ? AllowNormRing<AddRmsNormFwdKernel<true>>() : AllowNormRing<AddRmsNormFwdKernel<false>>());
-    kernel<<<n.ctas, n.groups * n.groupThreads, smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w,
-                                                                              (__nv_bfloat16*)xOut, (__nv_bfloat16*)h, (float*)rstd, (int)rows,
-                                                                              (int)hidden, n.groupThreads, eps);
-    return CheckLaunch("AddRmsNormFwd");
+    return Launched(LaunchDependent(kernel, n.ctas, n.groups * n.groupThreads, smem, (cudaStream_t)stream, 0, (const __nv_bfloat16*)x,
+                                    (const __nv_bfloat16*)delta, (const __nv_bfloat16*)w, (__nv_bfloat16*)xOut, (__nv_bfloat16*)h, (float*)rstd,
+                                    (int)rows, (int)hidden, n.groupThreads, eps),
+                    "AddRmsNormFwd");
 }
 
 uint32_t HcclFusedRmsNormBwdPartials(uint64_t rows)
@@ -563,23 +572,13 @@ HcclResult HcclFusedRmsNormBwd(const void* dh, const void* x, const void* w, con
                                                   n.groups > 1 ? (size_t)n.groups * hidden * 4 : (size_t)0);
     auto kernel = dxExtra ? RmsNormBwdKernel<true> : RmsNormBwdKernel<false>;
     CHK_RET(dxExtra ? AllowNormRing<RmsNormBwdKernel<true>>() : AllowNormRing<RmsNormBwdKernel<false>>());
-    kernel<<<nPart, n.groups * n.groupThreads, smem, (cudaStream_t)stream>>>((const __nv_bfloat16*)dh, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                                                         (const float*)rstd, (const __nv_bfloat16*)dxExtra, (__nv_bfloat16*)dx,
-                                                                         (float*)dwPartial, (int)rows, (int)hidden, n.groupThreads);
-    CHK_RET(CheckLaunch("RmsNormBwd"));
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((hidden + 31) / 32);
-    cfg.blockDim = dim3(32 * kReduceRows);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute early;
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, ReducePartialsKernel, (const float*)dwPartial, (__nv_bfloat16*)dw, (int)nPart, (int)hidden) != cudaSuccess)
-        return CheckLaunch("RmsNormBwd reduce");
-    return HCCL_SUCCESS;
+    CHK_RET(Launched(LaunchDependent(kernel, nPart, n.groups * n.groupThreads, smem, (cudaStream_t)stream, 0, (const __nv_bfloat16*)dh,
+                                     (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)rstd, (const __nv_bfloat16*)dxExtra,
+                                     (__nv_bfloat16*)dx, (float*)dwPartial, (int)rows, (int)hidden, n.groupThreads),
+                     "RmsNormBwd"));
+    return Launched(LaunchDependent(ReducePartialsKernel, (hidden + 31) / 32, 32 * kReduceRows, 0, (cudaStream_t)stream, 0, (const float*)dwPartial,
+                                    (__nv_bfloat16*)dw, (int)nPart, (int)hidden),
+                    "RmsNormBwd reduce");
 }
 
 HcclResult HcclFusedSwigluFwd(const void* gu, void* out, uint64_t rows, uint32_t f, hcclStream_t stream)
@@ -591,9 +590,9 @@ HcclResult HcclFusedSwigluFwd(const void* gu, void* out, uint64_t rows, uint32_t
     const bool big = SwigluBig(vecs);
     const size_t blocks = SwigluBlocks(vecs, big ? kSwiFwdVecs : 1);
     if (blocks > 0x7FFFFFFFull) return HCCL_E_PARA;
-    if (big) SwigluFwdKernel<kSwiFwdVecs><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f);
-    else SwigluFwdKernel<1><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f);
-    return CheckLaunch("SwigluFwd");
+    return Launched(LaunchDependent(big ? SwigluFwdKernel<kSwiFwdVecs> : SwigluFwdKernel<1>, (unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream, 0,
+                                    (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, (int)f),
+                    "SwigluFwd");
 }
 
 HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint64_t rows, uint32_t f, hcclStream_t stream)
@@ -605,9 +604,9 @@ HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint6
     const bool big = SwigluBig(vecs);
     const size_t blocks = SwigluBlocks(vecs, big ? kSwiBwdVecs : 1);
     if (blocks > 0x7FFFFFFFull) return HCCL_E_PARA;
-    if (big) SwigluBwdKernel<kSwiBwdVecs><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, rows, (int)f);
-    else SwigluBwdKernel<1><<<(unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, rows, (int)f);
-    return CheckLaunch("SwigluBwd");
+    return Launched(LaunchDependent(big ? SwigluBwdKernel<kSwiBwdVecs> : SwigluBwdKernel<1>, (unsigned)blocks, kSwiThreads, 0, (cudaStream_t)stream, 0,
+                                    (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, rows, (int)f),
+                    "SwigluBwd");
 }
 
 HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t outStride, const void* cosTable, const void* sinTable, uint64_t rows,
@@ -623,13 +622,11 @@ HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t 
     const uint32_t rowsPerBlock = perRow >= (uint32_t)kRopeThreads ? 1 : kRopeThreads / perRow;
     const uint64_t blocks = (rows + rowsPerBlock - 1) / rowsPerBlock;
     if (blocks > 0x7FFFFFFFull) return HCCL_E_PARA;
-#define HCCL_ROPE(H)                                                                                                                          \
-    RopeKernel<H><<<(unsigned)blocks, kRopeThreads, 0, (cudaStream_t)stream>>>(                                                               \
-        (const __nv_bfloat16*)in, (size_t)inStride, (__nv_bfloat16*)out, (size_t)outStride, (const float*)cosTable, (const float*)sinTable, rows, \
-        (int)nHeads, (int)headDim, backward ? -1.f : 1.f, (int)rowsPerBlock)
-    if (heads == 4) HCCL_ROPE(4); else if (heads == 2) HCCL_ROPE(2); else HCCL_ROPE(1);
-#undef HCCL_ROPE
-    return CheckLaunch("Rope");
+    return Launched(LaunchDependent(heads == 4 ? RopeKernel<4> : (heads == 2 ? RopeKernel<2> : RopeKernel<1>), (unsigned)blocks, kRopeThreads, 0,
+                                    (cudaStream_t)stream, 0, (const __nv_bfloat16*)in, (size_t)inStride, (__nv_bfloat16*)out, (size_t)outStride,
+                                    (const float*)cosTable, (const float*)sinTable, rows, (int)nHeads, (int)headDim, backward ? -1.f : 1.f,
+                                    (int)rowsPerBlock),
+                    "Rope");
 }
 
 }  // extern "C"

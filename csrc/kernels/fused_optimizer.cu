@@ -13,6 +13,7 @@
 #include <cstdint>
 #include "hccl/hccl_fused_ops.h"
 #include "../core/log.h"
+#include "dependent_launch.cuh"
 
 namespace hccl {
 namespace {
@@ -40,6 +41,8 @@ __device__ __forceinline__ float SqrtApprox(float x)
 // step[0] += 1, step[1] = 1 - beta1^step, step[2] = sqrt(1 - beta2^step)
 __global__ void AdamStepKernel(float* step, float beta1, float beta2)
 {
+    DependencyWait();
+    AllowDependents();
     const float s = step[0] + 1.0f;
     step[0] = s;
     step[1] = 1.0f - powf(beta1, s);
@@ -102,6 +105,7 @@ template <class TP, class TS>
 __global__ void __launch_bounds__(kAdamThreads, 4) AdamWKernel(const __grid_constant__ AdamBatch b, AdamScalars s, const float* __restrict__ step,
                                                             const float* __restrict__ lrDev)
 {
+    AllowDependents();
     // which tensor: last i with chunkStart[i] <= blockIdx.x
     uint32_t lo = 0, hi = b.n;
     while (hi - lo > 1) {
@@ -109,6 +113,7 @@ __global__ void __launch_bounds__(kAdamThreads, 4) AdamWKernel(const __grid_cons
         if (b.chunkStart[mid] <= blockIdx.x) lo = mid; else hi = mid;
     }
     const HcclAdamTensor& t = b.t[lo];
+    DependencyWait();
     if (lrDev) s.lr = *lrDev;
     const float decay = 1.0f - s.lr * s.weightDecay, stepSize = s.lr / step[1], rbc2s = 1.0f / step[2];
     constexpr int G = Vec<TP>::kElems < Vec<TS>::kElems ? Vec<TP>::kElems : Vec<TS>::kElems;     // elements per thread-iteration
@@ -226,8 +231,7 @@ HcclResult LaunchAdam(const HcclAdamTensor* tensors, uint32_t nTensors, const Ad
         }
         if (b.n == 0) break;
         b.chunkStart[b.n] = (uint32_t)chunks;
-        AdamWKernel<TP, TS><<<(unsigned)chunks, kAdamThreads, 0, stream>>>(b, s, step, lrDev);
-        if (cudaGetLastError() != cudaSuccess) return HCCL_E_RUNTIME;
+        if (LaunchDependent(AdamWKernel<TP, TS>, (unsigned)chunks, kAdamThreads, 0, stream, 0, b, s, step, lrDev) != cudaSuccess) return HCCL_E_RUNTIME;
     }
     return HCCL_SUCCESS;
 }
@@ -254,8 +258,7 @@ extern "C" HcclResult HcclFusedAdamW(const HcclAdamTensor* tensors, uint32_t nTe
     for (uint32_t i = 0; i < nTensors; ++i)
         if (tensors[i].numel != 0 && (!tensors[i].param || !tensors[i].grad || !tensors[i].expAvg || !tensors[i].expAvgSq)) return HCCL_E_PTR;
     cudaStream_t s = (cudaStream_t)stream;
-    AdamStepKernel<<<1, 1, 0, s>>>(stepState, beta1, beta2);
-    if (cudaGetLastError() != cudaSuccess) return HCCL_E_RUNTIME;
+    if (LaunchDependent(AdamStepKernel, 1, 1, 0, s, 0, stepState, beta1, beta2) != cudaSuccess) return HCCL_E_RUNTIME;
     const AdamScalars sc{lr, beta1, beta2, eps, weightDecay};
     if (paramType == HCCL_DATA_TYPE_BFP16 && stateType == HCCL_DATA_TYPE_BFP16) return LaunchAdam<__nv_bfloat16, __nv_bfloat16>(tensors, nTensors, sc, stepState, lrDev, s);
     if (paramType == HCCL_DATA_TYPE_FP32 && stateType == HCCL_DATA_TYPE_FP32) return LaunchAdam<float, float>(tensors, nTensors, sc, stepState, lrDev, s);

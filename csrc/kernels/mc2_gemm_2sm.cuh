@@ -149,7 +149,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int warp = threadIdx.x / 32;
     const int cta = (int)blockIdx.x;
     const uint32_t crank = ClusterCtaRank();
-    const uint32_t launchEpoch = *reinterpret_cast<volatile uint32_t*>(g.ctl + kCtlEpoch) + 1;
+    if (MODE == MODE_PLAIN) AllowDependents();
+    const uint32_t launchEpoch = MODE == MODE_PLAIN ? 0u : *reinterpret_cast<volatile uint32_t*>(g.ctl + kCtlEpoch) + 1;
 
     if (cta >= g.nGemmCtas) {
         const int worker = cta - g.nGemmCtas, nWorkers = (int)gridDim.x - g.nGemmCtas;
@@ -177,6 +178,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ClusterSync();               // the peer's barriers exist before anything arrives on them
         TcFenceAfter();
         const uint32_t tmemBase = *tmemBaseSlot;
+        if (MODE == MODE_PLAIN) DependencyWait();
         const int BN = g.bn;                        // column tile width of this launch (accumulators stay 256 columns apart)
         const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;
         const int tilesM2 = (g.M + 255) / 256;
@@ -385,6 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
     }
 
+    if (MODE == MODE_PLAIN) return;                    // no epochs
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();

@@ -56,6 +56,8 @@ inline int SplitSmemBytes(int bt)
     const int ring = SplitStages(bt) * SplitStageBytes(bt), partial = bt * 128 * 4;
     return (ring > partial ? ring : partial) + kSplitBarBytes + 1024;      // + slack for the 1024-byte alignment
 }
+constexpr int kSplitMaxSmemBytes = kSplitRingBytes + kSplitBarBytes + 1024;
+static_assert(kSplitMaxBt * 128 * 4 <= kSplitRingBytes, "the largest partial tile is no larger than the ring");
 
 __device__ __forceinline__ uint32_t SplitClusterRank()
 {
@@ -103,6 +105,7 @@ template <bool W_MN, bool X_MN>
 __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SplitArgs g)
 {
     extern __shared__ uint8_t smemRaw[];
+    AllowDependents();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
     const int stageBytes = SplitStageBytes(g.bt);
     const int ringBytes = g.stages * stageBytes, partialBytes = g.bt * 128 * 4;
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemBaseSlot;
+    DependencyWait();
 
     if (warp == 0) {
         if (ElectOne()) {

@@ -89,8 +89,7 @@ HcclResult LaunchGemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
         if (e != cudaSuccess) { HCCL_ERROR("fused matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
         return HCCL_SUCCESS;
     }
-    kernel<<<grid, kThreads, SmemLayout<BN>::kTotal, stream>>>(ta, tb, ta2, g, c);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)grid, kThreads, SmemLayout<BN>::kTotal, stream, 0, ta, tb, ta2, g, c);
     if (e != cudaSuccess) { HCCL_ERROR("matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -102,18 +101,23 @@ HcclResult LaunchGemm2Sm(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
     const CUtensorMap& ta2 = taOwn != nullptr ? *taOwn : ta;
     constexpr auto kernel = GemmKernel2Sm<A_MN, B_MN, MODE>;
     CHK_RET(AllowSharedMemory<kernel>(SmemLayout2::kTotal));
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = SmemLayout2::kTotal;
-    cfg.stream = stream;
-    cudaLaunchAttribute attrs[1];
-    attrs[0].id = cudaLaunchAttributeCooperative;
-    attrs[0].val.cooperative = cooperative ? 1 : 0;
-    cfg.attrs = attrs;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, ta2, g, c);
+    cudaError_t e;
+    if (cooperative) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = SmemLayout2::kTotal;
+        cfg.stream = stream;
+        cudaLaunchAttribute attrs[1];
+        attrs[0].id = cudaLaunchAttributeCooperative;
+        attrs[0].val.cooperative = 1;
+        cfg.attrs = attrs;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, ta2, g, c);
+    } else {
+        e = LaunchDependent(kernel, (unsigned)grid, kThreads, SmemLayout2::kTotal, stream, 0, ta, tb, ta2, g, c);
+    }
     if (e != cudaSuccess) { HCCL_ERROR("two-SM matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -123,13 +127,7 @@ HcclResult LaunchGemm2SmWide(const CUtensorMap& ta, const CUtensorMap& tb, const
 {
     constexpr auto kernel = GemmKernel2SmWide<A_MN, B_MN>;
     CHK_RET(AllowSharedMemory<kernel>(SmemLayoutWide::kTotal));
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = SmemLayoutWide::kTotal;
-    cfg.stream = stream;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ta, tb, g);
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)grid, kThreads, SmemLayoutWide::kTotal, stream, 0, ta, tb, g);
     if (e != cudaSuccess) { HCCL_ERROR("wide two-SM matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -137,22 +135,9 @@ HcclResult LaunchGemm2SmWide(const CUtensorMap& ta, const CUtensorMap& tb, const
 template <bool W_MN, bool X_MN>
 HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& g, int tiles, int split, cudaStream_t stream)
 {
-    auto kernel = GemmSplitKernel<W_MN, X_MN>;
-    const int smem = SplitSmemBytes(g.bt);
-    CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(tiles * split));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = (unsigned)split;
-    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    cfg.attrs = &cluster;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tw, tx, g);
+    constexpr auto kernel = GemmSplitKernel<W_MN, X_MN>;
+    CHK_RET(AllowSharedMemory<kernel>(kSplitMaxSmemBytes));
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split), kThreads, (size_t)SplitSmemBytes(g.bt), stream, (unsigned)split, tw, tx, g);
     if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }

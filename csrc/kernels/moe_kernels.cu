@@ -318,6 +318,6 @@ extern "C" HcclResult HcclMoeExpertOffsets(const int32_t* topkIdx, uint64_t nPai
     CHK_PTR_NULL(topkIdx);
     CHK_PTR_NULL(offsets);
     if (nExperts == 0 || nExperts > kRouteMaxExperts) { HCCL_ERROR("HcclMoeExpertOffsets: 1..%u experts supported (got %u)", kRouteMaxExperts, nExperts); return HCCL_E_PARA; }
-    MoeExpertOffsetsKernel<<<kRouteCtas, kRouteThreads, 0, (cudaStream_t)stream>>>(topkIdx, nPairs, nExperts, offsets);
-    return cudaGetLastError() == cudaSuccess ? HCCL_SUCCESS : HCCL_E_RUNTIME;
+    return LaunchDependent(MoeExpertOffsetsKernel, kRouteCtas, kRouteThreads, 0, (cudaStream_t)stream, 0, topkIdx, nPairs, nExperts, offsets) == cudaSuccess
+               ? HCCL_SUCCESS : HCCL_E_RUNTIME;
 }

@@ -19,6 +19,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "dependent_launch.cuh"
 
 namespace hccl {
 
@@ -68,6 +69,8 @@ static __global__ void __cluster_dims__(kRouteCtas, 1, 1) __launch_bounds__(kRou
     __shared__ uint32_t s_count[kRouteCounters];
     __shared__ uint32_t s_warp[kRouteThreads / 32];
     __shared__ uint32_t s_before[kRouteCtas];                    // pairs of the experts of each CTA before this one
+    DependencyWait();
+    AllowDependents();
     const uint32_t rank = route::ClusterRank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool everyCta = nExperts <= kRouteCounters;            // every CTA counts all experts
     const uint32_t perCta = (nExperts + kRouteCtas - 1) / kRouteCtas;

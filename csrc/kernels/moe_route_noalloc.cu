@@ -17,8 +17,7 @@ extern "C" HcclResult HcclMoeExpertOffsetsNoAlloc(const int32_t* topkIdx, uint64
                    HCCL_MOE_NOALLOC_MAX_EXPERTS);
         return HCCL_E_PARA;
     }
-    MoeExpertOffsetsKernel<<<kRouteCtas, kRouteThreads, 0, (cudaStream_t)stream>>>(topkIdx, nPairs, nExperts, offsets);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = LaunchDependent(MoeExpertOffsetsKernel, kRouteCtas, kRouteThreads, 0, (cudaStream_t)stream, 0, topkIdx, nPairs, nExperts, offsets);
     if (e != cudaSuccess) { HCCL_ERROR("HcclMoeExpertOffsetsNoAlloc: launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }

@@ -72,14 +72,15 @@ __device__ __forceinline__ void UmmaF16_2Sm(uint32_t tmemD, uint64_t descA, uint
         "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// Arrives on the barrier at the same offset in both CTAs once all MMAs issued so far have completed.
-__device__ __forceinline__ void UmmaCommit2Sm(uint64_t* bar)
+// Arrives on the barrier at the same offset in the CTAs of the mask (bit = cluster rank; the two of a pair) once all MMAs
+// issued so far have completed.
+__device__ __forceinline__ void UmmaCommitPair(uint64_t* bar, uint16_t mask)
 {
-    const uint16_t mask = 3;
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(SmemAddr(bar)),
                  "h"(mask)
                  : "memory");
 }
+__device__ __forceinline__ void UmmaCommit2Sm(uint64_t* bar) { UmmaCommitPair(bar, 3); }
 __device__ __forceinline__ void MbarArriveCluster(uint32_t clusterAddr)
 {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
@@ -94,6 +95,18 @@ __device__ __forceinline__ void TmemDealloc2(uint32_t taddr, uint32_t nCols)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(nCols) : "memory");
 }
 
+// Grouped raster: bands of `group` row tiles (8 unless asked otherwise), walked column by column, so that the ~74 tiles in
+// flight touch about 8 row tiles of A and 9 column tiles of B instead of all of A.
+constexpr int kRasterGroup = 8;
+__host__ __device__ __forceinline__ void GroupedTile(int t, int tilesM2, int tilesN, int group, int* mt2, int* nt)
+{
+    const int perBand = group * tilesN;
+    const int band = t / perBand, rem = t % perBand;
+    const int first = band * group;
+    const int rows = (tilesM2 - first) < group ? (tilesM2 - first) : group;
+    *mt2 = first + rem % rows;
+    *nt = rem / rows;
+}
 // Pair tile index -> (256-row tile, 256-column tile), same orders as TileCoord but in units of 256 rows.
 template <int MODE>
 __device__ __forceinline__ void TileCoord2(const GemmArgs& g, int t, int tilesM2, int* mt2, int* nt)
@@ -118,15 +131,7 @@ __device__ __forceinline__ void TileCoord2(const GemmArgs& g, int t, int tilesM2
         *mt2 = dstRank * rowTiles + rem % rowTiles;
         *nt = n;
     } else {
-        // grouped raster: bands of 8 row tiles, walked column by column, so that the ~74 tiles in flight touch about
-        // 8 row tiles of A and 9 column tiles of B instead of all of A
-        const int kGroup = g.rasterGroup > 0 ? g.rasterGroup : 8;
-        const int perBand = kGroup * g.tilesN;
-        const int band = t / perBand, rem = t % perBand;
-        const int first = band * kGroup;
-        const int rows = (tilesM2 - first) < kGroup ? (tilesM2 - first) : kGroup;
-        *mt2 = first + rem % rows;
-        *nt = rem / rows;
+        GroupedTile(t, tilesM2, g.tilesN, g.rasterGroup > 0 ? g.rasterGroup : kRasterGroup, mt2, nt);
     }
 }
 
@@ -149,7 +154,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int warp = threadIdx.x / 32;
     const int cta = (int)blockIdx.x;
     const uint32_t crank = ClusterCtaRank();
-    if (MODE == MODE_PLAIN) AllowDependents();
     const uint32_t launchEpoch = MODE == MODE_PLAIN ? 0u : *reinterpret_cast<volatile uint32_t*>(g.ctl + kCtlEpoch) + 1;
 
     if (cta >= g.nGemmCtas) {
@@ -178,11 +182,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ClusterSync();               // the peer's barriers exist before anything arrives on them
         TcFenceAfter();
         const uint32_t tmemBase = *tmemBaseSlot;
-        if (MODE == MODE_PLAIN) DependencyWait();
+        if (MODE == MODE_PLAIN) {
+            DependencyWait();
+            AllowDependents();          // not before: the split launch of the last tiles relies on it (mc2_gemm_2sm_split.cuh)
+        }
         const int BN = g.bn;                        // column tile width of this launch (accumulators stay 256 columns apart)
         const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;
         const int tilesM2 = (g.M + 255) / 256;
-        const int nTiles = tilesM2 * g.tilesN;
+        const int nTiles = MODE == MODE_PLAIN && g.tileLimit > 0 ? g.tileLimit : tilesM2 * g.tilesN;
         const int kBlocks = (g.K + kBK - 1) / kBK;
         // bytes of a stage in both CTAs.  An MN-major half tile of B comes in boxes of 64 columns, whole ones: at a
         // half width that is no multiple of 64 the last box brings columns of the neighbouring half (or tile) along,

@@ -54,12 +54,7 @@ struct WideOrder {
     // grouped raster over (256-row tile, pair of column tiles): bands of `group` row tiles, rows fastest
     __host__ __device__ void Position(int q, int* mt2, int* col) const
     {
-        const int perBand = group * cols;
-        const int band = q / perBand, rem = q % perBand;
-        const int first = band * group;
-        const int rows = (tilesM2 - first) < group ? (tilesM2 - first) : group;
-        *mt2 = first + rem % rows;
-        *col = rem / rows;
+        GroupedTile(q, tilesM2, cols, group, mt2, col);
     }
     __host__ __device__ WideItem Get(int t) const
     {
@@ -125,7 +120,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int BN = g.bn;
     const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;
     const int kBlocks = (g.K + kBK - 1) / kBK;
-    const WideOrder order((g.M + 255) / 256, g.tilesN, nPairs, g.rasterGroup > 0 ? g.rasterGroup : 8);
+    const WideOrder order((g.M + 255) / 256, g.tilesN, nPairs, g.rasterGroup > 0 ? g.rasterGroup : kRasterGroup);
     const int skew = kBlocks / 2 < kWideSkew ? kBlocks / 2 : kWideSkew;
 
     if (warp == 0) {

@@ -9,7 +9,7 @@
 #include "../core/log.h"
 #include "../core/per_device.h"
 #include "mc2_gemm_2sm_wide.cuh"
-#include "mc2_gemm_splitk.cuh"
+#include "mc2_gemm_2sm_split.cuh"
 
 namespace hccl {
 
@@ -140,6 +140,23 @@ HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const S
     const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split), kThreads, (size_t)SplitSmemBytes(g.bt), stream, (unsigned)split, tw, tx, g);
     if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
+}
+
+template <bool A_MN, bool B_MN>
+HcclResult LaunchGemm2SmSplit(const CUtensorMap& ta, const CUtensorMap& tb, const Split2Args& g, int tiles, int split, cudaStream_t stream)
+{
+    constexpr auto kernel = GemmKernel2SmSplit<A_MN, B_MN>;
+    CHK_RET(AllowSharedMemory<kernel>(SmemLayout2Split::kTotal));
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split * 2), kSplit2Threads, SmemLayout2Split::kTotal, stream, (unsigned)(2 * split), ta, tb, g);
+    if (e != cudaSuccess) { HCCL_ERROR("two-SM split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
+}
+HcclResult DispatchSplit2(bool aMn, bool bMn, const CUtensorMap& ta, const CUtensorMap& tb, const Split2Args& g, int tiles, int split, cudaStream_t s)
+{
+    if (!aMn && !bMn) return LaunchGemm2SmSplit<false, false>(ta, tb, g, tiles, split, s);
+    if (!aMn && bMn) return LaunchGemm2SmSplit<false, true>(ta, tb, g, tiles, split, s);
+    if (aMn && !bMn) return LaunchGemm2SmSplit<true, false>(ta, tb, g, tiles, split, s);
+    return LaunchGemm2SmSplit<true, true>(ta, tb, g, tiles, split, s);
 }
 
 template <int MODE>
@@ -293,6 +310,15 @@ int TwoSmColumnTile(int tilesM2, uint64_t n, int pairs, bool bMn)
     return best;
 }
 
+// CTA pairs per tile of a two-SM split launch.  Clusters of four, six and eight CTAs that fill an SM each fit 33, 22 and 15
+// times on a B200 (148 SMs in groups that no cluster crosses); more would run one after the other.
+int Split2Pairs(int tiles, int pairs)
+{
+    if (tiles * 74 <= 15 * pairs) return 4;
+    if (tiles * 74 <= 22 * pairs) return 3;
+    return tiles * 74 <= 33 * pairs ? 2 : 1;
+}
+
 HcclResult CheckShapes(uint64_t m, uint64_t n, uint64_t k)
 {
     if (m == 0 || n == 0 || k == 0 || m > (1u << 30) || n > (1u << 30) || k > (1u << 30)) return HCCL_E_PARA;
@@ -411,6 +437,20 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     // 512 x 4096 x 4096 26.6 -> 23.1, 1000 x 2048 x 2048 16.5 -> 16.1; with fewer tiles the split kernel is ahead: 300 x
     // 2048 x 4096 22.4 against 16.5).
     const bool twoSm = sw.twoSm && ((!narrow && m >= 256) || (m > 128 && k >= 2048 && (uint64_t)tilesM2 * ((n + 127) / 128) * 5 >= (uint64_t)pairs * 4));
+    // Two-SM tiles with the inner dimension split over a cluster of CTA pairs (see mc2_gemm_2sm_split.cuh): from 129 rows on, where
+    // 256 x 128 tiles do not outnumber the pairs and the inner dimension pays for the sum.  At 129 .. 192 rows a quarter and more
+    // of the 256 is padding, and the token split stays ahead where it has a long inner dimension (129 x 4096 x 14336: 28.9 us
+    // against 30.3).
+    const uint64_t tiles128 = (uint64_t)tilesM2 * ((n + 127) / 128);
+    if (sw.twoSm && m > 128 && k >= 2048 && tiles128 <= (uint64_t)pairs && (m > 192 || k < 4096 || twoSm)) {
+        p.route = MatmulRoute::TWO_SM_SPLIT;
+        p.bn = 128;
+        p.tilesM = tilesM2;
+        p.tilesN = (int)((n + 127) / 128);
+        p.split = Split2Pairs((int)tiles128, pairs);
+        p.grid = (int)tiles128 * 2 * p.split;
+        return p;
+    }
     // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
     // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
     // long (400 x 1024 x 1024: 10.3 us against 9.2 on the one-SM kernel, 300 x 2048 x 4096: 16.5 against 24.7).
@@ -451,6 +491,25 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     }
     p.route = MatmulRoute::TWO_SM;
     p.grid = std::min(2 * pairs, 2 * tilesM2 * p.tilesN);
+    // Full rounds of 256-wide tiles and a split launch for the last ones, where that costs less than a width that evens out the
+    // rounds (same units as TwoSmColumnTile; the split launch costs a share of a round and about 8 us, a k-block of a round
+    // 0.37).  It pays with MN-major B, whose narrower tiles are filled in whole boxes (sustained, us: 1024 x 10240 x 8192 with A
+    // transposed 157.8 -> 141.3, 1000 x 10240 x 8192 151.9 -> 140.7); with K-major B narrower tiles cost the same (1000 x 10240 x
+    // 8192 138.4 and 141.2).
+    const int tiles256 = tilesM2 * (int)((n + 255) / 256), rest = tiles256 % pairs;
+    const int restSplit = rest > 0 && tiles256 > pairs ? Split2Pairs(rest, pairs) : 1;
+    if (bMn && !sw.l2Hints && restSplit > 1 && k >= 16 * kBK) {
+        const int waves = (tilesM2 * p.tilesN + pairs - 1) / pairs, loaded = 2 * ((p.bn / 2 + 63) / 64 * 64);
+        const double perRound = 352.0, now = waves * ((p.bn + 2 * loaded) / 3.0 + 96);
+        const double split = (tiles256 / pairs) * perRound + perRound / restSplit + perRound * 8 / (0.37 * (double)((k + kBK - 1) / kBK));
+        if (split < 0.95 * now) {
+            p.bn = 256;
+            p.tilesN = (int)((n + 255) / 256);
+            p.grid = 2 * pairs;
+            p.restTiles = rest;
+            p.restSplit = restSplit;
+        }
+    }
     // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
     // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next
     // to the stream of the other, it is loaded "evict last", the streamed one "evict first", and the band covers
@@ -501,11 +560,23 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, plan.split, stream);
         return LaunchGemmSplit<true, true>(tw, tx, g, tiles, plan.split, stream);
     }
-    if (stalled != nullptr) return HCCL_E_NOT_SUPPORT;
+    if (stalled != nullptr && plan.route != MatmulRoute::TWO_SM_SPLIT) return HCCL_E_NOT_SUPPORT;
     CUtensorMap ta, tb;
     CHK_RET(MapA(&ta, a, m, k, aMn));
     // two-SM tiles: B is split between the two CTAs of a pair, each loads half of the B rows of a tile
     CHK_RET(MapB(&tb, b, n, k, bMn, plan.route == MatmulRoute::ONE_SM ? plan.bn : plan.bn / 2));
+    Split2Args split;
+    memset(&split, 0, sizeof(split));
+    split.M = (int)m; split.N = (int)n; split.K = (int)k;
+    split.out = (__nv_bfloat16*)out;
+    split.bn = plan.bn;
+    split.tilesM2 = (int)((m + 255) / 256);
+    split.tilesN = plan.tilesN;
+    split.stages = Split2Stages(plan.bn, bMn);
+    split.ctl = plain.ctl;
+    split.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
+    split.stalledCta = stalled != nullptr ? stalled->cta : -1;
+    if (plan.route == MatmulRoute::TWO_SM_SPLIT) return DispatchSplit2(aMn, bMn, ta, tb, split, split.tilesM2 * plan.tilesN, plan.split, stream);
     GemmArgs g;
     memset(&g, 0, sizeof(g));
     g.M = (int)m; g.N = (int)n; g.K = (int)k;
@@ -528,7 +599,13 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, plan.grid, stream);
         return LaunchGemm2SmWide<true, true>(ta, tb, g, plan.grid, stream);
     }
-    if (plan.route == MatmulRoute::TWO_SM) return DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
+    if (plan.route == MatmulRoute::TWO_SM) {
+        if (plan.restTiles > 0) g.tileLimit = split.firstTile = split.tilesM2 * plan.tilesN - plan.restTiles;
+        CHK_RET(DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream));
+        if (plan.restTiles == 0) return HCCL_SUCCESS;
+        split.rest = 1;
+        return DispatchSplit2(aMn, bMn, ta, tb, split, plan.restTiles, plan.restSplit, stream);
+    }
     if (plan.bn == 128) return DispatchLayout<128, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
     return DispatchLayout<256, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
 }

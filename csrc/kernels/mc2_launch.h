@@ -24,7 +24,7 @@ constexpr int kMc2AgBlocks = 8 * 512;   // arrival counters of the push-form All
 constexpr int kMc2CtlWords = 16 + 8 * 512;
 
 // How a plain matmul runs, from its sizes, the number of SMs and the switches of the environment.
-enum class MatmulRoute { SPLIT, ONE_SM, TWO_SM, WIDE };
+enum class MatmulRoute { SPLIT, ONE_SM, TWO_SM, WIDE, TWO_SM_SPLIT };
 struct MatmulSwitches {
     bool twoSm = true;                  // HCCL_MC2_2SM
     int wide = -1;                      // HCCL_MC2_WIDE: 0 never, 1 wherever one full round runs, -1 by the rule
@@ -33,8 +33,9 @@ struct MatmulSwitches {
 struct MatmulPlan {
     MatmulRoute route = MatmulRoute::ONE_SM;
     int bn = 0, tilesM = 0, tilesN = 0, grid = 0;
-    int bt = 0, split = 0;              // SPLIT: tokens per tile, CTAs per tile
+    int bt = 0, split = 0;              // SPLIT: tokens per tile, CTAs per tile; TWO_SM_SPLIT: CTA pairs per tile
     int wide = 0, singles = 0;          // WIDE: wide items, single ones
+    int restTiles = 0, restSplit = 0;   // TWO_SM: last tiles that a split launch computes, CTA pairs per tile of it
     int rasterGroup = 0, l2HintA = 0, l2HintB = 0;
 };
 MatmulSwitches MatmulSwitchesOfEnv();

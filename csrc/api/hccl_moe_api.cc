@@ -3,6 +3,7 @@
 #include <mutex>
 #include "../core/comm.h"
 #include "../core/log.h"
+#include "../core/per_device.h"
 #include "../kernels/moe_launch.h"
 #include "hccl/hccl_moe.h"
 
@@ -118,7 +119,9 @@ HcclResult HcclMoeCombine(HcclComm comm, const void* y, const float* topkWeight,
     for (int q = 0; q < c->nRanks; ++q) a.y[q] = (const __nv_bfloat16*)py[q];
     a.topkWeight = topkWeight; a.slotMap = slotMap; a.out = (__nv_bfloat16*)out;
     a.nTokens = (int)cfg->nTokens; a.hidden = (int)cfg->hidden; a.topk = (int)cfg->topk; a.capacity = cfg->capacity;
-    return LaunchMoeCombine(c->Target((cudaStream_t)stream), a, MoeBlocks(c, cfg->nTokens));
+    int nb = MoeBlocks(c, cfg->nTokens);
+    if (c->emulated()) nb = std::min(nb, std::max(1, SmCount() / c->nRanks));      // one block per SM (its ring), all ranks' in one grid
+    return LaunchMoeCombine(c->Target((cudaStream_t)stream), a, nb);
 }
 
 }  // extern "C"

@@ -452,14 +452,14 @@ void EmuGroup::Release(CommImpl*)
 }
 
 HcclResult EmuGroup::Post(int rank, const void* args, size_t argBytes, int nBlocks, int threads, const void* kernel,
-                          cudaStream_t stream)
+                          cudaStream_t stream, size_t smem)
 {
     std::lock_guard<std::mutex> lk(mu_);
     if (rank < 0 || rank >= nRanks_) return HCCL_E_INTERNAL;
     // One FIFO per rank: a rank may run ahead (an operator that needs several loops posts several launches before
     // the next rank is called); a launch is issued whenever every rank has an entry at the head of its queue.
     PendingPost post;
-    post.kernel = kernel; post.nBlocks = nBlocks; post.threads = threads;
+    post.kernel = kernel; post.nBlocks = nBlocks; post.threads = threads; post.smem = smem;
     post.args.assign((const char*)args, (const char*)args + argBytes);
     queues_[(size_t)rank].push_back(std::move(post));
     for (;;) {
@@ -486,10 +486,11 @@ HcclResult EmuGroup::Post(int rank, const void* args, size_t argBytes, int nBloc
         for (int r = 0; r < nRanks_; ++r) memcpy(launchArgs_.data() + (size_t)r * ab, queues_[(size_t)r].front().args.data(), ab);
         const void* fn = first.kernel;
         const int th = first.threads;
+        const size_t shared = first.smem;
         for (auto& q : queues_) q.pop_front();
         const DevComm* dc = dComms_;
         void* kargs[3] = {(void*)&dc, (void*)launchArgs_.data(), (void*)&nb};
-        cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)(nb * nRanks_)), dim3((unsigned)th), kargs, 0, stream);
+        cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)(nb * nRanks_)), dim3((unsigned)th), kargs, shared, stream);
         if (e != cudaSuccess) { HCCL_ERROR("cooperative launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     }
 }

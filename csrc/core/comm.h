@@ -146,7 +146,7 @@ public:
     static HcclResult Create(int nRanks, const HcclCommConfig* cfg, std::vector<CommImpl*>* comms);
     ~EmuGroup() override;
     HcclResult Post(int rank, const void* args, size_t argBytes, int nBlocks, int threads, const void* emuKernel,
-                    cudaStream_t stream) override;
+                    cudaStream_t stream, size_t smem) override;
     HcclResult MemAlloc(int rank, uint64_t size, SymSegment* seg);   // R matching calls -> one group allocation
     void Release(CommImpl* c);
     int nRanks() const { return nRanks_; }
@@ -163,7 +163,7 @@ private:
     DevComm* dComms_ = nullptr;            // device array [nRanks]
     std::vector<char> launchArgs_;         // the ranks' arguments side by side (EmuArgs), copied by the launch itself
     // launches posted by individual ranks and not yet issued
-    struct PendingPost { const void* kernel; int nBlocks, threads; std::vector<char> args; };
+    struct PendingPost { const void* kernel; int nBlocks, threads; size_t smem; std::vector<char> args; };
     std::vector<std::deque<PendingPost>> queues_;
     std::vector<DevComm> hostComms_;
     // pending group allocation

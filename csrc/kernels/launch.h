@@ -18,7 +18,7 @@ class EmuLauncher {
 public:
     virtual ~EmuLauncher() = default;
     virtual HcclResult Post(int rank, const void* args, size_t argBytes, int nBlocks, int threads,
-                            const void* emuKernel, cudaStream_t stream) = 0;
+                            const void* emuKernel, cudaStream_t stream, size_t smem = 0) = 0;
 };
 
 struct LaunchTarget {

@@ -18,6 +18,7 @@
 #include "launch.h"
 #include "moe_launch.h"
 #include "../core/log.h"
+#include "../core/per_device.h"
 
 namespace hccl {
 
@@ -193,26 +194,34 @@ struct DispatchBody {
 };
 
 // ------------------------------------------------------------------ combine
-// A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: up to kCombinePieces pieces (32 vectors of 16
-// bytes) of one token's row, fewer while that gives idle warps something to load.  A lane requests up to COPIES loads per
-// piece, UNROLL pieces at a time, before it uses the first: eight loads for every topk, which fit the 128 registers of a
-// thread (sixteen did not, and spilled).  Lane k keeps the k-th copy's address and weight and hands them round by shuffle.
-// Measured against a block per token, 8 emulated ranks, rows of 7168, top-8: 256 tokens (264 MB, the expert rows still being
-// written back) 91 -> 82 us, 64 55 -> 47, 8 45 -> 39, 1 15.6 -> 15.0; rows of 4096, top-2: 256 47 -> 26, 1 12.7 -> 13.0.
-constexpr int kCombinePieces = 4;
+// A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: pieces (32 vectors of 16 bytes) of one token's row,
+// whole rows where there are tokens enough, else as many parts as give every warp something to load.  Every thread owns a ring
+// of kCombineRing vectors in shared memory that asynchronous copies fill, 3 pieces of 8 copies (or 6 of 4, 12 of 2) ahead of
+// the arithmetic; it reads what it copied itself, so there is no hand-over.  The ring keeps up to 192 KiB per SM requested all
+// the time, where loads into registers (8 a thread: sixteen spilled) had 64 KiB, and nothing between a piece's sum and the
+// next piece's loads.  Lane k keeps the k-th copy's address and weight and hands them round by shuffle.
+// Measured against loads into registers, 8 emulated ranks, rows of 7168, top-8: 256 tokens (264 MB, the expert rows still being
+// written back) 83.6 -> 73.5 us, 64 50.4 -> 34.1, 8 41.9 -> 29.2, 1 16.4 -> 15.9; rows of 4096, top-2: 256 29.6 -> 28.4, 1 14.9 -> 14.0.
+constexpr int kCombineRing = 24;                                    // vectors per thread
+constexpr size_t kCombineSmem = (size_t)kCombineRing * kMoeThreads * 16;
 struct CombineBody {
     using Args = MoeCombineArgs;
     static constexpr int kThreads = kMoeThreads;
-    template <int COPIES, int UNROLL>
+    template <int COPIES>
     __device__ static void Tokens(const Args& a, int b, int nb)
     {
+        extern __shared__ __align__(16) uint8_t s_ring[];
+        constexpr int D = kCombineRing / COPIES;
         const int H = a.hidden, vecPerRow = H / 8, nPieces = (vecPerRow + 31) / 32;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t stride = (uint32_t)nb * kMoeWarps, all = (uint32_t)a.nTokens * nPieces;      // rows fit the GPU: far below 2^32
-        const int perItem = (int)min((all + stride - 1) / stride, (uint32_t)kCombinePieces);
-        const uint32_t parts = perItem > 0 ? (nPieces + perItem - 1) / perItem : 0, items = (uint32_t)a.nTokens * parts;
+        const uint32_t share = min((all + stride - 1) / stride, (uint32_t)nPieces);                 // pieces for every warp
+        const uint32_t parts = share > 0 ? ((uint32_t)nPieces + share - 1) / share : 0, items = (uint32_t)a.nTokens * parts;
+        const int perItem = parts > 0 ? (int)((nPieces + parts - 1) / parts) : 0;
+        const uint8_t* mine = s_ring + threadIdx.x * 16;            // slot s of this thread: s * kMoeThreads vectors further
+        const uint32_t mineAddr = (uint32_t)__cvta_generic_to_shared(mine);
         for (uint32_t it = b + warp * nb; it < items; it += stride) {
-            const int t = (int)(it / parts), first = (int)(it - t * parts) * perItem;
+            const int t = (int)(it / parts), first = (int)(it - t * parts) * perItem, n = min(perItem, nPieces - first);
             float wk = 0.f;
             unsigned long long srcK = 0;                            // 0: the copy was dropped
             if (lane < a.topk) {
@@ -222,43 +231,45 @@ struct CombineBody {
                     srcK = reinterpret_cast<unsigned long long>(a.y[sm >> 32] + (size_t)(uint32_t)sm * H);
                 }
             }
-            const int end = min((first + perItem) * 32, vecPerRow);
-            for (int v0 = first * 32 + lane; v0 - lane < end; v0 += 32 * UNROLL) {
-                uint4 raw[UNROLL][COPIES];
+            const uint32_t have = __ballot_sync(0xffffffffu, srcK != 0);
+            auto fetch = [&](int j) {                               // piece j of the item -> ring slots (j % D) * COPIES ..
+                const int v = (first + j) * 32 + lane;
 #pragma unroll
                 for (int k = 0; k < COPIES; ++k) {
                     const uint4* src = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, srcK, k));
-#pragma unroll
-                    for (int u = 0; u < UNROLL; ++u) {
-                        raw[u][k] = make_uint4(0, 0, 0, 0);
-                        if (src != nullptr && v0 + u * 32 < end) raw[u][k] = src[v0 + u * 32];
-                    }
+                    if (j < n && src != nullptr && v < vecPerRow)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mineAddr + (uint32_t)((j % D) * COPIES + k) * kMoeThreads * 16), "l"(src + v) : "memory");
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            for (int j = 0; j < D - 1; ++j) fetch(j);
+            for (int j = 0; j < n; ++j) {
+                fetch(j + D - 1);                                   // into the slots of piece j - 1, which is summed
+                asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+                const int v = (first + j) * 32 + lane;
+                float acc[8];
 #pragma unroll
-                for (int u = 0; u < UNROLL; ++u) {
-                    float acc[8];
+                for (int e = 0; e < 8; ++e) acc[e] = 0.f;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+                for (int k = 0; k < COPIES; ++k) {
+                    const float w = __shfl_sync(0xffffffffu, wk, k);
+                    if (have >> k & 1u) {
+                        const uint4 raw = *reinterpret_cast<const uint4*>(mine + (size_t)((j % D) * COPIES + k) * kMoeThreads * 16);
+                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-                    for (int k = 0; k < COPIES; ++k) {
-                        const float w = __shfl_sync(0xffffffffu, wk, k);
-                        if (k < a.topk) {
-                            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[u][k]);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float2 f = __bfloat1622float2(h[j]);
-                                acc[2 * j] += w * f.x;
-                                acc[2 * j + 1] += w * f.y;
-                            }
+                        for (int e = 0; e < 4; ++e) {
+                            const float2 f = __bfloat1622float2(h[e]);
+                            acc[2 * e] += w * f.x;
+                            acc[2 * e + 1] += w * f.y;
                         }
                     }
-                    if (v0 + u * 32 < end) {
-                        uint4 o;
-                        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+                }
+                if (v < vecPerRow) {
+                    uint4 o;
+                    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                        reinterpret_cast<uint4*>(a.out + (size_t)t * H)[v0 + u * 32] = o;
-                    }
+                    for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1]);
+                    reinterpret_cast<uint4*>(a.out + (size_t)t * H)[v] = o;
                 }
             }
         }
@@ -268,9 +279,9 @@ struct CombineBody {
         OpHead(c, b);
         const uint64_t e0 = LoadEpoch(c, b);
         if (RankBarrier(c, b, 0, e0 + 1, K_MOE_COMBINE)) {          // the peers' expert outputs are final
-            if (a.topk > 4) Tokens<8, 1>(a, b, nb);
-            else if (a.topk > 2) Tokens<4, 2>(a, b, nb);
-            else Tokens<2, 4>(a, b, nb);
+            if (a.topk > 4) Tokens<8>(a, b, nb);
+            else if (a.topk > 2) Tokens<4>(a, b, nb);
+            else Tokens<2>(a, b, nb);
         }
         RankBarrier(c, b, 0, e0 + 2, K_MOE_COMBINE);                 // nobody overwrites its outputs while a peer still reads
         StoreEpoch(c, b, e0 + 2);
@@ -280,11 +291,18 @@ struct CombineBody {
 static_assert(kMoeMaxTopk == 8, "CombineBody picks its copies by topk");
 
 template <class Body>
-HcclResult LaunchMoe(const LaunchTarget& t, const typename Body::Args& a, int nBlocks)
+HcclResult LaunchMoe(const LaunchTarget& t, const typename Body::Args& a, int nBlocks, size_t smem)
 {
+    static OncePerDevice allowed;
+    if (smem > 0)
+        CHK_RET(allowed([&]() -> HcclResult {
+            CHK_CUDA(cudaFuncSetAttribute(CollKernel<Body>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CHK_CUDA(cudaFuncSetAttribute(CollKernelEmu<Body>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            return HCCL_SUCCESS;
+        }));
     if (t.emu != nullptr)
-        return t.emu->Post(t.emuRank, &a, sizeof(a), nBlocks, Body::kThreads, reinterpret_cast<const void*>(&CollKernelEmu<Body>), t.stream);
-    CollKernel<Body><<<nBlocks, Body::kThreads, 0, t.stream>>>(*t.dev, a);
+        return t.emu->Post(t.emuRank, &a, sizeof(a), nBlocks, Body::kThreads, reinterpret_cast<const void*>(&CollKernelEmu<Body>), t.stream, smem);
+    CollKernel<Body><<<nBlocks, Body::kThreads, smem, t.stream>>>(*t.dev, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
@@ -303,8 +321,8 @@ HcclResult LaunchMoeCount(const int32_t* topkIdx, int nPairs, int nExperts, uint
     MoeCountKernel<<<blocks, 256, 0, stream>>>(topkIdx, nPairs, nExperts, counts, pos);
     return cudaGetLastError() == cudaSuccess ? HCCL_SUCCESS : HCCL_E_RUNTIME;
 }
-HcclResult LaunchMoeDispatch(const LaunchTarget& t, const MoeDispatchArgs& a, int nBlocks) { return LaunchMoe<DispatchBody>(t, a, nBlocks); }
-HcclResult LaunchMoeCombine(const LaunchTarget& t, const MoeCombineArgs& a, int nBlocks) { return LaunchMoe<CombineBody>(t, a, nBlocks); }
+HcclResult LaunchMoeDispatch(const LaunchTarget& t, const MoeDispatchArgs& a, int nBlocks) { return LaunchMoe<DispatchBody>(t, a, nBlocks, 0); }
+HcclResult LaunchMoeCombine(const LaunchTarget& t, const MoeCombineArgs& a, int nBlocks) { return LaunchMoe<CombineBody>(t, a, nBlocks, kCombineSmem); }
 
 }  // namespace hccl
 

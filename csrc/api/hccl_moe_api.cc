@@ -95,7 +95,8 @@ HcclResult HcclMoeDispatch(HcclComm comm, const void* x, const int32_t* topkIdx,
     }
     a.x = (const __nv_bfloat16*)x; a.topkIdx = topkIdx; a.counts = st->counts; a.pos = st->pos; a.slotMap = slotMap; a.recvOffsets = recvOffsets;
     a.nTokens = (int)cfg->nTokens; a.hidden = (int)cfg->hidden; a.topk = (int)cfg->topk; a.nExperts = (int)cfg->nExperts; a.capacity = cfg->capacity;
-    CHK_RET(LaunchMoeCount(topkIdx, (int)nPairs, (int)cfg->nExperts, st->counts, st->pos, (cudaStream_t)stream));
+    if (nPairs > (size_t)kMoeCountInDispatch) CHK_RET(LaunchMoeCount(topkIdx, (int)nPairs, (int)cfg->nExperts, st->counts, st->pos, (cudaStream_t)stream));
+    else a.counts = a.pos = nullptr;                 // every block of the dispatch kernel counts for itself
     // every rank launches the same grid: sized by a value all ranks share (the configured token count must match)
     return LaunchMoeDispatch(c->Target((cudaStream_t)stream), a, MoeBlocks(c, cfg->nTokens));
 }

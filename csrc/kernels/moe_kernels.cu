@@ -29,8 +29,9 @@ constexpr int kMoeWarps = kMoeThreads / 32;
 
 // ------------------------------------------------------------------ count + local positions
 // counts[e] = number of (token, k) pairs routed to global expert e; pos[t * K + k] = rank of the pair among this
-// rank's pairs for the same expert.  Up to kMoeCountOneBlock pairs (a decode step, a short prompt) one block counts in
-// shared memory and writes every count; more pairs are spread over blocks that share cleared global counters.
+// rank's pairs for the same expert.  Up to kMoeCountInDispatch pairs (a decode step) the dispatch kernel does this itself
+// (CountPairs); then up to kMoeCountOneBlock pairs (a short prompt) one block counts in shared memory and writes every count;
+// more pairs are spread over blocks that share cleared global counters.
 constexpr int kMoeCountOneBlock = 16384;
 __global__ void __launch_bounds__(1024) MoeCountOneBlockKernel(const int32_t* __restrict__ topkIdx, int nPairs, int nExperts, uint32_t* __restrict__ counts,
                                                                uint32_t* __restrict__ pos)
@@ -55,6 +56,46 @@ __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, 
     }
 }
 
+// The same inside one block for up to kMoeCountInDispatch pairs, in an order that depends on the pairs alone, so that every
+// block of a launch counts for itself and all agree: a warp takes a run of consecutive pairs, 32 at a time (lanes with the
+// same expert find each other by match.any), and a scan over the warps' counters gives each run its start.  It saves the
+// counting launch in front (2.1 .. 2.9 us and the boundary between the two) for 1 .. 5 us of the dispatch kernel: eight emulated
+// ranks, whose counting launches run one after the other, take 1149 -> 1120 us for a whole layer of 256 tokens.
+struct CountScratch {
+    uint16_t before[kMoeWarps][kMoeMaxExperts];       // pairs of an expert in a warp's run, then in the runs before it
+    uint16_t pos[kMoeCountInDispatch];                // position of a pair among the pairs of its expert in its warp's run
+    uint32_t count[kMoeMaxExperts];
+};
+__device__ __forceinline__ int CountRun(int nPairs) { return ((nPairs + kMoeWarps - 1) / kMoeWarps + 31) / 32 * 32; }
+__device__ __forceinline__ void CountPairs(const int32_t* __restrict__ topkIdx, int nPairs, int nExperts, CountScratch& s)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, run = CountRun(nPairs);
+    for (int e = lane; e < nExperts; e += 32) s.before[warp][e] = 0;
+    __syncwarp();
+    for (int i0 = warp * run; i0 < min((warp + 1) * run, nPairs); i0 += 32) {
+        const int i = i0 + lane, e = i < nPairs ? topkIdx[i] : -1;
+        const bool ok = e >= 0 && e < nExperts;
+        const uint32_t same = __match_any_sync(0xffffffffu, ok ? e : -1), below = same & ((1u << lane) - 1u);
+        const uint16_t start = ok ? s.before[warp][e] : 0;
+        __syncwarp();
+        if (ok && below == 0) s.before[warp][e] = (uint16_t)(start + __popc(same));
+        if (ok) s.pos[i] = (uint16_t)(start + __popc(below));
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nExperts; e += kMoeThreads) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < kMoeWarps; ++w) {
+            const uint16_t n = s.before[w][e];
+            s.before[w][e] = (uint16_t)sum;
+            sum += n;
+        }
+        s.count[e] = sum;
+    }
+    __syncthreads();
+}
+
 // ------------------------------------------------------------------ dispatch
 // Bound by the bytes written (topk fp8 copies of every row, over NVLink to the peers).  A WARP owns a token, or a part of
 // one while there are warps for it: a lane takes 16 elements of the row (two 16-byte loads), eight lanes share a
@@ -69,7 +110,11 @@ struct DispatchBody {
     {
         __shared__ uint32_t s_cnt[kMaxDevRanks * kMoeMaxExperts];   // [src][expert]
         __shared__ uint32_t s_base[kMoeMaxExperts];                 // slot base in the destination rank for (expert, src = me)
+        __shared__ CountScratch s_pairs;
         OpHead(c, b);
+        const bool counted = a.counts != nullptr;
+        if (!counted) CountPairs(a.topkIdx, a.nTokens * a.topk, a.nExperts, s_pairs);
+        const int run = CountRun(a.nTokens * a.topk);
         const int p = c.nRanks, me = c.rank;
         const int E = a.nExperts, perRank = E / p;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -77,7 +122,7 @@ struct DispatchBody {
         // phase 0: publish my counts in every rank's table, row `me` (each block row owns a private copy of the table)
         for (int i = threadIdx.x; i < p * E; i += kThreads) {
             const int q = i / E, e = i - q * E;
-            a.table[q][((size_t)b * kMaxDevRanks + me) * kMoeMaxExperts + e] = a.counts[e];
+            a.table[q][((size_t)b * kMaxDevRanks + me) * kMoeMaxExperts + e] = counted ? a.counts[e] : s_pairs.count[e];
         }
         bool ok = RankBarrier(c, b, 0, e0 + 1, K_MOE_DISPATCH);
         // phase 1: slot bases.  Destination rank d = e / perRank holds its experts one after the other; inside an expert the
@@ -133,7 +178,7 @@ struct DispatchBody {
             if (lane < a.topk) {
                 const int pair = t * a.topk + lane;
                 const int e = a.topkIdx[pair];
-                if (e >= 0 && e < E) sm = ((uint64_t)(e / perRank) << 32) | (uint64_t)(s_base[e] + a.pos[pair]);
+                if (e >= 0 && e < E) sm = ((uint64_t)(e / perRank) << 32) | (uint64_t)(s_base[e] + (counted ? a.pos[pair] : (uint32_t)s_pairs.before[pair / run][e] + s_pairs.pos[pair]));
                 if (part == 0) a.slotMap[pair] = sm;
                 if (sm != ~0ull && (uint32_t)sm >= a.capacity) sm = ~0ull;      // overflow: reported by the receiver's bounds check above
                 if (sm != ~0ull && part == 0) a.recvSrc[sm >> 32][(uint32_t)sm] = ((uint64_t)me << 32) | (uint32_t)pair;

@@ -10,13 +10,14 @@ namespace hccl {
 
 constexpr int kMoeMaxExperts = 512;
 constexpr int kMoeMaxTopk = 8;
+constexpr int kMoeCountInDispatch = 4096;   // pairs up to which the dispatch kernel counts them itself
 constexpr size_t kMoeTableBytes = (size_t)kMaxBlocks * kMaxDevRanks * kMoeMaxExperts * sizeof(uint32_t);
 
 struct MoeDispatchArgs {
     const __nv_bfloat16* x;            // [nTokens, hidden]
     const int32_t* topkIdx;            // [nTokens, topk] global expert ids (negative = dropped)
-    const uint32_t* counts;            // [nExperts] pairs per expert on this rank
-    const uint32_t* pos;               // [nTokens * topk] position of the pair among this rank's pairs of that expert
+    const uint32_t* counts;            // [nExperts] pairs per expert on this rank; null: the kernel counts
+    const uint32_t* pos;               // [nTokens * topk] position of the pair among this rank's pairs of that expert; null likewise
     uint64_t* slotMap;                 // [nTokens * topk] out: (destination rank << 32) | slot
     uint32_t* recvOffsets;             // [nExperts / nRanks + 1] out: where each local expert starts in the receive buffer
     uint32_t* table[kMaxDevRanks];     // count exchange table of every rank (symmetric)

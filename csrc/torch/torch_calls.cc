@@ -1,0 +1,298 @@
+// Calls of the C API with torch tensors, for hccl_b200/_calls.py: checks, output allocation, the current stream and the call
+// itself without Python or ctypes objects in between.  A decode step's operators take 4 .. 10 us on the device; with Python-level
+// allocations and ctypes a call of one took 10 .. 18 us of the host.
+//
+// Every function takes only what is plain: dense CUDA tensors that no transform, subclass, dispatch mode, forward-mode
+// gradient or tracer looks at, and that no gradient is recorded for.  For anything else it returns None and the caller goes
+// the general way (torch.autograd.Function, ctypes), which also words the errors.  An int is the HcclResult of a failed call.
+//
+// The functions of the C API come as addresses (`bind`), so that this module and the ctypes binding always use the same library.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <cstdint>
+
+namespace {
+
+using at::Tensor;
+
+struct Api {
+    int (*addRmsNormFwd)(const void*, const void*, const void*, void*, void*, void*, uint64_t, uint32_t, float, void*);
+    uint32_t (*rmsNormBwdPartials)(uint64_t);
+    int (*rmsNormBwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, uint64_t, uint32_t, void*);
+    int (*swigluFwd)(const void*, void*, uint64_t, uint32_t, void*);
+    int (*swigluBwd)(const void*, const void*, void*, uint64_t, uint32_t, void*);
+    int (*rope)(const void*, uint64_t, void*, uint64_t, const void*, const void*, uint64_t, uint32_t, uint32_t, int, void*);
+    int (*matmul)(const void*, const void*, void*, uint64_t, uint64_t, uint64_t, int, int, void*);
+    int (*expertOffsets)(const int32_t*, uint64_t, uint32_t, uint32_t*, void*);
+    int (*allReduce)(const void*, void*, uint64_t, int, int, void*, void*);
+    int (*reduceScatter)(const void*, void*, uint64_t, int, int, void*, void*);
+    int (*allGather)(const void*, void*, uint64_t, int, void*, void*);
+    int (*alltoAll)(const void*, uint64_t, int, const void*, uint64_t, int, void*, void*);
+};
+Api api;
+struct Slot { const char* name; void** at; };
+const Slot kSlots[] = {
+    {"HcclFusedAddRmsNormFwd", (void**)&api.addRmsNormFwd}, {"HcclFusedRmsNormBwdPartials", (void**)&api.rmsNormBwdPartials},
+    {"HcclFusedRmsNormBwd", (void**)&api.rmsNormBwd},       {"HcclFusedSwigluFwd", (void**)&api.swigluFwd},
+    {"HcclFusedSwigluBwd", (void**)&api.swigluBwd},         {"HcclFusedRope", (void**)&api.rope},
+    {"HcclMc2Matmul", (void**)&api.matmul},                 {"HcclMoeExpertOffsets", (void**)&api.expertOffsets},
+    {"HcclAllReduce", (void**)&api.allReduce},              {"HcclReduceScatter", (void**)&api.reduceScatter},
+    {"HcclAllGather", (void**)&api.allGather},              {"HcclAlltoAll", (void**)&api.alltoAll},
+};
+
+// A call that nothing but its own arithmetic is asked of: no tracer, no dispatch mode, no functional transform around it.
+bool PlainCall()
+{
+    return !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+           !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+// A dense CUDA tensor that nothing looks at and nothing is recorded for.
+bool Plain(const Tensor& t)
+{
+    return t.is_cuda() && t.layout() == at::kStrided && !(t.requires_grad() && c10::GradMode::is_enabled()) && !at::isTensorSubclassLike(t) &&
+           !t._fw_grad(0).defined();
+}
+const Tensor* Get(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+const Tensor* GetPlain(PyObject* o)
+{
+    const Tensor* t = Get(o);
+    return t != nullptr && Plain(*t) ? t : nullptr;
+}
+const Tensor* GetPlainBf16(PyObject* o)
+{
+    const Tensor* t = GetPlain(o);
+    return t != nullptr && t->scalar_type() == at::kBFloat16 && t->is_contiguous() ? t : nullptr;
+}
+void* Stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
+void* StreamOf(PyObject* o) { return o == Py_None ? Stream() : PyLong_AsVoidPtr(o); }
+PyObject* None() { Py_RETURN_NONE; }
+PyObject* Wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
+template <class... T> PyObject* WrapAll(T... t)
+{
+    PyObject* all[] = {Wrap(std::move(t))...};
+    PyObject* out = PyTuple_New(sizeof...(T));
+    for (size_t i = 0; i < sizeof...(T); ++i) PyTuple_SET_ITEM(out, i, all[i]);
+    return out;
+}
+// Errors of torch (out of memory among them) become the Python exceptions that torch's own functions raise.
+template <class F> PyObject* Guarded(F f)
+{
+    HANDLE_TH_ERRORS
+    return f();
+    END_HANDLE_TH_ERRORS
+}
+#define HCCL_ARGS(n) \
+    if (nargs != (n)) { PyErr_SetString(PyExc_TypeError, "wrong number of arguments"); return nullptr; }
+
+// (x, delta or None, weight, eps) -> (x_out or x, h, rstd)
+PyObject* AddRmsNorm(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(4)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetPlainBf16(a[0]), *w = GetPlainBf16(a[2]), *delta = a[1] == Py_None ? nullptr : GetPlainBf16(a[1]);
+        if (!x || !w || (a[1] != Py_None && !delta) || !PyFloat_Check(a[3]) || !PlainCall()) return None();
+        if (x->dim() == 0 || x->numel() == 0 || w->numel() != x->size(-1) || (delta && delta->sizes() != x->sizes())) return None();
+        const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
+        if (hidden % 8 != 0 || hidden > 8192) return None();
+        Tensor h = at::empty_like(*x), xOut = delta ? at::empty_like(*x) : *x, rstd = at::empty({(int64_t)rows}, x->options().dtype(at::kFloat));
+        const int r = api.addRmsNormFwd(x->const_data_ptr(), delta ? delta->const_data_ptr() : nullptr, w->const_data_ptr(),
+                                        delta ? xOut.mutable_data_ptr() : nullptr, h.mutable_data_ptr(), rstd.mutable_data_ptr(), rows, (uint32_t)hidden,
+                                        (float)PyFloat_AS_DOUBLE(a[3]), Stream());
+        if (r != 0) return PyLong_FromLong(r);
+        return WrapAll(std::move(xOut), std::move(h), std::move(rstd));
+    });
+}
+
+// (dh, x_out, weight, rstd, extra or None) -> (dx, dw)
+PyObject* RmsNormBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(5)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *dh = GetPlainBf16(a[0]), *x = GetPlainBf16(a[1]), *w = GetPlainBf16(a[2]), *rstd = GetPlain(a[3]);
+        const Tensor* extra = a[4] == Py_None ? nullptr : GetPlainBf16(a[4]);
+        if (!dh || !x || !w || !rstd || (a[4] != Py_None && !extra) || rstd->scalar_type() != at::kFloat || !rstd->is_contiguous() || !PlainCall()) return None();
+        if (x->numel() == 0 || dh->sizes() != x->sizes() || (extra && extra->sizes() != x->sizes())) return None();
+        const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
+        if (w->numel() != x->size(-1) || (uint64_t)rstd->numel() != rows) return None();
+        Tensor dx = at::empty_like(*x), dw = at::empty_like(*w);
+        Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), (int64_t)hidden}, x->options().dtype(at::kFloat));
+        const int r = api.rmsNormBwd(dh->const_data_ptr(), x->const_data_ptr(), w->const_data_ptr(), rstd->const_data_ptr(),
+                                     extra ? extra->const_data_ptr() : nullptr, dx.mutable_data_ptr(), partial.mutable_data_ptr(), dw.mutable_data_ptr(),
+                                     rows, (uint32_t)hidden, Stream());
+        if (r != 0) return PyLong_FromLong(r);
+        return WrapAll(std::move(dx), std::move(dw));
+    });
+}
+
+// (gate_up) -> out
+PyObject* SwigluFwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(1)
+    return Guarded([&]() -> PyObject* {
+        const Tensor* x = GetPlainBf16(a[0]);
+        if (!x || !PlainCall() || x->dim() == 0 || x->numel() == 0 || x->size(-1) % 16 != 0) return None();
+        const int64_t f = x->size(-1) / 2;
+        auto sizes = x->sizes().vec();
+        sizes.back() = f;
+        Tensor out = at::empty(sizes, x->options());
+        const int r = api.swigluFwd(x->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+// (gate_up, dout) -> dgate_up
+PyObject* SwigluBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(2)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetPlainBf16(a[0]), *dout = GetPlainBf16(a[1]);
+        if (!x || !dout || !PlainCall() || x->numel() == 0 || x->size(-1) % 16 != 0 || dout->numel() * 2 != x->numel()) return None();
+        const int64_t f = x->size(-1) / 2;
+        Tensor dx = at::empty_like(*x);
+        const int r = api.swigluBwd(x->const_data_ptr(), dout->const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(dx));
+    });
+}
+
+// (x [S, heads, D], cos, sin, backward) -> rotated x; rows of x may lie further apart than heads * D
+PyObject* Rope(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(4)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetPlain(a[0]), *c = GetPlain(a[1]), *s = GetPlain(a[2]);
+        if (!x || !c || !s || !PlainCall() || x->scalar_type() != at::kBFloat16 || x->dim() != 3 || x->numel() == 0) return None();
+        const int64_t rows = x->size(0), heads = x->size(1), d = x->size(2);
+        if (d % 16 != 0 || x->stride(2) != 1 || x->stride(1) != d || x->stride(0) < 0 || x->stride(0) % 8 != 0 || (uintptr_t)x->const_data_ptr() % 16 != 0)
+            return None();
+        for (const Tensor* t : {c, s})
+            if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() < rows * (d / 2)) return None();
+        const int backward = PyObject_IsTrue(a[3]);
+        Tensor out = at::empty({rows, heads, d}, x->options());
+        const int r = api.rope(x->const_data_ptr(), (uint64_t)x->stride(0), out.mutable_data_ptr(), (uint64_t)(heads * d), c->const_data_ptr(),
+                               s->const_data_ptr(), (uint64_t)rows, (uint32_t)heads, (uint32_t)d, backward, Stream());
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+// (a, b, trans_a, trans_b, out or None, stream or None) -> out
+PyObject* Matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs)
+{
+    HCCL_ARGS(6)
+    return Guarded([&]() -> PyObject* {
+        // operands that record gradients are taken as before: the product itself is not recorded
+        const Tensor *a = Get(args[0]), *b = Get(args[1]), *given = args[4] == Py_None ? nullptr : Get(args[4]);
+        if (!a || !b || (args[4] != Py_None && !given) || !PlainCall()) return None();
+        for (const Tensor* t : {a, b, given})
+            if (t && (!t->is_cuda() || t->layout() != at::kStrided || t->scalar_type() != at::kBFloat16 || t->dim() != 2 || at::isTensorSubclassLike(*t))) return None();
+        if (!a->is_contiguous() || !b->is_contiguous()) return None();
+        const bool ta = PyObject_IsTrue(args[2]), tb = PyObject_IsTrue(args[3]);
+        const int64_t m = a->size(ta ? 1 : 0), k = a->size(ta ? 0 : 1), n = b->size(tb ? 0 : 1);
+        if (b->size(tb ? 1 : 0) != k) return None();
+        void* stream = StreamOf(args[5]);
+        if (stream == nullptr && PyErr_Occurred()) return nullptr;
+        Tensor out = given ? *given : at::empty({m, n}, a->options());
+        const int r = api.matmul(a->const_data_ptr(), b->const_data_ptr(), out.data_ptr(), (uint64_t)m, (uint64_t)n, (uint64_t)k, ta, tb, stream);
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+// (topk_idx, n_experts, stream or None) -> offsets
+PyObject* ExpertOffsets(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(3)
+    return Guarded([&]() -> PyObject* {
+        const Tensor* idx = GetPlain(a[0]);
+        if (!idx || !PlainCall() || idx->scalar_type() != at::kInt || !idx->is_contiguous() || !PyLong_Check(a[1])) return None();
+        const long n = PyLong_AsLong(a[1]);
+        if (n <= 0 || n > 0x7FFFFFFFL) { PyErr_Clear(); return None(); }
+        void* stream = StreamOf(a[2]);
+        if (stream == nullptr && PyErr_Occurred()) return nullptr;
+        Tensor out = at::empty({n + 1}, idx->options());
+        const int r = api.expertOffsets(idx->const_data_ptr<int32_t>(), (uint64_t)idx->numel(), (uint32_t)n, (uint32_t*)out.mutable_data_ptr(), stream);
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+// HcclDataType of a tensor's elements, -1 where the general way has to look
+int TypeOf(const Tensor& t)
+{
+    switch (t.scalar_type()) {
+        case at::kFloat: return 4;
+        case at::kBFloat16: return 11;
+        default: return -1;
+    }
+}
+enum Which { ALL_REDUCE, REDUCE_SCATTER, ALL_GATHER, ALL_TO_ALL };
+// (which, communicator, send, recv, reduction, ranks, stream or None) -> HcclResult
+PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(7)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *send = Get(a[2]), *recv = Get(a[3]);
+        if (!send || !recv || !PlainCall()) return None();
+        for (const Tensor* t : {send, recv})
+            if (!t->is_cuda() || t->layout() != at::kStrided || !t->is_contiguous() || at::isTensorSubclassLike(*t)) return None();
+        const int type = TypeOf(*send), which = (int)PyLong_AsLong(a[0]), op = (int)PyLong_AsLong(a[4]), ranks = (int)PyLong_AsLong(a[5]);
+        void *comm = PyLong_AsVoidPtr(a[1]), *stream = StreamOf(a[6]);
+        if (PyErr_Occurred()) return nullptr;
+        if (type < 0 || TypeOf(*recv) != type || comm == nullptr || ranks < 1) return None();
+        const void* s = send->const_data_ptr();
+        void* r = recv->data_ptr();
+        const uint64_t nSend = (uint64_t)send->numel(), nRecv = (uint64_t)recv->numel();
+        int code = 0;
+        Py_BEGIN_ALLOW_THREADS          // as ctypes does: a first call may wait for the other ranks' threads
+        switch (which) {
+            case ALL_REDUCE: code = api.allReduce(s, r, nSend, type, op, comm, stream); break;
+            case REDUCE_SCATTER: code = api.reduceScatter(s, r, nRecv, type, op, comm, stream); break;
+            case ALL_GATHER: code = api.allGather(s, r, nSend, type, comm, stream); break;
+            default: code = api.alltoAll(s, nSend / (uint64_t)ranks, type, r, nSend / (uint64_t)ranks, type, comm, stream); break;
+        }
+        Py_END_ALLOW_THREADS
+        return PyLong_FromLong(code);
+    });
+}
+
+PyObject* Bind(PyObject*, PyObject* addresses)
+{
+    for (const Slot& s : kSlots) {
+        PyObject* v = PyDict_GetItemString(addresses, s.name);
+        void* p = v ? PyLong_AsVoidPtr(v) : nullptr;
+        if (p == nullptr) {
+            if (!PyErr_Occurred()) PyErr_Format(PyExc_KeyError, "no address of %s", s.name);
+            return nullptr;
+        }
+        *s.at = p;
+    }
+    Py_RETURN_NONE;
+}
+PyObject* Names(PyObject*, PyObject*)
+{
+    PyObject* out = PyList_New(0);
+    for (const Slot& s : kSlots) {
+        PyObject* n = PyUnicode_FromString(s.name);
+        PyList_Append(out, n);
+        Py_DECREF(n);
+    }
+    return out;
+}
+
+#define HCCL_FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr
+PyMethodDef methods[] = {
+    {"bind", Bind, METH_O, nullptr},           {"names", Names, METH_NOARGS, nullptr},      {"add_rms_norm", HCCL_FAST(AddRmsNorm)},
+    {"rms_norm_bwd", HCCL_FAST(RmsNormBwd)},   {"swiglu_fwd", HCCL_FAST(SwigluFwd)},        {"swiglu_bwd", HCCL_FAST(SwigluBwd)},
+    {"rope", HCCL_FAST(Rope)},                 {"matmul", HCCL_FAST(Matmul)},               {"expert_offsets", HCCL_FAST(ExpertOffsets)},
+    {"collective", HCCL_FAST(Collective)},     {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "hccl_b200_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_hccl_b200_torch() { return PyModule_Create(&module); }

@@ -9,12 +9,15 @@ header is newer.  Usage: ``python hccl_b200/build.py [--force] [--verbose] [--pt
 bootstrap, host engine, verifier) is compiled with AddressSanitizer; the CUDA objects are shared with the normal
 build.  Load it with ``HCCL_B200_LIB=<path> LD_PRELOAD=$(gcc -print-file-name=libasan.so)`` (the interpreter itself
 is not instrumented, so the runtime has to come first), ``ASAN_OPTIONS=detect_leaks=0``.
+Beside the library goes ``hccl_b200/lib/hccl_b200_torch.so``, a Python module built against torch's headers (where torch is
+installed).
 ``--cov`` builds ``build/lib/libhccl_b200_cov.so`` with ``--coverage``; after running tests against it
 (``HCCL_B200_LIB=<path>``), ``--cov-report`` prints the line coverage of every host source.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.util
 import os
 import subprocess
 import sys
@@ -27,6 +30,9 @@ LIB_DIR = ROOT / "hccl_b200" / "lib"
 LIB = LIB_DIR / "libhccl_b200.so"
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
+
+TORCH_SRC = CSRC / "torch" / "torch_calls.cc"          # a Python module of its own, against torch's headers
+TORCH_LIB = LIB_DIR / "hccl_b200_torch.so"
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -41,7 +47,7 @@ CXX_FLAGS = [
 
 def _sources():
     cu = sorted(CSRC.rglob("*.cu"))
-    cc = sorted(CSRC.rglob("*.cc"))
+    cc = sorted(p for p in CSRC.rglob("*.cc") if p != TORCH_SRC)
     return cu, cc
 
 
@@ -99,7 +105,31 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"linking failed:\n{r.stdout}\n{r.stderr}")
+    if importlib.util.find_spec("torch") is not None:
+        build_torch_calls(force, verbose)
     return LIB
+
+
+def build_torch_calls(force: bool = False, verbose: bool = False) -> Path:
+    """The Python module that makes the C API's calls with torch tensors (csrc/torch/torch_calls.cc).  It gets the C functions'
+    addresses at run time, so it is not linked to the library."""
+    if not force and TORCH_LIB.exists() and TORCH_LIB.stat().st_mtime >= TORCH_SRC.stat().st_mtime:
+        return TORCH_LIB
+    import sysconfig
+
+    import torch
+
+    home = Path(torch.__file__).resolve().parent
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-Wall", "-Wno-unused-function", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{home / 'include'}", f"-I{home / 'include/torch/csrc/api/include'}", f"-I{CUDA_HOME / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+           str(TORCH_SRC), "-o", str(TORCH_LIB), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling {TORCH_SRC.name} failed:\n{r.stdout}\n{r.stderr}")
+    return TORCH_LIB
 
 
 def _build_variant(obj_dir: Path, lib: Path, cxx_extra, link_extra, verbose: bool) -> Path:

@@ -16,6 +16,7 @@ import ctypes
 import torch
 import torch.nn.functional as F
 
+from .. import _calls
 from .._lib import lib
 from ..comm import _check
 
@@ -71,6 +72,13 @@ def rope_reference(x, cos, sin):
 class _AddRmsNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, delta, weight, eps):
+        ctx.has_delta = delta is not None
+        r = _calls.add_rms_norm(x, delta, weight, eps)
+        if r is not None:
+            x_out, h, rstd = _calls.result(r, "HcclFusedAddRmsNormFwd")
+            _count()
+            ctx.save_for_backward(x_out, weight, rstd)
+            return (x_out, h) if ctx.has_delta else h
         rows, hidden = x.numel() // x.shape[-1], x.shape[-1]
         x = x.contiguous()
         h = torch.empty_like(x)
@@ -84,7 +92,6 @@ class _AddRmsNorm(torch.autograd.Function):
                                           rows, hidden, float(eps), _s()), "HcclFusedAddRmsNormFwd")
         _count()
         ctx.save_for_backward(x_out, weight, rstd)
-        ctx.has_delta = delta is not None
         return (x_out, h) if delta is not None else h        # without delta the input itself is the residual stream
 
     @staticmethod
@@ -96,6 +103,11 @@ class _AddRmsNorm(torch.autograd.Function):
             dh = torch.zeros_like(x_out)
         dh = dh.contiguous()
         extra = dx_out.contiguous() if dx_out is not None else None
+        r = _calls.rms_norm_bwd(dh, x_out, weight, rstd, extra)
+        if r is not None:
+            dx, dw = _calls.result(r, "HcclFusedRmsNormBwd")
+            _count(2)
+            return dx, (dx if ctx.has_delta else None), dw, None
         dx = torch.empty_like(x_out)
         dw = torch.empty_like(weight)
         n_part = lib.HcclFusedRmsNormBwdPartials(rows)
@@ -110,6 +122,12 @@ class _Swiglu(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up):
         gate_up = gate_up.contiguous()
+        out = _calls.swiglu_fwd(gate_up)
+        if out is not None:
+            out = _calls.result(out, "HcclFusedSwigluFwd")
+            _count()
+            ctx.save_for_backward(gate_up)
+            return out
         f = gate_up.shape[-1] // 2
         rows = gate_up.numel() // gate_up.shape[-1]
         out = torch.empty(gate_up.shape[:-1] + (f,), device=gate_up.device, dtype=gate_up.dtype)
@@ -121,6 +139,11 @@ class _Swiglu(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         (gate_up,) = ctx.saved_tensors
+        dgu = _calls.swiglu_bwd(gate_up, dout.contiguous())
+        if dgu is not None:
+            dgu = _calls.result(dgu, "HcclFusedSwigluBwd")
+            _count()
+            return dgu
         f = gate_up.shape[-1] // 2
         rows = gate_up.numel() // gate_up.shape[-1]
         dgu = torch.empty_like(gate_up)
@@ -134,6 +157,12 @@ class _Rope(torch.autograd.Function):
     def forward(ctx, x, cos, sin):
         s, nh, d = x.shape
         assert x.stride(2) == 1 and x.stride(1) == d, "rope: heads must be packed inside a row"
+        out = _calls.rope(x, cos, sin, False)
+        if out is not None:
+            out = _calls.result(out, "HcclFusedRope")
+            _count()
+            ctx.save_for_backward(cos, sin)
+            return out
         out = torch.empty((s, nh, d), device=x.device, dtype=x.dtype)
         _check(lib.HcclFusedRope(_p(x), x.stride(0), _p(out), nh * d, _p(cos), _p(sin), s, nh, d, 0, _s()), "HcclFusedRope")
         _count()
@@ -145,6 +174,11 @@ class _Rope(torch.autograd.Function):
         cos, sin = ctx.saved_tensors
         s, nh, d = dout.shape
         dout = dout.contiguous()
+        dx = _calls.rope(dout, cos, sin, True)
+        if dx is not None:
+            dx = _calls.result(dx, "HcclFusedRope")
+            _count()
+            return dx, None, None
         dx = torch.empty_like(dout)
         _check(lib.HcclFusedRope(_p(dout), nh * d, _p(dx), nh * d, _p(cos), _p(sin), s, nh, d, 1, _s()), "HcclFusedRope")
         _count()
@@ -197,6 +231,11 @@ class _RopeQkv(torch.autograd.Function):
 # ----------------------------------------------------------------------------- public functions
 def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
     """``x_out = x + delta`` (``delta`` may be None) and ``h = rms_norm(x_out) * weight`` in one pass; returns both."""
+    r = _calls.add_rms_norm(x, delta, weight, eps) if use_kernels else None
+    if r is not None:                                        # no gradient is recorded: no autograd function either
+        x_out, h, _ = _calls.result(r, "HcclFusedAddRmsNormFwd")
+        _count()
+        return x_out, h
     if use_kernels and _native(x, delta, weight, hidden=x.shape[-1]):
         if delta is None:
             return x, _AddRmsNorm.apply(x, None, weight, eps)
@@ -205,6 +244,11 @@ def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
 
 
 def swiglu(gate_up, use_kernels: bool = True):
+    out = _calls.swiglu_fwd(gate_up) if use_kernels else None
+    if out is not None:
+        out = _calls.result(out, "HcclFusedSwigluFwd")
+        _count()
+        return out
     if use_kernels and _native(gate_up) and (gate_up.shape[-1] // 2) % 8 == 0:
         return _Swiglu.apply(gate_up)
     return swiglu_reference(gate_up)
@@ -217,6 +261,11 @@ def _rope_table(t, x) -> bool:
 
 def rope(x, cos, sin, use_kernels: bool = True):
     """x [S, heads, D] (row stride may exceed heads * D), cos / sin fp32 [S, D / 2]."""
+    out = _calls.rope(x, cos, sin, False) if use_kernels else None
+    if out is not None:
+        out = _calls.result(out, "HcclFusedRope")
+        _count()
+        return out
     if (use_kernels and _native(x) and x.shape[-1] % 16 == 0 and x.stride(2) == 1 and x.stride(1) == x.shape[-1] and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and _rope_table(cos, x) and _rope_table(sin, x)):
         return _Rope.apply(x, cos, sin)

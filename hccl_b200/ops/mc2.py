@@ -10,6 +10,7 @@ import ctypes
 
 import torch
 
+from .. import _calls
 from .._lib import lib
 from ..comm import Communicator, _check
 
@@ -29,6 +30,9 @@ def matmul(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: 
     ``trans_a=False``: ``a`` is ``[M, K]``; ``True``: ``a`` is ``[K, M]``.
     ``trans_b=True``: ``b`` is ``[N, K]`` (a Linear weight); ``False``: ``b`` is ``[K, N]``.
     """
+    r = _calls.matmul(a, b, trans_a, trans_b, out, None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _calls.result(r, "HcclMc2Matmul")
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_contiguous() and b.is_contiguous()
     m, k = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
     n = b.shape[0] if trans_b else b.shape[1]

@@ -13,7 +13,7 @@ import dataclasses
 
 import torch
 
-from .. import _lib
+from .. import _calls, _lib
 from .._lib import lib
 from ..comm import Communicator, _check
 
@@ -69,6 +69,9 @@ def dequantize(x_fp8: torch.Tensor, scales: torch.Tensor) -> torch.Tensor:
 
 def expert_offsets(topk_idx: torch.Tensor, n_experts: int, stream=None) -> torch.Tensor:
     """Row range of every expert when this rank's (token, expert) pairs are grouped by expert: int32 [n_experts + 1]."""
+    r = _calls.expert_offsets(topk_idx, n_experts, None if stream is None else stream.cuda_stream)
+    if r is not None:
+        return _calls.result(r, "HcclMoeExpertOffsets")
     assert topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
     out = torch.empty(n_experts + 1, dtype=torch.int32, device=topk_idx.device)
     s = stream if stream is not None else torch.cuda.current_stream()

@@ -18,6 +18,9 @@ uint32_t HcclFusedRmsNormBwdPartials(uint64_t rows);
 // dx = rstd * (dh * w) - x * rstd^3 * mean(dh * w * x) (+ dxExtra when not NULL), dw = sum_rows dh * x * rstd.
 HcclResult HcclFusedRmsNormBwd(const void* dh, const void* x, const void* w, const void* rstd, const void* dxExtra, void* dx, void* dwPartial,
                                void* dw, uint64_t rows, uint32_t hidden, hcclStream_t stream);
+// The same with dx written to a second buffer as well (dxCopy may be NULL).
+HcclResult HcclFusedRmsNormBwdCopy(const void* dh, const void* x, const void* w, const void* rstd, const void* dxExtra, void* dx, void* dxCopy,
+                                   void* dwPartial, void* dw, uint64_t rows, uint32_t hidden, hcclStream_t stream);
 // gu [rows, 2f] = [gate | up]: out [rows, f] = silu(gate) * up; backward writes dgu [rows, 2f].  f: multiple of 8.
 HcclResult HcclFusedSwigluFwd(const void* gu, void* out, uint64_t rows, uint32_t f, hcclStream_t stream);
 HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint64_t rows, uint32_t f, hcclStream_t stream);

@@ -26,7 +26,7 @@ using at::Tensor;
 struct Api {
     int (*addRmsNormFwd)(const void*, const void*, const void*, void*, void*, void*, uint64_t, uint32_t, float, void*);
     uint32_t (*rmsNormBwdPartials)(uint64_t);
-    int (*rmsNormBwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, uint64_t, uint32_t, void*);
+    int (*rmsNormBwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, uint64_t, uint32_t, void*);
     int (*swigluFwd)(const void*, void*, uint64_t, uint32_t, void*);
     int (*swigluBwd)(const void*, const void*, void*, uint64_t, uint32_t, void*);
     int (*rope)(const void*, uint64_t, void*, uint64_t, const void*, const void*, uint64_t, uint32_t, uint32_t, int, void*);
@@ -41,7 +41,7 @@ Api api;
 struct Slot { const char* name; void** at; };
 const Slot kSlots[] = {
     {"HcclFusedAddRmsNormFwd", (void**)&api.addRmsNormFwd}, {"HcclFusedRmsNormBwdPartials", (void**)&api.rmsNormBwdPartials},
-    {"HcclFusedRmsNormBwd", (void**)&api.rmsNormBwd},       {"HcclFusedSwigluFwd", (void**)&api.swigluFwd},
+    {"HcclFusedRmsNormBwdCopy", (void**)&api.rmsNormBwd},   {"HcclFusedSwigluFwd", (void**)&api.swigluFwd},
     {"HcclFusedSwigluBwd", (void**)&api.swigluBwd},         {"HcclFusedRope", (void**)&api.rope},
     {"HcclMc2Matmul", (void**)&api.matmul},                 {"HcclMoeExpertOffsets", (void**)&api.expertOffsets},
     {"HcclAllReduce", (void**)&api.allReduce},              {"HcclReduceScatter", (void**)&api.reduceScatter},
@@ -111,10 +111,10 @@ PyObject* AddRmsNorm(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     });
 }
 
-// (dh, x_out, weight, rstd, extra or None) -> (dx, dw)
+// (dh, x_out, weight, rstd, extra or None, a second copy of dx) -> (dx, dw, that copy or dx)
 PyObject* RmsNormBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
 {
-    HCCL_ARGS(5)
+    HCCL_ARGS(6)
     return Guarded([&]() -> PyObject* {
         const Tensor *dh = GetPlainBf16(a[0]), *x = GetPlainBf16(a[1]), *w = GetPlainBf16(a[2]), *rstd = GetPlain(a[3]);
         const Tensor* extra = a[4] == Py_None ? nullptr : GetPlainBf16(a[4]);
@@ -122,13 +122,14 @@ PyObject* RmsNormBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         if (x->numel() == 0 || dh->sizes() != x->sizes() || (extra && extra->sizes() != x->sizes())) return None();
         const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
         if (w->numel() != x->size(-1) || (uint64_t)rstd->numel() != rows) return None();
-        Tensor dx = at::empty_like(*x), dw = at::empty_like(*w);
+        const bool twice = PyObject_IsTrue(a[5]);
+        Tensor dx = at::empty_like(*x), dw = at::empty_like(*w), copy = twice ? at::empty_like(*x) : dx;
         Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), (int64_t)hidden}, x->options().dtype(at::kFloat));
         const int r = api.rmsNormBwd(dh->const_data_ptr(), x->const_data_ptr(), w->const_data_ptr(), rstd->const_data_ptr(),
-                                     extra ? extra->const_data_ptr() : nullptr, dx.mutable_data_ptr(), partial.mutable_data_ptr(), dw.mutable_data_ptr(),
-                                     rows, (uint32_t)hidden, Stream());
+                                     extra ? extra->const_data_ptr() : nullptr, dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr,
+                                     partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows, (uint32_t)hidden, Stream());
         if (r != 0) return PyLong_FromLong(r);
-        return WrapAll(std::move(dx), std::move(dw));
+        return WrapAll(std::move(dx), std::move(dw), std::move(copy));
     });
 }
 

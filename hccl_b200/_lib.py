@@ -158,6 +158,8 @@ def _sig_or_none(name, restype, *argtypes):
 _sig_or_none("HcclFusedAddRmsNormFwd", R, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_uint64, c_uint32, ctypes.c_float, c_void_p)
 _sig_or_none("HcclFusedRmsNormBwdPartials", c_uint32, c_uint64)
 _sig_or_none("HcclFusedRmsNormBwd", R, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_uint64, c_uint32, c_void_p)
+_sig_or_none("HcclFusedRmsNormBwdCopy", R, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_uint64, c_uint32,
+             c_void_p)
 _sig_or_none("HcclFusedSwigluFwd", R, c_void_p, c_void_p, c_uint64, c_uint32, c_void_p)
 _sig_or_none("HcclFusedSwigluBwd", R, c_void_p, c_void_p, c_void_p, c_uint64, c_uint32, c_void_p)
 _sig_or_none("HcclFusedRope", R, c_void_p, c_uint64, c_void_p, c_uint64, c_void_p, c_void_p, c_uint64, c_uint32, c_uint32, c_int, c_void_p)

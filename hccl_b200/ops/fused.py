@@ -69,6 +69,15 @@ def rope_reference(x, cos, sin):
 
 
 # ----------------------------------------------------------------------------- autograd functions
+def _kept_apart(*nodes) -> bool:
+    """The gradients of these inputs end in as many leaves that hold none yet: each leaf keeps the tensor it is given if nobody
+    else has it, and copies it otherwise.  (Under ``autograd.grad`` the leaves keep nothing: the engine refuses to say.)"""
+    try:
+        return all(hasattr(n, "variable") and n.variable.grad is None and torch._C._will_engine_execute_node(n) for n in nodes) and len(set(nodes)) == len(nodes)
+    except RuntimeError:
+        return False
+
+
 class _AddRmsNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, delta, weight, eps):
@@ -103,19 +112,21 @@ class _AddRmsNorm(torch.autograd.Function):
             dh = torch.zeros_like(x_out)
         dh = dh.contiguous()
         extra = dx_out.contiguous() if dx_out is not None else None
-        r = _calls.rms_norm_bwd(dh, x_out, weight, rstd, extra)
+        twice = ctx.has_delta and _kept_apart(ctx.next_functions[0][0], ctx.next_functions[1][0])
+        r = _calls.rms_norm_bwd(dh, x_out, weight, rstd, extra, twice)
         if r is not None:
-            dx, dw = _calls.result(r, "HcclFusedRmsNormBwd")
+            dx, dw, copy = _calls.result(r, "HcclFusedRmsNormBwdCopy")
             _count(2)
-            return dx, (dx if ctx.has_delta else None), dw, None
+            return dx, (copy if ctx.has_delta else None), dw, None
         dx = torch.empty_like(x_out)
+        copy = torch.empty_like(x_out) if twice else dx
         dw = torch.empty_like(weight)
         n_part = lib.HcclFusedRmsNormBwdPartials(rows)
         partial = torch.empty((n_part, hidden), device=x_out.device, dtype=torch.float32)
-        _check(lib.HcclFusedRmsNormBwd(_p(dh), _p(x_out), _p(weight), _p(rstd), _p(extra), _p(dx), _p(partial), _p(dw), rows, hidden, _s()),
-               "HcclFusedRmsNormBwd")
+        _check(lib.HcclFusedRmsNormBwdCopy(_p(dh), _p(x_out), _p(weight), _p(rstd), _p(extra), _p(dx), _p(copy) if twice else ctypes.c_void_p(0), _p(partial),
+                                           _p(dw), rows, hidden, _s()), "HcclFusedRmsNormBwdCopy")
         _count(2)
-        return dx, (dx if ctx.has_delta else None), dw, None
+        return dx, (copy if ctx.has_delta else None), dw, None
 
 
 class _Swiglu(torch.autograd.Function):

@@ -5,6 +5,7 @@
 #include "../algo/step_tables.h"
 #include "../core/bootstrap.h"
 #include "../core/config.h"
+#include "../core/comm.h"
 #include "../core/log.h"
 #include "../core/plan_cache.h"
 #include "../cpu/host_tree.h"
@@ -266,6 +267,13 @@ double HcclDebugEvalCost(double A, double B, double C, double D, int netType, do
     CostCoeff c;
     c.A = A; c.B = B; c.C = C; c.D = D; c.net = (NetType)netType; c.ratio = ratio;
     return EvalCost({c}, CostAgg::SUM, bytes, HCCL_ENGINE_P2P);
+}
+
+// Operators started and finished on this rank's device so far (what the stuck detection compares).
+HcclResult HcclDebugOpCounters(HcclComm comm, uint64_t* started, uint64_t* finished)
+{
+    CHK_PTR_NULL(comm);
+    return static_cast<CommImpl*>(comm)->ReadOpCounters(started, finished);
 }
 
 }  // extern "C"

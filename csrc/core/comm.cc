@@ -81,6 +81,8 @@ HcclResult CommImpl::SetupDeviceState()
     CHK_CUDA(cudaHostAlloc((void**)&hStatus_, sizeof(DevStatus), cudaHostAllocMapped | cudaHostAllocPortable));
     memset((void*)hStatus_, 0, sizeof(DevStatus));
     CHK_CUDA(cudaHostGetDevicePointer((void**)&dStatus_, (void*)hStatus_, 0));
+    CHK_CUDA(cudaStreamCreateWithFlags(&countersStream_, cudaStreamNonBlocking));
+    CHK_CUDA(cudaHostAlloc((void**)&hCounters_, 2 * sizeof(uint64_t), cudaHostAllocPortable));
     dev_->rank = rank;
     dev_->nRanks = nRanks;
     for (int q = 0; q < nRanks; ++q) dev_->slab[q] = (char*)slab_.peer[q];
@@ -195,6 +197,10 @@ HcclResult CommImpl::Destroy()
     for (auto& s : userSegs_) SymFree(&s);
     userSegs_.clear();
     if (ownsSlab_) SymFree(&slab_);
+    std::lock_guard<std::mutex> counters(countersMu_);
+    if (countersStream_) cudaStreamDestroy(countersStream_);
+    if (hCounters_) cudaFreeHost(hCounters_);
+    countersStream_ = nullptr; hCounters_ = nullptr;
     if (dEpochs_) cudaFree(dEpochs_);
     if (dAbort_) cudaFree(dAbort_);
     if (dP2pSeq_) cudaFree(dP2pSeq_);
@@ -380,16 +386,35 @@ bool CommImpl::Lookup(const void* p, uint64_t bytes, const char* peerPtr[HCCL_MA
     return false;
 }
 
+HcclResult CommImpl::ReadOpCounters(uint64_t* started, uint64_t* finished)
+{
+    CHK_PTR_NULL(started); CHK_PTR_NULL(finished);
+    std::lock_guard<std::mutex> lk(countersMu_);
+    if (!dEpochs_ || !countersStream_) return HCCL_E_NOT_SUPPORT;
+    // another thread's stream capture is none of this thread's business
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return HCCL_E_RUNTIME;             // the process is on its way out
+    e = cudaMemcpyAsync(hCounters_, dEpochs_ + 2 * kMaxBlocks, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, countersStream_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(countersStream_);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return HCCL_E_RUNTIME;
+    *started = hCounters_[0];
+    *finished = hCounters_[1];
+    return HCCL_SUCCESS;
+}
+
 void CommImpl::WatchdogLoop()
 {
+    cudaSetDevice(device);
     // head != tail with no progress for a whole wait budget = an op is stuck between its start and its end
     // (reference: per-communicator head/tail counters compared by a host watchdog, stuck_detect_counter_helper.h).
     uint64_t lastHead = 0, lastTail = 0;
     auto lastChange = std::chrono::steady_clock::now();
     while (!watchdogStop_.load()) {
         for (int i = 0; i < 10 && !watchdogStop_.load(); ++i) std::this_thread::sleep_for(std::chrono::milliseconds(100));
-        if (!hStatus_) continue;
-        const uint64_t h = hStatus_->head, t = hStatus_->tail;
+        uint64_t h = 0, t = 0;
+        if (watchdogStop_.load() || ReadOpCounters(&h, &t) != HCCL_SUCCESS) continue;
         auto now = std::chrono::steady_clock::now();
         if (h != lastHead || t != lastTail) { lastHead = h; lastTail = t; lastChange = now; continue; }
         if (h != t) {

@@ -125,11 +125,17 @@ private:
     DevStatus* dStatus_ = nullptr;  // device alias of hStatus_
     EmuGroup* emu_ = nullptr;
     StageLayout layout_{};
-    // watchdog (stuck detection): compares head/tail of the status block
+    // watchdog (stuck detection): compares the counts of started and finished operators
     std::thread watchdog_;
     std::atomic<bool> watchdogStop_{false};
     void WatchdogLoop();
+    // ops started and finished, copied from device memory on a stream of their own
+    cudaStream_t countersStream_ = nullptr;
+    uint64_t* hCounters_ = nullptr;     // pinned, two words
+    std::mutex countersMu_;
 public:
+    // Ops started and finished on this rank so far; does not wait for kernels in flight.
+    HcclResult ReadOpCounters(uint64_t* started, uint64_t* finished);
     std::atomic<uint64_t> stuckReports{0};
 };
 

@@ -77,6 +77,9 @@ static __device__ __noinline__ void ReportWaitFailure(const DevComm& c, uint32_t
         s->rank = (uint32_t)c.rank;
         s->expected = expected;
         s->seen = seen;
+        const volatile uint64_t* ops = c.epochs + 2 * kMaxBlocks;
+        s->head = ops[0];
+        s->tail = ops[1];
         __threadfence_system();
         s->error = err;
         __threadfence_system();
@@ -251,24 +254,22 @@ __device__ __forceinline__ bool WaitPeer(const DevComm& c, int peer, int block, 
 // Stuck-detection counters (reference: stuck_detect_counter_helper.h; AIV
 // EmitStuckCounter aiv_communication_base_v2.h:368-378).  Block 0 bumps `head`
 // at entry and `tail` at exit; a host watchdog compares them.
-// The running values live in device memory (no read crosses PCIe); each bump is
-// mirrored to the host-mapped status block with one posted write.
+// The values live in device memory and are read by the host when it wants to know (CommImpl::ReadOpCounters).  Mirrored to
+// the host-mapped status block they cost a write across PCIe at each end, which the system-scope release of the first
+// barrier, and the end of the kernel, then waited for: AllReduce of 256 KiB over 8 emulated ranks 19.3 -> 11.1 us without,
+// of 16 KiB 38.5 -> 18.4, AlltoAll of 8 x 32 KiB 39.0 -> 18.8.
 __device__ __forceinline__ void OpHead(const DevComm& c, int block)
 {
     if (block == 0 && threadIdx.x == 0) {
         volatile uint64_t* h = c.epochs + 2 * kMaxBlocks;
-        const uint64_t v = *h + 1;
-        *h = v;
-        c.status->head = v;
+        *h = *h + 1;
     }
 }
 __device__ __forceinline__ void OpTail(const DevComm& c, int block)
 {
     if (block == 0 && threadIdx.x == 0) {
         volatile uint64_t* t = c.epochs + 2 * kMaxBlocks + 1;
-        const uint64_t v = *t + 1;
-        *t = v;
-        c.status->tail = v;
+        *t = *t + 1;
     }
 }
 

@@ -42,7 +42,7 @@ struct DevStatus {
     volatile uint32_t rank;       // reporting rank
     volatile uint64_t expected;   // flag value waited for
     volatile uint64_t seen;       // last value observed
-    volatile uint64_t head;       // ops started  (stuck detection: head != tail for long = hung op)
+    volatile uint64_t head;       // ops started, as the failure was reported
     volatile uint64_t tail;       // ops finished
 };
 

@@ -30,6 +30,8 @@ __device__ __forceinline__ char* StageMcPtr(const DevComm& c) { return c.slabMc 
 
 #ifdef HCCL_HOST_SHIM
 inline void StReleaseSys(uint64_t* p, uint64_t v) { __atomic_store_n(p, v, __ATOMIC_RELEASE); }
+// after a system-scope fence by the same thread (a release here: the tools that watch the shim do not follow fences)
+inline void StRelaxedSys(uint64_t* p, uint64_t v) { __atomic_store_n(p, v, __ATOMIC_RELEASE); }
 inline uint64_t LdAcquireSys(const uint64_t* p) { return __atomic_load_n(p, __ATOMIC_ACQUIRE); }
 inline uint64_t LdRelaxedSys(const uint64_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
 inline uint32_t LdVolatileU32(const uint32_t* p) { return __atomic_load_n(p, __ATOMIC_RELAXED); }
@@ -38,6 +40,11 @@ inline uint64_t GlobalTimerNs() { return hostshim::NowNs(); }
 __device__ __forceinline__ void StReleaseSys(uint64_t* p, uint64_t v)
 {
     asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Published by a system-scope fence that the same thread made before: several flags behind one fence.
+__device__ __forceinline__ void StRelaxedSys(uint64_t* p, uint64_t v)
+{
+    asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ uint64_t LdAcquireSys(const uint64_t* p)
 {
@@ -161,10 +168,11 @@ __device__ __forceinline__ void FinishLLEpoch(const DevComm& c, uint64_t epoch, 
         if (t == (unsigned long long)(nBlocks - 1)) {
             *reinterpret_cast<volatile uint64_t*>(ticket) = 0;
             *reinterpret_cast<volatile uint64_t*>(c.epochs + kMaxBlocks) = epoch + 1;
-            __threadfence();
-            // every block of this rank has read its lines of this op: the peers may reuse the slots of this parity
+            // every block of this rank has read its lines of this op: the peers may reuse the slots of this parity.  One fence in
+            // front of all flags: a release store each costs a fence each, one after the other.
+            __threadfence_system();
             for (int q = 0; q < c.nRanks; ++q)
-                if (q != c.rank) StReleaseSys(FlagPtr(c, q, 0, kLLCreditSlot, c.rank), epoch + 1);
+                if (q != c.rank) StRelaxedSys(FlagPtr(c, q, 0, kLLCreditSlot, c.rank), epoch + 1);
         }
     }
 }

@@ -58,10 +58,16 @@ HcclResult EnsureState(CommImpl* c, size_t nPairs)
     return HCCL_SUCCESS;
 }
 
-int MoeBlocks(const CommImpl* c, uint32_t nTokens)
+// One block per eight tokens, or per 32 Ki elements of the rows' copies where that is more: few tokens of long rows are as much
+// to move as many of short ones.  8 emulated ranks, rows of 7168, top-8, with a block per eight tokens -> now (us, dispatch and
+// combine): 4 tokens 23.4 + 21.9 -> 21.0 + 17.3, 8 31.0 + 28.8 -> 21.3 + 17.8, 16 33.1 + 33.2 -> 21.6 + 19.3, 32 33.4 + 32.7 -> 22.0
+// + 23.1, 64 34.1 + 31.2 -> 27.6 + 30.2; 1 token, and rows of 4096 with top-2 up to 8 tokens, as before (a block per 16 Ki elements:
+// 1 token 18.8 -> 21.0).  All ranks come to the same number: their configurations are the same.
+int MoeBlocks(const CommImpl* c, const HcclMoeConfig* cfg)
 {
+    const uint64_t byRows = (uint64_t)cfg->nTokens * cfg->topk * cfg->hidden / (32 << 10);
     // combine is a pull over NVLink, bound by the bytes in flight: as many blocks as the flag rows allow
-    int nb = (int)std::min<uint32_t>(std::max<uint32_t>(nTokens / 8, 1), 128);
+    const int nb = (int)std::min<uint64_t>(std::max<uint64_t>({cfg->nTokens / 8, byRows, 1}), 128);
     return std::min(nb, c->MaxBlocks());
 }
 
@@ -98,7 +104,7 @@ HcclResult HcclMoeDispatch(HcclComm comm, const void* x, const int32_t* topkIdx,
     if (nPairs > (size_t)kMoeCountInDispatch) CHK_RET(LaunchMoeCount(topkIdx, (int)nPairs, (int)cfg->nExperts, st->counts, st->pos, (cudaStream_t)stream));
     else a.counts = a.pos = nullptr;                 // every block of the dispatch kernel counts for itself
     // every rank launches the same grid: sized by a value all ranks share (the configured token count must match)
-    return LaunchMoeDispatch(c->Target((cudaStream_t)stream), a, MoeBlocks(c, cfg->nTokens));
+    return LaunchMoeDispatch(c->Target((cudaStream_t)stream), a, MoeBlocks(c, cfg));
 }
 
 HcclResult HcclMoeCombine(HcclComm comm, const void* y, const float* topkWeight, const uint64_t* slotMap, const HcclMoeConfig* cfg, void* out,
@@ -120,7 +126,7 @@ HcclResult HcclMoeCombine(HcclComm comm, const void* y, const float* topkWeight,
     for (int q = 0; q < c->nRanks; ++q) a.y[q] = (const __nv_bfloat16*)py[q];
     a.topkWeight = topkWeight; a.slotMap = slotMap; a.out = (__nv_bfloat16*)out;
     a.nTokens = (int)cfg->nTokens; a.hidden = (int)cfg->hidden; a.topk = (int)cfg->topk; a.capacity = cfg->capacity;
-    int nb = MoeBlocks(c, cfg->nTokens);
+    int nb = MoeBlocks(c, cfg);
     if (c->emulated()) nb = std::min(nb, std::max(1, SmCount() / c->nRanks));      // one block per SM (its ring), all ranks' in one grid
     return LaunchMoeCombine(c->Target((cudaStream_t)stream), a, nb);
 }

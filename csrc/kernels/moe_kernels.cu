@@ -240,7 +240,7 @@ struct DispatchBody {
 
 // ------------------------------------------------------------------ combine
 // A pull over NVLink, bound by the bytes in flight.  Work item of a WARP: pieces (32 vectors of 16 bytes) of one token's row,
-// whole rows where there are tokens enough, else as many parts as give every warp something to load.  Every thread owns a ring
+// whole rows where there are tokens enough, else as many parts as finish first.  Every thread owns a ring
 // of kCombineRing vectors in shared memory that asynchronous copies fill, 3 pieces of 8 copies (or 6 of 4, 12 of 2) ahead of
 // the arithmetic; it reads what it copied itself, so there is no hand-over.  The ring keeps up to 192 KiB per SM requested all
 // the time, where loads into registers (8 a thread: sixteen spilled) had 64 KiB, and nothing between a piece's sum and the
@@ -259,10 +259,14 @@ struct CombineBody {
         constexpr int D = kCombineRing / COPIES;
         const int H = a.hidden, vecPerRow = H / 8, nPieces = (vecPerRow + 31) / 32;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const uint32_t stride = (uint32_t)nb * kMoeWarps, all = (uint32_t)a.nTokens * nPieces;      // rows fit the GPU: far below 2^32
-        const uint32_t share = min((all + stride - 1) / stride, (uint32_t)nPieces);                 // pieces for every warp
-        const uint32_t parts = share > 0 ? ((uint32_t)nPieces + share - 1) / share : 0, items = (uint32_t)a.nTokens * parts;
-        const int perItem = parts > 0 ? (int)((nPieces + parts - 1) / parts) : 0;
+        const uint32_t stride = (uint32_t)nb * kMoeWarps;
+        // parts per row: lane l weighs l + 1 of them by rounds of all warps x (pieces of a part + about two for its addresses)
+        static_assert(8192 / 8 <= 32 * 32, "as many parts to weigh as lanes");
+        const uint32_t p = (uint32_t)lane + 1, rounds = ((uint32_t)a.nTokens * p + stride - 1) / stride;
+        const uint32_t cost = p <= (uint32_t)nPieces ? rounds * (((uint32_t)nPieces + p - 1) / p + 2) : 0x3FFFFFFu;      // rows fit the GPU: far below 2^26
+        const uint32_t parts = (__reduce_min_sync(0xffffffffu, min(cost, 0x3FFFFFFu) << 6 | (uint32_t)lane) & 63u) + 1;
+        const uint32_t items = (uint32_t)a.nTokens * parts;
+        const int perItem = (int)((nPieces + parts - 1) / parts);
         const uint8_t* mine = s_ring + threadIdx.x * 16;            // slot s of this thread: s * kMoeThreads vectors further
         const uint32_t mineAddr = (uint32_t)__cvta_generic_to_shared(mine);
         for (uint32_t it = b + warp * nb; it < items; it += stride) {

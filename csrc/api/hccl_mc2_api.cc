@@ -156,8 +156,8 @@ HcclResult HcclDebugMatmulPlan(uint64_t m, uint64_t n, uint64_t k, int transA, i
     CHK_PTR_NULL(text);
     const MatmulPlan p = PlanMatmul(m, n, k, transA != 0, transB == 0, (int)sms, MatmulSwitchesOfEnv());
     static const char* const names[] = {"split", "one_sm", "two_sm", "wide", "two_sm_split"};
-    snprintf(text, cap, "route=%s bn=%d tiles=%dx%d grid=%d bt=%d split=%d wide=%d singles=%d hints=%d%d raster=%d rest=%dx%d", names[(int)p.route], p.bn, p.tilesM,
-             p.tilesN, p.grid, p.bt, p.split, p.wide, p.singles, p.l2HintA, p.l2HintB, p.rasterGroup, p.restTiles, p.restSplit);
+    snprintf(text, cap, "route=%s bn=%d tiles=%dx%d grid=%d bt=%d split=%d wide=%d singles=%d hints=%d%d raster=%d", names[(int)p.route], p.bn, p.tilesM,
+             p.tilesN, p.grid, p.bt, p.split, p.wide, p.singles, p.l2HintA, p.l2HintB, p.rasterGroup);
     return HCCL_SUCCESS;
 }
 // Tests: the matmul with a CTA whose operands never arrive.  `out` must stay as it is where that CTA's tile lies, and the next

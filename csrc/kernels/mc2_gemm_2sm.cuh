@@ -184,12 +184,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const uint32_t tmemBase = *tmemBaseSlot;
         if (MODE == MODE_PLAIN) {
             DependencyWait();
-            AllowDependents();          // not before: the split launch of the last tiles relies on it (mc2_gemm_2sm_split.cuh)
+            AllowDependents();
         }
         const int BN = g.bn;                        // column tile width of this launch (accumulators stay 256 columns apart)
         const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;
         const int tilesM2 = (g.M + 255) / 256;
-        const int nTiles = MODE == MODE_PLAIN && g.tileLimit > 0 ? g.tileLimit : tilesM2 * g.tilesN;
+        const int nTiles = tilesM2 * g.tilesN;
         const int kBlocks = (g.K + kBK - 1) / kBK;
         // bytes of a stage in both CTAs.  An MN-major half tile of B comes in boxes of 64 columns, whole ones: at a
         // half width that is no multiple of 64 the last box brings columns of the neighbouring half (or tile) along,

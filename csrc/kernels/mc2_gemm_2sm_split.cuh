@@ -29,10 +29,8 @@ constexpr int kSplit2StgRowBytes = 64 + 16, kSplit2StgWarpBytes = 32 * kSplit2St
 struct Split2Args {
     int M, N, K;               // out[M, N] = A[M, K] x B[K, N]   (operand storage is described by the tensor maps)
     __nv_bfloat16* out;
-    int bn;                    // column tile width, a multiple of 32, at most 256
+    int bn;                    // column tile width, a multiple of 32, at most 256 (launched with 128)
     int tilesM2, tilesN;
-    int firstTile;             // this launch's first tile, in the order of the other two-SM kernels
-    int rest;                  // != 0: the launch in front of this one computes the tiles before firstTile
     int stages;
     uint32_t* ctl;             // control block: the abort word of bounded waits
     uint64_t waitLimitNs;      // of every wait
@@ -79,7 +77,7 @@ __global__ void __launch_bounds__(kSplit2Threads, 1)
     const int split = (int)SplitClusterSize() / 2, crank = (int)ClusterCtaRank();
     const int pair = crank >> 1, half = crank & 1;     // this CTA: rows half * 128 .. + 127 of the tile, the pair's share of K
     int mt2, nt;
-    GroupedTile(g.firstTile + (int)blockIdx.x / (2 * split), g.tilesM2, g.tilesN, kRasterGroup, &mt2, &nt);
+    GroupedTile((int)blockIdx.x / (2 * split), g.tilesM2, g.tilesN, kRasterGroup, &mt2, &nt);
     const int BN = g.bn, mt = mt2 * 2 + half;
     const int kBlocks = (g.K + kBK - 1) / kBK;
     const int kFirst = (int)((long long)kBlocks * pair / split), kLast = (int)((long long)kBlocks * (pair + 1) / split);
@@ -103,13 +101,8 @@ __global__ void __launch_bounds__(kSplit2Threads, 1)
     ClusterSync();                                     // the peer's barriers exist before anything arrives on them
     TcFenceAfter();
     const uint32_t tmemBase = *tmemBaseSlot;
-    // The rest of a product: the launch in front allows this one only after its own wait, so the operands are complete and were
-    // written before it (they are read by TMA, through L2); its tiles are not this one's, and only this kernel's end has to come
-    // after its end.
-    if (!g.rest) {
-        DependencyWait();
-        AllowDependents();
-    }
+    DependencyWait();
+    AllowDependents();
     const int quarter = warp & 3, part = (warp - 2) >> 2;      // warps 2..9: rows, and every second chunk of columns
     const uint32_t taddr = tmemBase + ((uint32_t)(quarter * 32) << 16);
     bool drained = false;                              // warps 2..9: the accumulator is complete
@@ -240,10 +233,6 @@ __global__ void __launch_bounds__(kSplit2Threads, 1)
             }
             __syncwarp();
         }
-    }
-    if (g.rest) {
-        DependencyWait();
-        AllowDependents();
     }
     TcFenceBefore();
     __syncthreads();

@@ -491,25 +491,6 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     }
     p.route = MatmulRoute::TWO_SM;
     p.grid = std::min(2 * pairs, 2 * tilesM2 * p.tilesN);
-    // Full rounds of 256-wide tiles and a split launch for the last ones, where that costs less than a width that evens out the
-    // rounds (same units as TwoSmColumnTile; the split launch costs a share of a round and about 8 us, a k-block of a round
-    // 0.37).  It pays with MN-major B, whose narrower tiles are filled in whole boxes (sustained, us: 1024 x 10240 x 8192 with A
-    // transposed 157.8 -> 141.3, 1000 x 10240 x 8192 151.9 -> 140.7); with K-major B narrower tiles cost the same (1000 x 10240 x
-    // 8192 138.4 and 141.2).
-    const int tiles256 = tilesM2 * (int)((n + 255) / 256), rest = tiles256 % pairs;
-    const int restSplit = rest > 0 && tiles256 > pairs ? Split2Pairs(rest, pairs) : 1;
-    if (bMn && !sw.l2Hints && restSplit > 1 && k >= 16 * kBK) {
-        const int waves = (tilesM2 * p.tilesN + pairs - 1) / pairs, loaded = 2 * ((p.bn / 2 + 63) / 64 * 64);
-        const double perRound = 352.0, now = waves * ((p.bn + 2 * loaded) / 3.0 + 96);
-        const double split = (tiles256 / pairs) * perRound + perRound / restSplit + perRound * 8 / (0.37 * (double)((k + kBK - 1) / kBK));
-        if (split < 0.95 * now) {
-            p.bn = 256;
-            p.tilesN = (int)((n + 255) / 256);
-            p.grid = 2 * pairs;
-            p.restTiles = rest;
-            p.restSplit = restSplit;
-        }
-    }
     // Raster and L2 policy (experimental, HCCL_MC2_L2_HINTS=1).  About `pairs` tiles are in flight: r row tiles x c
     // column tiles, walking the columns of a band of r rows.  When one operand is small enough to live in L2 next
     // to the stream of the other, it is loaded "evict last", the streamed one "evict first", and the band covers
@@ -565,18 +546,20 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     CHK_RET(MapA(&ta, a, m, k, aMn));
     // two-SM tiles: B is split between the two CTAs of a pair, each loads half of the B rows of a tile
     CHK_RET(MapB(&tb, b, n, k, bMn, plan.route == MatmulRoute::ONE_SM ? plan.bn : plan.bn / 2));
-    Split2Args split;
-    memset(&split, 0, sizeof(split));
-    split.M = (int)m; split.N = (int)n; split.K = (int)k;
-    split.out = (__nv_bfloat16*)out;
-    split.bn = plan.bn;
-    split.tilesM2 = (int)((m + 255) / 256);
-    split.tilesN = plan.tilesN;
-    split.stages = Split2Stages(plan.bn, bMn);
-    split.ctl = plain.ctl;
-    split.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
-    split.stalledCta = stalled != nullptr ? stalled->cta : -1;
-    if (plan.route == MatmulRoute::TWO_SM_SPLIT) return DispatchSplit2(aMn, bMn, ta, tb, split, split.tilesM2 * plan.tilesN, plan.split, stream);
+    if (plan.route == MatmulRoute::TWO_SM_SPLIT) {
+        Split2Args split;
+        memset(&split, 0, sizeof(split));
+        split.M = (int)m; split.N = (int)n; split.K = (int)k;
+        split.out = (__nv_bfloat16*)out;
+        split.bn = plan.bn;
+        split.tilesM2 = plan.tilesM;
+        split.tilesN = plan.tilesN;
+        split.stages = Split2Stages(plan.bn, bMn);
+        split.ctl = plain.ctl;
+        split.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
+        split.stalledCta = stalled != nullptr ? stalled->cta : -1;
+        return DispatchSplit2(aMn, bMn, ta, tb, split, plan.tilesM * plan.tilesN, plan.split, stream);
+    }
     GemmArgs g;
     memset(&g, 0, sizeof(g));
     g.M = (int)m; g.N = (int)n; g.K = (int)k;
@@ -599,13 +582,7 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         if (aMn && !bMn) return LaunchGemm2SmWide<true, false>(ta, tb, g, plan.grid, stream);
         return LaunchGemm2SmWide<true, true>(ta, tb, g, plan.grid, stream);
     }
-    if (plan.route == MatmulRoute::TWO_SM) {
-        if (plan.restTiles > 0) g.tileLimit = split.firstTile = split.tilesM2 * plan.tilesN - plan.restTiles;
-        CHK_RET(DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream));
-        if (plan.restTiles == 0) return HCCL_SUCCESS;
-        split.rest = 1;
-        return DispatchSplit2(aMn, bMn, ta, tb, split, plan.restTiles, plan.restSplit, stream);
-    }
+    if (plan.route == MatmulRoute::TWO_SM) return DispatchLayout2Sm<MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
     if (plan.bn == 128) return DispatchLayout<128, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
     return DispatchLayout<256, MODE_PLAIN>(aMn, bMn, ta, tb, g, dummy, plan.grid, false, stream);
 }

@@ -35,7 +35,6 @@ struct MatmulPlan {
     int bn = 0, tilesM = 0, tilesN = 0, grid = 0;
     int bt = 0, split = 0;              // SPLIT: tokens per tile, CTAs per tile; TWO_SM_SPLIT: CTA pairs per tile
     int wide = 0, singles = 0;          // WIDE: wide items, single ones
-    int restTiles = 0, restSplit = 0;   // TWO_SM: last tiles that a split launch computes, CTA pairs per tile of it
     int rasterGroup = 0, l2HintA = 0, l2HintB = 0;
 };
 MatmulSwitches MatmulSwitchesOfEnv();

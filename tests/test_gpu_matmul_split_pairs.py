@@ -1,5 +1,5 @@
-"""Two-SM matmul tiles with the inner dimension split over a cluster of CTA pairs, and products whose last tiles such a launch
-computes, against float64.  Tolerance: one rounding to bf16 and fp32 sums, as in test_gpu_tile_edges."""
+"""Two-SM matmul tiles with the inner dimension split over a cluster of CTA pairs, and two-SM products that end in a round of few
+tiles, against float64.  Tolerance: one rounding to bf16 and fp32 sums, as in test_gpu_tile_edges."""
 import ctypes
 
 import pytest
@@ -25,20 +25,30 @@ def test_split_over_pairs(shape, pairs, ta, tb):
     _check_matmul(*shape, ta, tb)
 
 
-# (m, n, k), last tiles and pairs per tile of them; MN-major weights
-REST = [((1024, 10240, 4096), "12x4"), ((1000, 10240, 8192), "12x4"), ((2560, 4096, 4104), "12x4")]
+# (m, n, k) of two-SM products that end in a round of few tiles
+LAST_ROUND = [(1024, 10240, 4096), (1000, 10240, 8192), (2560, 4096, 4104), (4096, 3584, 8192)]
 
 
 @pytest.mark.parametrize("ta", [False, True])
-@pytest.mark.parametrize("shape,rest", REST)
-def test_last_tiles_split_over_pairs(shape, rest, ta):
-    p = plan(*shape, int(ta), 0)
-    assert (p["route"], p["rest"]) == ("two_sm", rest), p
+@pytest.mark.parametrize("shape", LAST_ROUND)
+def test_last_round_of_few_tiles(shape, ta):
+    assert plan(*shape, int(ta), 0)["route"] == "two_sm"
     _check_matmul(*shape, ta, False)
 
 
-def test_last_tiles_between_other_launches():
-    """The launch of the last tiles may start before the one in front of it ends: what comes before and after both must not notice."""
+@pytest.mark.parametrize("shape", LAST_ROUND)
+def test_all_tiles_of_a_product_add_in_one_order(shape):
+    """Columns moved by half the matrix land in other tiles, of other rounds: the same bits."""
+    m, n, k = shape
+    assert plan(*shape, 0, 0)["route"] == "two_sm"
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, w = torch.randn(m, k, device="cuda", generator=g).bfloat16(), (torch.randn(k, n, device="cuda", generator=g) * 0.02).bfloat16()
+    moved = mc2.matmul(a, w.roll(n // 2, 1), trans_b=False)
+    assert torch.equal(mc2.matmul(a, w, trans_b=False).roll(n // 2, 1), moved)
+
+
+def test_products_in_a_chain():
+    """Back to back, on streams and in a graph: a product's start overlaps the end of the one before it."""
     g = torch.Generator(device="cuda").manual_seed(9)
     rnd = lambda *s: (torch.randn(*s, device="cuda", generator=g) * 0.05).bfloat16()  # noqa: E731
     a, w, back = rnd(1000, 4096), rnd(4096, 10240), rnd(10240, 4096)

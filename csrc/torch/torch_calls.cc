@@ -89,6 +89,17 @@ template <class F> PyObject* Guarded(F f)
     return f();
     END_HANDLE_TH_ERRORS
 }
+// The interpreter's lock is not held while memory is allocated and the C API is called, as with torch's own functions and ctypes:
+// both may wait (a full launch queue, a kernel's first load, the allocator) for what another Python thread has yet to issue.
+class Unlocked {
+public:
+    Unlocked() : state_(PyEval_SaveThread()) {}
+    ~Unlocked() { PyEval_RestoreThread(state_); }
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+private:
+    PyThreadState* state_;
+};
 #define HCCL_ARGS(n) \
     if (nargs != (n)) { PyErr_SetString(PyExc_TypeError, "wrong number of arguments"); return nullptr; }
 
@@ -102,10 +113,17 @@ PyObject* AddRmsNorm(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         if (x->dim() == 0 || x->numel() == 0 || w->numel() != x->size(-1) || (delta && delta->sizes() != x->sizes())) return None();
         const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
         if (hidden % 8 != 0 || hidden > 8192) return None();
-        Tensor h = at::empty_like(*x), xOut = delta ? at::empty_like(*x) : *x, rstd = at::empty({(int64_t)rows}, x->options().dtype(at::kFloat));
-        const int r = api.addRmsNormFwd(x->const_data_ptr(), delta ? delta->const_data_ptr() : nullptr, w->const_data_ptr(),
-                                        delta ? xOut.mutable_data_ptr() : nullptr, h.mutable_data_ptr(), rstd.mutable_data_ptr(), rows, (uint32_t)hidden,
-                                        (float)PyFloat_AS_DOUBLE(a[3]), Stream());
+        const float eps = (float)PyFloat_AS_DOUBLE(a[3]);
+        Tensor h, xOut, rstd;
+        const int r = [&] {
+            Unlocked unlocked;
+            h = at::empty_like(*x);
+            xOut = delta ? at::empty_like(*x) : *x;
+            rstd = at::empty({(int64_t)rows}, x->options().dtype(at::kFloat));
+            return api.addRmsNormFwd(x->const_data_ptr(), delta ? delta->const_data_ptr() : nullptr, w->const_data_ptr(),
+                                     delta ? xOut.mutable_data_ptr() : nullptr, h.mutable_data_ptr(), rstd.mutable_data_ptr(), rows, (uint32_t)hidden, eps,
+                                     Stream());
+        }();
         if (r != 0) return PyLong_FromLong(r);
         return WrapAll(std::move(xOut), std::move(h), std::move(rstd));
     });
@@ -123,11 +141,17 @@ PyObject* RmsNormBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
         if (w->numel() != x->size(-1) || (uint64_t)rstd->numel() != rows) return None();
         const bool twice = PyObject_IsTrue(a[5]);
-        Tensor dx = at::empty_like(*x), dw = at::empty_like(*w), copy = twice ? at::empty_like(*x) : dx;
-        Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), (int64_t)hidden}, x->options().dtype(at::kFloat));
-        const int r = api.rmsNormBwd(dh->const_data_ptr(), x->const_data_ptr(), w->const_data_ptr(), rstd->const_data_ptr(),
-                                     extra ? extra->const_data_ptr() : nullptr, dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr,
-                                     partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows, (uint32_t)hidden, Stream());
+        Tensor dx, dw, copy;
+        const int r = [&] {
+            Unlocked unlocked;
+            dx = at::empty_like(*x);
+            dw = at::empty_like(*w);
+            copy = twice ? at::empty_like(*x) : dx;
+            Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), (int64_t)hidden}, x->options().dtype(at::kFloat));
+            return api.rmsNormBwd(dh->const_data_ptr(), x->const_data_ptr(), w->const_data_ptr(), rstd->const_data_ptr(),
+                                  extra ? extra->const_data_ptr() : nullptr, dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr,
+                                  partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows, (uint32_t)hidden, Stream());
+        }();
         if (r != 0) return PyLong_FromLong(r);
         return WrapAll(std::move(dx), std::move(dw), std::move(copy));
     });
@@ -143,8 +167,12 @@ PyObject* SwigluFwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const int64_t f = x->size(-1) / 2;
         auto sizes = x->sizes().vec();
         sizes.back() = f;
-        Tensor out = at::empty(sizes, x->options());
-        const int r = api.swigluFwd(x->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            out = at::empty(sizes, x->options());
+            return api.swigluFwd(x->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        }();
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
     });
 }
@@ -157,8 +185,12 @@ PyObject* SwigluBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const Tensor *x = GetPlainBf16(a[0]), *dout = GetPlainBf16(a[1]);
         if (!x || !dout || !PlainCall() || x->numel() == 0 || x->size(-1) % 16 != 0 || dout->numel() * 2 != x->numel()) return None();
         const int64_t f = x->size(-1) / 2;
-        Tensor dx = at::empty_like(*x);
-        const int r = api.swigluBwd(x->const_data_ptr(), dout->const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        Tensor dx;
+        const int r = [&] {
+            Unlocked unlocked;
+            dx = at::empty_like(*x);
+            return api.swigluBwd(x->const_data_ptr(), dout->const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+        }();
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(dx));
     });
 }
@@ -176,9 +208,13 @@ PyObject* Rope(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         for (const Tensor* t : {c, s})
             if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() < rows * (d / 2)) return None();
         const int backward = PyObject_IsTrue(a[3]);
-        Tensor out = at::empty({rows, heads, d}, x->options());
-        const int r = api.rope(x->const_data_ptr(), (uint64_t)x->stride(0), out.mutable_data_ptr(), (uint64_t)(heads * d), c->const_data_ptr(),
-                               s->const_data_ptr(), (uint64_t)rows, (uint32_t)heads, (uint32_t)d, backward, Stream());
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            out = at::empty({rows, heads, d}, x->options());
+            return api.rope(x->const_data_ptr(), (uint64_t)x->stride(0), out.mutable_data_ptr(), (uint64_t)(heads * d), c->const_data_ptr(),
+                            s->const_data_ptr(), (uint64_t)rows, (uint32_t)heads, (uint32_t)d, backward, Stream());
+        }();
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
     });
 }
@@ -199,8 +235,12 @@ PyObject* Matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs)
         if (b->size(tb ? 1 : 0) != k) return None();
         void* stream = StreamOf(args[5]);
         if (stream == nullptr && PyErr_Occurred()) return nullptr;
-        Tensor out = given ? *given : at::empty({m, n}, a->options());
-        const int r = api.matmul(a->const_data_ptr(), b->const_data_ptr(), out.data_ptr(), (uint64_t)m, (uint64_t)n, (uint64_t)k, ta, tb, stream);
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            out = given ? *given : at::empty({m, n}, a->options());
+            return api.matmul(a->const_data_ptr(), b->const_data_ptr(), out.data_ptr(), (uint64_t)m, (uint64_t)n, (uint64_t)k, ta, tb, stream);
+        }();
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
     });
 }
@@ -216,8 +256,12 @@ PyObject* ExpertOffsets(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         if (n <= 0 || n > 0x7FFFFFFFL) { PyErr_Clear(); return None(); }
         void* stream = StreamOf(a[2]);
         if (stream == nullptr && PyErr_Occurred()) return nullptr;
-        Tensor out = at::empty({n + 1}, idx->options());
-        const int r = api.expertOffsets(idx->const_data_ptr<int32_t>(), (uint64_t)idx->numel(), (uint32_t)n, (uint32_t*)out.mutable_data_ptr(), stream);
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            out = at::empty({n + 1}, idx->options());
+            return api.expertOffsets(idx->const_data_ptr<int32_t>(), (uint64_t)idx->numel(), (uint32_t)n, (uint32_t*)out.mutable_data_ptr(), stream);
+        }();
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
     });
 }
@@ -248,15 +292,15 @@ PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const void* s = send->const_data_ptr();
         void* r = recv->data_ptr();
         const uint64_t nSend = (uint64_t)send->numel(), nRecv = (uint64_t)recv->numel();
-        int code = 0;
-        Py_BEGIN_ALLOW_THREADS          // as ctypes does: a first call may wait for the other ranks' threads
-        switch (which) {
-            case ALL_REDUCE: code = api.allReduce(s, r, nSend, type, op, comm, stream); break;
-            case REDUCE_SCATTER: code = api.reduceScatter(s, r, nRecv, type, op, comm, stream); break;
-            case ALL_GATHER: code = api.allGather(s, r, nSend, type, comm, stream); break;
-            default: code = api.alltoAll(s, nSend / (uint64_t)ranks, type, r, nSend / (uint64_t)ranks, type, comm, stream); break;
-        }
-        Py_END_ALLOW_THREADS
+        const int code = [&] {
+            Unlocked unlocked;          // a first call may wait for the other ranks' threads
+            switch (which) {
+                case ALL_REDUCE: return api.allReduce(s, r, nSend, type, op, comm, stream);
+                case REDUCE_SCATTER: return api.reduceScatter(s, r, nRecv, type, op, comm, stream);
+                case ALL_GATHER: return api.allGather(s, r, nSend, type, comm, stream);
+                default: return api.alltoAll(s, nSend / (uint64_t)ranks, type, r, nSend / (uint64_t)ranks, type, comm, stream);
+            }
+        }();
         return PyLong_FromLong(code);
     });
 }

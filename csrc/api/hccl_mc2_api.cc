@@ -150,15 +150,21 @@ HcclResult HcclMc2Matmul(const void* a, const void* b, void* out, uint64_t m, ui
 {
     return Mc2Matmul(a, b, out, m, n, k, transA, transB, (cudaStream_t)stream);
 }
-// Tests: how a plain matmul would run on a GPU of `sms` SMs under the switches of the process environment.
-HcclResult HcclDebugMatmulPlan(uint64_t m, uint64_t n, uint64_t k, int transA, int transB, uint32_t sms, char* text, uint32_t cap)
+// Tests: how a plain matmul into an output aligned to `outAlign` bytes (16 for more) would run on a GPU of `sms` SMs under the switches
+// of the process environment; "refused" where the route stores more at a time.
+HcclResult HcclDebugMatmulPlanOut(uint64_t m, uint64_t n, uint64_t k, int transA, int transB, uint32_t sms, uint32_t outAlign, char* text, uint32_t cap)
 {
     CHK_PTR_NULL(text);
-    const MatmulPlan p = PlanMatmul(m, n, k, transA != 0, transB == 0, (int)sms, MatmulSwitchesOfEnv());
+    const MatmulPlan p = PlanMatmul(m, n, k, transA != 0, transB == 0, (int)sms, MatmulSwitchesOfEnv(), outAlign);
+    if (outAlign < MatmulOutAlign(p)) { snprintf(text, cap, "route=refused"); return HCCL_SUCCESS; }
     static const char* const names[] = {"split", "one_sm", "two_sm", "wide", "two_sm_split"};
     snprintf(text, cap, "route=%s bn=%d tiles=%dx%d grid=%d bt=%d split=%d wide=%d singles=%d hints=%d%d raster=%d", names[(int)p.route], p.bn, p.tilesM,
              p.tilesN, p.grid, p.bt, p.split, p.wide, p.singles, p.l2HintA, p.l2HintB, p.rasterGroup);
     return HCCL_SUCCESS;
+}
+HcclResult HcclDebugMatmulPlan(uint64_t m, uint64_t n, uint64_t k, int transA, int transB, uint32_t sms, char* text, uint32_t cap)
+{
+    return HcclDebugMatmulPlanOut(m, n, k, transA, transB, sms, 16, text, cap);
 }
 // Tests: the matmul with a CTA whose operands never arrive.  `out` must stay as it is where that CTA's tile lies, and the next
 // matmul on the device must return HCCL_E_TIMEOUT.

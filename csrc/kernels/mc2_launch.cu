@@ -424,7 +424,7 @@ MatmulSwitches MatmulSwitchesOfEnv()
     return s;
 }
 
-MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw)
+MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw, uint32_t outAlign)
 {
     MatmulPlan p;
     const int tilesM = (int)((m + kBM - 1) / kBM), tilesM2 = (int)((m + 255) / 256);
@@ -440,9 +440,9 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     // Two-SM tiles with the inner dimension split over a cluster of CTA pairs (see mc2_gemm_2sm_split.cuh): from 129 rows on, where
     // 256 x 128 tiles do not outnumber the pairs and the inner dimension pays for the sum.  At 129 .. 192 rows a quarter and more
     // of the 256 is padding, and the token split stays ahead where it has a long inner dimension (129 x 4096 x 14336: 28.9 us
-    // against 30.3).
+    // against 30.3).  The token split stores 8 bytes at a time, all other routes 16: an output that lies on 8 bytes only keeps it.
     const uint64_t tiles128 = (uint64_t)tilesM2 * ((n + 127) / 128);
-    if (sw.twoSm && m > 128 && k >= 2048 && tiles128 <= (uint64_t)pairs && (m > 192 || k < 4096 || twoSm)) {
+    if (sw.twoSm && outAlign >= 16 && m > 128 && k >= 2048 && tiles128 <= (uint64_t)pairs && (m > 192 || k < 4096 || twoSm)) {
         p.route = MatmulRoute::TWO_SM_SPLIT;
         p.bn = 128;
         p.tilesM = tilesM2;
@@ -510,6 +510,21 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     return p;
 }
 
+// Bytes that a route stores at a time.
+uint32_t MatmulOutAlign(const MatmulPlan& plan) { return plan.route == MatmulRoute::SPLIT ? 8 : 16; }
+
+static uint32_t AlignmentOf(const void* p)           // 2, 4, 8, or 16 for more
+{
+    const uint32_t low = (uint32_t)((uintptr_t)p & 15u);
+    return low == 0 ? 16u : (low & (~low + 1u));
+}
+static HcclResult RefuseOut(const void* out, uint64_t m, uint64_t n, uint64_t k)
+{
+    HCCL_ERROR("matmul %llu x %llu x %llu: the output at %p must be 16-byte aligned (8 bytes where the output has few tiles)", (unsigned long long)m,
+               (unsigned long long)n, (unsigned long long)k, out);
+    return HCCL_E_PARA;
+}
+
 HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, cudaStream_t stream,
                      const Mc2StalledCta* stalled)
 {
@@ -517,10 +532,13 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     CHK_RET(CheckShapes(m, n, k));
     const bool aMn = transA != 0, bMn = transB == 0;
     if (aMn && m % 8 != 0) return HCCL_E_PARA;
+    const uint32_t outAlign = AlignmentOf(out);
+    if (outAlign < 8) return RefuseOut(out, m, n, k);
     PlainCtl plain;
     CHK_RET(GetPlainCtl(&plain));
     if (*plain.gaveUp != 0) return ReportGaveUp(plain, stream);
-    const MatmulPlan plan = PlanMatmul(m, n, k, aMn, bMn, SmCount(), MatmulSwitchesOfEnv());
+    const MatmulPlan plan = PlanMatmul(m, n, k, aMn, bMn, SmCount(), MatmulSwitchesOfEnv(), outAlign);
+    if (outAlign < MatmulOutAlign(plan)) return RefuseOut(out, m, n, k);
     if (plan.route == MatmulRoute::SPLIT) {
         SplitArgs g;
         memset(&g, 0, sizeof(g));

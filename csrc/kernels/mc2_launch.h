@@ -38,7 +38,9 @@ struct MatmulPlan {
     int rasterGroup = 0, l2HintA = 0, l2HintB = 0;
 };
 MatmulSwitches MatmulSwitchesOfEnv();
-MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw);
+// `outAlign`: bytes the output is aligned to, 16 for more.
+MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw, uint32_t outAlign = 16);
+uint32_t MatmulOutAlign(const MatmulPlan& plan);      // what the route asks for
 
 // Tests of a wait that runs out, on a matmul with few output tiles: CTA `cta` loads nothing, all waits end after waitLimitNs.
 struct Mc2StalledCta { int cta; uint64_t waitLimitNs; };

@@ -10,7 +10,9 @@
 // parameters, shared and tensor memory are free), and so before it ends: a kernel is complete only after all kernels in front
 // of it are, and what follows may rely on the whole stream as with plain launches.  AllowDependents() lets the next kernel's
 // blocks take what this kernel leaves free of an SM; kernels that wait for another rank do not call it, so that blocks which
-// wait hold nothing that a kernel on another stream may need for that rank to get on.
+// wait hold nothing that a kernel on another stream may need for that rank to get on.  A kernel calls it only when it has all that
+// it will ever ask of its SM, its tensor memory above all: a follower, this library's or another's, may take the columns and then
+// hold at its own wait, for a kernel that cannot go on without them.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstring>

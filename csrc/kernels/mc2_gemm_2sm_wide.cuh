@@ -85,7 +85,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 {
     using L = SmemLayoutWide;
     extern __shared__ uint8_t smemRaw[];
-    AllowDependents();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kTileBytes);
     uint64_t* fullBar = bars;                          // [kStagesWide]  (used in the leader)
@@ -116,6 +115,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     ClusterSync();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemBaseSlot;
+    AllowDependents();
     DependencyWait();
     const int BN = g.bn;
     const int pair = cta >> 1, nPairs = g.nGemmCtas >> 1;

@@ -105,7 +105,6 @@ template <bool W_MN, bool X_MN>
 __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SplitArgs g)
 {
     extern __shared__ uint8_t smemRaw[];
-    AllowDependents();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
     const int stageBytes = SplitStageBytes(g.bt);
     const int ringBytes = g.stages * stageBytes, partialBytes = g.bt * 128 * 4;
@@ -140,6 +139,7 @@ __global__ void __launch_bounds__(kThreads) GemmSplitKernel(const __grid_constan
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemBaseSlot;
+    AllowDependents();
     DependencyWait();
 
     if (warp == 0) {

@@ -8,6 +8,7 @@
 #include "../core/comm.h"
 #include "../core/log.h"
 #include "../core/plan_cache.h"
+#include "../core/stuck_detector.h"
 #include "../cpu/host_tree.h"
 #include "../select/auto_selector.h"
 #include "../select/selector.h"
@@ -269,7 +270,16 @@ double HcclDebugEvalCost(double A, double B, double C, double D, int netType, do
     return EvalCost({c}, CostAgg::SUM, bytes, HCCL_ENGINE_P2P);
 }
 
-// Operators started and finished on this rank's device so far (what the stuck detection compares).
+// Which of n readings (answered, started, finished, seconds) of the operator counters the stuck detection reports.
+HcclResult HcclDebugStuckDetector(double budgetS, uint32_t n, const int* answered, const uint64_t* started, const uint64_t* finished, const double* nowS, int* reported)
+{
+    CHK_PTR_NULL(answered); CHK_PTR_NULL(started); CHK_PTR_NULL(finished); CHK_PTR_NULL(nowS); CHK_PTR_NULL(reported);
+    StuckDetector d(budgetS);
+    for (uint32_t i = 0; i < n; ++i) reported[i] = d.Observe(answered[i] != 0, started[i], finished[i], nowS[i]);
+    return HCCL_SUCCESS;
+}
+
+// Operators started and finished on this rank's device so far (what the stuck detection compares).  HCCL_E_AGAIN: no answer within a second.
 HcclResult HcclDebugOpCounters(HcclComm comm, uint64_t* started, uint64_t* finished)
 {
     CHK_PTR_NULL(comm);

@@ -7,6 +7,7 @@
 #include "../topo/topo.h"
 #include "log.h"
 #include "plan_cache.h"
+#include "stuck_detector.h"
 #include "../cpu/host_comm.h"
 
 namespace hccl {
@@ -70,6 +71,22 @@ StageLayout MakeStageLayout(uint64_t dataBytes, int nRanks)
     return l;
 }
 
+// The stream of the current device on which its communicators' counters are copied; it goes with the last of them.
+static std::shared_ptr<CUstream_st> CountersStream()
+{
+    static std::mutex mu;
+    static std::map<int, std::weak_ptr<CUstream_st>> streams;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    if (std::shared_ptr<CUstream_st> there = streams[device].lock()) return there;
+    cudaStream_t s = nullptr;
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+    std::shared_ptr<CUstream_st> made(s, [](cudaStream_t x) { cudaStreamDestroy(x); });
+    streams[device] = made;
+    return made;
+}
+
 HcclResult CommImpl::SetupDeviceState()
 {
     CHK_CUDA(cudaMalloc(&dEpochs_, kEpochWords * sizeof(uint64_t)));
@@ -81,7 +98,9 @@ HcclResult CommImpl::SetupDeviceState()
     CHK_CUDA(cudaHostAlloc((void**)&hStatus_, sizeof(DevStatus), cudaHostAllocMapped | cudaHostAllocPortable));
     memset((void*)hStatus_, 0, sizeof(DevStatus));
     CHK_CUDA(cudaHostGetDevicePointer((void**)&dStatus_, (void*)hStatus_, 0));
-    CHK_CUDA(cudaStreamCreateWithFlags(&countersStream_, cudaStreamNonBlocking));
+    countersStream_ = CountersStream();
+    if (!countersStream_) return HCCL_E_RUNTIME;
+    CHK_CUDA(cudaEventCreateWithFlags(&countersBack_, cudaEventDisableTiming));
     CHK_CUDA(cudaHostAlloc((void**)&hCounters_, 2 * sizeof(uint64_t), cudaHostAllocPortable));
     dev_->rank = rank;
     dev_->nRanks = nRanks;
@@ -198,9 +217,10 @@ HcclResult CommImpl::Destroy()
     userSegs_.clear();
     if (ownsSlab_) SymFree(&slab_);
     std::lock_guard<std::mutex> counters(countersMu_);
-    if (countersStream_) cudaStreamDestroy(countersStream_);
+    if (countersBack_) cudaEventDestroy(countersBack_);
     if (hCounters_) cudaFreeHost(hCounters_);
-    countersStream_ = nullptr; hCounters_ = nullptr;
+    countersStream_.reset();
+    countersBack_ = nullptr; hCounters_ = nullptr; countersAsked_ = false;
     if (dEpochs_) cudaFree(dEpochs_);
     if (dAbort_) cudaFree(dAbort_);
     if (dP2pSeq_) cudaFree(dP2pSeq_);
@@ -386,18 +406,37 @@ bool CommImpl::Lookup(const void* p, uint64_t bytes, const char* peerPtr[HCCL_MA
     return false;
 }
 
-HcclResult CommImpl::ReadOpCounters(uint64_t* started, uint64_t* finished)
+HcclResult CommImpl::ReadOpCounters(uint64_t* started, uint64_t* finished, int limitMs, const std::atomic<bool>* stop)
 {
     CHK_PTR_NULL(started); CHK_PTR_NULL(finished);
     std::lock_guard<std::mutex> lk(countersMu_);
     if (!dEpochs_ || !countersStream_) return HCCL_E_NOT_SUPPORT;
     // another thread's stream capture is none of this thread's business
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaSuccess) return HCCL_E_RUNTIME;             // the process is on its way out
-    e = cudaMemcpyAsync(hCounters_, dEpochs_ + 2 * kMaxBlocks, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, countersStream_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(countersStream_);
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return HCCL_E_RUNTIME;             // the process is on its way out
+    const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(limitMs);
+    bool earlier = countersAsked_;      // the answer on its way is to an earlier call: it frees the buffer, then the device is asked again
+    cudaError_t e = cudaSuccess;
+    for (;;) {
+        if (!countersAsked_) {
+            e = cudaMemcpyAsync(hCounters_, dEpochs_ + 2 * kMaxBlocks, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, countersStream_.get());
+            if (e == cudaSuccess) e = cudaEventRecord(countersBack_, countersStream_.get());
+            if (e != cudaSuccess) break;
+            countersAsked_ = true;
+        }
+        e = cudaEventQuery(countersBack_);
+        if (e == cudaSuccess) {
+            countersAsked_ = false;
+            if (!earlier) break;
+            earlier = false;
+            continue;
+        }
+        if (e == cudaErrorNotReady) cudaGetLastError();          // no error that the thread's next check should find
+        if (e != cudaErrorNotReady || (stop != nullptr && stop->load()) || std::chrono::steady_clock::now() >= until) break;
+        std::this_thread::sleep_for(std::chrono::microseconds(200));
+    }
     cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaErrorNotReady) return HCCL_E_AGAIN;
     if (e != cudaSuccess) return HCCL_E_RUNTIME;
     *started = hCounters_[0];
     *finished = hCounters_[1];
@@ -407,24 +446,18 @@ HcclResult CommImpl::ReadOpCounters(uint64_t* started, uint64_t* finished)
 void CommImpl::WatchdogLoop()
 {
     cudaSetDevice(device);
-    // head != tail with no progress for a whole wait budget = an op is stuck between its start and its end
-    // (reference: per-communicator head/tail counters compared by a host watchdog, stuck_detect_counter_helper.h).
-    uint64_t lastHead = 0, lastTail = 0;
-    auto lastChange = std::chrono::steady_clock::now();
+    StuckDetector detector((double)DeriveTimeouts(cfg.execTimeoutNs).fullNs * 1e-9);
     while (!watchdogStop_.load()) {
         for (int i = 0; i < 10 && !watchdogStop_.load(); ++i) std::this_thread::sleep_for(std::chrono::milliseconds(100));
         uint64_t h = 0, t = 0;
-        if (watchdogStop_.load() || ReadOpCounters(&h, &t) != HCCL_SUCCESS) continue;
-        auto now = std::chrono::steady_clock::now();
-        if (h != lastHead || t != lastTail) { lastHead = h; lastTail = t; lastChange = now; continue; }
-        if (h != t) {
-            const double idle = std::chrono::duration<double>(now - lastChange).count();
-            if (idle * 1e9 > (double)DeriveTimeouts(cfg.execTimeoutNs).fullNs) {
-                stuckReports.fetch_add(1);
-                HCCL_ERROR("comm %s rank %d: stuck detection: %llu ops started, %llu finished, no progress for %.0f s",
-                           name.c_str(), rank, (unsigned long long)h, (unsigned long long)t, idle);
-                lastChange = now;
-            }
+        if (watchdogStop_.load()) break;
+        const HcclResult r = ReadOpCounters(&h, &t, 1000, &watchdogStop_);
+        if (watchdogStop_.load() || (r != HCCL_SUCCESS && r != HCCL_E_AGAIN)) continue;
+        if (detector.Observe(r == HCCL_SUCCESS, h, t, std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count())) {
+            stuckReports.fetch_add(1);
+            HCCL_ERROR("comm %s rank %d: stuck detection: %llu ops started, %llu finished, no progress for %.0f s%s", name.c_str(), rank,
+                       (unsigned long long)detector.started(), (unsigned long long)detector.finished(), detector.idleS(),
+                       r == HCCL_SUCCESS ? "" : " (the device does not answer)");
         }
     }
 }

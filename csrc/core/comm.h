@@ -129,13 +129,17 @@ private:
     std::thread watchdog_;
     std::atomic<bool> watchdogStop_{false};
     void WatchdogLoop();
-    // ops started and finished, copied from device memory on a stream of their own
-    cudaStream_t countersStream_ = nullptr;
+    // ops started and finished, copied from device memory on a stream that all communicators of the device share
+    std::shared_ptr<CUstream_st> countersStream_;
+    cudaEvent_t countersBack_ = nullptr;
+    bool countersAsked_ = false;        // a copy is on its way; countersBack_ is behind it
     uint64_t* hCounters_ = nullptr;     // pinned, two words
     std::mutex countersMu_;
 public:
-    // Ops started and finished on this rank so far; does not wait for kernels in flight.
-    HcclResult ReadOpCounters(uint64_t* started, uint64_t* finished);
+    // Ops started and finished on this rank so far.  The device is asked and waited for, `limitMs` at most and only until `*stop`:
+    // HCCL_E_AGAIN then, and the next call looks for the same answer.  Normally the copy passes kernels in flight, but where
+    // streams share a hardware queue (CUDA_DEVICE_MAX_CONNECTIONS, more streams than queues) it may lie behind them.
+    HcclResult ReadOpCounters(uint64_t* started, uint64_t* finished, int limitMs = 1000, const std::atomic<bool>* stop = nullptr);
     std::atomic<uint64_t> stuckReports{0};
 };
 

@@ -2,19 +2,22 @@
 // itself without Python or ctypes objects in between.  A decode step's operators take 4 .. 10 us on the device; with Python-level
 // allocations and ctypes a call of one took 10 .. 18 us of the host.
 //
-// Every function takes only what is plain: dense CUDA tensors that no transform, subclass, dispatch mode, forward-mode
-// gradient or tracer looks at, and that no gradient is recorded for.  For anything else it returns None and the caller goes
-// the general way (torch.autograd.Function, ctypes), which also words the errors.  An int is the HcclResult of a failed call.
+// Every function takes only what is plain: dense CUDA tensors that no transform, subclass, dispatch or function mode,
+// forward-mode gradient or tracer looks at, and that no gradient is recorded for.  For anything else it returns None and the
+// caller goes the general way (torch.autograd.Function, ctypes), which also words the errors.  An int is the HcclResult of a
+// failed call.
 //
 // The functions of the C API come as addresses (`bind`), so that this module and the ctypes binding always use the same library.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <cstdint>
@@ -48,10 +51,20 @@ const Slot kSlots[] = {
     {"HcclAllGather", (void**)&api.allGather},              {"HcclAlltoAll", (void**)&api.alltoAll},
 };
 
-// A call that nothing but its own arithmetic is asked of: no tracer, no dispatch mode, no functional transform around it.
+// The function mode behind torch.set_default_device and `with torch.device(...)`.  It gives a device to factory calls that name
+// none; these calls name theirs, so that it has nothing to see here.
+PyTypeObject* defaultDeviceMode = nullptr;
+bool FunctionModes()
+{
+    if (!at::impl::torch_function_mode_enabled()) return false;
+    for (int64_t i = 0; i < at::impl::PythonTorchFunctionTLS::stack_len(); ++i)
+        if (Py_TYPE(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter())) != defaultDeviceMode) return true;
+    return false;
+}
+// A call that nothing but its own arithmetic is asked of: no tracer, no mode, no functional transform around it.
 bool PlainCall()
 {
-    return !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+    return !FunctionModes() && !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
            !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 // A dense CUDA tensor that nothing looks at and nothing is recorded for.
@@ -60,7 +73,8 @@ bool Plain(const Tensor& t)
     return t.is_cuda() && t.layout() == at::kStrided && !(t.requires_grad() && c10::GradMode::is_enabled()) && !at::isTensorSubclassLike(t) &&
            !t._fw_grad(0).defined();
 }
-const Tensor* Get(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+// Tensors and parameters themselves: a subclass may have a __torch_function__ of its own.
+const Tensor* Get(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
 const Tensor* GetPlain(PyObject* o)
 {
     const Tensor* t = Get(o);
@@ -74,6 +88,13 @@ const Tensor* GetPlainBf16(PyObject* o)
 void* Stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 void* StreamOf(PyObject* o) { return o == Py_None ? Stream() : PyLong_AsVoidPtr(o); }
 PyObject* None() { Py_RETURN_NONE; }
+// An argument that is not what it is here (a float where an int is meant, say): the general way makes of it what it can.
+bool Odd()
+{
+    const bool odd = PyErr_Occurred() != nullptr;
+    if (odd) PyErr_Clear();
+    return odd;
+}
 PyObject* Wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
 template <class... T> PyObject* WrapAll(T... t)
 {
@@ -141,6 +162,7 @@ PyObject* RmsNormBwd(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
         if (w->numel() != x->size(-1) || (uint64_t)rstd->numel() != rows) return None();
         const bool twice = PyObject_IsTrue(a[5]);
+        if (Odd()) return None();
         Tensor dx, dw, copy;
         const int r = [&] {
             Unlocked unlocked;
@@ -208,6 +230,7 @@ PyObject* Rope(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         for (const Tensor* t : {c, s})
             if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() < rows * (d / 2)) return None();
         const int backward = PyObject_IsTrue(a[3]);
+        if (Odd()) return None();
         Tensor out;
         const int r = [&] {
             Unlocked unlocked;
@@ -231,10 +254,10 @@ PyObject* Matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs)
             if (t && (!t->is_cuda() || t->layout() != at::kStrided || t->scalar_type() != at::kBFloat16 || t->dim() != 2 || at::isTensorSubclassLike(*t))) return None();
         if (!a->is_contiguous() || !b->is_contiguous()) return None();
         const bool ta = PyObject_IsTrue(args[2]), tb = PyObject_IsTrue(args[3]);
+        void* stream = StreamOf(args[5]);
+        if (Odd()) return None();
         const int64_t m = a->size(ta ? 1 : 0), k = a->size(ta ? 0 : 1), n = b->size(tb ? 0 : 1);
         if (b->size(tb ? 1 : 0) != k) return None();
-        void* stream = StreamOf(args[5]);
-        if (stream == nullptr && PyErr_Occurred()) return nullptr;
         Tensor out;
         const int r = [&] {
             Unlocked unlocked;
@@ -253,9 +276,8 @@ PyObject* ExpertOffsets(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         const Tensor* idx = GetPlain(a[0]);
         if (!idx || !PlainCall() || idx->scalar_type() != at::kInt || !idx->is_contiguous() || !PyLong_Check(a[1])) return None();
         const long n = PyLong_AsLong(a[1]);
-        if (n <= 0 || n > 0x7FFFFFFFL) { PyErr_Clear(); return None(); }
         void* stream = StreamOf(a[2]);
-        if (stream == nullptr && PyErr_Occurred()) return nullptr;
+        if (Odd() || n <= 0 || n > 0x7FFFFFFFL) return None();
         Tensor out;
         const int r = [&] {
             Unlocked unlocked;
@@ -287,8 +309,7 @@ PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
             if (!t->is_cuda() || t->layout() != at::kStrided || !t->is_contiguous() || at::isTensorSubclassLike(*t)) return None();
         const int type = TypeOf(*send), which = (int)PyLong_AsLong(a[0]), op = (int)PyLong_AsLong(a[4]), ranks = (int)PyLong_AsLong(a[5]);
         void *comm = PyLong_AsVoidPtr(a[1]), *stream = StreamOf(a[6]);
-        if (PyErr_Occurred()) return nullptr;
-        if (type < 0 || TypeOf(*recv) != type || comm == nullptr || ranks < 1) return None();
+        if (Odd() || type < 0 || TypeOf(*recv) != type || comm == nullptr || ranks < 1) return None();
         const void* s = send->const_data_ptr();
         void* r = recv->data_ptr();
         const uint64_t nSend = (uint64_t)send->numel(), nRecv = (uint64_t)recv->numel();
@@ -307,6 +328,14 @@ PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
 
 PyObject* Bind(PyObject*, PyObject* addresses)
 {
+    if (defaultDeviceMode == nullptr) {
+        PyObject* devices = PyImport_ImportModule("torch.utils._device");
+        PyObject* mode = devices ? PyObject_GetAttrString(devices, "DeviceContext") : nullptr;
+        if (mode && PyType_Check(mode)) defaultDeviceMode = reinterpret_cast<PyTypeObject*>(mode);          // kept
+        else Py_XDECREF(mode);
+        Py_XDECREF(devices);
+        PyErr_Clear();                 // another torch without it: its default devices go the general way
+    }
     for (const Slot& s : kSlots) {
         PyObject* v = PyDict_GetItemString(addresses, s.name);
         void* p = v ? PyLong_AsVoidPtr(v) : nullptr;

@@ -110,6 +110,52 @@ def test_transforms_modes_and_tracers_see_the_operators():
     assert traced == [None]
 
 
+def test_torch_function_sees_the_operators():
+    """Subclasses and modes that know __torch_function__ only: what they get is what the general way gives them."""
+    from torch.overrides import TorchFunctionMode
+
+    class Named(torch.Tensor):
+        pass
+
+    x, d, w = _rnd(4, 64), _rnd(4, 64, seed=1), _rnd(64)
+    c, s = _tables(4, 16)
+    n = x.as_subclass(Named)
+    assert _calls.add_rms_norm(n, None, w, 1e-5) is None and _calls.add_rms_norm(x, d.as_subclass(Named), w, 1e-5) is None
+    assert _calls.swiglu_fwd(n) is None and _calls.rope(n.view(4, 4, 16), c, s, False) is None
+    assert _calls.matmul(n, x, False, True, None, None) is None and _calls.expert_offsets(torch.zeros(4, device="cuda", dtype=torch.int32).as_subclass(Named), 4, None) is None
+    x_out, h = fused.add_rms_norm(n, d, w, 1e-5)
+    assert type(x_out) is Named and type(h) is Named
+    want = fused.add_rms_norm(x, d, w, 1e-5)
+    assert torch.equal(torch.Tensor(x_out), torch.Tensor(want[0])) and torch.equal(torch.Tensor(h), torch.Tensor(want[1]))
+    assert _calls.swiglu_fwd(torch.nn.Parameter(x, requires_grad=False)) is not None
+    seen = []
+
+    class Count(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    with Count():
+        assert _calls.swiglu_fwd(x) is None
+        fused.swiglu(x)
+    assert seen
+    with torch.device("cpu"):                                                   # a default device is no such mode
+        assert _calls.swiglu_fwd(x) is not None
+        with Count():
+            assert _calls.swiglu_fwd(x) is None
+    assert _calls.swiglu_fwd(x) is not None
+
+
+def test_arguments_of_other_types_are_left_to_the_general_way():
+    a, b = _rnd(8, 16), _rnd(8, 16, seed=1)
+    assert _calls.matmul(a, b, torch.zeros(2), True, None, None) is None        # no truth value
+    assert _calls.matmul(a, b, False, True, None, "a stream") is None
+    assert _calls.expert_offsets(torch.zeros(4, device="cuda", dtype=torch.int32), 4, 1.5) is None
+    assert _calls.collective(0, 1, a.float(), b.float(), 0.0, 2, None) is None
+    with pytest.raises(RuntimeError):
+        mc2.matmul(a, b, trans_a=torch.zeros(2))
+
+
 def test_saved_tensor_hooks_are_called():
     x, w = _rnd(4, 64).requires_grad_(), _rnd(64).requires_grad_()
     packed = []

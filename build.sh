@@ -54,7 +54,7 @@ if [ $pkg -eq 1 ]; then
   cp -r csrc/include/hccl "$root/include/"
   tar -C . --exclude='__pycache__' --exclude='*.so' -cf - hccl_b200 | tar -C "$root/python" -xf -
   mkdir -p "$root/python/hccl_b200/lib" && cp hccl_b200/lib/libhccl_b200.so "$root/python/hccl_b200/lib/"
-  if [ -f hccl_b200/lib/hccl_b200_torch.so ]; then cp hccl_b200/lib/hccl_b200_torch.so "$root/python/hccl_b200/lib/"; fi
+  for f in hccl_b200/lib/hccl_b200_torch.*.so; do if [ -f "$f" ]; then cp "$f" "$root/python/hccl_b200/lib/"; fi; done
   cp -r examples docs README.md "$root/"
   tar -C "$stage" -czf "dist/hccl_b200-$version.tar.gz" "hccl_b200-$version"
   rm -rf "$stage"

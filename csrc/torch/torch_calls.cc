@@ -21,24 +21,28 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <cstdint>
+#include "hccl/hccl.h"
+#include "hccl/hccl_fused_ops.h"
+#include "hccl/hccl_mc2.h"
+#include "hccl/hccl_moe.h"
 
 namespace {
 
 using at::Tensor;
 
 struct Api {
-    int (*addRmsNormFwd)(const void*, const void*, const void*, void*, void*, void*, uint64_t, uint32_t, float, void*);
-    uint32_t (*rmsNormBwdPartials)(uint64_t);
-    int (*rmsNormBwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, uint64_t, uint32_t, void*);
-    int (*swigluFwd)(const void*, void*, uint64_t, uint32_t, void*);
-    int (*swigluBwd)(const void*, const void*, void*, uint64_t, uint32_t, void*);
-    int (*rope)(const void*, uint64_t, void*, uint64_t, const void*, const void*, uint64_t, uint32_t, uint32_t, int, void*);
-    int (*matmul)(const void*, const void*, void*, uint64_t, uint64_t, uint64_t, int, int, void*);
-    int (*expertOffsets)(const int32_t*, uint64_t, uint32_t, uint32_t*, void*);
-    int (*allReduce)(const void*, void*, uint64_t, int, int, void*, void*);
-    int (*reduceScatter)(const void*, void*, uint64_t, int, int, void*, void*);
-    int (*allGather)(const void*, void*, uint64_t, int, void*, void*);
-    int (*alltoAll)(const void*, uint64_t, int, const void*, uint64_t, int, void*, void*);
+    decltype(&HcclFusedAddRmsNormFwd) addRmsNormFwd;
+    decltype(&HcclFusedRmsNormBwdPartials) rmsNormBwdPartials;
+    decltype(&HcclFusedRmsNormBwdCopy) rmsNormBwd;
+    decltype(&HcclFusedSwigluFwd) swigluFwd;
+    decltype(&HcclFusedSwigluBwd) swigluBwd;
+    decltype(&HcclFusedRope) rope;
+    decltype(&HcclMc2Matmul) matmul;
+    decltype(&HcclMoeExpertOffsets) expertOffsets;
+    decltype(&HcclAllReduce) allReduce;
+    decltype(&HcclReduceScatter) reduceScatter;
+    decltype(&HcclAllGather) allGather;
+    decltype(&HcclAlltoAll) alltoAll;
 };
 Api api;
 struct Slot { const char* name; void** at; };
@@ -288,13 +292,13 @@ PyObject* ExpertOffsets(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     });
 }
 
-// HcclDataType of a tensor's elements, -1 where the general way has to look
-int TypeOf(const Tensor& t)
+// HcclDataType of a tensor's elements, HCCL_DATA_TYPE_RESERVED where the general way has to look
+HcclDataType TypeOf(const Tensor& t)
 {
     switch (t.scalar_type()) {
-        case at::kFloat: return 4;
-        case at::kBFloat16: return 11;
-        default: return -1;
+        case at::kFloat: return HCCL_DATA_TYPE_FP32;
+        case at::kBFloat16: return HCCL_DATA_TYPE_BFP16;
+        default: return HCCL_DATA_TYPE_RESERVED;
     }
 }
 enum Which { ALL_REDUCE, REDUCE_SCATTER, ALL_GATHER, ALL_TO_ALL };
@@ -307,11 +311,12 @@ PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         if (!send || !recv || !PlainCall()) return None();
         for (const Tensor* t : {send, recv})
             if (!t->is_cuda() || t->layout() != at::kStrided || !t->is_contiguous() || at::isTensorSubclassLike(*t)) return None();
-        const int type = TypeOf(*send), which = (int)PyLong_AsLong(a[0]), op = (int)PyLong_AsLong(a[4]), ranks = (int)PyLong_AsLong(a[5]);
+        const HcclDataType type = TypeOf(*send);
+        const int which = (int)PyLong_AsLong(a[0]), ranks = (int)PyLong_AsLong(a[5]);
+        const HcclReduceOp op = (HcclReduceOp)PyLong_AsLong(a[4]);
         void *comm = PyLong_AsVoidPtr(a[1]), *stream = StreamOf(a[6]);
-        if (Odd() || type < 0 || TypeOf(*recv) != type || comm == nullptr || ranks < 1) return None();
-        const void* s = send->const_data_ptr();
-        void* r = recv->data_ptr();
+        if (Odd() || type == HCCL_DATA_TYPE_RESERVED || TypeOf(*recv) != type || comm == nullptr || ranks < 1) return None();
+        void *s = const_cast<void*>(send->const_data_ptr()), *r = recv->data_ptr();
         const uint64_t nSend = (uint64_t)send->numel(), nRecv = (uint64_t)recv->numel();
         const int code = [&] {
             Unlocked unlocked;          // a first call may wait for the other ranks' threads

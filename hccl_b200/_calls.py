@@ -1,7 +1,8 @@
-"""Calls of the C API with torch tensors through the native module ``lib/hccl_b200_torch.so`` (csrc/torch/torch_calls.cc).
+"""Calls of the C API with torch tensors through the native module of csrc/torch/torch_calls.cc.
 
 Each function takes what is plain and returns ``None`` for everything else; the caller then goes the general way through
-``torch.autograd.Function`` and ctypes.  Where the module is not there (a library without it, another torch) that is every call.
+``torch.autograd.Function`` and ctypes.  Where the module is not there (a library without it; a Python or a torch other than
+the ones it was built for, which its file name holds) that is every call.
 ``result`` turns the answer into the outputs, or raises for the ``HcclResult`` of a call that failed.
 """
 from __future__ import annotations
@@ -10,14 +11,12 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import warnings
-from pathlib import Path
 
 import torch          # its libraries have to be loaded before the module's
 
 from ._lib import lib
+from .build import torch_lib
 from .comm import _check
-
-_PATH = Path(__file__).resolve().parent / "lib" / "hccl_b200_torch.so"
 
 
 def _nothing(*_):
@@ -25,15 +24,16 @@ def _nothing(*_):
 
 
 def _load():
+    path = torch_lib()
     try:
-        loader = importlib.machinery.ExtensionFileLoader("hccl_b200_torch", str(_PATH))
+        loader = importlib.machinery.ExtensionFileLoader("hccl_b200_torch", str(path))
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("hccl_b200_torch", loader))
         loader.exec_module(module)
         module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in module.names()})
         return module
     except (ImportError, AttributeError) as e:
         if torch.cuda.is_available():
-            warnings.warn(f"{_PATH.name} cannot be loaded ({e}): calls take the slower way through ctypes; `python hccl_b200/build.py` builds it")
+            warnings.warn(f"{path.name} cannot be loaded ({e}): calls take the slower way through ctypes; `python hccl_b200/build.py` builds it")
         return None
 
 

@@ -9,8 +9,8 @@ header is newer.  Usage: ``python hccl_b200/build.py [--force] [--verbose] [--pt
 bootstrap, host engine, verifier) is compiled with AddressSanitizer; the CUDA objects are shared with the normal
 build.  Load it with ``HCCL_B200_LIB=<path> LD_PRELOAD=$(gcc -print-file-name=libasan.so)`` (the interpreter itself
 is not instrumented, so the runtime has to come first), ``ASAN_OPTIONS=detect_leaks=0``.
-Beside the library goes ``hccl_b200/lib/hccl_b200_torch.so``, a Python module built against torch's headers (where torch is
-installed).
+Beside the library goes ``hccl_b200/lib/hccl_b200_torch.<Python ABI>.torch-<version>.so``, a Python module built against torch's
+headers (where torch is installed, with CUDA).
 ``--cov`` builds ``build/lib/libhccl_b200_cov.so`` with ``--coverage``; after running tests against it
 (``HCCL_B200_LIB=<path>``), ``--cov-report`` prints the line coverage of every host source.
 """
@@ -21,6 +21,8 @@ import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
+import warnings
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -32,7 +34,6 @@ CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 
 TORCH_SRC = CSRC / "torch" / "torch_calls.cc"          # a Python module of its own, against torch's headers
-TORCH_LIB = LIB_DIR / "hccl_b200_torch.so"
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -110,26 +111,42 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
     return LIB
 
 
-def build_torch_calls(force: bool = False, verbose: bool = False) -> Path:
-    """The Python module that makes the C API's calls with torch tensors (csrc/torch/torch_calls.cc).  It gets the C functions'
-    addresses at run time, so it is not linked to the library."""
-    if not force and TORCH_LIB.exists() and TORCH_LIB.stat().st_mtime >= TORCH_SRC.stat().st_mtime:
-        return TORCH_LIB
-    import sysconfig
+def torch_lib() -> Path:
+    """Where that module lies for this Python and this torch.  It inlines their data layouts, so its name holds both: another
+    version does not find it, instead of loading it as long as its symbols resolve."""
+    import torch
 
+    return LIB_DIR / f"hccl_b200_torch.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so"
+
+
+def build_torch_calls(force: bool = False, verbose: bool = False) -> Path | None:
+    """The Python module that makes the C API's calls with torch tensors (csrc/torch/torch_calls.cc).  It gets the C functions'
+    addresses at run time, so it is not linked to the library, and the library does not need it: where it cannot be built (a torch
+    without CUDA) that is a warning."""
+    out = torch_lib()
+    newest = max(p.stat().st_mtime for p in (TORCH_SRC, *(CSRC / "include").rglob("*.h")))
+    for old in LIB_DIR.glob("hccl_b200_torch*.so"):          # also those of other versions: they call the C API as it was
+        if force or old.stat().st_mtime < newest:
+            old.unlink()
+    if out.exists():
+        return out
     import torch
 
     home = Path(torch.__file__).resolve().parent
     LIB_DIR.mkdir(parents=True, exist_ok=True)
+    part = out.with_suffix(".part")
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-Wall", "-Wno-unused-function", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           f"-I{home / 'include'}", f"-I{home / 'include/torch/csrc/api/include'}", f"-I{CUDA_HOME / 'include'}", f"-I{sysconfig.get_paths()['include']}",
-           str(TORCH_SRC), "-o", str(TORCH_LIB), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda"]
+           f"-I{CSRC / 'include'}", f"-I{home / 'include'}", f"-I{home / 'include/torch/csrc/api/include'}", f"-I{CUDA_HOME / 'include'}",
+           f"-I{sysconfig.get_paths()['include']}", str(TORCH_SRC), "-o", str(part), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10",
+           "-lc10_cuda"]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"compiling {TORCH_SRC.name} failed:\n{r.stdout}\n{r.stderr}")
-    return TORCH_LIB
+        warnings.warn(f"{TORCH_SRC.name} cannot be compiled against torch {torch.__version__}; calls with tensors take the slower way through ctypes:\n{r.stdout}\n{r.stderr}")
+        return None
+    part.replace(out)
+    return out
 
 
 def _build_variant(obj_dir: Path, lib: Path, cxx_extra, link_extra, verbose: bool) -> Path:

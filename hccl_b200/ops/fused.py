@@ -112,7 +112,7 @@ class _AddRmsNorm(torch.autograd.Function):
             dh = torch.zeros_like(x_out)
         dh = dh.contiguous()
         extra = dx_out.contiguous() if dx_out is not None else None
-        twice = ctx.has_delta and _kept_apart(ctx.next_functions[0][0], ctx.next_functions[1][0])
+        twice = ctx.has_delta and hasattr(lib, "HcclFusedRmsNormBwdCopy") and _kept_apart(ctx.next_functions[0][0], ctx.next_functions[1][0])
         r = _calls.rms_norm_bwd(dh, x_out, weight, rstd, extra, twice)
         if r is not None:
             dx, dw, copy = _calls.result(r, "HcclFusedRmsNormBwdCopy")
@@ -123,8 +123,12 @@ class _AddRmsNorm(torch.autograd.Function):
         dw = torch.empty_like(weight)
         n_part = lib.HcclFusedRmsNormBwdPartials(rows)
         partial = torch.empty((n_part, hidden), device=x_out.device, dtype=torch.float32)
-        _check(lib.HcclFusedRmsNormBwdCopy(_p(dh), _p(x_out), _p(weight), _p(rstd), _p(extra), _p(dx), _p(copy) if twice else ctypes.c_void_p(0), _p(partial),
-                                           _p(dw), rows, hidden, _s()), "HcclFusedRmsNormBwdCopy")
+        if twice:
+            _check(lib.HcclFusedRmsNormBwdCopy(_p(dh), _p(x_out), _p(weight), _p(rstd), _p(extra), _p(dx), _p(copy), _p(partial), _p(dw), rows, hidden,
+                                               _s()), "HcclFusedRmsNormBwdCopy")
+        else:                                   # also what a library without the other has
+            _check(lib.HcclFusedRmsNormBwd(_p(dh), _p(x_out), _p(weight), _p(rstd), _p(extra), _p(dx), _p(partial), _p(dw), rows, hidden, _s()),
+                   "HcclFusedRmsNormBwd")
         _count(2)
         return dx, (copy if ctx.has_delta else None), dw, None
 

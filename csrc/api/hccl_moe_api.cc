@@ -30,7 +30,7 @@ namespace {
 HcclResult CheckCfg(const CommImpl* c, const HcclMoeConfig* cfg)
 {
     if (!cfg) return HCCL_E_PTR;
-    if (cfg->hidden == 0 || cfg->hidden % 128 != 0 || cfg->hidden > 8192) { HCCL_ERROR("MoE: hidden must be a multiple of 128 up to 8192 (got %u)", cfg->hidden); return HCCL_E_PARA; }
+    if (cfg->hidden == 0 || cfg->hidden % 128 != 0 || cfg->hidden > (uint32_t)kMoeMaxHidden) { HCCL_ERROR("MoE: hidden must be a multiple of 128 up to %d (got %u)", kMoeMaxHidden, cfg->hidden); return HCCL_E_PARA; }
     if (cfg->topk == 0 || cfg->topk > (uint32_t)kMoeMaxTopk) { HCCL_ERROR("MoE: topk must be 1..%d (got %u)", kMoeMaxTopk, cfg->topk); return HCCL_E_PARA; }
     if (cfg->nExperts == 0 || cfg->nExperts > (uint32_t)kMoeMaxExperts || cfg->nExperts % (uint32_t)c->nRanks != 0) {
         HCCL_ERROR("MoE: the number of experts must be a multiple of the %d ranks, at most %d (got %u)", c->nRanks, kMoeMaxExperts, cfg->nExperts);

@@ -439,8 +439,11 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     const bool twoSm = sw.twoSm && ((!narrow && m >= 256) || (m > 128 && k >= 2048 && (uint64_t)tilesM2 * ((n + 127) / 128) * 5 >= (uint64_t)pairs * 4));
     // Two-SM tiles with the inner dimension split over a cluster of CTA pairs (see mc2_gemm_2sm_split.cuh): from 129 rows on, where
     // 256 x 128 tiles do not outnumber the pairs and the inner dimension pays for the sum.  At 129 .. 192 rows a quarter and more
-    // of the 256 is padding, and the token split stays ahead where it has a long inner dimension (129 x 4096 x 14336: 28.9 us
-    // against 30.3).  The token split stores 8 bytes at a time, all other routes 16: an output that lies on 8 bytes only keeps it.
+    // of the 256 is padding, and with an inner dimension of 4096 and more the token split keeps them.  Token split and pairs, us,
+    // back to back: 129 x 4096 x 4096 13.7 and 13.9, x 8192 20.6 and 21.2, x 14336 31.8 and 32.5, 129 x 7168 x 4096 18.5 and 19.1, 160 x
+    // 4096 x 4096 13.7 and 13.9.  The line is not the best one: the pairs are ahead at few columns (129 x 1024 x 8192 15.9 and 14.0,
+    // 160 x 2048 x 8192 17.2 and 16.3) and from 176 rows on (176 x 4096 x 4096 14.6 and 13.9, 192 x 1024 x 8192 18.4 and 14.1, 192 x 4096 x
+    // 14336 35.3 and 32.4); moving it changes the order in which those products are summed.  The token split stores 8 bytes at a time, all other routes 16: an output that lies on 8 bytes only keeps it.
     const uint64_t tiles128 = (uint64_t)tilesM2 * ((n + 127) / 128);
     if (sw.twoSm && outAlign >= 16 && m > 128 && k >= 2048 && tiles128 <= (uint64_t)pairs && (m > 192 || k < 4096 || twoSm)) {
         p.route = MatmulRoute::TWO_SM_SPLIT;

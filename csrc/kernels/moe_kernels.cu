@@ -59,8 +59,9 @@ __global__ void MoeCountKernel(const int32_t* __restrict__ topkIdx, int nPairs, 
 // The same inside one block for up to kMoeCountInDispatch pairs, in an order that depends on the pairs alone, so that every
 // block of a launch counts for itself and all agree: a warp takes a run of consecutive pairs, 32 at a time (lanes with the
 // same expert find each other by match.any), and a scan over the warps' counters gives each run its start.  It saves the
-// counting launch in front (2.1 .. 2.9 us and the boundary between the two) for 1 .. 5 us of the dispatch kernel: eight emulated
-// ranks, whose counting launches run one after the other, take 1149 -> 1120 us for a whole layer of 256 tokens.
+// counting launch in front (2.1 .. 2.9 us and the boundary between the two) for 1 .. 5 us of the dispatch kernel; up to where that
+// pays stands beside kMoeCountInDispatch.  Eight emulated ranks, whose counting launches run one after the other, take 1149 -> 1120
+// us for a whole layer of 256 tokens.
 struct CountScratch {
     uint16_t before[kMoeWarps][kMoeMaxExperts];       // pairs of an expert in a warp's run, then in the runs before it
     uint16_t pos[kMoeCountInDispatch];                // position of a pair among the pairs of its expert in its warp's run
@@ -261,7 +262,7 @@ struct CombineBody {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t stride = (uint32_t)nb * kMoeWarps;
         // parts per row: lane l weighs l + 1 of them by rounds of all warps x (pieces of a part + about two for its addresses)
-        static_assert(8192 / 8 <= 32 * 32, "as many parts to weigh as lanes");
+        static_assert(kMoeMaxHidden / 8 <= 32 * 32, "no row has more pieces, and so parts to weigh, than a warp has lanes");
         const uint32_t p = (uint32_t)lane + 1, rounds = ((uint32_t)a.nTokens * p + stride - 1) / stride;
         const uint32_t cost = p <= (uint32_t)nPieces ? rounds * (((uint32_t)nPieces + p - 1) / p + 2) : 0x3FFFFFFu;      // rows fit the GPU: far below 2^26
         const uint32_t parts = (__reduce_min_sync(0xffffffffu, min(cost, 0x3FFFFFFu) << 6 | (uint32_t)lane) & 63u) + 1;

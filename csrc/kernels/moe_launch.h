@@ -10,7 +10,13 @@ namespace hccl {
 
 constexpr int kMoeMaxExperts = 512;
 constexpr int kMoeMaxTopk = 8;
-constexpr int kMoeCountInDispatch = 4096;   // pairs up to which the dispatch kernel counts them itself
+constexpr int kMoeMaxHidden = 8192;
+// Pairs up to which the dispatch kernel counts them itself.  Against one counting launch in front, which is what a rank with a GPU of
+// its own saves (one rank, rows of 7168, top-8, us, in the kernel and with the launch): launched one by one 8 pairs 14.6 and 18.0, 512
+// 16.8 and 20.4, 2048 28.0 and 30.6, 4096 40.0 and 40.8, where the two meet; in a CUDA graph, where a launch costs less, 8 pairs 14.6 and
+// 15.3, 512 19.8 and 20.2, 1024 23.7 and 23.4, 2048 31.6 and 30.7, 4096 43.4 and 41.1.  Two emulated ranks, whose launches run one after the other,
+// gain at every size and either way (4096 pairs 42.5 and 48.0, in a graph 45.7 and 46.7).
+constexpr int kMoeCountInDispatch = 4096;
 constexpr size_t kMoeTableBytes = (size_t)kMaxBlocks * kMaxDevRanks * kMoeMaxExperts * sizeof(uint32_t);
 
 struct MoeDispatchArgs {

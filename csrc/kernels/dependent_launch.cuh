@@ -40,7 +40,9 @@ cudaError_t LaunchDependent(void (*kernel)(Params...), unsigned grid, unsigned b
     attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = cluster > 0 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();             // the caller has it: the check behind the next <<<>>> shall not find it
+    return e;
 }
 
 }  // namespace hccl

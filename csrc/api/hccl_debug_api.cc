@@ -285,5 +285,11 @@ HcclResult HcclDebugOpCounters(HcclComm comm, uint64_t* started, uint64_t* finis
     CHK_PTR_NULL(comm);
     return static_cast<CommImpl*>(comm)->ReadOpCounters(started, finished);
 }
+// The readings that follow lie behind what `stream` holds now, as a copy does that shares a hardware queue with a stuck operator.
+HcclResult HcclDebugOpCountersBehind(HcclComm comm, hcclStream_t stream)
+{
+    CHK_PTR_NULL(comm);
+    return static_cast<CommImpl*>(comm)->ReadOpCountersBehind((cudaStream_t)stream);
+}
 
 }  // extern "C"

@@ -443,6 +443,18 @@ HcclResult CommImpl::ReadOpCounters(uint64_t* started, uint64_t* finished, int l
     return HCCL_SUCCESS;
 }
 
+HcclResult CommImpl::ReadOpCountersBehind(cudaStream_t stream)
+{
+    std::lock_guard<std::mutex> lk(countersMu_);
+    if (!countersStream_) return HCCL_E_NOT_SUPPORT;
+    cudaEvent_t e = nullptr;
+    CHK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaError_t r = cudaEventRecord(e, stream);
+    if (r == cudaSuccess) r = cudaStreamWaitEvent(countersStream_.get(), e, 0);
+    cudaEventDestroy(e);
+    return r == cudaSuccess ? HCCL_SUCCESS : HCCL_E_RUNTIME;
+}
+
 void CommImpl::WatchdogLoop()
 {
     cudaSetDevice(device);

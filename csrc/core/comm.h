@@ -140,6 +140,8 @@ public:
     // HCCL_E_AGAIN then, and the next call looks for the same answer.  Normally the copy passes kernels in flight, but where
     // streams share a hardware queue (CUDA_DEVICE_MAX_CONNECTIONS, more streams than queues) it may lie behind them.
     HcclResult ReadOpCounters(uint64_t* started, uint64_t* finished, int limitMs = 1000, const std::atomic<bool>* stop = nullptr);
+    // Tests: the readings that follow lie behind what `stream` holds now.
+    HcclResult ReadOpCountersBehind(cudaStream_t stream);
     std::atomic<uint64_t> stuckReports{0};
 };
 

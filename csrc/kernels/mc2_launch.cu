@@ -1,5 +1,7 @@
 // Instantiation, tensor-map encoding and launch of the MC2 kernels (sm_100a).
 #include "mc2_launch.h"
+#include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <string>
@@ -137,7 +139,7 @@ HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const S
 {
     constexpr auto kernel = GemmSplitKernel<W_MN, X_MN>;
     CHK_RET(AllowSharedMemory<kernel>(kSplitMaxSmemBytes));
-    const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split), kThreads, (size_t)SplitSmemBytes(g.bt), stream, (unsigned)split, tw, tx, g);
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split), SplitThreads(g.bt), (size_t)SplitSmemBytes(g.barOffset), stream, (unsigned)split, tw, tx, g);
     if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -424,6 +426,124 @@ MatmulSwitches MatmulSwitchesOfEnv()
     return s;
 }
 
+namespace {
+
+// Estimated time of a small product on each kernel, in us on a B200.  Up to some 50 us a matmul is bound by what one SM takes in
+// (a k-block of a tile comes at 110 .. 145 GB/s from L2), by what a k-block costs at least, by a tile's drain and by whole rounds
+// of tiles, so the best kernel and cut are those that balance these four.  Fitted to 11000 timed calls (8 .. 8000 rows, 64 .. 16000
+// columns, inner dimensions of 64 .. 16000; cluster launches in a graph): off by 12 % (two-SM), 14 % (pairs), 17 % (token split),
+// 19 % (one-SM) in the root mean square, most of it in common; taking the best estimate instead of the best time costs 2-3 %.
+struct SmallProduct {
+    uint64_t m, n, k;
+    int kBlocks, sms;
+    double hbmUs;              // every operand and the output once at 6.3 TB/s
+    SmallProduct(uint64_t m, uint64_t n, uint64_t k, int sms)
+        : m(m), n(n), k(k), kBlocks((int)((k + kBK - 1) / kBK)), sms(sms), hbmUs(2.0 * ((double)m * k + (double)n * k + (double)m * n) / 6.3e6) {}
+};
+uint64_t CeilDiv(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
+double FourNorm(double a, double b) { return std::sqrt(std::sqrt(a * a * a * a + b * b * b * b)); }
+// CTAs of `cluster` that run together, one per SM (clusters stay within groups of SMs: 33 of four, 15 of eight on 148)
+double ResidentCtas(int cluster, int sms) { return cluster == 8 ? sms * (120. / 148) : (cluster >= 4 ? sms * (132. / 148) : sms); }
+
+double SplitUs(const SmallProduct& s, bool aMn, int bt, int wr, int split, bool* lone)
+{
+    // rows of MN-major activations with fewer than 64 tokens come in pieces that all CTAs read from the same few lines
+    const double block = 0.142 + (aMn && s.m < 64 ? 0.45 * (64 - (double)s.m) / 56 : 0);
+    const double ctas = (double)(CeilDiv(s.m, bt) * CeilDiv(s.n, wr) * split), resident = ResidentCtas(split, s.sms);
+    *lone = ctas <= resident;                                   // one per SM: the ring may take its whole shared memory
+    const double rounds = std::ceil(ctas / (resident * (*lone ? 1 : 2))), perSm = *lone ? 1 : std::min(2.0, std::ceil(ctas / resident));
+    const int stageBytes = SplitStageBytes(bt, wr), stages = SplitStages(bt, wr, *lone ? kSplitLoneRingBytes : kSplitRingBytes);
+    const double kb = std::ceil((double)s.kBlocks / split), tile = perSm * bt * wr / 16384.;
+    const double loads = rounds * kb * std::max({block, perSm * stageBytes / 145e3, 0.142 * 6 / stages});
+    const double hbm = 0.87 * s.hbmUs * std::pow(std::max(1.0, s.sms / std::min(ctas, resident)), 0.6);      // fewer SMs keep fewer bytes on their way
+    return 2.1 + (wr == 64 ? 0.8 : 0) + std::max(loads, hbm) + rounds * (2.1 * tile + (split > 1 ? 1.15 + 1.05 * tile : 0));
+}
+double OneSmUs(const SmallProduct& s, int bn)
+{
+    const double rounds = (double)CeilDiv(CeilDiv(s.m, kBM) * CeilDiv(s.n, bn), s.sms);
+    const double loads = s.kBlocks * (128 + bn) * 128 / 128.5e3, drain = 0.8 * bn / 128;
+    return 0.72 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 0.77 * rounds;
+}
+double PairsUs(const SmallProduct& s, int bn, int split)
+{
+    static const double resident[] = {0, 74, 66, 66, 60};       // CTA pairs
+    const double rounds = std::ceil((double)(CeilDiv(s.m, 256) * CeilDiv(s.n, bn) * split) / (resident[split] * s.sms / 148));
+    const double loads = std::ceil((double)s.kBlocks / split) * (128 + bn / 2) * 128 / 114.5e3, drain = 3.07 * bn / 128;
+    return 0.8 + std::max(rounds * (loads + drain + (split > 1 ? 2.54 : 0)), 3.07 + s.hbmUs);
+}
+double TwoSmUs(const SmallProduct& s, int bn)
+{
+    const double rounds = (double)CeilDiv(CeilDiv(s.m, 256) * CeilDiv(s.n, bn), s.sms / 2);
+    const double loads = s.kBlocks * (128 + bn / 2) * 128 / 111.7e3, drain = 0.72 * bn / 128;
+    return 1.73 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 1.6 * rounds;
+}
+// Another kernel, or another cut for the same one, is taken where its estimate is lower by more than the two are off against each other.
+constexpr double kOtherKernel = 0.87, kOtherCut = 0.9;
+
+// Best cut for the token split, its estimate in *us.
+MatmulPlan BestSplit(const SmallProduct& s, bool aMn, double* us)
+{
+    MatmulPlan best;
+    *us = 1e30;
+    for (int most : {128, 64, 32}) {
+        // equal token tiles of at most `most` (MN-major activations come in boxes of 64)
+        const int unit = aMn ? 64 : 16, parts = (int)CeilDiv(s.m, most);
+        const int bt = (int)(CeilDiv(CeilDiv(s.m, parts), unit) * unit);
+        if (bt > most || (parts > 1 && parts == (int)CeilDiv(s.m, 2 * most))) continue;
+        // smaller token tiles read the weights more often: from L2, where they fit it; 32 tokens were timed up to 128 rows
+        if (parts > (int)CeilDiv(s.m, 128) && s.n * s.k * 2 > (64u << 20)) continue;
+        if (most == 32 && s.m > 128) continue;
+        for (int wr : {128, 64}) {
+            if (wr == 64 && aMn) continue;
+            for (int split : {1, 2, 4, 8}) {
+                if (split > 1 && s.kBlocks < 2 * split) break;
+                bool lone;
+                const double t = SplitUs(s, aMn, bt, wr, split, &lone);
+                if (t >= *us) continue;
+                *us = t;
+                best.route = MatmulRoute::SPLIT;
+                best.bt = bt;
+                best.bn = wr;
+                best.tilesM = (int)CeilDiv(s.m, bt);
+                best.tilesN = (int)CeilDiv(s.n, wr);
+                best.split = split;
+                best.grid = best.tilesM * best.tilesN * split;
+                best.ring = lone ? kSplitLoneRingBytes : kSplitRingBytes;
+            }
+        }
+    }
+    return best;
+}
+// 256 x 256 tiles shared by two to four CTA pairs, where that takes less than `most`; no plan otherwise.
+MatmulPlan BestPairs256(const SmallProduct& s, double most)
+{
+    MatmulPlan p;
+    for (int split = 2; split <= kSplit2MaxPairs; ++split) {
+        const double t = s.kBlocks >= 2 * split ? PairsUs(s, 256, split) : 1e30;
+        if (t >= most) continue;
+        most = t;
+        p.route = MatmulRoute::TWO_SM_SPLIT;
+        p.bn = 256;
+        p.tilesM = (int)CeilDiv(s.m, 256);
+        p.tilesN = (int)CeilDiv(s.n, 256);
+        p.split = split;
+        p.grid = p.tilesM * p.tilesN * 2 * split;
+    }
+    return p;
+}
+MatmulPlan OneSmPlan(uint64_t m, uint64_t n, int bn, int sms)
+{
+    MatmulPlan p;
+    p.route = MatmulRoute::ONE_SM;
+    p.bn = bn;
+    p.tilesM = (int)CeilDiv(m, kBM);
+    p.tilesN = (int)CeilDiv(n, bn);
+    p.grid = std::min(sms, p.tilesM * p.tilesN);
+    return p;
+}
+
+}  // namespace
+
 MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms, const MatmulSwitches& sw, uint32_t outAlign)
 {
     MatmulPlan p;
@@ -452,7 +572,11 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.tilesN = (int)((n + 127) / 128);
         p.split = Split2Pairs((int)tiles128, pairs);
         p.grid = (int)tiles128 * 2 * p.split;
-        return p;
+        // long inner dimensions: 256 x 256 tiles, which bring a third fewer bytes per SM, shared by two to four pairs (255 x 5192 x 9888
+        // 37.1 -> 29.3 us, 137 x 5976 x 8048 45.3 -> 30.6)
+        const SmallProduct s(m, n, k, sms);
+        const MatmulPlan wide = BestPairs256(s, kOtherKernel * PairsUs(s, 128, p.split));
+        return wide.grid > 0 ? wide : p;
     }
     // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
     // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
@@ -465,19 +589,29 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.bn = 128;
         p.tilesM = (int)((m + p.bt - 1) / p.bt);
         p.tilesN = (int)((n + 127) / 128);
-        // two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile)
+        // Two CTAs per SM, at least four k-blocks each (16 x 8192 x 8192: 34.9, 29.7, 26.7 us with 1, 2, 4 CTAs per tile).  Where that is
+        // at most one tile for two SMs, another cut if its estimate is clearly lower, or 128 x 128 tiles where many tokens come with
+        // a short inner dimension (128 x 8192 x 256: 4.2 us split, 3.5 on the one-SM kernel).
         const int tiles = p.tilesM * p.tilesN, kBlocks = (int)((k + kBK - 1) / kBK);
-        p.split = std::max(1, std::min({kSplitMaxCluster, 2 * sms / tiles, kBlocks / 4}));
+        p.split = std::max(1, std::min({4, 2 * sms / tiles, kBlocks / 4}));
         p.grid = tiles * p.split;
-        return p;
+        bool lone;
+        const SmallProduct s(m, n, k, sms);
+        double us = SplitUs(s, aMn, p.bt, p.bn, p.split, &lone);
+        p.ring = lone ? kSplitLoneRingBytes : kSplitRingBytes;
+        if (tiles * 2 > sms) return p;
+        double bestUs;
+        const MatmulPlan best = BestSplit(s, aMn, &bestUs);
+        if (bestUs < kOtherCut * us) { p = best; us = bestUs; }
+        return m > 64 && outAlign >= 16 && OneSmUs(s, 128) < kOtherKernel * us ? OneSmPlan(m, n, 128, sms) : p;
     }
     if (!twoSm) {
-        p.route = MatmulRoute::ONE_SM;
-        p.bn = narrow ? 128 : 256;
-        p.tilesM = tilesM;
-        p.tilesN = (int)((n + p.bn - 1) / p.bn);
-        p.grid = std::min(sms, p.tilesM * p.tilesN);
-        return p;
+        p = OneSmPlan(m, n, narrow ? 128 : 256, sms);
+        if (!narrow || outAlign < 16) return p;
+        double us;
+        const SmallProduct s(m, n, k, sms);
+        const MatmulPlan split = BestSplit(s, aMn, &us);
+        return us < kOtherKernel * OneSmUs(s, p.bn) ? split : p;
     }
     p.bn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
     p.tilesN = (int)((n + p.bn - 1) / p.bn);
@@ -491,6 +625,21 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.wide = order.wide;
         p.singles = order.items - order.wide;
         return p;
+    }
+    // Short inner dimensions, where the drain of a tile is longer than its math: one-SM tiles, of which twice as many are under way
+    // (1000 x 4096 x 256 7.1 -> 4.6 us, 2048 x 8192 x 256 15.6 -> 12.1; larger outputs stay, 2248 x 4368 x 192 11.1 -> 7.6 is the
+    // last kind that was timed).  Long ones with few tiles: 256 x 256 tiles that pairs share (255 x 5192 x 9888 37.1 -> 29.3 us).
+    if (!sw.l2Hints && outAlign >= 16 && sw.wide != 1 && m * n <= (1u << 24)) {
+        const SmallProduct s(m, n, k, sms);
+        double best = kOtherKernel * TwoSmUs(s, p.bn);
+        MatmulPlan other;
+        for (int bn : {128, 256}) {
+            const double us = OneSmUs(s, bn);
+            if (us < best) { best = us; other = OneSmPlan(m, n, bn, sms); }
+        }
+        const MatmulPlan pairs256 = BestPairs256(s, best);
+        if (pairs256.grid > 0) return pairs256;
+        if (other.grid > 0) return other;
     }
     p.route = MatmulRoute::TWO_SM;
     p.grid = std::min(2 * pairs, 2 * tilesM2 * p.tilesN);
@@ -528,6 +677,19 @@ static HcclResult RefuseOut(const void* out, uint64_t m, uint64_t n, uint64_t k)
     return HCCL_E_PARA;
 }
 
+// Plans of the sizes that this thread multiplied last: weighing the cuts of a small product takes a microsecond of the host.
+static MatmulPlan RecentPlan(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, uint32_t outAlign)
+{
+    struct Entry { uint64_t m, n, k; int sms; uint32_t form; MatmulPlan plan; };
+    static thread_local Entry recent[64] = {};
+    const int sms = SmCount();
+    const uint32_t form = (aMn ? 1u : 0u) | (bMn ? 2u : 0u) | outAlign << 2;
+    Entry& e = recent[((m * 0x9E3779B97F4A7C15ull) ^ (n * 0xC2B2AE3D27D4EB4Full) ^ (k * 0x165667B19E3779F9ull) ^ form) >> 7 & 63u];
+    if (e.m != m || e.n != n || e.k != k || e.sms != sms || e.form != form)
+        e = {m, n, k, sms, form, PlanMatmul(m, n, k, aMn, bMn, sms, MatmulSwitchesOfEnv(), outAlign)};
+    return e.plan;
+}
+
 HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64_t n, uint64_t k, int transA, int transB, cudaStream_t stream,
                      const Mc2StalledCta* stalled)
 {
@@ -540,7 +702,7 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
     PlainCtl plain;
     CHK_RET(GetPlainCtl(&plain));
     if (*plain.gaveUp != 0) return ReportGaveUp(plain, stream);
-    const MatmulPlan plan = PlanMatmul(m, n, k, aMn, bMn, SmCount(), MatmulSwitchesOfEnv(), outAlign);
+    const MatmulPlan plan = RecentPlan(m, n, k, aMn, bMn, outAlign);
     if (outAlign < MatmulOutAlign(plan)) return RefuseOut(out, m, n, k);
     if (plan.route == MatmulRoute::SPLIT) {
         SplitArgs g;
@@ -549,13 +711,15 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         g.out = (__nv_bfloat16*)out;
         g.bt = plan.bt;
         g.tilesM = plan.tilesM;
-        g.stages = SplitStages(g.bt);
+        g.wr = plan.bn;
+        g.stages = std::max(1, std::min(SplitStages(g.bt, g.wr, plan.ring), (int)(((k + kBK - 1) / kBK + plan.split - 1) / plan.split)));
+        g.barOffset = SplitBarOffset(g.bt, g.wr, g.stages, plan.split);
         g.ctl = plain.ctl;
         g.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
         g.stalledCta = stalled != nullptr ? stalled->cta : -1;
         const int tiles = plan.tilesM * plan.tilesN;
         CUtensorMap tw, tx;
-        CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, 128, kBK));
+        CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, (uint32_t)g.wr, kBK));
         CHK_RET(aMn ? MakeMap(&tx, a, k, m, kBK, 64) : MakeMap(&tx, a, m, k, (uint32_t)g.bt, kBK));
         if (!bMn && !aMn) return LaunchGemmSplit<false, false>(tw, tx, g, tiles, plan.split, stream);
         if (!bMn && aMn) return LaunchGemmSplit<false, true>(tw, tx, g, tiles, plan.split, stream);

@@ -33,7 +33,8 @@ struct MatmulSwitches {
 struct MatmulPlan {
     MatmulRoute route = MatmulRoute::ONE_SM;
     int bn = 0, tilesM = 0, tilesN = 0, grid = 0;
-    int bt = 0, split = 0;              // SPLIT: tokens per tile, CTAs per tile; TWO_SM_SPLIT: CTA pairs per tile
+    int bt = 0, split = 0;              // SPLIT: tokens per tile (bn: weight rows), CTAs per tile; TWO_SM_SPLIT: CTA pairs per tile
+    int ring = 0;                       // SPLIT: bytes of shared memory for stages
     int wide = 0, singles = 0;          // WIDE: wide items, single ones
     int rasterGroup = 0, l2HintA = 0, l2HintB = 0;
 };

@@ -1,0 +1,51 @@
+"""Products of few tiles: every kernel and cut that the estimates choose among, at the edges of its tiles."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from test_gpu_tile_edges import LAYOUTS, _check_matmul
+from test_matmul_plan import plan
+
+# (m, n, k) with [N, K] weights: one token to 128, single CTAs and clusters of two to eight, k-blocks shared evenly and not, whole
+# and ragged inner dimensions, columns that end inside a tile, several token tiles
+CUTS = [((1, 64, 16000), {"split": "8", "bn": "128"}), ((16, 1000, 8200), {"split": "8", "bn": "64"}), ((17, 136, 4104), {"split": "8", "bt": "32"}),
+        ((33, 8, 1000), {"split": "8", "bt": "32"}), ((65, 264, 2056), {"split": "8", "bt": "32"}), ((32, 4096, 8192), {"split": "4", "bn": "128"}),
+        ((100, 520, 136), {"split": "1", "bt": "32"}), ((72, 1000, 72), {"split": "1", "bt": "32"}), ((128, 8192, 1032), {"split": "1", "bt": "64"}),
+        ((256, 128, 1000), {"split": "8", "bn": "64"}), ((136, 200, 1000), {"split": "8", "bt": "48"})]
+
+
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("shape,cut", CUTS)
+def test_token_split(shape, cut, ta, tb):
+    p = plan(*shape)
+    assert p["route"] == "split" and {k: p[k] for k in cut} == cut, p
+    m, n, k = shape
+    _check_matmul(m + (-m % 8 if ta else 0), n, k, ta, tb)
+
+
+# short inner dimensions on one-SM tiles, long ones with few rows on 256 x 256 tiles that pairs share
+OTHERS = [((1000, 4104, 72), "one_sm", {"bn": "256"}), ((520, 7304, 200), "one_sm", {"bn": "256"}), ((200, 10248, 200), "one_sm", {"bn": "128"}),
+          ((120, 7000, 256), "one_sm", {"bn": "128"}), ((255, 5192, 9888), "two_sm_split", {"bn": "256", "split": "3"}),
+          ((300, 2056, 12008), "two_sm_split", {"bn": "256", "split": "3"})]
+
+
+@pytest.mark.parametrize("ta,tb", LAYOUTS)
+@pytest.mark.parametrize("shape,route,cut", OTHERS)
+def test_other_kernels(shape, route, cut, ta, tb):
+    p = plan(*shape)
+    assert p["route"] == route and {k: p[k] for k in cut} == cut, p
+    m, n, k = shape
+    _check_matmul(m + (-m % 8 if ta else 0), n, k, ta, tb)
+
+
+def test_a_row_that_does_not_depend_on_the_buffer_next_to_it():
+    """The last columns of a 64-row tile lie beyond the matrix: nothing is written there."""
+    from hccl_b200.ops import mc2
+    m, n, k = 3, 72, 8200
+    whole = torch.full((m * n + 64,), 7.0, device="cuda", dtype=torch.bfloat16)
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    mc2.matmul(a, b, out=whole[:m * n].view(m, n))
+    want = (a.double() @ b.double().t()).float()
+    assert ((whole[:m * n].view(m, n).float() - want).norm() / want.norm()).item() < 3e-3
+    assert (whole[m * n:] == 7).all()

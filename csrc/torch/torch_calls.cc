@@ -3,9 +3,13 @@
 // allocations and ctypes a call of one took 10 .. 18 us of the host.
 //
 // Every function takes only what is plain: dense CUDA tensors that no transform, subclass, dispatch or function mode,
-// forward-mode gradient or tracer looks at, and that no gradient is recorded for.  For anything else it returns None and the
-// caller goes the general way (torch.autograd.Function, ctypes), which also words the errors.  An int is the HcclResult of a
-// failed call.
+// forward-mode gradient or tracer looks at, and (but for those of the second part) that no gradient is recorded for.  For
+// anything else it returns None and the caller goes the general way (torch.autograd.Function, ctypes), which also words the
+// errors.  An int is the HcclResult of a failed call.
+//
+// The second part (add_rms_norm_grad, swiglu_grad, rope_grad, linear) records gradients: nodes of autograd's graph in the place of
+// Python functions, whose passes through the interpreter took 100 us of the host for a norm forward and backward and 250 for the
+// FFN half of a layer, several times what the kernels of a small one take.
 //
 // The functions of the C API come as addresses (`bind`), so that this module and the ctypes binding always use the same library.
 #define PY_SSIZE_T_CLEAN
@@ -17,9 +21,15 @@
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/PyInterpreter.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/accumulate_grad.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
+#include <atomic>
 #include <cstdint>
 #include "hccl/hccl.h"
 #include "hccl/hccl_fused_ops.h"
@@ -331,6 +341,323 @@ PyObject* Collective(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     });
 }
 
+// ----------------------------------------------------------------------------- calls that record gradients
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+std::atomic<int64_t> launches{0};                  // kernels of the nodes' backward passes (benchmark accounting)
+PyObject* errorClass = nullptr;                    // what a failed call raises, (code, function)
+
+// In a backward pass, which runs on a thread of its own without the interpreter's lock.
+void CheckBackward(int code, const char* what)
+{
+    if (code == 0) return;
+    const PyGILState_STATE lock = PyGILState_Ensure();
+    PyObject* error = errorClass ? PyObject_CallFunction(errorClass, "is", code, what) : nullptr;
+    if (error != nullptr) {
+        PyErr_SetObject(reinterpret_cast<PyObject*>(Py_TYPE(error)), error);
+        Py_DECREF(error);
+    } else if (!PyErr_Occurred()) {
+        PyErr_Format(PyExc_RuntimeError, "%s failed (%d)", what, code);
+    }
+    python_error e;
+    e.persist();
+    PyGILState_Release(lock);
+    throw e;
+}
+// A dense bf16 CUDA tensor that nothing but the recording of gradients looks at.
+const Tensor* GetRecordable(PyObject* o, bool contiguous = true)
+{
+    const Tensor* t = Get(o);
+    if (t == nullptr || !t->is_cuda() || t->layout() != at::kStrided || t->scalar_type() != at::kBFloat16 || at::isTensorSubclassLike(*t) ||
+        t->_fw_grad(0).defined() || (contiguous && !t->is_contiguous()))
+        return nullptr;
+    return t;
+}
+bool Records(std::initializer_list<const Tensor*> inputs)
+{
+    if (!c10::GradMode::is_enabled()) return false;
+    for (const Tensor* t : inputs)
+        if (t != nullptr && t->requires_grad()) return true;
+    return false;
+}
+template <class... T> void TakeInputs(const std::shared_ptr<Node>& node, const T&... inputs) { node->set_next_edges(torch::autograd::collect_next_edges(inputs...)); }
+void GiveOutput(const std::shared_ptr<Node>& node, const Tensor& out)
+{
+    const uint32_t nr = node->add_input_metadata(out);
+    torch::autograd::impl::set_gradient_edge(out, {node, nr});
+}
+// The gradient of an input ends in a leaf that holds none yet: the leaf keeps the tensor it is given if nobody else has it, and
+// copies it otherwise.  (Under autograd.grad the leaves keep nothing.)
+torch::autograd::AccumulateGrad* EmptyLeaf(const torch::autograd::Edge& edge)
+{
+    auto* leaf = dynamic_cast<torch::autograd::AccumulateGrad*>(edge.function.get());
+    if (leaf == nullptr || leaf->variable.grad().defined()) return nullptr;
+    const auto* executed = torch::autograd::get_current_graph_task_exec_info();
+    if (executed == nullptr) return nullptr;
+    if (executed->empty()) return leaf;
+    const auto it = executed->find(leaf);
+    return it != executed->end() && it->second.needed_ && !it->second.captures_ ? leaf : nullptr;
+}
+
+struct AddRmsNormNode : Node {
+    SavedVariable xOut, weight, rstd;
+    bool hasDelta = false;
+    std::string name() const override { return "_AddRmsNormBackward"; }
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        xOut.reset_data();
+        weight.reset_data();
+        rstd.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override
+    {
+        Tensor x, w, r;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            x = xOut.unpack(hasDelta ? shared_from_this() : nullptr);
+            w = weight.unpack();
+            r = rstd.unpack();
+        }
+        c10::AutoGradMode off(false);
+        const Tensor extra = hasDelta && grads[0].defined() ? grads[0].contiguous() : Tensor();
+        const Tensor& given = grads[hasDelta ? 1 : 0];
+        const Tensor dh = given.defined() ? given.contiguous() : at::zeros_like(x);
+        const torch::autograd::AccumulateGrad* first = hasDelta ? EmptyLeaf(next_edge(0)) : nullptr;
+        const torch::autograd::AccumulateGrad* second = first ? EmptyLeaf(next_edge(1)) : nullptr;
+        const bool twice = second != nullptr && first != second;
+        const int64_t hidden = x.size(-1);
+        const uint64_t rows = (uint64_t)(x.numel() / hidden);
+        Tensor dx = at::empty_like(x), copy = twice ? at::empty_like(x) : dx, dw = at::empty_like(w);
+        Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), hidden}, x.options().dtype(at::kFloat));
+        CheckBackward(api.rmsNormBwd(dh.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), r.const_data_ptr(), extra.defined() ? extra.const_data_ptr() : nullptr,
+                                     dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr, partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows,
+                                     (uint32_t)hidden, Stream()),
+                      "HcclFusedRmsNormBwdCopy");
+        launches += 2;
+        if (!hasDelta) return {std::move(dx), std::move(dw)};
+        return {std::move(dx), std::move(copy), std::move(dw)};
+    }
+};
+// (x, delta or None, weight, eps) -> (x_out or x, h)
+PyObject* AddRmsNormGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(4)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetRecordable(a[0]), *w = GetRecordable(a[2]), *delta = a[1] == Py_None ? nullptr : GetRecordable(a[1]);
+        if (!x || !w || (a[1] != Py_None && !delta) || !PyFloat_Check(a[3]) || !Records({x, w, delta}) || !PlainCall()) return None();
+        if (x->dim() == 0 || x->numel() == 0 || w->numel() != x->size(-1) || (delta && delta->sizes() != x->sizes())) return None();
+        const uint64_t hidden = (uint64_t)x->size(-1), rows = (uint64_t)x->numel() / hidden;
+        if (hidden % 8 != 0 || hidden > 8192) return None();
+        const float eps = (float)PyFloat_AS_DOUBLE(a[3]);
+        Tensor h, xOut;
+        const int r = [&] {
+            Unlocked unlocked;
+            c10::AutoGradMode off(false);
+            h = at::empty_like(*x);
+            xOut = delta ? at::empty_like(*x) : *x;
+            Tensor rstd = at::empty({(int64_t)rows}, x->options().dtype(at::kFloat));
+            const int code = api.addRmsNormFwd(x->const_data_ptr(), delta ? delta->const_data_ptr() : nullptr, w->const_data_ptr(),
+                                               delta ? xOut.mutable_data_ptr() : nullptr, h.mutable_data_ptr(), rstd.mutable_data_ptr(), rows, (uint32_t)hidden, eps,
+                                               Stream());
+            if (code != 0) return code;
+            auto node = std::make_shared<AddRmsNormNode>();
+            node->hasDelta = delta != nullptr;
+            if (delta) TakeInputs(node, *x, *delta, *w);
+            else TakeInputs(node, *x, *w);
+            if (delta) GiveOutput(node, xOut);
+            GiveOutput(node, h);
+            node->xOut = SavedVariable(xOut, delta != nullptr);
+            node->weight = SavedVariable(*w, false);
+            node->rstd = SavedVariable(rstd, false);
+            return 0;
+        }();
+        if (r != 0) return PyLong_FromLong(r);
+        return WrapAll(std::move(xOut), std::move(h));
+    });
+}
+
+struct SwigluNode : Node {
+    SavedVariable gateUp;
+    std::string name() const override { return "_SwigluBackward"; }
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        gateUp.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        Tensor x;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            x = gateUp.unpack();
+        }
+        c10::AutoGradMode off(false);
+        const Tensor dout = grads[0].contiguous();
+        const int64_t f = x.size(-1) / 2;
+        Tensor dx = at::empty_like(x);
+        CheckBackward(api.swigluBwd(x.const_data_ptr(), dout.const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x.numel() / (2 * f)), (uint32_t)f, Stream()),
+                      "HcclFusedSwigluBwd");
+        launches += 1;
+        return {std::move(dx)};
+    }
+};
+// (gate_up) -> out
+PyObject* SwigluGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(1)
+    return Guarded([&]() -> PyObject* {
+        const Tensor* x = GetRecordable(a[0]);
+        if (!x || !Records({x}) || !PlainCall() || x->dim() == 0 || x->numel() == 0 || x->size(-1) % 16 != 0) return None();
+        const int64_t f = x->size(-1) / 2;
+        auto sizes = x->sizes().vec();
+        sizes.back() = f;
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            c10::AutoGradMode off(false);
+            out = at::empty(sizes, x->options());
+            const int code = api.swigluFwd(x->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
+            if (code != 0) return code;
+            auto node = std::make_shared<SwigluNode>();
+            TakeInputs(node, *x);
+            GiveOutput(node, out);
+            node->gateUp = SavedVariable(*x, false);
+            return 0;
+        }();
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+struct RopeNode : Node {
+    SavedVariable cos, sin;
+    std::string name() const override { return "_RopeBackward"; }
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        cos.reset_data();
+        sin.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        Tensor c, s;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            c = cos.unpack();
+            s = sin.unpack();
+        }
+        c10::AutoGradMode off(false);
+        const Tensor dout = grads[0].contiguous();
+        const int64_t rows = dout.size(0), heads = dout.size(1), d = dout.size(2);
+        Tensor dx = at::empty_like(dout);
+        CheckBackward(api.rope(dout.const_data_ptr(), (uint64_t)(heads * d), dx.mutable_data_ptr(), (uint64_t)(heads * d), c.const_data_ptr(), s.const_data_ptr(),
+                               (uint64_t)rows, (uint32_t)heads, (uint32_t)d, 1, Stream()),
+                      "HcclFusedRope");
+        launches += 1;
+        return {std::move(dx)};
+    }
+};
+// (x [S, heads, D], cos, sin) -> rotated x
+PyObject* RopeGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(3)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetRecordable(a[0], false), *c = GetPlain(a[1]), *s = GetPlain(a[2]);
+        if (!x || !c || !s || !Records({x}) || !PlainCall() || x->dim() != 3 || x->numel() == 0) return None();
+        const int64_t rows = x->size(0), heads = x->size(1), d = x->size(2);
+        if (d % 16 != 0 || x->stride(2) != 1 || x->stride(1) != d || x->stride(0) < 0 || x->stride(0) % 8 != 0 || (uintptr_t)x->const_data_ptr() % 16 != 0)
+            return None();
+        for (const Tensor* t : {c, s})
+            if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() < rows * (d / 2)) return None();
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            c10::AutoGradMode off(false);
+            out = at::empty({rows, heads, d}, x->options());
+            const int code = api.rope(x->const_data_ptr(), (uint64_t)x->stride(0), out.mutable_data_ptr(), (uint64_t)(heads * d), c->const_data_ptr(),
+                                      s->const_data_ptr(), (uint64_t)rows, (uint32_t)heads, (uint32_t)d, 0, Stream());
+            if (code != 0) return code;
+            auto node = std::make_shared<RopeNode>();
+            TakeInputs(node, *x);
+            GiveOutput(node, out);
+            node->cos = SavedVariable(*c, false);
+            node->sin = SavedVariable(*s, false);
+            return 0;
+        }();
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+
+struct LinearNode : Node {
+    SavedVariable x, weight;
+    Tensor counter;                                // int64 on the host: kernels launched
+    std::string name() const override { return "_LinearBackward"; }
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        x.reset_data();
+        weight.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override
+    {
+        if (!grads[0].defined()) return {Tensor(), Tensor()};
+        Tensor in, w;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            in = x.unpack();
+            w = weight.unpack();
+        }
+        c10::AutoGradMode off(false);
+        const Tensor dy = grads[0].contiguous();
+        const uint64_t rows = (uint64_t)dy.size(0), n = (uint64_t)dy.size(1), k = (uint64_t)in.size(1);
+        Tensor dw = at::empty({(int64_t)n, (int64_t)k}, dy.options()), dx = at::empty({(int64_t)rows, (int64_t)k}, dy.options());
+        CheckBackward(api.matmul(dy.const_data_ptr(), in.const_data_ptr(), dw.mutable_data_ptr(), n, k, rows, 1, 0, Stream()), "HcclMc2Matmul");
+        CheckBackward(api.matmul(dy.const_data_ptr(), w.const_data_ptr(), dx.mutable_data_ptr(), rows, k, n, 0, 0, Stream()), "HcclMc2Matmul");
+        __atomic_fetch_add(counter.mutable_data_ptr<int64_t>(), 2, __ATOMIC_RELAXED);
+        return {std::move(dx), std::move(dw)};
+    }
+};
+// (x [rows, k], weight [n, k], counter of launches) -> x @ weight^T
+PyObject* Linear(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(3)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *x = GetRecordable(a[0]), *w = GetRecordable(a[1]), *counter = Get(a[2]);
+        if (!x || !w || !counter || counter->scalar_type() != at::kLong || counter->numel() != 1 || !counter->is_cpu() || !PlainCall()) return None();
+        if (x->dim() != 2 || w->dim() != 2 || x->numel() == 0 || w->numel() == 0 || x->size(1) != w->size(1)) return None();
+        const bool record = Records({x, w});
+        Tensor out;
+        const int r = [&] {
+            Unlocked unlocked;
+            c10::AutoGradMode off(false);
+            out = at::empty({x->size(0), w->size(0)}, x->options());
+            const int code = api.matmul(x->const_data_ptr(), w->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)x->size(0), (uint64_t)w->size(0),
+                                        (uint64_t)x->size(1), 0, 1, Stream());
+            if (code != 0) return code;
+            if (!record) return 0;
+            auto node = std::make_shared<LinearNode>();
+            TakeInputs(node, *x, *w);
+            GiveOutput(node, out);
+            node->x = SavedVariable(*x, false);
+            node->weight = SavedVariable(*w, false);
+            node->counter = *counter;
+            return 0;
+        }();
+        return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
+    });
+}
+PyObject* Launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launches.load()); }
+PyObject* Raises(PyObject*, PyObject* error)
+{
+    Py_INCREF(error);
+    Py_XSETREF(errorClass, error);
+    Py_RETURN_NONE;
+}
+
 PyObject* Bind(PyObject*, PyObject* addresses)
 {
     if (defaultDeviceMode == nullptr) {
@@ -368,7 +695,9 @@ PyMethodDef methods[] = {
     {"bind", Bind, METH_O, nullptr},           {"names", Names, METH_NOARGS, nullptr},      {"add_rms_norm", HCCL_FAST(AddRmsNorm)},
     {"rms_norm_bwd", HCCL_FAST(RmsNormBwd)},   {"swiglu_fwd", HCCL_FAST(SwigluFwd)},        {"swiglu_bwd", HCCL_FAST(SwigluBwd)},
     {"rope", HCCL_FAST(Rope)},                 {"matmul", HCCL_FAST(Matmul)},               {"expert_offsets", HCCL_FAST(ExpertOffsets)},
-    {"collective", HCCL_FAST(Collective)},     {nullptr, nullptr, 0, nullptr},
+    {"collective", HCCL_FAST(Collective)},     {"add_rms_norm_grad", HCCL_FAST(AddRmsNormGrad)},
+    {"swiglu_grad", HCCL_FAST(SwigluGrad)},    {"rope_grad", HCCL_FAST(RopeGrad)},          {"linear", HCCL_FAST(Linear)},
+    {"launches", Launches, METH_NOARGS, nullptr}, {"raises", Raises, METH_O, nullptr},      {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "hccl_b200_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

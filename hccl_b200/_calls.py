@@ -16,7 +16,7 @@ import torch          # its libraries have to be loaded before the module's
 
 from ._lib import lib
 from .build import torch_lib
-from .comm import _check
+from .comm import HcclError, _check
 
 
 def _nothing(*_):
@@ -29,6 +29,7 @@ def _load():
         loader = importlib.machinery.ExtensionFileLoader("hccl_b200_torch", str(path))
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("hccl_b200_torch", loader))
         loader.exec_module(module)
+        module.raises(HcclError)
         module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in module.names()})
         return module
     except (ImportError, AttributeError) as e:
@@ -41,6 +42,13 @@ _module = _load()
 add_rms_norm, rms_norm_bwd, swiglu_fwd, swiglu_bwd, rope, matmul, expert_offsets, collective = (
     getattr(_module, name, _nothing)
     for name in ("add_rms_norm", "rms_norm_bwd", "swiglu_fwd", "swiglu_bwd", "rope", "matmul", "expert_offsets", "collective"))
+# the same where gradients are recorded (``linear``: recorded or not)
+add_rms_norm_grad, swiglu_grad, rope_grad, linear = (getattr(_module, name, _nothing) for name in ("add_rms_norm_grad", "swiglu_grad", "rope_grad", "linear"))
+
+
+def launches() -> int:
+    """Kernels that the backward passes of these have launched (``linear`` counts in the tensor it is given)."""
+    return _module.launches() if _module is not None else 0
 
 
 def result(r, what: str):

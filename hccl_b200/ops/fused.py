@@ -21,12 +21,18 @@ from .._lib import lib
 from ..comm import _check
 
 
-LAUNCHES = 0          # kernels of this module launched so far (benchmark accounting)
+_launches = 0
 
 
 def _count(n=1):
-    global LAUNCHES
-    LAUNCHES += n
+    global _launches
+    _launches += n
+
+
+def __getattr__(name):
+    if name == "LAUNCHES":          # kernels of this module launched so far (benchmark accounting)
+        return _launches + _calls.launches()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _p(t):
@@ -251,6 +257,11 @@ def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
         x_out, h, _ = _calls.result(r, "HcclFusedAddRmsNormFwd")
         _count()
         return x_out, h
+    r = _calls.add_rms_norm_grad(x, delta, weight, eps) if use_kernels else None
+    if r is not None:
+        x_out, h = _calls.result(r, "HcclFusedAddRmsNormFwd")
+        _count()
+        return x_out, h
     if use_kernels and _native(x, delta, weight, hidden=x.shape[-1]):
         if delta is None:
             return x, _AddRmsNorm.apply(x, None, weight, eps)
@@ -260,6 +271,8 @@ def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
 
 def swiglu(gate_up, use_kernels: bool = True):
     out = _calls.swiglu_fwd(gate_up) if use_kernels else None
+    if out is None and use_kernels:
+        out = _calls.swiglu_grad(gate_up)
     if out is not None:
         out = _calls.result(out, "HcclFusedSwigluFwd")
         _count()
@@ -277,6 +290,8 @@ def _rope_table(t, x) -> bool:
 def rope(x, cos, sin, use_kernels: bool = True):
     """x [S, heads, D] (row stride may exceed heads * D), cos / sin fp32 [S, D / 2]."""
     out = _calls.rope(x, cos, sin, False) if use_kernels else None
+    if out is None and use_kernels:
+        out = _calls.rope_grad(x, cos, sin)
     if out is not None:
         out = _calls.result(out, "HcclFusedRope")
         _count()

@@ -20,6 +20,7 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
+from .. import _calls
 from ..ops import mc2
 
 
@@ -39,7 +40,7 @@ class TPContext:
             self.world = dist.get_world_size(group) if dist.is_initialized() else 1
             self.rank = dist.get_rank(group) if dist.is_initialized() else 0
         self._sym = {}
-        self.launches = 0                 # kernels of this library launched (bench accounting)
+        self._launches, self._launched = 0, torch.zeros(1, dtype=torch.int64, device="cpu")      # here, and by native backward passes
         # AllGather->Matmul form: "push" (every rank writes its shard into the others' symmetric gathered buffers) or
         # "pull" (every rank reads the peers' symmetric shards)
         import os
@@ -52,6 +53,15 @@ class TPContext:
         if fused_ops is None:
             fused_ops = impl == "hccl"
         self.fused_ops = bool(fused_ops) and str(device).startswith("cuda") and os.environ.get("HCCL_FUSED_ELEMENTWISE", "1") != "0"
+
+    @property
+    def launches(self):
+        """Kernels of this library launched (bench accounting)."""
+        return self._launches + int(self._launched)
+
+    @launches.setter
+    def launches(self, n):
+        self._launches = n - int(self._launched)
 
     # ---- collectives on whole tensors, either arm (used for what is not a fused matmul: the embedding exchange and
     # the gradients of replicated parameters)
@@ -132,6 +142,15 @@ def _mm(ctx, a, b, **kw):
     A = a.t() if kw.get("trans_a", False) else a
     B = b.t() if kw.get("trans_b", True) else b
     return A @ B
+
+
+def _alone(ctx, x, weight):
+    """``x @ W^T`` on one rank, where the native call takes it; ``None`` goes through the functions below."""
+    out = _calls.linear(x, weight, ctx._launched) if ctx.world == 1 and ctx.impl == "hccl" else None
+    if out is not None:
+        out = _calls.result(out, "HcclMc2Matmul")
+        ctx._launches += 1
+    return out
 
 
 class _ColumnParallel(torch.autograd.Function):
@@ -228,7 +247,8 @@ class ColumnParallelLinear(torch.nn.Module):
         self.weight = torch.nn.Parameter(torch.randn(out_features // ctx.world, in_features, device=ctx.device, dtype=torch.float32).mul_(std).to(ctx.dtype))
 
     def forward(self, x_shard):
-        return _ColumnParallel.apply(x_shard, self.weight, self.ctx, self.key)
+        out = _alone(self.ctx, x_shard, self.weight)
+        return out if out is not None else _ColumnParallel.apply(x_shard, self.weight, self.ctx, self.key)
 
 
 class RowParallelLinear(torch.nn.Module):
@@ -243,4 +263,5 @@ class RowParallelLinear(torch.nn.Module):
         self.weight = torch.nn.Parameter(torch.randn(out_features, in_features // ctx.world, device=ctx.device, dtype=torch.float32).mul_(std).to(ctx.dtype))
 
     def forward(self, x):
-        return _RowParallel.apply(x, self.weight, self.ctx, self.key)
+        out = _alone(self.ctx, x, self.weight)
+        return out if out is not None else _RowParallel.apply(x, self.weight, self.ctx, self.key)

@@ -430,75 +430,78 @@ namespace {
 
 // Estimated time of a small product on each kernel, in us on a B200.  Up to some 50 us a matmul is bound by what one SM takes in
 // (a k-block of a tile comes at 110 .. 145 GB/s from L2), by what a k-block costs at least, by a tile's drain and by whole rounds
-// of tiles, so the best kernel and cut are those that balance these four.  Fitted to 11000 timed calls (8 .. 8000 rows, 64 .. 16000
-// columns, inner dimensions of 64 .. 16000; cluster launches in a graph): off by 12 % (two-SM), 14 % (pairs), 17 % (token split),
-// 19 % (one-SM) in the root mean square, most of it in common; taking the best estimate instead of the best time costs 2-3 %.
+// of tiles, so the best kernel and cut are those that balance these four.  Fitted to 16000 timed calls (8 .. 8000 rows, 64 .. 16000
+// columns, inner dimensions of 64 .. 16000, back to back in a graph): off by 8 % (two-SM), 12 % (one-SM, pairs) and 15 % (token split) in
+// the root mean square; taking the best estimate instead of the best time costs 2-3 %.
 struct SmallProduct {
     uint64_t m, n, k;
     int kBlocks, sms;
+    bool aMn;
+    double a, b;               // rows that lie on 16 bytes only, not on 32, take the copy engine 1.6 times as long
     double hbmUs;              // every operand and the output once at 6.3 TB/s
-    SmallProduct(uint64_t m, uint64_t n, uint64_t k, int sms)
-        : m(m), n(n), k(k), kBlocks((int)((k + kBK - 1) / kBK)), sms(sms), hbmUs(2.0 * ((double)m * k + (double)n * k + (double)m * n) / 6.3e6) {}
+    SmallProduct(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, int sms)
+        : m(m), n(n), k(k), kBlocks((int)((k + kBK - 1) / kBK)), sms(sms), aMn(aMn), a((aMn ? m : k) % 16 != 0 ? 1.6 : 1.0), b((bMn ? n : k) % 16 != 0 ? 1.6 : 1.0),
+          hbmUs(2.0 * ((double)m * k + (double)n * k + (double)m * n) / 6.3e6) {}
 };
 uint64_t CeilDiv(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 double FourNorm(double a, double b) { return std::sqrt(std::sqrt(a * a * a * a + b * b * b * b)); }
 // CTAs of `cluster` that run together, one per SM (clusters stay within groups of SMs: 33 of four, 15 of eight on 148)
 double ResidentCtas(int cluster, int sms) { return cluster == 8 ? sms * (120. / 148) : (cluster >= 4 ? sms * (132. / 148) : sms); }
 
-double SplitUs(const SmallProduct& s, bool aMn, int bt, int wr, int split, bool* lone)
+double SplitUs(const SmallProduct& s, int bt, int wr, int split, bool* lone)
 {
     // rows of MN-major activations with fewer than 64 tokens come in pieces that all CTAs read from the same few lines
-    const double block = 0.142 + (aMn && s.m < 64 ? 0.45 * (64 - (double)s.m) / 56 : 0);
+    const double block = 0.134 + (s.aMn && s.m < 64 ? 0.45 * (64 - (double)s.m) / 56 : 0);
     const double ctas = (double)(CeilDiv(s.m, bt) * CeilDiv(s.n, wr) * split), resident = ResidentCtas(split, s.sms);
     *lone = ctas <= resident;                                   // one per SM: the ring may take its whole shared memory
     const double rounds = std::ceil(ctas / (resident * (*lone ? 1 : 2))), perSm = *lone ? 1 : std::min(2.0, std::ceil(ctas / resident));
-    const int stageBytes = SplitStageBytes(bt, wr), stages = SplitStages(bt, wr, *lone ? kSplitLoneRingBytes : kSplitRingBytes);
+    const int stages = SplitStages(bt, wr, *lone ? kSplitLoneRingBytes : kSplitRingBytes);
     const double kb = std::ceil((double)s.kBlocks / split), tile = perSm * bt * wr / 16384.;
-    const double loads = rounds * kb * std::max({block, perSm * stageBytes / 145e3, 0.142 * 6 / stages});
-    const double hbm = 0.87 * s.hbmUs * std::pow(std::max(1.0, s.sms / std::min(ctas, resident)), 0.6);      // fewer SMs keep fewer bytes on their way
-    return 2.1 + (wr == 64 ? 0.8 : 0) + std::max(loads, hbm) + rounds * (2.1 * tile + (split > 1 ? 1.15 + 1.05 * tile : 0));
+    const double loads = rounds * kb * std::max({block, perSm * (wr * s.b + bt * s.a) * 128 / 143.6e3, 0.134 * 6 / stages});
+    const double hbm = 0.88 * s.hbmUs * std::pow(std::max(1.0, s.sms / std::min(ctas, resident)), 0.6);      // fewer SMs keep fewer bytes on their way
+    return 2.2 + (wr == 64 ? 0.7 : 0) + std::max(loads, hbm) + rounds * (1.85 * tile + (split > 1 ? 1.1 + 1.1 * tile : 0));
 }
 double OneSmUs(const SmallProduct& s, int bn)
 {
     const double rounds = (double)CeilDiv(CeilDiv(s.m, kBM) * CeilDiv(s.n, bn), s.sms);
-    const double loads = s.kBlocks * (128 + bn) * 128 / 128.5e3, drain = 0.8 * bn / 128;
-    return 0.72 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 0.77 * rounds;
+    const double loads = s.kBlocks * (128 * s.a + bn * s.b) * 128 / 138.3e3, drain = 0.77 * bn / 128;
+    return 0.87 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 0.71 * rounds;
 }
 double PairsUs(const SmallProduct& s, int bn, int split)
 {
     static const double resident[] = {0, 74, 66, 66, 60};       // CTA pairs
     const double rounds = std::ceil((double)(CeilDiv(s.m, 256) * CeilDiv(s.n, bn) * split) / (resident[split] * s.sms / 148));
-    const double loads = std::ceil((double)s.kBlocks / split) * (128 + bn / 2) * 128 / 114.5e3, drain = 3.07 * bn / 128;
-    return 0.8 + std::max(rounds * (loads + drain + (split > 1 ? 2.54 : 0)), 3.07 + s.hbmUs);
+    const double loads = std::ceil((double)s.kBlocks / split) * (128 * s.a + bn / 2 * s.b) * 128 / 127.2e3, drain = 3.13 * bn / 128;
+    return 0.8 + std::max(rounds * (loads + drain + (split > 1 ? 2.47 : 0)), 3.13 + s.hbmUs);
 }
 double TwoSmUs(const SmallProduct& s, int bn)
 {
     const double rounds = (double)CeilDiv(CeilDiv(s.m, 256) * CeilDiv(s.n, bn), s.sms / 2);
-    const double loads = s.kBlocks * (128 + bn / 2) * 128 / 111.7e3, drain = 0.72 * bn / 128;
-    return 1.73 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 1.6 * rounds;
+    const double loads = s.kBlocks * (128 * s.a + bn / 2 * s.b) * 128 / 123.6e3, drain = 0.68 * bn / 128;
+    return 1.97 + std::max(s.hbmUs, rounds * FourNorm(loads, drain)) + drain + 1.48 * rounds;
 }
 // Another kernel, or another cut for the same one, is taken where its estimate is lower by more than the two are off against each other.
 constexpr double kOtherKernel = 0.87, kOtherCut = 0.9;
 
 // Best cut for the token split, its estimate in *us.
-MatmulPlan BestSplit(const SmallProduct& s, bool aMn, double* us)
+MatmulPlan BestSplit(const SmallProduct& s, double* us)
 {
     MatmulPlan best;
     *us = 1e30;
     for (int most : {128, 64, 32}) {
         // equal token tiles of at most `most` (MN-major activations come in boxes of 64)
-        const int unit = aMn ? 64 : 16, parts = (int)CeilDiv(s.m, most);
+        const int unit = s.aMn ? 64 : 16, parts = (int)CeilDiv(s.m, most);
         const int bt = (int)(CeilDiv(CeilDiv(s.m, parts), unit) * unit);
         if (bt > most || (parts > 1 && parts == (int)CeilDiv(s.m, 2 * most))) continue;
         // smaller token tiles read the weights more often: from L2, where they fit it; 32 tokens were timed up to 128 rows
         if (parts > (int)CeilDiv(s.m, 128) && s.n * s.k * 2 > (64u << 20)) continue;
         if (most == 32 && s.m > 128) continue;
         for (int wr : {128, 64}) {
-            if (wr == 64 && aMn) continue;
+            if (wr == 64 && s.aMn) continue;
             for (int split : {1, 2, 4, 8}) {
                 if (split > 1 && s.kBlocks < 2 * split) break;
                 bool lone;
-                const double t = SplitUs(s, aMn, bt, wr, split, &lone);
+                const double t = SplitUs(s, bt, wr, split, &lone);
                 if (t >= *us) continue;
                 *us = t;
                 best.route = MatmulRoute::SPLIT;
@@ -574,9 +577,16 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.grid = (int)tiles128 * 2 * p.split;
         // long inner dimensions: 256 x 256 tiles, which bring a third fewer bytes per SM, shared by two to four pairs (255 x 5192 x 9888
         // 37.1 -> 29.3 us, 137 x 5976 x 8048 45.3 -> 30.6)
-        const SmallProduct s(m, n, k, sms);
-        const MatmulPlan wide = BestPairs256(s, kOtherKernel * PairsUs(s, 128, p.split));
-        return wide.grid > 0 ? wide : p;
+        const SmallProduct s(m, n, k, aMn, bMn, sms);
+        double us = PairsUs(s, 128, p.split);
+        const MatmulPlan wide = BestPairs256(s, kOtherKernel * us);
+        if (wide.grid > 0) return wide;
+        // One or two column tiles (a router's logits): token tiles of 64 and clusters of eight keep more SMs busy (256 x 128 x 8192 11.3 -> 6.4
+        // us, 244 x 208 x 10520 18.6 -> 10.6, 637 x 72 x 2784 8.7 -> 5.8).  They are ahead at 2048 as well (512 x 128 x 2048 8.0 and 5.0) and
+        // up to some thousand columns by less (256 x 1024 x 8192 12.9 and 10.5): there the pairs and their order of sums stay.
+        if (n > 256 || s.kBlocks <= 36) return p;
+        const MatmulPlan split = BestSplit(s, &us);
+        return us < kOtherKernel * PairsUs(s, 128, p.split) ? split : p;
     }
     // Inner dimension split over clusters: up to 96 rows always (at 128 rows and 57344 columns the 256-wide one-SM tiles win,
     // 166 against 174 us), beyond that where the output leaves SMs idle; from 129 rows on only if the inner dimension is
@@ -596,12 +606,12 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.split = std::max(1, std::min({4, 2 * sms / tiles, kBlocks / 4}));
         p.grid = tiles * p.split;
         bool lone;
-        const SmallProduct s(m, n, k, sms);
-        double us = SplitUs(s, aMn, p.bt, p.bn, p.split, &lone);
+        const SmallProduct s(m, n, k, aMn, bMn, sms);
+        double us = SplitUs(s, p.bt, p.bn, p.split, &lone);
         p.ring = lone ? kSplitLoneRingBytes : kSplitRingBytes;
         if (tiles * 2 > sms) return p;
         double bestUs;
-        const MatmulPlan best = BestSplit(s, aMn, &bestUs);
+        const MatmulPlan best = BestSplit(s, &bestUs);
         if (bestUs < kOtherCut * us) { p = best; us = bestUs; }
         return m > 64 && outAlign >= 16 && OneSmUs(s, 128) < kOtherKernel * us ? OneSmPlan(m, n, 128, sms) : p;
     }
@@ -609,9 +619,22 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p = OneSmPlan(m, n, narrow ? 128 : 256, sms);
         if (!narrow || outAlign < 16) return p;
         double us;
-        const SmallProduct s(m, n, k, sms);
-        const MatmulPlan split = BestSplit(s, aMn, &us);
-        return us < kOtherKernel * OneSmUs(s, p.bn) ? split : p;
+        const SmallProduct s(m, n, k, aMn, bMn, sms);
+        const MatmulPlan split = BestSplit(s, &us);
+        const double oneSm = OneSmUs(s, p.bn);
+        // outputs of more than one round of one-SM tiles that two-SM tiles cover in one (759 x 3824 x 1552 16.4 -> 11.1 us, 269 x 8056 x 1448
+        // 21.5 -> 15.3)
+        const int bn2 = TwoSmColumnTile(tilesM2, n, pairs, bMn);
+        if (sw.twoSm && m > 128 && TwoSmUs(s, bn2) < std::min(us, kOtherKernel * oneSm)) {
+            p = MatmulPlan();
+            p.route = MatmulRoute::TWO_SM;
+            p.bn = bn2;
+            p.tilesM = tilesM;
+            p.tilesN = (int)CeilDiv(n, bn2);
+            p.grid = std::min(2 * pairs, 2 * tilesM2 * p.tilesN);
+            return p;
+        }
+        return us < kOtherKernel * oneSm ? split : p;
     }
     p.bn = TwoSmColumnTile(tilesM2, n, pairs, bMn);
     p.tilesN = (int)((n + p.bn - 1) / p.bn);
@@ -630,7 +653,7 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
     // (1000 x 4096 x 256 7.1 -> 4.6 us, 2048 x 8192 x 256 15.6 -> 12.1; larger outputs stay, 2248 x 4368 x 192 11.1 -> 7.6 is the
     // last kind that was timed).  Long ones with few tiles: 256 x 256 tiles that pairs share (255 x 5192 x 9888 37.1 -> 29.3 us).
     if (!sw.l2Hints && outAlign >= 16 && sw.wide != 1 && m * n <= (1u << 24)) {
-        const SmallProduct s(m, n, k, sms);
+        const SmallProduct s(m, n, k, aMn, bMn, sms);
         double best = kOtherKernel * TwoSmUs(s, p.bn);
         MatmulPlan other;
         for (int bn : {128, 256}) {

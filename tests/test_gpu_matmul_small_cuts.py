@@ -9,10 +9,11 @@ from test_matmul_plan import plan
 
 # (m, n, k) with [N, K] weights: one token to 128, single CTAs and clusters of two to eight, k-blocks shared evenly and not, whole
 # and ragged inner dimensions, columns that end inside a tile, several token tiles
-CUTS = [((1, 64, 16000), {"split": "8", "bn": "128"}), ((16, 1000, 8200), {"split": "8", "bn": "64"}), ((17, 136, 4104), {"split": "8", "bt": "32"}),
+CUTS = [((1, 64, 16000), {"split": "8", "bn": "128"}), ((16, 1000, 8200), {"split": "8", "bn": "128"}), ((17, 136, 4104), {"split": "8", "bt": "32"}),
         ((33, 8, 1000), {"split": "8", "bt": "32"}), ((65, 264, 2056), {"split": "8", "bt": "32"}), ((32, 4096, 8192), {"split": "4", "bn": "128"}),
         ((100, 520, 136), {"split": "1", "bt": "32"}), ((72, 1000, 72), {"split": "1", "bt": "32"}), ((128, 8192, 1032), {"split": "1", "bt": "64"}),
-        ((256, 128, 1000), {"split": "8", "bn": "64"}), ((136, 200, 1000), {"split": "8", "bt": "48"})]
+        ((256, 128, 1000), {"split": "8", "bn": "64"}), ((136, 200, 1000), {"split": "8", "bt": "48"}),
+        ((250, 136, 8200), {"split": "8", "bt": "64"}), ((1000, 72, 2504), {"split": "4", "bt": "64"})]
 
 
 @pytest.mark.parametrize("ta,tb", LAYOUTS)
@@ -27,7 +28,7 @@ def test_token_split(shape, cut, ta, tb):
 # short inner dimensions on one-SM tiles, long ones with few rows on 256 x 256 tiles that pairs share
 OTHERS = [((1000, 4104, 72), "one_sm", {"bn": "256"}), ((520, 7304, 200), "one_sm", {"bn": "256"}), ((200, 10248, 200), "one_sm", {"bn": "128"}),
           ((120, 7000, 256), "one_sm", {"bn": "128"}), ((255, 5192, 9888), "two_sm_split", {"bn": "256", "split": "3"}),
-          ((300, 2056, 12008), "two_sm_split", {"bn": "256", "split": "3"})]
+          ((300, 2056, 12008), "two_sm_split", {"bn": "256", "split": "3"}), ((759, 3824, 1552), "two_sm", {"bn": "160"})]
 
 
 @pytest.mark.parametrize("ta,tb", LAYOUTS)

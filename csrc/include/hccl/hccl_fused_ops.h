@@ -30,6 +30,12 @@ HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint6
 HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t outStride, const void* cosTable, const void* sinTable, uint64_t rows,
                          uint32_t nHeads, uint32_t headDim, int backward, hcclStream_t stream);
 
+// Gradient of an embedding table, every row of it: dTable[r] = sum of dy[t] over the tokens t with ids[t] == r, in token order in fp32,
+// zero where there is none.  ids: int64 [tokens], at most 8192 (others are HCCL_E_NOT_SUPPORT; ids outside the table are left out); dy
+// [tokens, hidden], dTable [vocab, hidden]: bf16, hidden a multiple of 8; marks: scratch of vocab bytes, 16-byte aligned.
+HcclResult HcclFusedEmbeddingBwd(const int64_t* ids, const void* dy, void* dTable, void* marks, uint64_t tokens, uint64_t vocab, uint32_t hidden,
+                                 hcclStream_t stream);
+
 // AdamW (decoupled weight decay, bias correction as torch.optim.AdamW) over a list of tensors: one launch per 80
 // tensors plus one for the step counter.  `tensors` is a HOST array; it travels in the kernels' parameter space, so
 // nothing is uploaded or allocated and the call can be captured in a CUDA graph.  paramType is the storage type of

@@ -505,6 +505,82 @@ __global__ void __launch_bounds__(kRopeThreads) RopeKernel(const __nv_bfloat16* 
     }
 }
 
+// Gradient of an embedding table.  Bound by the rows it writes, nearly all of them zero: 67 MB for 4096 rows of 8192 beside 17 MB
+// of 1024 tokens' gradients.  One kernel writes every row once in place of a fill and a second pass over the rows in use;
+// which rows are in use is marked before, so that the others need not look for their tokens.  A block takes up to 256
+// vectors of a row; if its row is in use it goes through the ids, 256 at a time, keeps the places of its tokens in order and adds their
+// gradients, eight loads at a time (a token that is every tenth of the text has hundreds).  Eager, with what autograd adds (us, before on
+// PyTorch's kernels -> now): 4096 x 8192, 1024 tokens 73 -> 50; 32000 x 4096, 4096 tokens 488 -> 153, one of them every tenth 469 -> 148;
+// 128256 x 8192, 8192 tokens 1791 -> 1047 (2.1 GB written).
+constexpr int kEmbThreads = 256;
+constexpr uint64_t kEmbMaxTokens = 8192;          // beyond, rows in use would read more ids than gradients
+__global__ void __launch_bounds__(1024) EmbeddingMarkKernel(const long long* __restrict__ ids, uint32_t tokens, uint8_t* __restrict__ marks, uint32_t vocab)
+{
+    DependencyWait();
+    AllowDependents();
+    for (uint32_t i = threadIdx.x; i < (vocab + 15) / 16; i += blockDim.x) {
+        if (i * 16 + 16 <= vocab) reinterpret_cast<uint4*>(marks)[i] = make_uint4(0, 0, 0, 0);
+        else for (uint32_t k = i * 16; k < vocab; ++k) marks[k] = 0;
+    }
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < tokens; t += blockDim.x) {
+        const long long id = ids[t];
+        if (id >= 0 && id < (long long)vocab) marks[id] = 1;
+    }
+}
+__global__ void __launch_bounds__(kEmbThreads) EmbeddingBwdKernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
+                                                                  __nv_bfloat16* __restrict__ dTable, const uint8_t* __restrict__ marks, uint32_t tokens,
+                                                                  int hidden, int chunks)
+{
+    DependencyWait();
+    AllowDependents();
+    __shared__ uint32_t s_hits[kEmbThreads / 32];
+    __shared__ uint16_t s_list[kEmbThreads];
+    const uint32_t row = blockIdx.x / (uint32_t)chunks;
+    const int v = (int)(blockIdx.x - row * (uint32_t)chunks) * kEmbThreads + (int)threadIdx.x, nVec = hidden / 8;
+    const bool mine = v < nVec;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (marks[row] != 0) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        long long id = threadIdx.x < tokens ? ids[threadIdx.x] : -1;
+        for (uint32_t base = 0; base < tokens; base += kEmbThreads) {
+            const bool hit = id == (long long)row;
+            const uint32_t following = base + kEmbThreads + threadIdx.x;
+            id = following < tokens ? ids[following] : -1;
+            if (__syncthreads_count(hit) == 0) continue;
+            const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+            if (lane == 0) s_hits[warp] = hits;
+            __syncthreads();
+            int before = 0, n = 0;
+#pragma unroll
+            for (int w = 0; w < kEmbThreads / 32; ++w) {
+                if (w < warp) before += __popc(s_hits[w]);
+                n += __popc(s_hits[w]);
+            }
+            if (hit) s_list[before + __popc(hits & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
+            __syncthreads();
+            const __nv_bfloat16* from = dy + (size_t)base * hidden;
+            constexpr int U = 8;
+            for (int i = 0; mine && i < n; i += U) {
+                uint4 raw[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (i + u < n) raw[u] = reinterpret_cast<const uint4*>(from + (size_t)s_list[i + u] * hidden)[v];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (i + u >= n) break;
+                    float f[8];
+                    Unpack8(raw[u], f);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[k] += f[k];
+                }
+            }
+            __syncthreads();                          // the list is read, the next 256 ids may take its place
+        }
+    }
+    if (mine) reinterpret_cast<uint4*>(dTable + (size_t)row * hidden)[v] = Pack8(acc);
+}
+
 // Lets a norm kernel take the largest ring the norm kernels use.
 template <auto KERNEL> HcclResult AllowNormRing()
 {
@@ -645,6 +721,20 @@ HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t 
                                     (const float*)cosTable, (const float*)sinTable, rows, (int)nHeads, (int)headDim, backward ? -1.f : 1.f,
                                     (int)rowsPerBlock),
                     "Rope");
+}
+
+HcclResult HcclFusedEmbeddingBwd(const int64_t* ids, const void* dy, void* dTable, void* marks, uint64_t tokens, uint64_t vocab, uint32_t hidden,
+                                 hcclStream_t stream)
+{
+    CHK_PTR_NULL(ids); CHK_PTR_NULL(dy); CHK_PTR_NULL(dTable); CHK_PTR_NULL(marks);
+    if (hidden == 0 || hidden % 8 != 0 || !Aligned16(dy) || !Aligned16(dTable) || !Aligned16(marks) || (reinterpret_cast<uintptr_t>(ids) & 7u) != 0) return HCCL_E_PARA;
+    const uint64_t chunks = (hidden / 8 + kEmbThreads - 1) / kEmbThreads;
+    if (tokens > kEmbMaxTokens || vocab * chunks > 0x7FFFFFFFull || hidden > 0x7FFFFFFFu) return HCCL_E_NOT_SUPPORT;
+    if (vocab == 0) return HCCL_SUCCESS;
+    CHK_RET(Launched(LaunchDependent(EmbeddingMarkKernel, 1, 1024, 0, (cudaStream_t)stream, 0, reinterpret_cast<const long long*>(ids), (uint32_t)tokens,
+                                     (uint8_t*)marks, (uint32_t)vocab), "EmbeddingMark"));
+    return Launched(LaunchDependent(EmbeddingBwdKernel, (unsigned)(vocab * chunks), kEmbThreads, 0, (cudaStream_t)stream, 0, reinterpret_cast<const long long*>(ids),
+                                    (const __nv_bfloat16*)dy, (__nv_bfloat16*)dTable, (const uint8_t*)marks, (uint32_t)tokens, (int)hidden, (int)chunks), "EmbeddingBwd");
 }
 
 }  // extern "C"

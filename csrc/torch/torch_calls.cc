@@ -7,7 +7,7 @@
 // anything else it returns None and the caller goes the general way (torch.autograd.Function, ctypes), which also words the
 // errors.  An int is the HcclResult of a failed call.
 //
-// The second part (add_rms_norm_grad, swiglu_grad, rope_grad, linear) records gradients: nodes of autograd's graph in the place of
+// The second part (add_rms_norm_grad, swiglu_grad, rope_grad, linear, embedding) records gradients: nodes of autograd's graph in the place of
 // Python functions, whose passes through the interpreter took 100 us of the host for a norm forward and backward and 250 for the
 // FFN half of a layer, several times what the kernels of a small one take.
 //
@@ -48,6 +48,7 @@ struct Api {
     decltype(&HcclFusedSwigluBwd) swigluBwd;
     decltype(&HcclFusedRope) rope;
     decltype(&HcclMc2Matmul) matmul;
+    decltype(&HcclFusedEmbeddingBwd) embeddingBwd;
     decltype(&HcclMoeExpertOffsets) expertOffsets;
     decltype(&HcclAllReduce) allReduce;
     decltype(&HcclReduceScatter) reduceScatter;
@@ -60,6 +61,7 @@ const Slot kSlots[] = {
     {"HcclFusedAddRmsNormFwd", (void**)&api.addRmsNormFwd}, {"HcclFusedRmsNormBwdPartials", (void**)&api.rmsNormBwdPartials},
     {"HcclFusedRmsNormBwdCopy", (void**)&api.rmsNormBwd},   {"HcclFusedSwigluFwd", (void**)&api.swigluFwd},
     {"HcclFusedSwigluBwd", (void**)&api.swigluBwd},         {"HcclFusedRope", (void**)&api.rope},
+    {"HcclFusedEmbeddingBwd", (void**)&api.embeddingBwd},
     {"HcclMc2Matmul", (void**)&api.matmul},                 {"HcclMoeExpertOffsets", (void**)&api.expertOffsets},
     {"HcclAllReduce", (void**)&api.allReduce},              {"HcclReduceScatter", (void**)&api.reduceScatter},
     {"HcclAllGather", (void**)&api.allGather},              {"HcclAlltoAll", (void**)&api.alltoAll},
@@ -650,6 +652,55 @@ PyObject* Linear(PyObject*, PyObject* const* a, Py_ssize_t nargs)
         return r != 0 ? PyLong_FromLong(r) : Wrap(std::move(out));
     });
 }
+struct EmbeddingNode : Node {
+    SavedVariable ids;
+    int64_t vocab = 0;
+    std::string name() const override { return "_EmbeddingBackward"; }
+    void release_variables() override
+    {
+        std::lock_guard<std::mutex> lock(mutex_);
+        ids.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        Tensor i;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            i = ids.unpack();
+        }
+        c10::AutoGradMode off(false);
+        const Tensor dy = grads[0].contiguous();
+        Tensor dTable = at::empty({vocab, dy.size(1)}, dy.options()), marks = at::empty({vocab}, dy.options().dtype(at::kByte));
+        CheckBackward(api.embeddingBwd(i.const_data_ptr<int64_t>(), dy.const_data_ptr(), dTable.mutable_data_ptr(), marks.mutable_data_ptr(), (uint64_t)dy.size(0),
+                                       (uint64_t)vocab, (uint32_t)dy.size(1), Stream()),
+                      "HcclFusedEmbeddingBwd");
+        launches += 2;
+        return {std::move(dTable)};
+    }
+};
+// (ids [tokens], table [vocab, hidden]) -> the rows
+PyObject* Embedding(PyObject*, PyObject* const* a, Py_ssize_t nargs)
+{
+    HCCL_ARGS(2)
+    return Guarded([&]() -> PyObject* {
+        const Tensor *ids = GetPlain(a[0]), *table = GetRecordable(a[1]);
+        if (!ids || !table || !Records({table}) || !PlainCall() || ids->scalar_type() != at::kLong || ids->dim() != 1 || !ids->is_contiguous()) return None();
+        if (table->dim() != 2 || table->numel() == 0 || ids->numel() == 0 || ids->numel() > 8192 || table->size(1) % 8 != 0 || table->size(0) > (1 << 24)) return None();
+        Tensor out;
+        {
+            Unlocked unlocked;
+            c10::AutoGradMode off(false);
+            out = at::embedding(*table, *ids);
+            auto node = std::make_shared<EmbeddingNode>();
+            TakeInputs(node, *table);
+            GiveOutput(node, out);
+            node->ids = SavedVariable(*ids, false);
+            node->vocab = table->size(0);
+        }
+        return Wrap(std::move(out));
+    });
+}
 PyObject* Launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launches.load()); }
 PyObject* Raises(PyObject*, PyObject* error)
 {
@@ -697,6 +748,7 @@ PyMethodDef methods[] = {
     {"rope", HCCL_FAST(Rope)},                 {"matmul", HCCL_FAST(Matmul)},               {"expert_offsets", HCCL_FAST(ExpertOffsets)},
     {"collective", HCCL_FAST(Collective)},     {"add_rms_norm_grad", HCCL_FAST(AddRmsNormGrad)},
     {"swiglu_grad", HCCL_FAST(SwigluGrad)},    {"rope_grad", HCCL_FAST(RopeGrad)},          {"linear", HCCL_FAST(Linear)},
+    {"embedding", HCCL_FAST(Embedding)},
     {"launches", Launches, METH_NOARGS, nullptr}, {"raises", Raises, METH_O, nullptr},      {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "hccl_b200_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -43,7 +43,8 @@ add_rms_norm, rms_norm_bwd, swiglu_fwd, swiglu_bwd, rope, matmul, expert_offsets
     getattr(_module, name, _nothing)
     for name in ("add_rms_norm", "rms_norm_bwd", "swiglu_fwd", "swiglu_bwd", "rope", "matmul", "expert_offsets", "collective"))
 # the same where gradients are recorded (``linear``: recorded or not)
-add_rms_norm_grad, swiglu_grad, rope_grad, linear = (getattr(_module, name, _nothing) for name in ("add_rms_norm_grad", "swiglu_grad", "rope_grad", "linear"))
+add_rms_norm_grad, swiglu_grad, rope_grad, linear, embedding = (
+    getattr(_module, name, _nothing) for name in ("add_rms_norm_grad", "swiglu_grad", "rope_grad", "linear", "embedding"))
 
 
 def launches() -> int:

@@ -87,7 +87,7 @@ class DecoderLayer(torch.nn.Module):
         q, k, v = fused.rope_qkv(qkv, cos, sin, self.hq, self.hkv, use_kernels=k_)
         attn = F.scaled_dot_product_attention(q.transpose(0, 1)[None], k.transpose(0, 1)[None], v.transpose(0, 1)[None], is_causal=True,
                                               enable_gqa=self.hq != self.hkv)
-        attn = attn[0].transpose(0, 1).reshape(s, self.hq * d)
+        attn = attn.squeeze(0).transpose(0, 1).reshape(s, self.hq * d)      # (the backward pass of attn[0] fills and copies a tensor)
         x, h = fused.add_rms_norm(x, self.o(attn), self.ffn_norm, cfg.norm_eps, use_kernels=k_)
         return x, self.down(fused.swiglu(self.gate_up(h), use_kernels=k_))
 
@@ -179,7 +179,7 @@ class LlamaStack(torch.nn.Module):
         s = token_ids.shape[0]
         p = self.ctx.world
         assert s % p == 0
-        x = F.embedding(token_ids, self.embed) if p == 1 else _ShardedEmbedding.apply(token_ids, self.embed, self.ctx)
+        x = fused.embedding(token_ids, self.embed, use_kernels=self.ctx.fused_ops) if p == 1 else _ShardedEmbedding.apply(token_ids, self.embed, self.ctx)
         if self._rope is None or self._rope[0].shape[0] != s:
             self._rope = rope_tables(s, self.cfg.head_dim, self.cfg.rope_theta, x.device)
         cos, sin = self._rope

@@ -4,6 +4,7 @@
 * ``swiglu(gate_up)`` -> ``silu(gate) * up`` for ``gate_up = [gate | up]`` along the last dimension
 * ``rope(x, cos, sin)`` -> rotary embedding ("rotate halves") of ``x [S, heads, D]``; ``x`` may be a column slice
   of a wider projection output (row stride larger than ``heads * D``)
+* ``embedding(ids, table)`` -> ``table[ids]`` with the table's gradient written in one pass over its rows
 * ``rope_qkv(qkv, cos, sin, hq, hkv)`` -> ``(q, k, v)`` of a projection output ``[S, (hq + 2 hkv) * D]`` with q and k rotated
 
 CUDA bf16 tensors run the hand-written kernels (csrc/kernels/fused_elementwise.cu); anything else (CPU tensors, other
@@ -271,9 +272,7 @@ def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
 
 def swiglu(gate_up, use_kernels: bool = True):
     out = _calls.swiglu_fwd(gate_up) if use_kernels else None
-    if out is None and use_kernels:
-        out = _calls.swiglu_grad(gate_up)
-    if out is not None:
+    if out is not None or use_kernels and (out := _calls.swiglu_grad(gate_up)) is not None:
         out = _calls.result(out, "HcclFusedSwigluFwd")
         _count()
         return out
@@ -290,9 +289,7 @@ def _rope_table(t, x) -> bool:
 def rope(x, cos, sin, use_kernels: bool = True):
     """x [S, heads, D] (row stride may exceed heads * D), cos / sin fp32 [S, D / 2]."""
     out = _calls.rope(x, cos, sin, False) if use_kernels else None
-    if out is None and use_kernels:
-        out = _calls.rope_grad(x, cos, sin)
-    if out is not None:
+    if out is not None or use_kernels and (out := _calls.rope_grad(x, cos, sin)) is not None:
         out = _calls.result(out, "HcclFusedRope")
         _count()
         return out
@@ -312,3 +309,9 @@ def rope_qkv(qkv, cos, sin, hq: int, hkv: int, use_kernels: bool = True):
     q = rope(qkv[:, :hq * d].view(s, hq, d), cos, sin, use_kernels=use_kernels)
     k = rope(qkv[:, hq * d:(hq + hkv) * d].view(s, hkv, d), cos, sin, use_kernels=use_kernels)
     return q, k, qkv[:, (hq + hkv) * d:].view(s, hkv, d)
+
+
+def embedding(ids, table, use_kernels: bool = True):
+    """Rows ``ids`` of ``table [vocab, hidden]``.  Up to 8192 tokens the table's gradient is this library's kernel."""
+    out = _calls.embedding(ids, table) if use_kernels else None
+    return out if out is not None else F.embedding(ids, table)

@@ -1,0 +1,76 @@
+"""The embedding's gradient kernel: every row of the table, the rows in use summed in token order."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from hccl_b200 import Result, _calls
+from hccl_b200._lib import lib
+from hccl_b200.ops import fused
+
+
+def _case(tokens, vocab, hidden, skew=False, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    ids = torch.randint(0, vocab, (tokens,), device="cuda", generator=g)
+    if skew:                                             # every other token is the same one
+        ids[::2] = vocab - 1
+    return ids, torch.randn(vocab, hidden, device="cuda", generator=g).bfloat16(), torch.randn(tokens, hidden, device="cuda", generator=g).bfloat16()
+
+
+def _want(ids, dy, vocab):
+    return torch.zeros(vocab, dy.shape[1], device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+
+
+# one token, ids at the edges of the 256 that are looked at together, rows of one vector and of several blocks, a table that is no
+# multiple of 16 rows, many tokens of one id
+@pytest.mark.parametrize("tokens,vocab,hidden,skew", [(1, 1, 8, False), (255, 17, 64, False), (256, 1000, 2048, False), (257, 33, 2056, True), (1024, 4096, 8192, False),
+                                                      (2000, 5, 520, True), (8192, 50000, 128, True)])
+def test_against_64_bits(tokens, vocab, hidden, skew):
+    ids, table, dy = _case(tokens, vocab, hidden, skew)
+    t = table.clone().requires_grad_()
+    out = fused.embedding(ids, t)
+    assert out.grad_fn.name() == "_EmbeddingBackward" and torch.equal(out, table[ids])
+    out.backward(dy)
+    want = _want(ids, dy, vocab)
+    # sums in fp32, one rounding to bf16 (half a unit in the last of 8 places)
+    bound = want.abs() * 2 ** -8 + torch.zeros_like(want).index_add_(0, ids, dy.double().abs()) * tokens * 2 ** -24 + 1e-30
+    assert ((t.grad.double() - want).abs() <= bound).all()
+    assert (t.grad[torch.bincount(ids, minlength=vocab) == 0] == 0).all()
+    again = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+    assert torch.equal(again, t.grad)
+
+
+def test_what_is_left_to_pytorch():
+    ids, table, _ = _case(40, 64, 64)
+    assert _calls.embedding(ids, table) is None                                            # nothing is recorded
+    t = table.clone().requires_grad_()
+    for i, w in ((ids.int(), t), (ids.view(8, 5), t), (ids, t.detach().float().requires_grad_()), (ids.repeat(300), t), (ids[:0], t), (ids.cpu(), t)):
+        assert _calls.embedding(i, w) is None
+    assert fused.embedding(ids.view(8, 5), t).shape == (8, 5, 64) and fused.embedding(ids, table).grad_fn is None
+
+
+def test_calls_that_are_refused():
+    p, s = ctypes.c_void_p(1 << 20), torch.cuda.current_stream().cuda_stream
+    bwd = lib.HcclFusedEmbeddingBwd
+    bwd.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_uint64] * 2 + [ctypes.c_uint32, ctypes.c_void_p]
+    assert bwd(p, p, p, p, 8193, 10, 64, s) == Result.E_NOT_SUPPORT
+    assert bwd(p, p, p, p, 8, 10, 60, s) == Result.E_PARA and bwd(p, ctypes.c_void_p((1 << 20) + 8), p, p, 8, 10, 64, s) == Result.E_PARA
+    assert bwd(p, p, p, p, 8, 0, 64, s) == 0
+
+
+def test_captured_and_side_stream():
+    ids, table, dy = _case(300, 128, 256)
+    t = table.clone().requires_grad_()
+    want = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.autograd.grad(fused.embedding(ids, t), t, dy)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            got = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+        g.replay()
+    side.synchronize()
+    assert torch.equal(got, want)

@@ -61,11 +61,13 @@ const Slot kSlots[] = {
     {"HcclFusedAddRmsNormFwd", (void**)&api.addRmsNormFwd}, {"HcclFusedRmsNormBwdPartials", (void**)&api.rmsNormBwdPartials},
     {"HcclFusedRmsNormBwdCopy", (void**)&api.rmsNormBwd},   {"HcclFusedSwigluFwd", (void**)&api.swigluFwd},
     {"HcclFusedSwigluBwd", (void**)&api.swigluBwd},         {"HcclFusedRope", (void**)&api.rope},
-    {"HcclFusedEmbeddingBwd", (void**)&api.embeddingBwd},
     {"HcclMc2Matmul", (void**)&api.matmul},                 {"HcclMoeExpertOffsets", (void**)&api.expertOffsets},
     {"HcclAllReduce", (void**)&api.allReduce},              {"HcclReduceScatter", (void**)&api.reduceScatter},
     {"HcclAllGather", (void**)&api.allGather},              {"HcclAlltoAll", (void**)&api.alltoAll},
 };
+
+// Functions that only the backward passes of recorded calls use.
+const Slot kBackwardSlots[] = {{"HcclFusedEmbeddingBwd", (void**)&api.embeddingBwd}};
 
 // The function mode behind torch.set_default_device and `with torch.device(...)`.  It gives a device to factory calls that name
 // none; these calls name theirs, so that it has nothing to see here.
@@ -384,6 +386,8 @@ bool Records(std::initializer_list<const Tensor*> inputs)
         if (t != nullptr && t->requires_grad()) return true;
     return false;
 }
+// Owned as autograd owns its own nodes: long chains of them are freed one by one, not in each other's destructors.
+template <class T> std::shared_ptr<T> NewNode() { return std::shared_ptr<T>(new T(), torch::autograd::deleteNode); }
 template <class... T> void TakeInputs(const std::shared_ptr<Node>& node, const T&... inputs) { node->set_next_edges(torch::autograd::collect_next_edges(inputs...)); }
 void GiveOutput(const std::shared_ptr<Node>& node, const Tensor& out)
 {
@@ -465,7 +469,7 @@ PyObject* AddRmsNormGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
                                                delta ? xOut.mutable_data_ptr() : nullptr, h.mutable_data_ptr(), rstd.mutable_data_ptr(), rows, (uint32_t)hidden, eps,
                                                Stream());
             if (code != 0) return code;
-            auto node = std::make_shared<AddRmsNormNode>();
+            auto node = NewNode<AddRmsNormNode>();
             node->hasDelta = delta != nullptr;
             if (delta) TakeInputs(node, *x, *delta, *w);
             else TakeInputs(node, *x, *w);
@@ -524,7 +528,7 @@ PyObject* SwigluGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
             out = at::empty(sizes, x->options());
             const int code = api.swigluFwd(x->const_data_ptr(), out.mutable_data_ptr(), (uint64_t)(x->numel() / (2 * f)), (uint32_t)f, Stream());
             if (code != 0) return code;
-            auto node = std::make_shared<SwigluNode>();
+            auto node = NewNode<SwigluNode>();
             TakeInputs(node, *x);
             GiveOutput(node, out);
             node->gateUp = SavedVariable(*x, false);
@@ -583,7 +587,7 @@ PyObject* RopeGrad(PyObject*, PyObject* const* a, Py_ssize_t nargs)
             const int code = api.rope(x->const_data_ptr(), (uint64_t)x->stride(0), out.mutable_data_ptr(), (uint64_t)(heads * d), c->const_data_ptr(),
                                       s->const_data_ptr(), (uint64_t)rows, (uint32_t)heads, (uint32_t)d, 0, Stream());
             if (code != 0) return code;
-            auto node = std::make_shared<RopeNode>();
+            auto node = NewNode<RopeNode>();
             TakeInputs(node, *x);
             GiveOutput(node, out);
             node->cos = SavedVariable(*c, false);
@@ -641,7 +645,7 @@ PyObject* Linear(PyObject*, PyObject* const* a, Py_ssize_t nargs)
                                         (uint64_t)x->size(1), 0, 1, Stream());
             if (code != 0) return code;
             if (!record) return 0;
-            auto node = std::make_shared<LinearNode>();
+            auto node = NewNode<LinearNode>();
             TakeInputs(node, *x, *w);
             GiveOutput(node, out);
             node->x = SavedVariable(*x, false);
@@ -685,14 +689,14 @@ PyObject* Embedding(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     HCCL_ARGS(2)
     return Guarded([&]() -> PyObject* {
         const Tensor *ids = GetPlain(a[0]), *table = GetRecordable(a[1]);
-        if (!ids || !table || !Records({table}) || !PlainCall() || ids->scalar_type() != at::kLong || ids->dim() != 1 || !ids->is_contiguous()) return None();
+        if (api.embeddingBwd == nullptr || !ids || !table || !Records({table}) || !PlainCall() || ids->scalar_type() != at::kLong || ids->dim() != 1 || !ids->is_contiguous()) return None();
         if (table->dim() != 2 || table->numel() == 0 || ids->numel() == 0 || ids->numel() > 8192 || table->size(1) % 8 != 0 || table->size(0) > (1 << 24)) return None();
         Tensor out;
         {
             Unlocked unlocked;
             c10::AutoGradMode off(false);
             out = at::embedding(*table, *ids);
-            auto node = std::make_shared<EmbeddingNode>();
+            auto node = NewNode<EmbeddingNode>();
             TakeInputs(node, *table);
             GiveOutput(node, out);
             node->ids = SavedVariable(*ids, false);
@@ -709,6 +713,19 @@ PyObject* Raises(PyObject*, PyObject* error)
     Py_RETURN_NONE;
 }
 
+PyObject* BindSlots(const Slot* slots, size_t n, PyObject* addresses)
+{
+    for (size_t i = 0; i < n; ++i) {
+        PyObject* v = PyDict_GetItemString(addresses, slots[i].name);
+        void* p = v ? PyLong_AsVoidPtr(v) : nullptr;
+        if (p == nullptr) {
+            if (!PyErr_Occurred()) PyErr_Format(PyExc_KeyError, "no address of %s", slots[i].name);
+            return nullptr;
+        }
+        *slots[i].at = p;
+    }
+    Py_RETURN_NONE;
+}
 PyObject* Bind(PyObject*, PyObject* addresses)
 {
     if (defaultDeviceMode == nullptr) {
@@ -719,27 +736,21 @@ PyObject* Bind(PyObject*, PyObject* addresses)
         Py_XDECREF(devices);
         PyErr_Clear();                 // another torch without it: its default devices go the general way
     }
-    for (const Slot& s : kSlots) {
-        PyObject* v = PyDict_GetItemString(addresses, s.name);
-        void* p = v ? PyLong_AsVoidPtr(v) : nullptr;
-        if (p == nullptr) {
-            if (!PyErr_Occurred()) PyErr_Format(PyExc_KeyError, "no address of %s", s.name);
-            return nullptr;
-        }
-        *s.at = p;
-    }
-    Py_RETURN_NONE;
+    return BindSlots(kSlots, sizeof(kSlots) / sizeof(kSlots[0]), addresses);
 }
-PyObject* Names(PyObject*, PyObject*)
+PyObject* BindBackward(PyObject*, PyObject* addresses) { return BindSlots(kBackwardSlots, sizeof(kBackwardSlots) / sizeof(kBackwardSlots[0]), addresses); }
+PyObject* NamesOf(const Slot* slots, size_t n)
 {
     PyObject* out = PyList_New(0);
-    for (const Slot& s : kSlots) {
-        PyObject* n = PyUnicode_FromString(s.name);
-        PyList_Append(out, n);
-        Py_DECREF(n);
+    for (size_t i = 0; i < n; ++i) {
+        PyObject* name = PyUnicode_FromString(slots[i].name);
+        PyList_Append(out, name);
+        Py_DECREF(name);
     }
     return out;
 }
+PyObject* Names(PyObject*, PyObject*) { return NamesOf(kSlots, sizeof(kSlots) / sizeof(kSlots[0])); }
+PyObject* BackwardNames(PyObject*, PyObject*) { return NamesOf(kBackwardSlots, sizeof(kBackwardSlots) / sizeof(kBackwardSlots[0])); }
 
 #define HCCL_FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr
 PyMethodDef methods[] = {
@@ -749,6 +760,7 @@ PyMethodDef methods[] = {
     {"collective", HCCL_FAST(Collective)},     {"add_rms_norm_grad", HCCL_FAST(AddRmsNormGrad)},
     {"swiglu_grad", HCCL_FAST(SwigluGrad)},    {"rope_grad", HCCL_FAST(RopeGrad)},          {"linear", HCCL_FAST(Linear)},
     {"embedding", HCCL_FAST(Embedding)},
+    {"bind_backward", BindBackward, METH_O, nullptr}, {"backward_names", BackwardNames, METH_NOARGS, nullptr},
     {"launches", Launches, METH_NOARGS, nullptr}, {"raises", Raises, METH_O, nullptr},      {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "hccl_b200_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -31,6 +31,8 @@ def _load():
         loader.exec_module(module)
         module.raises(HcclError)
         module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in module.names()})
+        if all(hasattr(lib, name) for name in module.backward_names()):
+            module.bind_backward({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in module.backward_names()})
         return module
     except (ImportError, AttributeError) as e:
         if torch.cuda.is_available():

@@ -39,3 +39,16 @@ def test_every_pair_has_a_slot_of_its_own(tokens, topk, experts, same):
     assert comms[0].async_error() == hb.Result.SUCCESS
     for c in comms:
         c.destroy()
+
+
+# one CTA adds up and scans up to 1024 experts, eight share them beyond; every CTA counts up to 8192
+@pytest.mark.parametrize("experts", [1, 31, 256, 1023, 1024, 1025, 8192, 8193])
+@pytest.mark.parametrize("pairs", [1, 4097, 65536])
+def test_expert_offsets_at_the_edges(experts, pairs):
+    from hccl_b200.ops.moe import expert_offsets
+    g = torch.Generator(device="cuda").manual_seed(experts)
+    ids = [torch.randint(-1, experts, (pairs,), device="cuda", generator=g, dtype=torch.int32) for _ in range(4)]
+    got = [expert_offsets(i, experts) for i in ids]                     # back to back: one starts under the other's end
+    for i, off in zip(ids, got):
+        n = torch.bincount(i[i >= 0].long(), minlength=experts)
+        assert torch.equal(off, torch.cat((n.new_zeros(1), n.cumsum(0))).int())

@@ -15,7 +15,7 @@
 //     CTAs in rank order (one fixed order, no atomics, no workspace) and stores them as bf16.  The order depends on the number of
 //     CTAs per tile and so on the shape: a row's fp32 sum may differ in its last place from that of a call with more rows.
 // The drain is a serial chain of a few warps: with more than 32 tokens eight warps share it, and a tile that nobody shares does not
-// pass through shared memory (128 x 1024 x 256 8.4 -> 2.9 us, 64 x 1024 x 256 5.5 -> 2.9).  Sending the partials to their owner
+// pass through shared memory (101 x 288 x 72 5.2 -> 2.8 us, 128 x 2048 x 512 7.0 -> 3.4).  Sending the partials to their owner
 // instead of fetching them was slower (128 x 10240 x 8192 35.6 against 34.4 us).
 // Measured against the one-SM kernel on 128 x 128 tiles (us, bf16, weight [N, K]): 16 x 8192 x 8192 47.5 -> 26.8 (5.0
 // TB/s), 64 x 8192 x 8192 48.4 -> 28.8; against its 256-wide form 16 x 57344 x 8192 160.6 -> 142.4 (6.6 TB/s), 64 x 57344 x 8192

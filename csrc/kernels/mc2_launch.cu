@@ -576,7 +576,7 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         p.split = Split2Pairs((int)tiles128, pairs);
         p.grid = (int)tiles128 * 2 * p.split;
         // long inner dimensions: 256 x 256 tiles, which bring a third fewer bytes per SM, shared by two to four pairs (255 x 5192 x 9888
-        // 37.1 -> 29.3 us, 137 x 5976 x 8048 45.3 -> 30.6)
+        // 37.1 -> 29.3 us, 193 x 5256 x 4216 26.6 -> 20.0)
         const SmallProduct s(m, n, k, aMn, bMn, sms);
         double us = PairsUs(s, 128, p.split);
         const MatmulPlan wide = BestPairs256(s, kOtherKernel * us);
@@ -650,8 +650,8 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         return p;
     }
     // Short inner dimensions, where the drain of a tile is longer than its math: one-SM tiles, of which twice as many are under way
-    // (1000 x 4096 x 256 7.1 -> 4.6 us, 2048 x 8192 x 256 15.6 -> 12.1; larger outputs stay, 2248 x 4368 x 192 11.1 -> 7.6 is the
-    // last kind that was timed).  Long ones with few tiles: 256 x 256 tiles that pairs share (255 x 5192 x 9888 37.1 -> 29.3 us).
+    // (1000 x 4096 x 256 7.1 -> 4.6 us, 2048 x 8192 x 256 15.6 -> 12.1; outputs of more than 2^24 elements were not timed on
+    // both and stay).  Long ones with few tiles: 256 x 256 tiles that pairs share (255 x 5192 x 9888 37.1 -> 29.3 us).
     if (!sw.l2Hints && outAlign >= 16 && sw.wide != 1 && m * n <= (1u << 24)) {
         const SmallProduct s(m, n, k, aMn, bMn, sms);
         double best = kOtherKernel * TwoSmUs(s, p.bn);

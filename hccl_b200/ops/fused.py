@@ -253,11 +253,13 @@ class _RopeQkv(torch.autograd.Function):
 # ----------------------------------------------------------------------------- public functions
 def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
     """``x_out = x + delta`` (``delta`` may be None) and ``h = rms_norm(x_out) * weight`` in one pass; returns both."""
+    global _launches
     r = _calls.add_rms_norm(x, delta, weight, eps) if use_kernels else None
     if r is not None:                                        # no gradient is recorded: no autograd function either
-        x_out, h, _ = _calls.result(r, "HcclFusedAddRmsNormFwd")
-        _count()
-        return x_out, h
+        if type(r) is int:
+            _check(r, "HcclFusedAddRmsNormFwd")
+        _launches += 1
+        return r[0], r[1]
     r = _calls.add_rms_norm_grad(x, delta, weight, eps) if use_kernels else None
     if r is not None:
         x_out, h = _calls.result(r, "HcclFusedAddRmsNormFwd")
@@ -271,10 +273,12 @@ def add_rms_norm(x, delta, weight, eps: float = 1e-5, use_kernels: bool = True):
 
 
 def swiglu(gate_up, use_kernels: bool = True):
+    global _launches
     out = _calls.swiglu_fwd(gate_up) if use_kernels else None
     if out is not None or use_kernels and (out := _calls.swiglu_grad(gate_up)) is not None:
-        out = _calls.result(out, "HcclFusedSwigluFwd")
-        _count()
+        if type(out) is int:
+            _check(out, "HcclFusedSwigluFwd")
+        _launches += 1
         return out
     if use_kernels and _native(gate_up) and (gate_up.shape[-1] // 2) % 8 == 0:
         return _Swiglu.apply(gate_up)
@@ -288,10 +292,12 @@ def _rope_table(t, x) -> bool:
 
 def rope(x, cos, sin, use_kernels: bool = True):
     """x [S, heads, D] (row stride may exceed heads * D), cos / sin fp32 [S, D / 2]."""
+    global _launches
     out = _calls.rope(x, cos, sin, False) if use_kernels else None
     if out is not None or use_kernels and (out := _calls.rope_grad(x, cos, sin)) is not None:
-        out = _calls.result(out, "HcclFusedRope")
-        _count()
+        if type(out) is int:
+            _check(out, "HcclFusedRope")
+        _launches += 1
         return out
     if (use_kernels and _native(x) and x.shape[-1] % 16 == 0 and x.stride(2) == 1 and x.stride(1) == x.shape[-1] and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and _rope_table(cos, x) and _rope_table(sin, x)):

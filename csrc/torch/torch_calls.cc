@@ -79,12 +79,12 @@ bool FunctionModes()
         if (Py_TYPE(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter())) != defaultDeviceMode) return true;
     return false;
 }
-// A call that nothing but its own arithmetic is asked of: no tracer, no mode, no functional transform around it.
-bool PlainCall()
+bool HasModes()
 {
-    return !FunctionModes() && !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
-           !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+    return c10::impl::TorchDispatchModeTLS::any_modes_set() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
+// A call that nothing but its own arithmetic is asked of: no tracer, no mode, no functional transform around it.
+bool PlainCall() { return !FunctionModes() && !torch::jit::tracer::isTracing() && !HasModes(); }
 // A dense CUDA tensor that nothing looks at and nothing is recorded for.
 bool Plain(const Tensor& t)
 {
@@ -673,6 +673,9 @@ struct EmbeddingNode : Node {
             std::lock_guard<std::mutex> lock(mutex_);
             i = ids.unpack();
         }
+        // A gradient that is recorded itself (create_graph), batched, dual, a subclass or seen by a mode takes PyTorch's operator, which
+        // all of these look into.
+        if (!Plain(grads[0]) || !Plain(i) || HasModes()) return {at::embedding_dense_backward(grads[0], i, vocab, -1, false)};
         c10::AutoGradMode off(false);
         const Tensor dy = grads[0].contiguous();
         Tensor dTable = at::empty({vocab, dy.size(1)}, dy.options()), marks = at::empty({vocab}, dy.options().dtype(at::kByte));

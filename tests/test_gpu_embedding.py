@@ -51,6 +51,23 @@ def test_what_is_left_to_pytorch():
     assert fused.embedding(ids.view(8, 5), t).shape == (8, 5, 64) and fused.embedding(ids, table).grad_fn is None
 
 
+def test_gradients_that_are_looked_at():
+    """Recorded, batched and dual gradients: what PyTorch's embedding makes of them."""
+    import torch.autograd.forward_ad as fwd
+    import torch.nn.functional as F
+    ids, table, dy = _case(40, 64, 64)
+    t, up, tangent = table.clone().requires_grad_(), dy.clone().requires_grad_(), _case(40, 64, 64, seed=1)[2]
+    got, want = ([torch.autograd.grad(f(ids, t), t, up, create_graph=True)[0]] for f in (fused.embedding, F.embedding))
+    for g in (got, want):                                                                  # the penalty's gradient goes through the table's
+        g.append(torch.autograd.grad(g[0].float().square().sum(), up)[0])
+        f = fused.embedding if g is got else F.embedding
+        g.append(torch.autograd.grad(f(ids, t), t, torch.stack((dy, 2 * dy, -dy)), is_grads_batched=True)[0])
+        with fwd.dual_level():
+            g += fwd.unpack_dual(torch.autograd.grad(f(ids, t), t, fwd.make_dual(dy, tangent))[0])
+    assert got[1].abs().sum() > 0 and got[4] is not None
+    assert all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
+
+
 def test_calls_that_are_refused():
     p, s = ctypes.c_void_p(1 << 20), torch.cuda.current_stream().cuda_stream
     bwd = lib.HcclFusedEmbeddingBwd

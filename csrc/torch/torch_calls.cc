@@ -677,7 +677,8 @@ struct EmbeddingNode : Node {
         // all of these look into.
         if (!Plain(grads[0]) || !Plain(i) || HasModes()) return {at::embedding_dense_backward(grads[0], i, vocab, -1, false)};
         c10::AutoGradMode off(false);
-        const Tensor dy = grads[0].contiguous();
+        Tensor dy = grads[0].contiguous();
+        if ((uintptr_t)dy.const_data_ptr() % 16 != 0) dy = dy.clone();      // a packed view that does not begin on 16 bytes
         Tensor dTable = at::empty({vocab, dy.size(1)}, dy.options()), marks = at::empty({vocab}, dy.options().dtype(at::kByte));
         CheckBackward(api.embeddingBwd(i.const_data_ptr<int64_t>(), dy.const_data_ptr(), dTable.mutable_data_ptr(), marks.mutable_data_ptr(), (uint64_t)dy.size(0),
                                        (uint64_t)vocab, (uint32_t)dy.size(1), Stream()),

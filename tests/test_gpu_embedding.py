@@ -68,6 +68,17 @@ def test_gradients_that_are_looked_at():
     assert all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
 
 
+def test_gradients_that_begin_anywhere():
+    """A packed view into a larger buffer at an odd element, and one that is not packed."""
+    ids, table, dy = _case(40, 64, 64)
+    t = table.clone().requires_grad_()
+    want = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+    odd = torch.cat((dy.new_zeros(1), dy.flatten()))[1:].view(40, 64)
+    assert odd.data_ptr() % 16 != 0
+    for g in (odd, dy.t().contiguous().t()):
+        assert torch.equal(torch.autograd.grad(fused.embedding(ids, t), t, g)[0], want)
+
+
 def test_calls_that_are_refused():
     p, s = ctypes.c_void_p(1 << 20), torch.cuda.current_stream().cuda_stream
     bwd = lib.HcclFusedEmbeddingBwd

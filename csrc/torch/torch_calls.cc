@@ -394,6 +394,8 @@ void GiveOutput(const std::shared_ptr<Node>& node, const Tensor& out)
     const uint32_t nr = node->add_input_metadata(out);
     torch::autograd::impl::set_gradient_edge(out, {node, nr});
 }
+// The gradient of a node's only output; zeros where what used that output gave none, as functions in Python get them.
+Tensor GradientOf(const Node& node, const Tensor& given) { return given.defined() ? given : node.input_metadata(0).zeros_like(); }
 // The gradient of an input ends in a leaf that holds none yet: the leaf keeps the tensor it is given if nobody else has it, and
 // copies it otherwise.  (Under autograd.grad the leaves keep nothing.)
 torch::autograd::AccumulateGrad* EmptyLeaf(const torch::autograd::Edge& edge)
@@ -495,14 +497,13 @@ struct SwigluNode : Node {
     }
     variable_list apply(variable_list&& grads) override
     {
-        if (!grads[0].defined()) return {Tensor()};
         Tensor x;
         {
             std::lock_guard<std::mutex> lock(mutex_);
             x = gateUp.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dout = grads[0].contiguous();
+        const Tensor dout = GradientOf(*this, grads[0]).contiguous();
         const int64_t f = x.size(-1) / 2;
         Tensor dx = at::empty_like(x);
         CheckBackward(api.swigluBwd(x.const_data_ptr(), dout.const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x.numel() / (2 * f)), (uint32_t)f, Stream()),
@@ -549,7 +550,6 @@ struct RopeNode : Node {
     }
     variable_list apply(variable_list&& grads) override
     {
-        if (!grads[0].defined()) return {Tensor()};
         Tensor c, s;
         {
             std::lock_guard<std::mutex> lock(mutex_);
@@ -557,7 +557,7 @@ struct RopeNode : Node {
             s = sin.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dout = grads[0].contiguous();
+        const Tensor dout = GradientOf(*this, grads[0]).contiguous();
         const int64_t rows = dout.size(0), heads = dout.size(1), d = dout.size(2);
         Tensor dx = at::empty_like(dout);
         CheckBackward(api.rope(dout.const_data_ptr(), (uint64_t)(heads * d), dx.mutable_data_ptr(), (uint64_t)(heads * d), c.const_data_ptr(), s.const_data_ptr(),
@@ -610,7 +610,6 @@ struct LinearNode : Node {
     }
     variable_list apply(variable_list&& grads) override
     {
-        if (!grads[0].defined()) return {Tensor(), Tensor()};
         Tensor in, w;
         {
             std::lock_guard<std::mutex> lock(mutex_);
@@ -618,7 +617,7 @@ struct LinearNode : Node {
             w = weight.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dy = grads[0].contiguous();
+        const Tensor dy = GradientOf(*this, grads[0]).contiguous();
         const uint64_t rows = (uint64_t)dy.size(0), n = (uint64_t)dy.size(1), k = (uint64_t)in.size(1);
         Tensor dw = at::empty({(int64_t)n, (int64_t)k}, dy.options()), dx = at::empty({(int64_t)rows, (int64_t)k}, dy.options());
         CheckBackward(api.matmul(dy.const_data_ptr(), in.const_data_ptr(), dw.mutable_data_ptr(), n, k, rows, 1, 0, Stream()), "HcclMc2Matmul");

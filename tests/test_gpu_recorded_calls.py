@@ -82,6 +82,28 @@ def test_only_some_outputs_and_inputs(way):
         assert not fused.add_rms_norm(x, d, w, 1e-5)[1].requires_grad
 
 
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_outputs_whose_gradient_is_undefined(way):
+    """Every leaf gets zeros, not nothing: an optimizer steps the ones and skips the others."""
+    leaves, outs, _ = _layer()
+    sum(_NoGradient.apply(o).float().sum() for o in outs).backward()
+    assert all(t.grad is not None and not t.grad.any() for t in leaves)
+    for f, x in ((fused.swiglu, _rnd(8, 64)), (lambda t: fused.rope(t.view(8, 1, 64), torch.ones(8, 32, device="cuda"), torch.zeros(8, 32, device="cuda")), _rnd(8, 64)),
+                 (ColumnParallelLinear(64, 128, TPContext(None), "up"), _rnd(8, 64))):
+        x.requires_grad_()
+        _NoGradient.apply(f(x)).sum().backward()
+        assert x.grad is not None and not x.grad.any()
+
+
 def test_what_autograd_checks_is_checked(way):
     x, w = _rnd(9, 64).requires_grad_(), _rnd(64).requires_grad_()
     y = fused.swiglu(fused.add_rms_norm(x * 1, None, w, 1e-5)[1])

@@ -28,7 +28,9 @@
 #include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/library.h>
 #include <atomic>
 #include <cstdint>
 #include "hccl/hccl.h"
@@ -395,7 +397,7 @@ void GiveOutput(const std::shared_ptr<Node>& node, const Tensor& out)
     torch::autograd::impl::set_gradient_edge(out, {node, nr});
 }
 // The gradient of a node's only output; zeros where what used that output gave none, as functions in Python get them.
-Tensor GradientOf(const Node& node, const Tensor& given) { return given.defined() ? given : node.input_metadata(0).zeros_like(); }
+Tensor GradientOf(const torch::autograd::InputMetadata& output, const Tensor& given) { return given.defined() ? given : output.zeros_like(); }
 // The gradient of an input ends in a leaf that holds none yet: the leaf keeps the tensor it is given if nobody else has it, and
 // copies it otherwise.  (Under autograd.grad the leaves keep nothing.)
 torch::autograd::AccumulateGrad* EmptyLeaf(const torch::autograd::Edge& edge)
@@ -408,6 +410,118 @@ torch::autograd::AccumulateGrad* EmptyLeaf(const torch::autograd::Edge& edge)
     const auto it = executed->find(leaf);
     return it != executed->end() && it->second.needed_ && !it->second.captures_ ? leaf : nullptr;
 }
+
+// ---- gradients of plain tensors: what the nodes' backward passes launch
+// (dx, dw, dx or, if that is asked for, a second copy of it)
+std::tuple<Tensor, Tensor, Tensor> NormGradient(const Tensor& dh, const Tensor& x, const Tensor& w, const Tensor& rstd, const Tensor& extra, bool twice)
+{
+    const int64_t hidden = x.size(-1);
+    const uint64_t rows = (uint64_t)(x.numel() / hidden);
+    Tensor dx = at::empty_like(x), copy = twice ? at::empty_like(x) : dx, dw = at::empty_like(w);
+    Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), hidden}, x.options().dtype(at::kFloat));
+    CheckBackward(api.rmsNormBwd(dh.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), rstd.const_data_ptr(), extra.defined() ? extra.const_data_ptr() : nullptr,
+                                 dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr, partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows,
+                                 (uint32_t)hidden, Stream()),
+                  "HcclFusedRmsNormBwdCopy");
+    launches += 2;
+    return {std::move(dx), std::move(dw), std::move(copy)};
+}
+Tensor SwigluGradient(const Tensor& dout, const Tensor& x)
+{
+    const int64_t f = x.size(-1) / 2;
+    Tensor dx = at::empty_like(x);
+    CheckBackward(api.swigluBwd(x.const_data_ptr(), dout.const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x.numel() / (2 * f)), (uint32_t)f, Stream()),
+                  "HcclFusedSwigluBwd");
+    launches += 1;
+    return dx;
+}
+Tensor RopeGradient(const Tensor& dout, const Tensor& cos, const Tensor& sin)
+{
+    const int64_t rows = dout.size(0), heads = dout.size(1), d = dout.size(2);
+    Tensor dx = at::empty_like(dout);
+    CheckBackward(api.rope(dout.const_data_ptr(), (uint64_t)(heads * d), dx.mutable_data_ptr(), (uint64_t)(heads * d), cos.const_data_ptr(), sin.const_data_ptr(),
+                           (uint64_t)rows, (uint32_t)heads, (uint32_t)d, 1, Stream()),
+                  "HcclFusedRope");
+    launches += 1;
+    return dx;
+}
+// (dx, dw)
+std::tuple<Tensor, Tensor> LinearGradient(const Tensor& dy, const Tensor& x, const Tensor& w)
+{
+    const uint64_t rows = (uint64_t)dy.size(0), n = (uint64_t)dy.size(1), k = (uint64_t)x.size(1);
+    Tensor dw = at::empty({(int64_t)n, (int64_t)k}, dy.options()), dx = at::empty({(int64_t)rows, (int64_t)k}, dy.options());
+    CheckBackward(api.matmul(dy.const_data_ptr(), x.const_data_ptr(), dw.mutable_data_ptr(), n, k, rows, 1, 0, Stream()), "HcclMc2Matmul");
+    CheckBackward(api.matmul(dy.const_data_ptr(), w.const_data_ptr(), dx.mutable_data_ptr(), rows, k, n, 0, 0, Stream()), "HcclMc2Matmul");
+    return {std::move(dx), std::move(dw)};
+}
+
+// ---- the same as operators of torch, for compiled backward passes (compiled autograd): its graph traces the nodes with tensors that have
+// no memory, holds these operators and launches when it runs
+using torch::dynamo::autograd::CompiledNodeArgs;
+using torch::dynamo::autograd::SwapSavedVariables;
+namespace ops {
+std::tuple<Tensor, Tensor> Norm(const Tensor& dh, const Tensor& x, const Tensor& w, const Tensor& rstd, const std::optional<Tensor>& extra)
+{
+    auto [dx, dw, copy] = NormGradient(dh.contiguous(), x.contiguous(), w.contiguous(), rstd.contiguous(), extra ? extra->contiguous() : Tensor(), false);
+    return {std::move(dx), std::move(dw)};
+}
+Tensor Swiglu(const Tensor& dout, const Tensor& x) { return SwigluGradient(dout.contiguous(), x.contiguous()); }
+Tensor Rope(const Tensor& dout, const Tensor& cos, const Tensor& sin) { return RopeGradient(dout.contiguous(), cos.contiguous(), sin.contiguous()); }
+std::tuple<Tensor, Tensor> Linear(const Tensor& dy, const Tensor& x, const Tensor& w)
+{
+    auto out = LinearGradient(dy.contiguous(), x.contiguous(), w.contiguous());
+    launches += 2;
+    return out;
+}
+Tensor PackedLike(const Tensor& t) { return at::empty_symint(t.sym_sizes(), t.options()); }
+void Define()
+{
+    if (c10::Dispatcher::singleton().findSchema({"hccl_b200::linear_backward", ""})) return;       // by another copy of this module
+    static torch::Library lib(torch::Library::FRAGMENT, "hccl_b200", std::nullopt, __FILE__, __LINE__);
+    lib.def("norm_backward(Tensor dh, Tensor x, Tensor weight, Tensor rstd, Tensor? extra) -> (Tensor, Tensor)");
+    lib.def("swiglu_backward(Tensor dout, Tensor gate_up) -> Tensor");
+    lib.def("rope_backward(Tensor dout, Tensor cos, Tensor sin) -> Tensor");
+    lib.def("linear_backward(Tensor dy, Tensor x, Tensor weight) -> (Tensor, Tensor)");
+    lib.impl("norm_backward", torch::dispatch(c10::DispatchKey::CUDA, Norm));
+    lib.impl("swiglu_backward", torch::dispatch(c10::DispatchKey::CUDA, Swiglu));
+    lib.impl("rope_backward", torch::dispatch(c10::DispatchKey::CUDA, Rope));
+    lib.impl("linear_backward", torch::dispatch(c10::DispatchKey::CUDA, Linear));
+    lib.impl("norm_backward", torch::dispatch(c10::DispatchKey::Meta, [](const Tensor&, const Tensor& x, const Tensor& w, const Tensor&, const std::optional<Tensor>&) {
+                 return std::tuple<Tensor, Tensor>(PackedLike(x), PackedLike(w));
+             }));
+    lib.impl("swiglu_backward", torch::dispatch(c10::DispatchKey::Meta, [](const Tensor&, const Tensor& x) { return PackedLike(x); }));
+    lib.impl("rope_backward", torch::dispatch(c10::DispatchKey::Meta, [](const Tensor& dout, const Tensor&, const Tensor&) { return PackedLike(dout); }));
+    lib.impl("linear_backward", torch::dispatch(c10::DispatchKey::Meta, [](const Tensor&, const Tensor& x, const Tensor& w) {
+                 return std::tuple<Tensor, Tensor>(PackedLike(x), PackedLike(w));
+             }));
+}
+template <class F> c10::TypedOperatorHandle<F> Find(const char* name) { return c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<F>(); }
+}  // namespace ops
+using torch::autograd::InputMetadata;
+using torch::dynamo::autograd::IValuePacker;
+using torch::dynamo::autograd::PackedArgs;
+// A node's backward pass as a call in the graph of a compiled one: `apply` gets the gradients and what is read from `saved`, in the place of
+// which stands what the trace has given for it.
+template <class... T> class Traced {
+public:
+    Traced(SwapSavedVariables& trace, T&... saved) : trace_(trace), saved_(saved...) { std::apply([&](auto&... s) { (trace_.before(s), ...); }, saved_); }
+    ~Traced() { std::apply([&](auto&... s) { (trace_.after(s), ...); }, saved_); }
+    Traced(const Traced&) = delete;
+    Traced& operator=(const Traced&) = delete;
+    template <class... A> variable_list Call(const Node& node, const variable_list& grads, variable_list (*apply)(const variable_list&, const std::vector<c10::IValue>&),
+                                             const A&... args) const
+    {
+        const auto& compiler = torch::dynamo::autograd::getPyCompilerInterface();
+        const std::string name = compiler->bind_function(trace_.get_py_compiler(), node.name(), apply, {IValuePacker<A>::packed_type()...}, true, true);
+        PackedArgs packed;
+        (packed.pack(args), ...);
+        return compiler->call_function(trace_.get_py_compiler(), "apply_functional", name, grads, packed.vec(),
+                                       IValuePacker<std::vector<std::optional<InputMetadata>>>::pack(torch::dynamo::autograd::get_input_metadata(node.next_edges())));
+    }
+private:
+    SwapSavedVariables& trace_;
+    std::tuple<T&...> saved_;
+};
 
 struct AddRmsNormNode : Node {
     SavedVariable xOut, weight, rstd;
@@ -435,17 +549,33 @@ struct AddRmsNormNode : Node {
         const Tensor dh = given.defined() ? given.contiguous() : at::zeros_like(x);
         const torch::autograd::AccumulateGrad* first = hasDelta ? EmptyLeaf(next_edge(0)) : nullptr;
         const torch::autograd::AccumulateGrad* second = first ? EmptyLeaf(next_edge(1)) : nullptr;
-        const bool twice = second != nullptr && first != second;
-        const int64_t hidden = x.size(-1);
-        const uint64_t rows = (uint64_t)(x.numel() / hidden);
-        Tensor dx = at::empty_like(x), copy = twice ? at::empty_like(x) : dx, dw = at::empty_like(w);
-        Tensor partial = at::empty({(int64_t)api.rmsNormBwdPartials(rows), hidden}, x.options().dtype(at::kFloat));
-        CheckBackward(api.rmsNormBwd(dh.const_data_ptr(), x.const_data_ptr(), w.const_data_ptr(), r.const_data_ptr(), extra.defined() ? extra.const_data_ptr() : nullptr,
-                                     dx.mutable_data_ptr(), twice ? copy.mutable_data_ptr() : nullptr, partial.mutable_data_ptr(), dw.mutable_data_ptr(), rows,
-                                     (uint32_t)hidden, Stream()),
-                      "HcclFusedRmsNormBwdCopy");
-        launches += 2;
+        auto [dx, dw, copy] = NormGradient(dh, x, w, r, extra, second != nullptr && first != second);
         if (!hasDelta) return {std::move(dx), std::move(dw)};
+        return {std::move(dx), std::move(copy), std::move(dw)};
+    }
+    void compiled_args(CompiledNodeArgs& args) const override
+    {
+        args.collect(hasDelta);
+        args.collect(xOut, hasDelta);
+        args.collect(weight, false);
+        args.collect(rstd, false);
+    }
+    variable_list apply_with_saved(const variable_list& grads, SwapSavedVariables& saved) override
+    {
+        const Traced traced(saved, xOut, weight, rstd);
+        return traced.Call(*this, grads, Compiled, xOut.unpack(hasDelta ? shared_from_this() : nullptr), weight.unpack(), rstd.unpack(), hasDelta);
+    }
+    static variable_list Compiled(const variable_list& grads, const std::vector<c10::IValue>& args)
+    {
+        PackedArgs packed(args);
+        const Tensor x = packed.unpack<Tensor>(), w = packed.unpack<Tensor>(), r = packed.unpack<Tensor>();
+        const bool hasDelta = packed.unpack<bool>();
+        const Tensor& dh = grads[hasDelta ? 1 : 0];
+        const std::optional<Tensor> extra = hasDelta && grads[0].defined() ? std::optional<Tensor>(grads[0]) : std::nullopt;
+        static const auto op = ops::Find<decltype(ops::Norm)>("hccl_b200::norm_backward");
+        auto [dx, dw] = op.call(dh.defined() ? dh : at::zeros_like(x), x, w, r, extra);
+        if (!hasDelta) return {std::move(dx), std::move(dw)};
+        Tensor copy = dx.clone();
         return {std::move(dx), std::move(copy), std::move(dw)};
     }
 };
@@ -503,13 +633,24 @@ struct SwigluNode : Node {
             x = gateUp.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dout = GradientOf(*this, grads[0]).contiguous();
-        const int64_t f = x.size(-1) / 2;
-        Tensor dx = at::empty_like(x);
-        CheckBackward(api.swigluBwd(x.const_data_ptr(), dout.const_data_ptr(), dx.mutable_data_ptr(), (uint64_t)(x.numel() / (2 * f)), (uint32_t)f, Stream()),
-                      "HcclFusedSwigluBwd");
-        launches += 1;
-        return {std::move(dx)};
+        return {SwigluGradient(GradientOf(input_metadata(0), grads[0]).contiguous(), x)};
+    }
+    void compiled_args(CompiledNodeArgs& args) const override
+    {
+        args.collect(gateUp, false);
+        args.collect(input_metadata(0));
+    }
+    variable_list apply_with_saved(const variable_list& grads, SwapSavedVariables& saved) override
+    {
+        const Traced traced(saved, gateUp, mutable_input_metadata(0));
+        return traced.Call(*this, grads, Compiled, gateUp.unpack(), input_metadata(0));
+    }
+    static variable_list Compiled(const variable_list& grads, const std::vector<c10::IValue>& args)
+    {
+        PackedArgs packed(args);
+        const Tensor x = packed.unpack<Tensor>();
+        static const auto op = ops::Find<decltype(ops::Swiglu)>("hccl_b200::swiglu_backward");
+        return {op.call(GradientOf(packed.unpack<InputMetadata>(), grads[0]), x)};
     }
 };
 // (gate_up) -> out
@@ -557,14 +698,25 @@ struct RopeNode : Node {
             s = sin.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dout = GradientOf(*this, grads[0]).contiguous();
-        const int64_t rows = dout.size(0), heads = dout.size(1), d = dout.size(2);
-        Tensor dx = at::empty_like(dout);
-        CheckBackward(api.rope(dout.const_data_ptr(), (uint64_t)(heads * d), dx.mutable_data_ptr(), (uint64_t)(heads * d), c.const_data_ptr(), s.const_data_ptr(),
-                               (uint64_t)rows, (uint32_t)heads, (uint32_t)d, 1, Stream()),
-                      "HcclFusedRope");
-        launches += 1;
-        return {std::move(dx)};
+        return {RopeGradient(GradientOf(input_metadata(0), grads[0]).contiguous(), c, s)};
+    }
+    void compiled_args(CompiledNodeArgs& args) const override
+    {
+        args.collect(cos, false);
+        args.collect(sin, false);
+        args.collect(input_metadata(0));
+    }
+    variable_list apply_with_saved(const variable_list& grads, SwapSavedVariables& saved) override
+    {
+        const Traced traced(saved, cos, sin, mutable_input_metadata(0));
+        return traced.Call(*this, grads, Compiled, cos.unpack(), sin.unpack(), input_metadata(0));
+    }
+    static variable_list Compiled(const variable_list& grads, const std::vector<c10::IValue>& args)
+    {
+        PackedArgs packed(args);
+        const Tensor c = packed.unpack<Tensor>(), s = packed.unpack<Tensor>();
+        static const auto op = ops::Find<decltype(ops::Rope)>("hccl_b200::rope_backward");
+        return {op.call(GradientOf(packed.unpack<InputMetadata>(), grads[0]), c, s)};
     }
 };
 // (x [S, heads, D], cos, sin) -> rotated x
@@ -617,12 +769,27 @@ struct LinearNode : Node {
             w = weight.unpack();
         }
         c10::AutoGradMode off(false);
-        const Tensor dy = GradientOf(*this, grads[0]).contiguous();
-        const uint64_t rows = (uint64_t)dy.size(0), n = (uint64_t)dy.size(1), k = (uint64_t)in.size(1);
-        Tensor dw = at::empty({(int64_t)n, (int64_t)k}, dy.options()), dx = at::empty({(int64_t)rows, (int64_t)k}, dy.options());
-        CheckBackward(api.matmul(dy.const_data_ptr(), in.const_data_ptr(), dw.mutable_data_ptr(), n, k, rows, 1, 0, Stream()), "HcclMc2Matmul");
-        CheckBackward(api.matmul(dy.const_data_ptr(), w.const_data_ptr(), dx.mutable_data_ptr(), rows, k, n, 0, 0, Stream()), "HcclMc2Matmul");
+        auto [dx, dw] = LinearGradient(GradientOf(input_metadata(0), grads[0]).contiguous(), in, w);
         __atomic_fetch_add(counter.mutable_data_ptr<int64_t>(), 2, __ATOMIC_RELAXED);
+        return {std::move(dx), std::move(dw)};
+    }
+    void compiled_args(CompiledNodeArgs& args) const override
+    {
+        args.collect(x, false);
+        args.collect(weight, false);
+        args.collect(input_metadata(0));
+    }
+    variable_list apply_with_saved(const variable_list& grads, SwapSavedVariables& saved) override
+    {
+        const Traced traced(saved, x, weight, mutable_input_metadata(0));
+        return traced.Call(*this, grads, Compiled, x.unpack(), weight.unpack(), input_metadata(0));
+    }
+    static variable_list Compiled(const variable_list& grads, const std::vector<c10::IValue>& args)
+    {
+        PackedArgs packed(args);
+        const Tensor in = packed.unpack<Tensor>(), w = packed.unpack<Tensor>();
+        static const auto op = ops::Find<decltype(ops::Linear)>("hccl_b200::linear_backward");
+        auto [dx, dw] = op.call(GradientOf(packed.unpack<InputMetadata>(), grads[0]), in, w);
         return {std::move(dx), std::move(dw)};
     }
 };
@@ -685,6 +852,23 @@ struct EmbeddingNode : Node {
         launches += 2;
         return {std::move(dTable)};
     }
+    void compiled_args(CompiledNodeArgs& args) const override
+    {
+        args.collect(ids, false);
+        args.collect(vocab);
+    }
+    variable_list apply_with_saved(const variable_list& grads, SwapSavedVariables& saved) override
+    {
+        const Traced traced(saved, ids);
+        return traced.Call(*this, grads, Compiled, ids.unpack(), vocab);
+    }
+    static variable_list Compiled(const variable_list& grads, const std::vector<c10::IValue>& args)
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        PackedArgs packed(args);
+        const Tensor i = packed.unpack<Tensor>();
+        return {at::embedding_dense_backward(grads[0], i, packed.unpack<int64_t>(), -1, false)};
+    }
 };
 // (ids [tokens], table [vocab, hidden]) -> the rows
 PyObject* Embedding(PyObject*, PyObject* const* a, Py_ssize_t nargs)
@@ -731,6 +915,7 @@ PyObject* BindSlots(const Slot* slots, size_t n, PyObject* addresses)
 }
 PyObject* Bind(PyObject*, PyObject* addresses)
 {
+    if (Guarded([]() -> PyObject* { ops::Define(); return Py_None; }) == nullptr) return nullptr;
     if (defaultDeviceMode == nullptr) {
         PyObject* devices = PyImport_ImportModule("torch.utils._device");
         PyObject* mode = devices ? PyObject_GetAttrString(devices, "DeviceContext") : nullptr;

@@ -19,7 +19,7 @@ def _rnd(*shape, seed=0):
 @pytest.fixture(params=["native", "python"])
 def way(request, monkeypatch):
     if request.param == "python":
-        for name in NAMES:
+        for name in NAMES + ("embedding",):
             monkeypatch.setattr(_calls, name, _calls._nothing)
     else:
         assert _calls._module is not None
@@ -123,6 +123,28 @@ def test_what_autograd_checks_is_checked(way):
     assert len(seen) == 1 and seen[0] is h or torch.equal(seen[0], h)
     y.sum().backward()
     assert len(seen) == 2
+
+
+def test_compiled_backward_passes(way):
+    """Compiled autograd takes the nodes into its graph, which then launches what the nodes launch."""
+    from torch._dynamo import compiled_autograd
+    want, launched = None, []
+    for compiled in (False, True, True):                                         # the second time the graph is used again
+        before = fused.LAUNCHES
+        leaves, outs, ctx = _layer()                                             # no tensor has more than two uses: sums have one order
+        table = _rnd(64, 256, seed=5).requires_grad_()
+        loss = sum(o.float().square().sum() for o in outs) + fused.embedding(torch.arange(39, -1, -1, device="cuda"), table).float().square().sum()
+        if compiled:
+            with compiled_autograd._enable(torch.compile(backend="eager")):
+                loss.backward()
+        else:
+            loss.backward()
+        launched.append(fused.LAUNCHES - before + ctx.launches)
+        got = [t.grad for t in leaves + [table]]
+        want = want or got
+        assert all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
+        assert len({t.data_ptr() for t in got}) == len(got)                      # every leaf has a gradient of its own
+    assert launched[1:] == [launched[0] - (2 if way == "native" else 0)] * 2    # the embedding's gradient is PyTorch's there
 
 
 def test_a_refused_backward_call_raises_what_a_refused_call_raises(way):

@@ -30,9 +30,13 @@ HcclResult HcclFusedSwigluBwd(const void* gu, const void* dout, void* dgu, uint6
 HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t outStride, const void* cosTable, const void* sinTable, uint64_t rows,
                          uint32_t nHeads, uint32_t headDim, int backward, hcclStream_t stream);
 
-// Gradient of an embedding table, every row of it: dTable[r] = sum of dy[t] over the tokens t with ids[t] == r, in token order in fp32,
-// zero where there is none.  ids: int64 [tokens], at most 8192 (others are HCCL_E_NOT_SUPPORT; ids outside the table are left out); dy
-// [tokens, hidden], dTable [vocab, hidden]: bf16, hidden a multiple of 8; marks: scratch of vocab bytes, 16-byte aligned.
+// Gradient of an embedding table, every row of it: dTable[r] = sum of dy[t] over the tokens t with ids[t] == r, zero where there is none.
+// Sums are in fp32, in token order up to 128 tokens of a row, beyond in an order that depends on their number only.  ids: int64
+// [tokens], at most 8192 (others are HCCL_E_NOT_SUPPORT; ids outside the table are left out); dy [tokens, hidden], dTable [vocab, hidden]:
+// bf16, hidden a multiple of 8; scratch: 8 bytes per token, 16-byte aligned.
+HcclResult HcclFusedEmbeddingGrad(const int64_t* ids, const void* dy, void* dTable, void* scratch, uint64_t tokens, uint64_t vocab, uint32_t hidden,
+                                  hcclStream_t stream);
+// The same with scratch of its own, allocated and freed in stream order; `marks` (vocab bytes, 16-byte aligned) is not used any more.
 HcclResult HcclFusedEmbeddingBwd(const int64_t* ids, const void* dy, void* dTable, void* marks, uint64_t tokens, uint64_t vocab, uint32_t hidden,
                                  hcclStream_t stream);
 

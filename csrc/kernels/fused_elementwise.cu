@@ -506,79 +506,192 @@ __global__ void __launch_bounds__(kRopeThreads) RopeKernel(const __nv_bfloat16* 
 }
 
 // Gradient of an embedding table.  Bound by the rows it writes, nearly all of them zero: 67 MB for 4096 rows of 8192 beside 17 MB
-// of 1024 tokens' gradients.  One kernel writes every row once in place of a fill and a second pass over the rows in use;
-// which rows are in use is marked before, so that the others need not look for their tokens.  A block takes up to 256
-// vectors of a row; if its row is in use it goes through the ids, 256 at a time, keeps the places of its tokens in order and adds their
-// gradients, eight loads at a time (a token that is every tenth of the text has hundreds).  Eager, with what autograd adds (us, before on
-// PyTorch's kernels -> now): 4096 x 8192, 1024 tokens 73 -> 50; 32000 x 4096, 4096 tokens 488 -> 153, one of them every tenth 469 -> 148;
-// 128256 x 8192, 8192 tokens 1791 -> 1047 (2.1 GB written).
+// of 1024 tokens' gradients, 2.1 GB for 128256.  Two kernels.  The first fills the table with zeros, and some of its blocks meanwhile sort
+// the tokens by their ids: a token's place is the number of tokens with a smaller id and of earlier ones with its own, counted against
+// all ids in shared memory.  The second writes the rows in use.  Few tokens of one id (nearly all rows): a thread owns a vector of the
+// row and adds its tokens in order; a block takes up to 256 vectors of four rows, or more rows if they are short.  More than kEmbLong
+// (padding, a separator): a block takes 16 vectors, 16 groups of threads each every 16th token, so that a row is shared by up to 64 SMs.
+// Measured against marks of the rows in use and one block per 2048 columns of every row, which went through all ids and added a row's
+// tokens alone (tokens, table, us back to back in a graph): 1024, 4096 x 8192 35.3 -> 17.9 (102 MB); 8192, 4096 x 8192 231 -> 93; 8192,
+// 128256 x 8192 1042 -> 346 (2.3 GB, 6.6 TB/s); 1024, 128256 x 8192 853 -> 290; 4096, 32000 x 4096 147 -> 54; 8192, 1048576 x 64 1491 -> 38;
+// all 8192 tokens of one id 958 -> 110 at 4096 x 8192 and 775 -> 90 at 50000 x 768; 8192, 32 x 8192 (256 tokens of every id) 58.8 -> 62.8.
+// With autograd around it a call takes 0.13 .. 1.01 of PyTorch's time at 190 sizes and mixes of ids (1 .. 8192 tokens, 32 .. 16777216 rows);
+// with the kernels before it took up to three times as long for large tables of few tokens and for frequent ids.
 constexpr int kEmbThreads = 256;
-constexpr uint64_t kEmbMaxTokens = 8192;          // beyond, rows in use would read more ids than gradients
-__global__ void __launch_bounds__(1024) EmbeddingMarkKernel(const long long* __restrict__ ids, uint32_t tokens, uint8_t* __restrict__ marks, uint32_t vocab)
+constexpr uint64_t kEmbMaxTokens = 8192;          // sorted by counting: the work grows with the square of the tokens
+constexpr int kEmbRanked = 32;                    // tokens that a block finds the places of
+constexpr int kEmbFillVecs = 8;                   // 16-byte vectors that a thread fills, 32 KiB per block
+constexpr int kEmbLong = 128;
+constexpr int kEmbPlaces = 4;                     // places that a thread takes in turn where tokens are not frequent
+constexpr int kEmbSlice = 16;                     // vectors of a row that a block takes where a token is frequent
+
+// A place in the order of ids: its token and the id, 0x7FFFFFFF where that is no row of the table.  The blocks that find the places read
+// the ids each for itself: ids that another stream is still writing, which a program has no right to, may leave places unwritten, so the
+// second kernel takes every number of a place within its bounds.
+struct alignas(8) EmbPlace { int token, id; };
+
+__device__ __forceinline__ void EmbeddingRank(const long long* __restrict__ ids, int tokens, int vocab, int base, EmbPlace* __restrict__ places)
 {
-    DependencyWait();
-    AllowDependents();
-    for (uint32_t i = threadIdx.x; i < (vocab + 15) / 16; i += blockDim.x) {
-        if (i * 16 + 16 <= vocab) reinterpret_cast<uint4*>(marks)[i] = make_uint4(0, 0, 0, 0);
-        else for (uint32_t k = i * 16; k < vocab; ++k) marks[k] = 0;
+    constexpr int kWarps = kEmbThreads / 32;
+    __shared__ __align__(16) int s_id[kEmbMaxTokens];
+    __shared__ int s_before[kWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, padded = (tokens + 3) & ~3;
+    constexpr int U = 8;                              // ids that a thread requests at a time
+    for (int t0 = threadIdx.x; t0 < padded; t0 += U * kEmbThreads) {
+        long long id[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) id[u] = t0 + u * kEmbThreads < tokens ? ids[t0 + u * kEmbThreads] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (t0 + u * kEmbThreads < padded) s_id[t0 + u * kEmbThreads] = id[u] >= 0 && id[u] < (long long)vocab ? (int)id[u] : 0x7FFFFFFF;
     }
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < tokens; t += blockDim.x) {
-        const long long id = ids[t];
-        if (id >= 0 && id < (long long)vocab) marks[id] = 1;
+    // lane: a token of this block; warp: an eighth of the ids it is compared with, four at a time (base is a multiple of four).  Ids of
+    // tokens in front of the block count if they are no larger, the others if they are smaller.
+    const int t = base + lane, mine = t < tokens ? s_id[t] : -1;
+    const int quads = padded / 4, q0 = quads * warp / kWarps, q1 = quads * (warp + 1) / kWarps, qBase = min(max(base / 4, q0), q1);
+    const int4* quad = reinterpret_cast<const int4*>(s_id);
+    int before = 0;
+#pragma unroll 4
+    for (int q = q0; q < qBase; ++q) {
+        const int4 o = quad[q];
+        before += (o.x <= mine) + (o.y <= mine) + (o.z <= mine) + (o.w <= mine);
     }
+#pragma unroll 4
+    for (int q = qBase; q < q1; ++q) {
+        const int4 o = quad[q];
+        before += (o.x < mine) + (o.y < mine) + (o.z < mine) + (o.w < mine);
+    }
+    s_before[warp][lane] = before;
+    __syncthreads();
+    if (warp != 0) return;
+    before = __popc(__match_any_sync(0xFFFFFFFFu, mine) & ((1u << lane) - 1u));       // and those of the block itself with the same id
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) before += s_before[w][lane];
+    if (t < tokens) places[before] = {t, mine};
 }
-__global__ void __launch_bounds__(kEmbThreads) EmbeddingBwdKernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
-                                                                  __nv_bfloat16* __restrict__ dTable, const uint8_t* __restrict__ marks, uint32_t tokens,
-                                                                  int hidden, int chunks)
+__global__ void __launch_bounds__(kEmbThreads) EmbeddingSortKernel(const long long* __restrict__ ids, uint4* __restrict__ dTable, uint64_t vecs,
+                                                                   EmbPlace* __restrict__ places, int tokens, int vocab, int ranking)
 {
     DependencyWait();
     AllowDependents();
-    __shared__ uint32_t s_hits[kEmbThreads / 32];
-    __shared__ uint16_t s_list[kEmbThreads];
-    const uint32_t row = blockIdx.x / (uint32_t)chunks;
-    const int v = (int)(blockIdx.x - row * (uint32_t)chunks) * kEmbThreads + (int)threadIdx.x, nVec = hidden / 8;
-    const bool mine = v < nVec;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (marks[row] != 0) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        long long id = threadIdx.x < tokens ? ids[threadIdx.x] : -1;
-        for (uint32_t base = 0; base < tokens; base += kEmbThreads) {
-            const bool hit = id == (long long)row;
-            const uint32_t following = base + kEmbThreads + threadIdx.x;
-            id = following < tokens ? ids[following] : -1;
-            if (__syncthreads_count(hit) == 0) continue;
-            const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
-            if (lane == 0) s_hits[warp] = hits;
-            __syncthreads();
-            int before = 0, n = 0;
-#pragma unroll
-            for (int w = 0; w < kEmbThreads / 32; ++w) {
-                if (w < warp) before += __popc(s_hits[w]);
-                n += __popc(s_hits[w]);
-            }
-            if (hit) s_list[before + __popc(hits & ((1u << lane) - 1u))] = (uint16_t)threadIdx.x;
-            __syncthreads();
-            const __nv_bfloat16* from = dy + (size_t)base * hidden;
-            constexpr int U = 8;
-            for (int i = 0; mine && i < n; i += U) {
-                uint4 raw[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (i + u < n) raw[u] = reinterpret_cast<const uint4*>(from + (size_t)s_list[i + u] * hidden)[v];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (i + u >= n) break;
-                    float f[8];
-                    Unpack8(raw[u], f);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[k] += f[k];
-                }
-            }
-            __syncthreads();                          // the list is read, the next 256 ids may take its place
-        }
+    if ((int)blockIdx.x < ranking) {
+        EmbeddingRank(ids, tokens, vocab, (int)blockIdx.x * kEmbRanked, places);
+        return;
     }
-    if (mine) reinterpret_cast<uint4*>(dTable + (size_t)row * hidden)[v] = Pack8(acc);
+    const uint64_t first = (uint64_t)((int)blockIdx.x - ranking) * (kEmbThreads * kEmbFillVecs) + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < kEmbFillVecs; ++u) {
+        const uint64_t v = first + (uint64_t)u * kEmbThreads;
+        if (v < vecs) dTable[v] = make_uint4(0, 0, 0, 0);
+    }
+}
+__device__ __forceinline__ void AddVector(float (&acc)[8], const uint4& raw)
+{
+    float f[8];
+    Unpack8(raw, f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[k] += f[k];
+}
+// acc += vector `v` of every `STEP`-th of the places [at, end).  The tokens of the next eight are requested behind the vectors of these: one
+// after the other, in the branches that the ends of a row make of it, eight took 3 us.
+template <int STEP>
+__device__ __forceinline__ void EmbeddingAdd(float (&acc)[8], const EmbPlace* __restrict__ places, int at, int end, int tokens, const __nv_bfloat16* __restrict__ dy,
+                                             int hidden, int v)
+{
+    constexpr int U = 8;
+    int token[U];
+    auto request = [&] {
+#pragma unroll
+        for (int u = 0; u < U; ++u) token[u] = (int)min((unsigned)places[min(at + u * STEP, end - 1)].token, (unsigned)tokens - 1);
+    };
+    if (at < end) request();
+    while (at < end) {
+        uint4 raw[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            raw[u] = make_uint4(0, 0, 0, 0);
+            if (at + u * STEP < end) raw[u] = reinterpret_cast<const uint4*>(dy + (size_t)token[u] * hidden)[v];
+        }
+        at += U * STEP;
+        if (at < end) request();
+#pragma unroll
+        for (int u = 0; u < U; ++u) AddVector(acc, raw[u]);
+    }
+}
+// `slots` x `slices` blocks for frequent tokens in front, a slot for every kEmbLong-th place; the others take kEmbPlaces places per `lanes`
+// threads, a row of more than kEmbThreads vectors in `chunks` blocks.
+__global__ void __launch_bounds__(kEmbThreads, 4) EmbeddingRowsKernel(const EmbPlace* __restrict__ places, const __nv_bfloat16* __restrict__ dy,
+                                                                   __nv_bfloat16* __restrict__ dTable, int tokens, int vocab, int hidden, int slots, int slices,
+                                                                   int chunks, int lanes)
+{
+    DependencyWait();
+    AllowDependents();
+    const int nVec = hidden / 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    int block = (int)blockIdx.x;
+    if (block < slots * slices) {
+        constexpr int kGroups = kEmbThreads / kEmbSlice;
+        __shared__ float s_sum[kGroups][kEmbSlice][8];
+        // more than kEmbLong places hold a multiple of it: the first one's blocks take the row, from its first place to its end
+        const int at = block / slices * kEmbLong, tid = (int)threadIdx.x, id = places[at].id;
+        if ((unsigned)id >= (unsigned)vocab) return;
+        const int back = __syncthreads_count(tid < kEmbLong && at - 1 - tid >= 0 && places[at - 1 - tid].id == id);
+        if (back == kEmbLong) return;
+        const int far = at + 32 * __syncthreads_count(at + 32 * (tid + 1) < tokens && places[at + 32 * (tid + 1)].id == id);
+        const int first = at - back, end = far + __syncthreads_count(tid < 32 && far + tid < tokens && places[far + tid].id == id);
+        if (end - first <= kEmbLong) return;
+        const int lane = threadIdx.x % kEmbSlice, group = threadIdx.x / kEmbSlice, v = block % slices * kEmbSlice + lane;
+        if (v < nVec) EmbeddingAdd<kGroups>(acc, places, first + group, end, tokens, dy, hidden, v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s_sum[group][lane][k] = acc[k];
+        __syncthreads();
+        if (group != 0 || v >= nVec) return;
+        for (int g = 1; g < kGroups; ++g) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] += s_sum[g][lane][k];
+        }
+        reinterpret_cast<uint4*>(dTable + (size_t)id * hidden)[v] = Pack8(acc);
+        return;
+    }
+    block -= slots * slices;
+    const int place = (block / chunks * (kEmbThreads / lanes) + (int)threadIdx.x / lanes) * kEmbPlaces, v = block % chunks * kEmbThreads + (int)threadIdx.x % lanes;
+    if (place >= tokens || v >= nVec) return;
+    auto at = [&](int i) { return places[min(i, tokens - 1)]; };
+    auto vector = [&](int token) { return reinterpret_cast<const uint4*>(dy + (size_t)min((unsigned)token, (unsigned)tokens - 1) * hidden)[v]; };
+    EmbPlace p[kEmbPlaces + 1];
+    bool mine[kEmbPlaces];                            // a row begins here that is not left to the blocks above
+    uint4 raw[kEmbPlaces];
+#pragma unroll
+    for (int j = 0; j <= kEmbPlaces; ++j) p[j] = at(place + j);
+    int previous = place > 0 ? places[place - 1].id : -1;
+#pragma unroll
+    for (int j = 0; j < kEmbPlaces; ++j) {
+        mine[j] = place + j < tokens && p[j].id != previous && (unsigned)p[j].id < (unsigned)vocab && !(place + j + kEmbLong < tokens && at(place + j + kEmbLong).id == p[j].id);
+        previous = p[j].id;
+        if (mine[j]) raw[j] = vector(p[j].token);
+    }
+#pragma unroll
+    for (int j = 0; j < kEmbPlaces; ++j) {
+        if (!mine[j]) continue;
+        Unpack8(raw[j], acc);
+        bool more = place + j + 1 < tokens && p[j + 1].id == p[j].id;
+        for (int i = place + j + 1; more; i += 4) {
+            EmbPlace q[4];
+            uint4 next[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) q[u] = at(i + u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                more = i + u < tokens && q[u].id == p[j].id;
+                next[u] = make_uint4(0, 0, 0, 0);
+                if (more) next[u] = vector(q[u].token);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) AddVector(acc, next[u]);
+        }
+        reinterpret_cast<uint4*>(dTable + (size_t)p[j].id * hidden)[v] = Pack8(acc);
+    }
 }
 
 // Lets a norm kernel take the largest ring the norm kernels use.
@@ -723,18 +836,44 @@ HcclResult HcclFusedRope(const void* in, uint64_t inStride, void* out, uint64_t 
                     "Rope");
 }
 
+HcclResult HcclFusedEmbeddingGrad(const int64_t* ids, const void* dy, void* dTable, void* scratch, uint64_t tokens, uint64_t vocab, uint32_t hidden,
+                                  hcclStream_t stream)
+{
+    CHK_PTR_NULL(ids); CHK_PTR_NULL(dy); CHK_PTR_NULL(dTable); CHK_PTR_NULL(scratch);
+    if (hidden == 0 || hidden % 8 != 0 || !Aligned16(dy) || !Aligned16(dTable) || !Aligned16(scratch) || (reinterpret_cast<uintptr_t>(ids) & 7u) != 0) return HCCL_E_PARA;
+    const uint64_t nVec = hidden / 8, chunks = (nVec + kEmbThreads - 1) / kEmbThreads;
+    if (tokens > kEmbMaxTokens || hidden > 0x7FFFFFFFu || vocab > 0x7FFFFFFFull / chunks) return HCCL_E_NOT_SUPPORT;
+    if (vocab == 0) return HCCL_SUCCESS;
+    const uint64_t vecs = vocab * nVec, perBlock = (uint64_t)kEmbThreads * kEmbFillVecs, filling = (vecs + perBlock - 1) / perBlock;
+    const uint64_t ranking = (tokens + kEmbRanked - 1) / kEmbRanked;
+    const uint64_t slots = tokens > kEmbLong ? (tokens + kEmbLong - 1) / kEmbLong : 0, slices = (nVec + kEmbSlice - 1) / kEmbSlice;
+    int lanes = 1;
+    while (lanes < kEmbThreads && (uint64_t)lanes < nVec) lanes *= 2;
+    const uint64_t perRowBlock = (uint64_t)(kEmbThreads / lanes) * kEmbPlaces, rows = (tokens + perRowBlock - 1) / perRowBlock * chunks;
+    if (ranking + filling > 0x7FFFFFFFull || slots * slices + rows > 0x7FFFFFFFull) return HCCL_E_NOT_SUPPORT;
+    CHK_RET(Launched(LaunchDependent(EmbeddingSortKernel, (unsigned)(ranking + filling), kEmbThreads, 0, (cudaStream_t)stream, 0, reinterpret_cast<const long long*>(ids),
+                                     (uint4*)dTable, vecs, (EmbPlace*)scratch, (int)tokens, (int)vocab, (int)ranking), "EmbeddingSort"));
+    if (tokens == 0) return HCCL_SUCCESS;
+    return Launched(LaunchDependent(EmbeddingRowsKernel, (unsigned)(slots * slices + rows), kEmbThreads, 0, (cudaStream_t)stream, 0, (const EmbPlace*)scratch,
+                                    (const __nv_bfloat16*)dy, (__nv_bfloat16*)dTable, (int)tokens, (int)vocab, (int)hidden, (int)slots, (int)slices, (int)chunks, lanes),
+                    "EmbeddingRows");
+}
+
 HcclResult HcclFusedEmbeddingBwd(const int64_t* ids, const void* dy, void* dTable, void* marks, uint64_t tokens, uint64_t vocab, uint32_t hidden,
                                  hcclStream_t stream)
 {
-    CHK_PTR_NULL(ids); CHK_PTR_NULL(dy); CHK_PTR_NULL(dTable); CHK_PTR_NULL(marks);
-    if (hidden == 0 || hidden % 8 != 0 || !Aligned16(dy) || !Aligned16(dTable) || !Aligned16(marks) || (reinterpret_cast<uintptr_t>(ids) & 7u) != 0) return HCCL_E_PARA;
-    const uint64_t chunks = (hidden / 8 + kEmbThreads - 1) / kEmbThreads;
-    if (tokens > kEmbMaxTokens || vocab * chunks > 0x7FFFFFFFull || hidden > 0x7FFFFFFFu) return HCCL_E_NOT_SUPPORT;
-    if (vocab == 0) return HCCL_SUCCESS;
-    CHK_RET(Launched(LaunchDependent(EmbeddingMarkKernel, 1, 1024, 0, (cudaStream_t)stream, 0, reinterpret_cast<const long long*>(ids), (uint32_t)tokens,
-                                     (uint8_t*)marks, (uint32_t)vocab), "EmbeddingMark"));
-    return Launched(LaunchDependent(EmbeddingBwdKernel, (unsigned)(vocab * chunks), kEmbThreads, 0, (cudaStream_t)stream, 0, reinterpret_cast<const long long*>(ids),
-                                    (const __nv_bfloat16*)dy, (__nv_bfloat16*)dTable, (const uint8_t*)marks, (uint32_t)tokens, (int)hidden, (int)chunks), "EmbeddingBwd");
+    CHK_PTR_NULL(marks);
+    if (!Aligned16(marks)) return HCCL_E_PARA;
+    if (tokens > kEmbMaxTokens) return HCCL_E_NOT_SUPPORT;
+    void* scratch = nullptr;
+    if (const cudaError_t e = cudaMallocAsync(&scratch, std::max<uint64_t>(tokens, 1) * sizeof(EmbPlace), (cudaStream_t)stream); e != cudaSuccess) {
+        cudaGetLastError();
+        HCCL_ERROR("no scratch for the embedding's gradient: %s", cudaGetErrorString(e));
+        return HCCL_E_RUNTIME;
+    }
+    const HcclResult r = HcclFusedEmbeddingGrad(ids, dy, dTable, scratch, tokens, vocab, hidden, stream);
+    CHK_CUDA(cudaFreeAsync(scratch, (cudaStream_t)stream));
+    return r;
 }
 
 }  // extern "C"

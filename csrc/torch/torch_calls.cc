@@ -50,7 +50,7 @@ struct Api {
     decltype(&HcclFusedSwigluBwd) swigluBwd;
     decltype(&HcclFusedRope) rope;
     decltype(&HcclMc2Matmul) matmul;
-    decltype(&HcclFusedEmbeddingBwd) embeddingBwd;
+    decltype(&HcclFusedEmbeddingGrad) embeddingGrad;
     decltype(&HcclMoeExpertOffsets) expertOffsets;
     decltype(&HcclAllReduce) allReduce;
     decltype(&HcclReduceScatter) reduceScatter;
@@ -69,7 +69,7 @@ const Slot kSlots[] = {
 };
 
 // Functions that only the backward passes of recorded calls use.
-const Slot kBackwardSlots[] = {{"HcclFusedEmbeddingBwd", (void**)&api.embeddingBwd}};
+const Slot kBackwardSlots[] = {{"HcclFusedEmbeddingGrad", (void**)&api.embeddingGrad}};
 
 // The function mode behind torch.set_default_device and `with torch.device(...)`.  It gives a device to factory calls that name
 // none; these calls name theirs, so that it has nothing to see here.
@@ -845,10 +845,10 @@ struct EmbeddingNode : Node {
         c10::AutoGradMode off(false);
         Tensor dy = grads[0].contiguous();
         if ((uintptr_t)dy.const_data_ptr() % 16 != 0) dy = dy.clone();      // a packed view that does not begin on 16 bytes
-        Tensor dTable = at::empty({vocab, dy.size(1)}, dy.options()), marks = at::empty({vocab}, dy.options().dtype(at::kByte));
-        CheckBackward(api.embeddingBwd(i.const_data_ptr<int64_t>(), dy.const_data_ptr(), dTable.mutable_data_ptr(), marks.mutable_data_ptr(), (uint64_t)dy.size(0),
-                                       (uint64_t)vocab, (uint32_t)dy.size(1), Stream()),
-                      "HcclFusedEmbeddingBwd");
+        Tensor dTable = at::empty({vocab, dy.size(1)}, dy.options()), scratch = at::empty({8 * dy.size(0)}, dy.options().dtype(at::kByte));
+        CheckBackward(api.embeddingGrad(i.const_data_ptr<int64_t>(), dy.const_data_ptr(), dTable.mutable_data_ptr(), scratch.mutable_data_ptr(), (uint64_t)dy.size(0),
+                                        (uint64_t)vocab, (uint32_t)dy.size(1), Stream()),
+                      "HcclFusedEmbeddingGrad");
         launches += 2;
         return {std::move(dTable)};
     }
@@ -876,7 +876,7 @@ PyObject* Embedding(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     HCCL_ARGS(2)
     return Guarded([&]() -> PyObject* {
         const Tensor *ids = GetPlain(a[0]), *table = GetRecordable(a[1]);
-        if (api.embeddingBwd == nullptr || !ids || !table || !Records({table}) || !PlainCall() || ids->scalar_type() != at::kLong || ids->dim() != 1 || !ids->is_contiguous()) return None();
+        if (api.embeddingGrad == nullptr || !ids || !table || !Records({table}) || !PlainCall() || ids->scalar_type() != at::kLong || ids->dim() != 1 || !ids->is_contiguous()) return None();
         if (table->dim() != 2 || table->numel() == 0 || ids->numel() == 0 || ids->numel() > 8192 || table->size(1) % 8 != 0 || table->size(0) > (1 << 24)) return None();
         Tensor out;
         {

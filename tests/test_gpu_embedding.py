@@ -42,6 +42,41 @@ def test_against_64_bits(tokens, vocab, hidden, skew):
     assert torch.equal(again, t.grad)
 
 
+# ids that are more frequent than one thread adds up alone (128), at the edges of that, of rows, of the vectors and places a block takes
+@pytest.mark.parametrize("tokens,vocab,hidden,often", [(129, 1, 8, 129), (300, 40, 120, 128), (300, 40, 128, 129), (515, 9, 136, 257), (1000, 4, 2056, 640),
+                                                       (8192, 300, 1032, 8192), (8192, 5000, 8, 4000)])
+def test_frequent_ids(tokens, vocab, hidden, often):
+    ids, _, dy = _case(tokens, vocab, hidden)
+    if vocab > 1:
+        ids %= vocab - 1
+        ids[torch.randperm(tokens, device="cuda")[:often]] = vocab - 1
+    t = torch.zeros(vocab, hidden, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    got = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+    want = _want(ids, dy, vocab)
+    bound = want.abs() * 2 ** -8 + torch.zeros_like(want).index_add_(0, ids, dy.double().abs()) * tokens * 2 ** -24 + 1e-30
+    assert ((got.double() - want).abs() <= bound).all()
+    assert torch.equal(got, torch.autograd.grad(fused.embedding(ids, t), t, dy)[0])
+
+
+@pytest.mark.parametrize("scratch", [True, False])
+def test_the_c_functions(scratch):
+    """With scratch and without; ids outside the table, and no tokens at all."""
+    ids, _, dy = _case(200, 50, 72)
+    ids[::3] = 50
+    ids[1::5] = -1
+    out, s = torch.full((50, 72), 7.0, device="cuda", dtype=torch.bfloat16), torch.cuda.current_stream().cuda_stream
+    call = lib.HcclFusedEmbeddingGrad if scratch else lib.HcclFusedEmbeddingBwd
+    call.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_uint64] * 2 + [ctypes.c_uint32, ctypes.c_void_p]
+    extra = torch.empty(8 * 200 if scratch else 50, device="cuda", dtype=torch.uint8)
+    assert call(ids.data_ptr(), dy.data_ptr(), out.data_ptr(), extra.data_ptr(), 200, 50, 72, s) == 0
+    keep = (ids >= 0) & (ids < 50)
+    want = _want(ids[keep], dy[keep], 50)
+    assert ((out.double() - want).norm() / want.norm()).item() < 4e-3
+    assert call(ids.data_ptr(), dy.data_ptr(), out.data_ptr(), extra.data_ptr(), 0, 50, 72, s) == 0 and not out.any()
+    assert call(ids.data_ptr(), dy.data_ptr(), out.data_ptr(), extra.data_ptr(), 8193, 50, 72, s) == Result.E_NOT_SUPPORT
+    assert call(ids.data_ptr(), dy.data_ptr(), out.data_ptr(), extra.data_ptr(), 8, 1 << 63, 4096, s) == Result.E_NOT_SUPPORT
+
+
 def test_what_is_left_to_pytorch():
     ids, table, _ = _case(40, 64, 64)
     assert _calls.embedding(ids, table) is None                                            # nothing is recorded

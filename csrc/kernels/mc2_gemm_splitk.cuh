@@ -252,7 +252,10 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
     const int perQuarter = g.wr / 4, myRow = quarter * perQuarter + lane;
     const bool hasRow = lane < perQuarter;
     if (split == 1) {
-        // straight to memory: a pair of lanes swaps halves, so that each stores two columns of every second token
+        // straight to memory: a pair of lanes swaps halves, so that each stores two columns of every second token.  All of the tile or nothing:
+        // of two warps that wait for the same accumulator, one may have given up just before it was complete.
+        __syncthreads();
+        drained = drained && *gaveUp == 0;
         const int col = hasRow ? col0 + (myRow & ~1) : g.N;
         for (int c = part * 16; drained && c < tokens; c += chunkStep) {
             uint32_t v[16];
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
             }
         }
         TcFenceBefore();
-        __syncthreads();
+        __syncthreads();                                 // the accumulator is read
     } else {
         // every CTA leaves its partial tile in its own idle ring, [token][column], before the cluster meets
         float* mine = reinterpret_cast<float*>(smem) + myRow;

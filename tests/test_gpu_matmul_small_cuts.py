@@ -50,3 +50,33 @@ def test_a_row_that_does_not_depend_on_the_buffer_next_to_it():
     want = (a.double() @ b.double().t()).float()
     assert ((whole[:m * n].view(m, n).float() - want).norm() / want.norm()).item() < 3e-3
     assert (whole[m * n:] == 7).all()
+
+
+def test_a_lone_tile_is_stored_whole_or_not_at_all():
+    """Waits that run out anywhere in the middle of the work, in warps of one tile that look at different times."""
+    import ctypes
+    from hccl_b200._lib import lib
+    from hccl_b200.comm import HcclError
+    from hccl_b200.ops import mc2
+    m, n, k = 128, 8192, 1024
+    p = plan(m, n, k)
+    assert (p["route"], p["split"], p["bt"], p["bn"]) == ("split", "1", "64", "128")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, b = torch.randn(m, k, device="cuda", generator=g).bfloat16(), torch.randn(n, k, device="cuda", generator=g).bfloat16()
+    want = mc2.matmul(a, b)
+    f = lib.HcclDebugMatmulStalled
+    f.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_uint64] * 3 + [ctypes.c_int] * 3 + [ctypes.c_uint64, ctypes.c_void_p]
+    stored = 0
+    for limit in [0, 200, 500, 1000] + list(range(1500, 4500, 100)) + [6000, 1_000_000]:
+        out = torch.full((m, n), 7.0, device="cuda", dtype=torch.bfloat16)
+        assert f(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, 0, 1, -1, limit, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        tiles, wanted = (t.view(2, 64, 64, 128).transpose(1, 2).reshape(128, -1) for t in (out, want))
+        whole, untouched = (tiles == wanted).all(1), (tiles == 7.0).all(1)
+        assert (whole | untouched).all(), limit
+        stored += int(whole.sum())
+        try:                                                                     # a launch that gave up is reported to the next call
+            mc2.matmul(a, b)
+        except HcclError:
+            pass
+    assert stored >= 128 and torch.equal(mc2.matmul(a, b), want)

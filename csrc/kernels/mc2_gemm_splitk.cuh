@@ -20,8 +20,8 @@
 // Measured against the one-SM kernel on 128 x 128 tiles (us, bf16, weight [N, K]): 16 x 8192 x 8192 47.5 -> 26.8 (5.0
 // TB/s), 64 x 8192 x 8192 48.4 -> 28.8; against its 256-wide form 16 x 57344 x 8192 160.6 -> 142.4 (6.6 TB/s), 64 x 57344 x 8192
 // 162.3 -> 151.0.  Clusters of at most four, 128 x 128 tiles and 108 KiB rings -> chosen per shape (back to back in a graph): 128 x 2048 x
-// 8192 18.2 -> 11.7 (3.3 TB/s), 128 x 1024 x 8192 13.8 -> 9.4, 16 x 1024 x 8192 7.5 -> 5.7, 64 x 4096 x 8192 17.7 -> 14.9, 128 x 8192 x 1024
-// 9.6 -> 6.0, 64 x 2048 x 512 5.1 -> 3.4, 128 x 4096 x 4096 14.6 -> 11.4, 33 x 128 x 13048 15.9 -> 10.0.
+// 8192 18.2 -> 11.4 (3.4 TB/s), 128 x 1024 x 8192 13.8 -> 9.2, 16 x 1024 x 8192 7.5 -> 5.7, 64 x 4096 x 8192 17.7 -> 14.9, 128 x 8192 x 1024
+// 9.4 -> 5.6, 64 x 2048 x 512 5.1 -> 3.6, 128 x 4096 x 4096 14.6 -> 11.4, 33 x 128 x 13048 15.9 -> 10.0.
 // Warp roles and waits are those of the other kernels (mc2_gemm.cuh): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5
 // or 2-9 drain the accumulator; every wait is bounded, and a CTA that gave one up tells its cluster, which then stores nothing of
 // the tile: what its shared memory holds is no partial sum.
@@ -33,19 +33,20 @@ namespace mc2 {
 
 constexpr int kSplitMaxBt = 128;
 constexpr int kSplitMaxCluster = 8;               // the portable cluster size
-// one warp per quarter of the accumulator lanes, two where there are many tokens to drain
-__host__ __device__ constexpr int SplitThreads(int bt) { return bt <= 32 ? 192 : 320; }
 constexpr int kSplitMaxThreads = 320;
 constexpr int kSplitMaxStages = 12;
 constexpr int kSplitRingBytes = 108 * 1024;                  // two CTAs per SM
 constexpr int kSplitLoneRingBytes = 200 * 1024;              // one CTA per SM
+// One warp per quarter of the accumulator lanes to drain it, two where there are many tokens and no neighbour on the SM whose main loop
+// runs meanwhile (128 x 8192 x 1024 6.33 us with one, 5.64 with two; with a neighbour 64 x 10240 x 8192 30.04 and 30.30; 8 tokens in a tile of 64,
+// 8 x 11520 x 448 with MN-major tokens, 8.4 and 8.8).
+inline int SplitThreads(int tokens, int ringBytes) { return tokens <= 32 || ringBytes == kSplitRingBytes ? 192 : kSplitMaxThreads; }
 constexpr int kSplitBarBytes = 256;
 
 struct SplitArgs {
     int M, N, K;               // out[M, N] = X[M, K] x W[N, K]^T   (operand storage is described by the tensor maps)
     __nv_bfloat16* out;
     int bt;                    // tokens per tile
-    int wr;                    // weight rows (output columns) per tile: 128 or 64
     int tilesM;                // token tiles; the tile index runs over them first, so that they share a weight tile in L2
     int stages;
     int barOffset;             // barriers behind the ring and the partial tile
@@ -114,27 +115,26 @@ __device__ __forceinline__ void TmemLd32x16(uint32_t taddr, uint32_t (&r)[16])
         : "memory");
 }
 
-// This CTA's share of the tokens: the partial tiles of the cluster (at most R) added in rank order, every CTA's piece of 4 columns
+// This CTA's share of the tokens: the partial tiles of the cluster's R CTAs added in rank order, every CTA's piece of 4 columns
 // requested before the first is added.
-template <int R>
-__device__ __forceinline__ void SplitAddPartials(const SplitArgs& g, uint8_t* smem, uint32_t* gaveUp, int split, int crank, int tokens, int row0, int col0)
+template <int R, int WR>
+__device__ __forceinline__ void SplitAddPartials(const SplitArgs& g, uint8_t* smem, uint32_t* gaveUp, int crank, int tokens, int row0, int col0)
 {
     uint32_t lost = 0;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        if (r < split) lost |= LdCluster1(SmemAddr(gaveUp), (uint32_t)r);
-    const int quadBits = g.wr == 128 ? 5 : 4, t0 = tokens * crank / split, t1 = tokens * (crank + 1) / split;
+    for (int r = 0; r < R; ++r) lost |= LdCluster1(SmemAddr(gaveUp), (uint32_t)r);
+    constexpr int quadBits = WR == 128 ? 5 : 4;
+    const int t0 = tokens * crank / R, t1 = tokens * (crank + 1) / R;
     const uint32_t base = SmemAddr(smem);
+#pragma unroll 1
     for (int i = (t0 << quadBits) + (int)threadIdx.x; i < t1 << quadBits; i += (int)blockDim.x) {
         const int t = i >> quadBits, c = (i - (t << quadBits)) * 4;
         float4 p[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (r < split) p[r] = LdCluster4(base + (uint32_t)i * 16, (uint32_t)r);
+        for (int r = 0; r < R; ++r) p[r] = LdCluster4(base + (uint32_t)i * 16, (uint32_t)r);
         float4 a = p[0];
 #pragma unroll
-        for (int r = 1; r < R; ++r)
-            if (r < split) { a.x += p[r].x; a.y += p[r].y; a.z += p[r].z; a.w += p[r].w; }
+        for (int r = 1; r < R; ++r) { a.x += p[r].x; a.y += p[r].y; a.z += p[r].z; a.w += p[r].w; }
         if (col0 + c < g.N && lost == 0) {               // N is a multiple of 8
             const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
             *reinterpret_cast<uint2*>(g.out + (size_t)(row0 + t) * g.N + col0 + c) =
@@ -143,12 +143,16 @@ __device__ __forceinline__ void SplitAddPartials(const SplitArgs& g, uint8_t* sm
     }
 }
 
-template <bool W_MN, bool X_MN>
+// One kernel for every height of a weight tile (WR) and cluster size (R), with loops that are not unrolled over tokens: what a launch of a
+// few microseconds fetches of its code shows.  As values of the launch they cost 0.1 .. 0.3 us (us, values -> kernels: 16 x 7168 x 2048 8.27 -> 8.14, 256 x 128 x 8192
+// 6.38 -> 6.18, 128 x 2048 x 8192 11.74 -> 11.37, 64 x 10240 x 8192 30.67 -> 30.26, 128 x 8192 x 1024 5.83 -> 5.61).
+template <bool W_MN, bool X_MN, int WR, int R>
 __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SplitArgs g)
 {
     extern __shared__ uint8_t smemRaw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
-    const int stageBytes = SplitStageBytes(g.bt, g.wr), wBytes = g.wr * kBK * 2;
+    const int stageBytes = SplitStageBytes(g.bt, WR);
+    constexpr int wBytes = WR * kBK * 2;
     uint64_t* fullBar = reinterpret_cast<uint64_t*>(smem + g.barOffset);
     uint64_t* emptyBar = fullBar + kSplitMaxStages;
     uint64_t* tmemFull = fullBar + 2 * kSplitMaxStages;
@@ -157,11 +161,11 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
     volatile uint32_t* abortWord = g.ctl + kCtlAbort;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
-    const int split = (int)SplitClusterSize(), crank = (int)SplitClusterRank();
-    const int tile = (int)blockIdx.x / split;
-    const int row0 = (tile % g.tilesM) * g.bt, col0 = (tile / g.tilesM) * g.wr;
+    const int crank = R == 1 ? 0 : (int)SplitClusterRank();
+    const int tile = (int)blockIdx.x / R;
+    const int row0 = (tile % g.tilesM) * g.bt, col0 = (tile / g.tilesM) * WR;
     const int kBlocks = (g.K + kBK - 1) / kBK;
-    const int kFirst = (int)((long long)kBlocks * crank / split), kLast = (int)((long long)kBlocks * (crank + 1) / split);
+    const int kFirst = (int)((long long)kBlocks * crank / R), kLast = (int)((long long)kBlocks * (crank + 1) / R);
     const uint32_t tmemCols = g.bt <= 32 ? 32u : (g.bt <= 64 ? 64u : 128u);
 
     if (threadIdx.x == 0) {
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
                     TmaLoad2D(sw, &tmW, &fullBar[stage], kb * kBK, col0);
                 } else {
                     TmaLoad2D(sw, &tmW, &fullBar[stage], col0, kb * kBK);
-                    if (g.wr > 64) TmaLoad2D(sw + 64 * kBK * 2, &tmW, &fullBar[stage], col0 + 64, kb * kBK);
+                    if (WR > 64) TmaLoad2D(sw + 64 * kBK * 2, &tmW, &fullBar[stage], col0 + 64, kb * kBK);
                 }
                 if (!X_MN) {
                     TmaLoad2D(sx, &tmX, &fullBar[stage], kb * kBK, row0);
@@ -213,7 +217,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
         }
     } else if (warp == 1) {
         if (ElectOne()) {
-            const uint32_t idesc = InstrDescF16(g.wr, g.bt, true, W_MN, X_MN);
+            const uint32_t idesc = InstrDescF16(WR, g.bt, true, W_MN, X_MN);
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -249,14 +253,16 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
     const uint32_t taddr = tmemBase + ((uint32_t)(quarter * 32) << 16);
     const bool odd = (lane & 1) != 0;
     // 64 rows lie in the first 16 lanes of every quarter
-    const int perQuarter = g.wr / 4, myRow = quarter * perQuarter + lane;
+    constexpr int perQuarter = WR / 4;
+    const int myRow = quarter * perQuarter + lane;
     const bool hasRow = lane < perQuarter;
-    if (split == 1) {
+    if (R == 1) {
         // straight to memory: a pair of lanes swaps halves, so that each stores two columns of every second token.  All of the tile or nothing:
         // of two warps that wait for the same accumulator, one may have given up just before it was complete.
         __syncthreads();
         drained = drained && *gaveUp == 0;
         const int col = hasRow ? col0 + (myRow & ~1) : g.N;
+#pragma unroll 1
         for (int c = part * 16; drained && c < tokens; c += chunkStep) {
             uint32_t v[16];
             TmemLd32x16(taddr + (uint32_t)c, v);
@@ -275,20 +281,20 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) GemmSplitKernel(const __g
     } else {
         // every CTA leaves its partial tile in its own idle ring, [token][column], before the cluster meets
         float* mine = reinterpret_cast<float*>(smem) + myRow;
+#pragma unroll 1
         for (int c = part * 16; drained && c < tokens; c += chunkStep) {
             uint32_t v[16];
             TmemLd32x16(taddr + (uint32_t)c, v);
             TmemLdWait();
             if (hasRow) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) mine[(c + j) * g.wr] = __uint_as_float(v[j]);
+                for (int j = 0; j < 16; ++j) mine[(c + j) * WR] = __uint_as_float(v[j]);
             }
         }
         TcFenceBefore();
         __syncthreads();
         SplitClusterSync();
-        if (split <= 4) SplitAddPartials<4>(g, smem, const_cast<uint32_t*>(gaveUp), split, crank, tokens, row0, col0);
-        else SplitAddPartials<kSplitMaxCluster>(g, smem, const_cast<uint32_t*>(gaveUp), split, crank, tokens, row0, col0);
+        SplitAddPartials<R, WR>(g, smem, const_cast<uint32_t*>(gaveUp), crank, tokens, row0, col0);
         __syncthreads();
         SplitClusterSync();                              // nobody leaves while a peer still reads its partial
     }

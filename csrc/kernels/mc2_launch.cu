@@ -134,14 +134,29 @@ HcclResult LaunchGemm2SmWide(const CUtensorMap& ta, const CUtensorMap& tb, const
     return HCCL_SUCCESS;
 }
 
-template <bool W_MN, bool X_MN>
-HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& g, int tiles, int split, cudaStream_t stream)
+template <bool W_MN, bool X_MN, int WR, int R>
+HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& g, const MatmulPlan& p, cudaStream_t stream)
 {
-    constexpr auto kernel = GemmSplitKernel<W_MN, X_MN>;
+    constexpr auto kernel = GemmSplitKernel<W_MN, X_MN, WR, R>;
     CHK_RET(AllowSharedMemory<kernel>(kSplitMaxSmemBytes));
-    const cudaError_t e = LaunchDependent(kernel, (unsigned)(tiles * split), SplitThreads(g.bt), (size_t)SplitSmemBytes(g.barOffset), stream, (unsigned)split, tw, tx, g);
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)p.grid, SplitThreads(std::min(g.M, g.bt), p.ring), (size_t)SplitSmemBytes(g.barOffset), stream, (unsigned)p.split, tw, tx, g);
     if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
+}
+template <bool W_MN, bool X_MN, int WR>
+HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& g, const MatmulPlan& p, cudaStream_t stream)
+{
+    switch (p.split) {
+        case 1: return LaunchGemmSplit<W_MN, X_MN, WR, 1>(tw, tx, g, p, stream);
+        case 2: return LaunchGemmSplit<W_MN, X_MN, WR, 2>(tw, tx, g, p, stream);
+        case 3:                                                  // tiles of 128 rows only (PlanMatmul)
+            if constexpr (WR == 128) return LaunchGemmSplit<W_MN, X_MN, WR, 3>(tw, tx, g, p, stream);
+            break;
+        case 4: return LaunchGemmSplit<W_MN, X_MN, WR, 4>(tw, tx, g, p, stream);
+        case 8: return LaunchGemmSplit<W_MN, X_MN, WR, 8>(tw, tx, g, p, stream);
+        default: break;
+    }
+    return HCCL_E_INTERNAL;                                      // no cut of PlanMatmul
 }
 
 template <bool A_MN, bool B_MN>
@@ -734,20 +749,22 @@ HcclResult Mc2Matmul(const void* a, const void* b, void* out, uint64_t m, uint64
         g.out = (__nv_bfloat16*)out;
         g.bt = plan.bt;
         g.tilesM = plan.tilesM;
-        g.wr = plan.bn;
-        g.stages = std::max(1, std::min(SplitStages(g.bt, g.wr, plan.ring), (int)(((k + kBK - 1) / kBK + plan.split - 1) / plan.split)));
-        g.barOffset = SplitBarOffset(g.bt, g.wr, g.stages, plan.split);
+        // all stages also where a CTA has fewer k-blocks: two CTAs of half a ring each would share an SM while others are idle (5 x 15248 x 248
+        // 4.4 us with as many stages as k-blocks, 3.5 with all)
+        g.stages = SplitStages(g.bt, plan.bn, plan.ring);
+        g.barOffset = SplitBarOffset(g.bt, plan.bn, g.stages, plan.split);
         g.ctl = plain.ctl;
         g.waitLimitNs = stalled != nullptr ? stalled->waitLimitNs : kWaitLimitNs;
         g.stalledCta = stalled != nullptr ? stalled->cta : -1;
-        const int tiles = plan.tilesM * plan.tilesN;
         CUtensorMap tw, tx;
-        CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, (uint32_t)g.wr, kBK));
+        CHK_RET(bMn ? MakeMap(&tw, b, k, n, kBK, 64) : MakeMap(&tw, b, n, k, (uint32_t)plan.bn, kBK));
         CHK_RET(aMn ? MakeMap(&tx, a, k, m, kBK, 64) : MakeMap(&tx, a, m, k, (uint32_t)g.bt, kBK));
-        if (!bMn && !aMn) return LaunchGemmSplit<false, false>(tw, tx, g, tiles, plan.split, stream);
-        if (!bMn && aMn) return LaunchGemmSplit<false, true>(tw, tx, g, tiles, plan.split, stream);
-        if (bMn && !aMn) return LaunchGemmSplit<true, false>(tw, tx, g, tiles, plan.split, stream);
-        return LaunchGemmSplit<true, true>(tw, tx, g, tiles, plan.split, stream);
+        if (plan.bn == 64)                                       // never with MN-major tokens (BestSplit)
+            return bMn ? LaunchGemmSplit<true, false, 64>(tw, tx, g, plan, stream) : LaunchGemmSplit<false, false, 64>(tw, tx, g, plan, stream);
+        if (!bMn && !aMn) return LaunchGemmSplit<false, false, 128>(tw, tx, g, plan, stream);
+        if (!bMn && aMn) return LaunchGemmSplit<false, true, 128>(tw, tx, g, plan, stream);
+        if (bMn && !aMn) return LaunchGemmSplit<true, false, 128>(tw, tx, g, plan, stream);
+        return LaunchGemmSplit<true, true, 128>(tw, tx, g, plan, stream);
     }
     if (stalled != nullptr && plan.route != MatmulRoute::TWO_SM_SPLIT) return HCCL_E_NOT_SUPPORT;
     CUtensorMap ta, tb;

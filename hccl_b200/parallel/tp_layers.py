@@ -60,7 +60,7 @@ class TPContext:
         return self._launches + int(self._launched)
 
     @launches.setter
-    def launches(self, n):
+    def launches(self, n):          # `+=` from outside loses what a backward pass on another thread counts in the middle of it
         self._launches = n - int(self._launched)
 
     # ---- collectives on whole tensors, either arm (used for what is not a fused matmul: the embedding exchange and
@@ -74,7 +74,7 @@ class TPContext:
             buf.copy_(send)
             recv = torch.empty_like(send)
             self.comm.all_to_all(buf, recv)
-            self.launches += 1
+            self._launches += 1
             return recv
         recv = torch.empty_like(send)
         dist.all_to_all_single(recv, send.contiguous(), group=self.group)
@@ -86,7 +86,7 @@ class TPContext:
             return t
         if self.impl == "hccl":
             self.comm.all_reduce(t)
-            self.launches += 1
+            self._launches += 1
         else:
             dist.all_reduce(t, group=self.group)
         return t
@@ -137,7 +137,7 @@ def _reduce_scatter_rows(ctx, full):
 
 def _mm(ctx, a, b, **kw):
     if ctx.impl == "hccl":
-        ctx.launches += 1
+        ctx._launches += 1
         return mc2.matmul(a, b, **kw)
     A = a.t() if kw.get("trans_a", False) else a
     B = b.t() if kw.get("trans_b", True) else b
@@ -171,7 +171,7 @@ class _ColumnParallel(torch.autograd.Function):
                 a = ctx.sym_buffer(("cp_in", key), x_shard.shape)
                 a.copy_(x_shard)
                 out, gathered = mc2.all_gather_matmul(ctx.comm, a, weight)
-            ctx.launches += 1
+            ctx._launches += 1
         else:
             gathered = torch.empty((x_shard.shape[0] * ctx.world, x_shard.shape[1]), device=x_shard.device, dtype=x_shard.dtype)
             dist.all_gather_into_tensor(gathered, x_shard.contiguous(), group=ctx.group)
@@ -190,7 +190,7 @@ class _ColumnParallel(torch.autograd.Function):
             dx = _mm(ctx, dy, weight, trans_b=False)
         elif ctx.impl == "hccl":
             dx = mc2.matmul_reduce_scatter(ctx.comm, dy, weight, weight_is_kn=True)
-            ctx.launches += 1
+            ctx._launches += 1
         else:
             dx = _reduce_scatter_rows(ctx, dy @ weight)
         return dx, dw, None, None
@@ -205,7 +205,7 @@ class _RowParallel(torch.autograd.Function):
         if ctx.world == 1:
             return _mm(ctx, x, weight)
         if ctx.impl == "hccl":
-            ctx.launches += 1
+            ctx._launches += 1
             return mc2.matmul_reduce_scatter(ctx.comm, x.contiguous(), weight)
         return _reduce_scatter_rows(ctx, x @ weight.t())
 
@@ -226,7 +226,7 @@ class _RowParallel(torch.autograd.Function):
                 a = ctx.sym_buffer(("rp_dy", fctx.key), dy_shard.shape)
                 a.copy_(dy_shard)
                 dx, dy_full = mc2.all_gather_matmul(ctx.comm, a, weight, weight_is_kn=True)
-            ctx.launches += 1
+            ctx._launches += 1
         else:
             dy_full = torch.empty((dy_shard.shape[0] * ctx.world, dy_shard.shape[1]), device=dy_shard.device, dtype=dy_shard.dtype)
             dist.all_gather_into_tensor(dy_full, dy_shard, group=ctx.group)

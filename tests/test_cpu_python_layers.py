@@ -149,3 +149,23 @@ def test_norm_kernels_refuse_row_counts_they_cannot_number():
     for rows in (1 << 31, (1 << 32) + 5):
         assert lib.HcclFusedAddRmsNormFwd(p, ctypes.c_void_p(0), p, ctypes.c_void_p(0), p, p, rows, 8, 1e-5, ctypes.c_void_p(0)) == 1
         assert lib.HcclFusedRmsNormBwd(p, p, p, p, ctypes.c_void_p(0), p, p, p, rows, 8, ctypes.c_void_p(0)) == 1
+
+
+def test_launches_counted_while_a_backward_pass_counts(monkeypatch):
+    """A matmul's count is not lost where a native backward pass, on its own thread, counts between two looks at its counter."""
+    from hccl_b200.parallel import TPContext, tp_layers
+
+    class Counting:
+        def __init__(self):
+            self.n = 0
+
+        def __int__(self):
+            self.n += 2
+            return self.n
+
+    ctx = TPContext(None, impl="hccl", device="cpu")
+    ctx._launched = Counting()
+    monkeypatch.setattr(tp_layers.mc2, "matmul", lambda a, b, **kw: a @ b)
+    for _ in range(3):
+        tp_layers._mm(ctx, torch.ones(2, 2), torch.ones(2, 2))
+    assert ctx.launches == 3 + 2

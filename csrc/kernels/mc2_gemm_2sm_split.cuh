@@ -29,7 +29,7 @@ constexpr int kSplit2StgRowBytes = 64 + 16, kSplit2StgWarpBytes = 32 * kSplit2St
 struct Split2Args {
     int M, N, K;               // out[M, N] = A[M, K] x B[K, N]   (operand storage is described by the tensor maps)
     __nv_bfloat16* out;
-    int bn;                    // column tile width, a multiple of 32, at most 256 (launched with 128)
+    int bn;                    // column tile width, a multiple of 32, at most 256 (launched with 128 and 256)
     int tilesM2, tilesN;
     int stages;
     uint32_t* ctl;             // control block: the abort word of bounded waits

@@ -5,7 +5,7 @@
 // 2 GFLOP.  A one-tile-per-SM kernel leaves most SMs idle (64 tiles of 128 columns) and pads the tokens to a 128-row
 // operand.  So here
 //   * the WEIGHT is the 128- or 64-row operand of tcgen05.mma (cta_group::1) and the tokens are the narrow one (N = bt, a multiple
-//     of 16): a stage is 16 KiB of weights plus bt * 128 bytes of activations;
+//     of 16): a stage is 16 or 8 KiB of weights plus bt * 128 bytes of activations;
 //   * a cluster of `split` CTAs (at most 8) works on one 128 x bt tile, CTA r on the r-th share of the k-blocks.  Long streams of
 //     weights want about two CTAs per SM: the stage ring takes at most half of an SM's shared memory, so that one CTA's start and
 //     end run under its neighbour's main loop.  Outputs of few tiles are bound by what one CTA gets through (a k-block of 64 takes
@@ -23,8 +23,8 @@
 // 8192 18.2 -> 11.4 (3.4 TB/s), 128 x 1024 x 8192 13.8 -> 9.2, 16 x 1024 x 8192 7.5 -> 5.7, 64 x 4096 x 8192 17.7 -> 14.9, 128 x 8192 x 1024
 // 9.4 -> 5.6, 64 x 2048 x 512 5.1 -> 3.6, 128 x 4096 x 4096 14.6 -> 11.4, 33 x 128 x 13048 15.9 -> 10.0.
 // Warp roles and waits are those of the other kernels (mc2_gemm.cuh): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5
-// or 2-9 drain the accumulator; every wait is bounded, and a CTA that gave one up tells its cluster, which then stores nothing of
-// the tile: what its shared memory holds is no partial sum.
+// or 2-9 drain the accumulator; every wait is bounded, and a CTA that gave one up tells its cluster, or the warps of its
+// own that would store, and nothing of the tile is stored: what its shared memory holds is no partial sum.
 #pragma once
 #include "mc2_gemm.cuh"
 

@@ -597,8 +597,10 @@ MatmulPlan PlanMatmul(uint64_t m, uint64_t n, uint64_t k, bool aMn, bool bMn, in
         const MatmulPlan wide = BestPairs256(s, kOtherKernel * us);
         if (wide.grid > 0) return wide;
         // One or two column tiles (a router's logits): token tiles of 64 and clusters of eight keep more SMs busy (256 x 128 x 8192 11.3 -> 6.4
-        // us, 244 x 208 x 10520 18.6 -> 10.6, 637 x 72 x 2784 8.7 -> 5.8).  They are ahead at 2048 as well (512 x 128 x 2048 8.0 and 5.0) and
-        // up to some thousand columns by less (256 x 1024 x 8192 12.9 and 10.5): there the pairs and their order of sums stay.
+        // us, 244 x 208 x 10520 18.6 -> 10.6, 637 x 72 x 2784 8.7 -> 5.8).  Neither
+        // line is where the two cross.  Columns: the token split is ahead up to some thousand, by less (256 x 1024 x 8192 12.9 and 10.5), and a line
+        // further out would change the order of sums of projections, not of routers only.  k-blocks: it is ahead at 2048 as well (512 x 128 x 2048 8.0
+        // and 5.0); inner dimensions up to 2248 stay because the tests of the pairs' kernel ask for it there, on products small enough to test.
         if (n > 256 || s.kBlocks <= 36) return p;
         const MatmulPlan split = BestSplit(s, &us);
         return us < kOtherKernel * PairsUs(s, 128, p.split) ? split : p;

@@ -120,7 +120,7 @@ def test_what_autograd_checks_is_checked(way):
     h.register_hook(lambda g: seen.append(g) or 2 * g)
     with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t) or t.cpu(), lambda t: t.cuda()):
         y = fused.swiglu(h)
-    assert len(seen) == 1 and seen[0] is h or torch.equal(seen[0], h)
+    assert len(seen) == 1 and torch.equal(seen[0], h)
     y.sum().backward()
     assert len(seen) == 2
 
@@ -178,3 +178,42 @@ def test_streams_and_checkpoints(way):
     torch.cuda.current_stream().wait_stream(side)
     got = torch.autograd.grad(y.float().square().sum(), [x, w])                  # the nodes run on their forward pass's stream
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_recorded_gradients_anomaly_mode_and_batches(way):
+    """Gradients that are themselves to be recorded come without a graph, batches of them are refused; anomaly mode sees the nodes."""
+    x, w = _rnd(8, 64).requires_grad_(), _rnd(64).requires_grad_()
+    h = fused.add_rms_norm(x, None, w, 1e-5)[1]
+    up = _rnd(8, 64, seed=5).requires_grad_()
+    assert not any(g.requires_grad for g in torch.autograd.grad(h, [x, w], up, create_graph=True))
+    h = fused.add_rms_norm(x, None, w, 1e-5)[1]
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(h, x, torch.stack((up.detach(), up.detach())), is_grads_batched=True)
+    with torch.autograd.set_detect_anomaly(True):
+        y = fused.swiglu(fused.add_rms_norm(x, None, w, 1e-5)[1])
+        want = torch.autograd.grad(y, x, torch.ones_like(y), retain_graph=True)[0]
+        with pytest.raises(RuntimeError, match="nan"):
+            torch.autograd.grad(y, x, torch.full_like(y, float("nan")))
+    assert torch.equal(want, torch.autograd.grad(fused.swiglu(fused.add_rms_norm(x, None, w, 1e-5)[1]), x, torch.ones_like(y))[0])
+
+
+# one leaf for both inputs, a leaf that holds a gradient beside one that does not (either way round), inputs that are no leaves
+@pytest.mark.parametrize("case", ["same", "first", "second", "results"])
+def test_leaves_and_what_they_hold(case, way):
+    x, w = _rnd(16, 64, seed=1).requires_grad_(), _rnd(64, seed=3)
+    d = x if case == "same" else _rnd(16, 64, seed=2).requires_grad_()
+    held = {"first": x, "second": d}.get(case)
+    if held is not None:
+        held.grad = torch.ones_like(held)
+    a, b = (x * 1, d * 1) if case == "results" else (x, d)
+    x_out, h = fused.add_rms_norm(a, b, w, 1e-5)
+    ups = [_rnd(16, 64, seed=6), _rnd(16, 64, seed=7)]
+    one = torch.autograd.grad([x_out, h], a if case == "results" else x, ups, retain_graph=True)[0]
+    torch.autograd.backward([x_out, h], ups)
+    if case == "same":
+        assert torch.equal(x.grad, one)                          # the sum of both inputs' parts, which `grad` gives too
+        return
+    assert all(torch.equal(t.grad, one + 1 if t is held else one) for t in (x, d))
+    assert x.grad.data_ptr() != d.grad.data_ptr()
+    x.grad.zero_()
+    assert torch.equal(d.grad, one + 1 if d is held else one)

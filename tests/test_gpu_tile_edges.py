@@ -365,15 +365,19 @@ def test_matmul_as_the_first_work_of_a_thread(m, n):
     assert torch.equal(out, want)
 
 
-# the stalled CTA alone on its tile, and one of a cluster of four: its peers hold good partials and must not store sums either
-@pytest.mark.parametrize("cta,k", [(0, 128), (0, 2048), (2, 2048)])
-def test_matmul_that_gives_up_a_wait(cta, k):
+# the stalled CTA alone on its tile, and the first and another one of clusters of two to eight: their peers hold good partials and must
+# not store sums either
+@pytest.mark.parametrize("cta,k,split", [(0, 128, 1), (1, 456, 2), (2, 712, 3), (0, 1024, 4), (2, 1024, 4), (0, 2048, 8), (2, 2048, 8), (7, 2048, 8)])
+def test_matmul_that_gives_up_a_wait(cta, k, split):
     """A CTA whose operands never arrive gives up after a short limit: nothing of its tile is stored, the next matmul on the
     device reports it, the one after that runs."""
     import ctypes
     from hccl_b200 import Result
     from hccl_b200._lib import lib
     from hccl_b200.comm import HcclError
+    from test_matmul_plan import plan
+    p = plan(16, 128, k)
+    assert p["route"] == "split" and p["split"] == str(split)
     g = torch.Generator(device="cuda").manual_seed(k)
     a, b = _rnd(g, 16, k), _rnd(g, 128, k)
     out = torch.full((16, 128), 7.0, device="cuda", dtype=torch.bfloat16)

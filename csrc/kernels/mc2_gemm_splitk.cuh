@@ -37,10 +37,13 @@ constexpr int kSplitMaxThreads = 320;
 constexpr int kSplitMaxStages = 12;
 constexpr int kSplitRingBytes = 108 * 1024;                  // two CTAs per SM
 constexpr int kSplitLoneRingBytes = 200 * 1024;              // one CTA per SM
-// One warp per quarter of the accumulator lanes to drain it, two where there are many tokens and no neighbour on the SM whose main loop
-// runs meanwhile (128 x 8192 x 1024 6.33 us with one, 5.64 with two; with a neighbour 64 x 10240 x 8192 30.04 and 30.30; 8 tokens in a tile of 64,
-// 8 x 11520 x 448 with MN-major tokens, 8.4 and 8.8).
-inline int SplitThreads(int tokens, int ringBytes) { return tokens <= 32 || ringBytes == kSplitRingBytes ? 192 : kSplitMaxThreads; }
+// One warp per quarter of the accumulator lanes to drain it, 16 tokens at a time; two where there is more to drain and no neighbour on the
+// SM whose main loop runs meanwhile.  128 x 8192 x 1024 6.33 us with one, 5.64 with two; 32 x 8192 x 256 3.10 and 2.78; in clusters, whose CTAs drain
+// into shared memory, only from 32 tokens on (20 x 1728 x 3064 5.50 and 5.62); with a neighbour 64 x 10240 x 8192 30.04 and 30.30.
+inline int SplitThreads(int tokens, int split, int ringBytes)
+{
+    return tokens <= (split == 1 ? 16 : 32) || ringBytes == kSplitRingBytes ? 192 : kSplitMaxThreads;
+}
 constexpr int kSplitBarBytes = 256;
 
 struct SplitArgs {

@@ -139,7 +139,7 @@ HcclResult LaunchGemmSplit(const CUtensorMap& tw, const CUtensorMap& tx, const S
 {
     constexpr auto kernel = GemmSplitKernel<W_MN, X_MN, WR, R>;
     CHK_RET(AllowSharedMemory<kernel>(kSplitMaxSmemBytes));
-    const cudaError_t e = LaunchDependent(kernel, (unsigned)p.grid, SplitThreads(std::min(g.M, g.bt), p.ring), (size_t)SplitSmemBytes(g.barOffset), stream, (unsigned)p.split, tw, tx, g);
+    const cudaError_t e = LaunchDependent(kernel, (unsigned)p.grid, SplitThreads(std::min(g.M, g.bt), p.split, p.ring), (size_t)SplitSmemBytes(g.barOffset), stream, (unsigned)p.split, tw, tx, g);
     if (e != cudaSuccess) { HCCL_ERROR("split matmul launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }

@@ -840,8 +840,8 @@ struct EmbeddingNode : Node {
             i = ids.unpack();
         }
         // A gradient that is recorded itself (create_graph), batched, dual, a subclass or seen by a mode takes PyTorch's operator, which
-        // all of these look into.
-        if (!Plain(grads[0]) || !Plain(i) || HasModes()) return {at::embedding_dense_backward(grads[0], i, vocab, -1, false)};
+        // all of these look into; ids that a hook has given back in another form too.
+        if (!Plain(grads[0]) || !Plain(i) || i.scalar_type() != at::kLong || !i.is_contiguous() || HasModes()) return {at::embedding_dense_backward(grads[0], i, vocab, -1, false)};
         c10::AutoGradMode off(false);
         Tensor dy = grads[0].contiguous();
         if ((uintptr_t)dy.const_data_ptr() % 16 != 0) dy = dy.clone();      // a packed view that does not begin on 16 bytes

@@ -103,6 +103,16 @@ def test_gradients_that_are_looked_at():
     assert all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
 
 
+def test_ids_that_a_hook_gives_back_as_it_likes():
+    ids, table, dy = _case(40, 64, 64)
+    t = table.clone().requires_grad_()
+    want = torch.autograd.grad(fused.embedding(ids, t), t, dy)[0]
+    for unpack in (lambda i: i.int(), lambda i: torch.stack((i, i), 1)[:, 0]):
+        with torch.autograd.graph.saved_tensors_hooks(lambda i: i, unpack):
+            out = fused.embedding(ids, t)
+        assert torch.equal(torch.autograd.grad(out, t, dy)[0], want)
+
+
 def test_gradients_that_begin_anywhere():
     """A packed view into a larger buffer at an odd element, and one that is not packed."""
     ids, table, dy = _case(40, 64, 64)

@@ -13,6 +13,8 @@ dtypes, hidden > 8192) takes the equivalent PyTorch expression, which is also th
 from __future__ import annotations
 
 import ctypes
+import sys
+import types
 
 import torch
 import torch.nn.functional as F
@@ -30,10 +32,20 @@ def _count(n=1):
     _launches += n
 
 
-def __getattr__(name):
-    if name == "LAUNCHES":          # kernels of this module launched so far (benchmark accounting)
+class _Module(types.ModuleType):
+    """This module: its count of launches is made of two, and can be set like the variable it looks like."""
+
+    @property
+    def LAUNCHES(self):          # kernels of this module launched so far (benchmark accounting)
         return _launches + _calls.launches()
-    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+    @LAUNCHES.setter
+    def LAUNCHES(self, n):
+        global _launches
+        _launches = n - _calls.launches()
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def _p(t):

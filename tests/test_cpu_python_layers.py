@@ -169,3 +169,18 @@ def test_launches_counted_while_a_backward_pass_counts(monkeypatch):
     for _ in range(3):
         tp_layers._mm(ctx, torch.ones(2, 2), torch.ones(2, 2))
     assert ctx.launches == 3 + 2
+
+
+def test_the_count_of_launches_can_be_set(monkeypatch):
+    before = fused.LAUNCHES
+    try:
+        fused.LAUNCHES = 0
+        fused._count(3)
+        assert fused.LAUNCHES == 3
+        monkeypatch.setattr(fused._calls, "launches", lambda: 10)        # native backward passes count too
+        assert fused.LAUNCHES == 13
+        fused.LAUNCHES = 5
+        assert fused.LAUNCHES == 5
+    finally:
+        monkeypatch.undo()
+        fused.LAUNCHES = before

@@ -460,15 +460,32 @@ std::tuple<Tensor, Tensor> LinearGradient(const Tensor& dy, const Tensor& x, con
 using torch::dynamo::autograd::CompiledNodeArgs;
 using torch::dynamo::autograd::SwapSavedVariables;
 namespace ops {
+// Anyone can call an operator: what the nodes know of their tensors is checked here.
+template <class... T> bool Bf16(const T&... t) { return ((t.scalar_type() == at::kBFloat16) && ...); }
 std::tuple<Tensor, Tensor> Norm(const Tensor& dh, const Tensor& x, const Tensor& w, const Tensor& rstd, const std::optional<Tensor>& extra)
 {
+    TORCH_CHECK(Bf16(dh, x, w) && rstd.scalar_type() == at::kFloat && x.dim() > 0 && x.numel() > 0 && x.size(-1) % 8 == 0 && x.size(-1) <= 8192 &&
+                    dh.sizes() == x.sizes() && w.numel() == x.size(-1) && rstd.numel() == x.numel() / x.size(-1) && (!extra || (Bf16(*extra) && extra->sizes() == x.sizes())),
+                "norm_backward: tensors of other types or sizes than a norm has");
     auto [dx, dw, copy] = NormGradient(dh.contiguous(), x.contiguous(), w.contiguous(), rstd.contiguous(), extra ? extra->contiguous() : Tensor(), false);
     return {std::move(dx), std::move(dw)};
 }
-Tensor Swiglu(const Tensor& dout, const Tensor& x) { return SwigluGradient(dout.contiguous(), x.contiguous()); }
-Tensor Rope(const Tensor& dout, const Tensor& cos, const Tensor& sin) { return RopeGradient(dout.contiguous(), cos.contiguous(), sin.contiguous()); }
+Tensor Swiglu(const Tensor& dout, const Tensor& x)
+{
+    TORCH_CHECK(Bf16(dout, x) && x.dim() > 0 && x.numel() > 0 && x.size(-1) % 16 == 0 && dout.numel() * 2 == x.numel(), "swiglu_backward: tensors of other types or sizes than SwiGLU has");
+    return SwigluGradient(dout.contiguous(), x.contiguous());
+}
+Tensor Rope(const Tensor& dout, const Tensor& cos, const Tensor& sin)
+{
+    TORCH_CHECK(Bf16(dout) && dout.dim() == 3 && dout.numel() > 0 && dout.size(2) % 16 == 0, "rope_backward: no bf16 gradient [rows, heads, a multiple of 16]");
+    for (const Tensor* t : {&cos, &sin})
+        TORCH_CHECK(t->scalar_type() == at::kFloat && t->numel() >= dout.size(0) * (dout.size(2) / 2), "rope_backward: no fp32 table that holds every row");
+    return RopeGradient(dout.contiguous(), cos.contiguous(), sin.contiguous());
+}
 std::tuple<Tensor, Tensor> Linear(const Tensor& dy, const Tensor& x, const Tensor& w)
 {
+    TORCH_CHECK(Bf16(dy, x, w) && dy.dim() == 2 && x.dim() == 2 && w.dim() == 2 && dy.size(0) == x.size(0) && dy.size(1) == w.size(0) && x.size(1) == w.size(1),
+                "linear_backward: tensors of other types or sizes than a linear layer has");
     auto out = LinearGradient(dy.contiguous(), x.contiguous(), w.contiguous());
     launches += 2;
     return out;

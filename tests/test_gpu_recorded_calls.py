@@ -147,6 +147,21 @@ def test_compiled_backward_passes(way):
     assert launched[1:] == [launched[0] - (2 if way == "native" else 0)] * 2    # the embedding's gradient is PyTorch's there
 
 
+def test_the_operators_of_compiled_passes_check_what_they_are_given():
+    op = torch.ops.hccl_b200
+    x, w, r = _rnd(8, 64), _rnd(64), torch.ones(8, device="cuda")
+    table = torch.ones(8, 32, device="cuda")
+    for f, args in ((op.norm_backward, (x[:4], x, w, r, None)), (op.norm_backward, (x, x, w[:32], r, None)), (op.norm_backward, (x, x, w, r[:4], None)),
+                    (op.norm_backward, (x, x, w, r, x[:4])), (op.norm_backward, (x.float(), x, w, r, None)), (op.swiglu_backward, (x, x)), (op.swiglu_backward, (x[:, :32].half(), x)),
+                    (op.rope_backward, (x, table, table)), (op.rope_backward, (x.view(8, 1, 64), table[:4], table)), (op.rope_backward, (x.view(8, 1, 64), table.half(), table)),
+                    (op.linear_backward, (x, x, _rnd(32, 64))), (op.linear_backward, (x[:4], x, _rnd(64, 64))), (op.linear_backward, (x, x, w))):
+        with pytest.raises(RuntimeError):
+            f(*args)
+    dx, dw = op.norm_backward(x, x, w, r, None)
+    assert dx.shape == x.shape and dw.shape == w.shape
+    assert [t.shape for t in op.linear_backward(x.to("meta"), x.to("meta"), _rnd(64, 64).to("meta"))] == [(8, 64), (64, 64)]
+
+
 def test_a_refused_backward_call_raises_what_a_refused_call_raises(way):
     ctx = TPContext(None)
     layer = ColumnParallelLinear(64, 128, ctx, "odd")
